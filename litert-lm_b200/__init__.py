@@ -412,9 +412,13 @@ class ops:
         """Split-KV decode attention over caller-owned DEVICE buffers (raw addresses); allocates
         nothing: the split partials live in a fixed array inside the library (8 MiB per GPU).
         For callers that must not allocate device memory at call time."""
-        _call("B200LmOps_AttentionDecodeStatic", device, C.c_void_p(q_dev), C.c_void_p(k_pages_dev),
-              C.c_void_p(v_pages_dev), C.c_void_p(page_table_dev), batch, s, hq, hkv, hd, window, int(kv_bf16), nsplit,
-              C.c_void_p(out_dev), C.c_void_p(stream) if stream else None)
+        # called once per layer and step: the addresses go straight through (argtypes turn them into pointers)
+        err = C.c_char_p()
+        code = (_lib or load_library()).B200LmOps_AttentionDecodeStatic(
+            device, q_dev, k_pages_dev, v_pages_dev, page_table_dev, batch, s, hq, hkv, hd, window, kv_bf16, nsplit, out_dev,
+            stream or None, C.byref(err))
+        if code != OK:
+            _check(code, err)
 
     @staticmethod
     def attention_decode_static_status(stream: int = 0, device: int = 0) -> int:

@@ -11,11 +11,16 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200lm.so")
-SOURCES = ["lib.cu"]
+# one translation unit per kernel family and cache type, compiled side by side
+SOURCES = ["lib.cu"] + [f"{k}_{t}.cu" for k in ("decode_fused", "decode_stream", "decode_wide", "attn_mma") for t in ("f32", "bf16")]
+
+
 def _deps():
     """Every file the translation unit can include."""
     inc = os.path.join(HERE, "..", "include")
@@ -41,18 +46,26 @@ def needs_build() -> bool:
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
         return LIB
-    cmd = [nvcc_path(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
-           "-Xcompiler", "-fPIC,-O2", "-shared", "-o", LIB] + [os.path.join(CSRC, s) for s in SOURCES]
+    flags = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2"]
     if verbose:
-        cmd.insert(1, "-Xptxas=-v")
+        flags.insert(0, "-Xptxas=-v")
     env = dict(os.environ)
     env.pop("CC", None)
     env.pop("CXX", None)
-    res = subprocess.run(cmd, capture_output=True, text=True, env=env)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-    if verbose:
-        print(res.stderr)
+    nvcc = nvcc_path()
+
+    def run(cmd) -> None:
+        res = subprocess.run(cmd, capture_output=True, text=True, env=env)
+        if res.returncode != 0:
+            raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
+        if verbose:
+            print(res.stderr)
+
+    with tempfile.TemporaryDirectory() as tmp:
+        objs = [os.path.join(tmp, s + ".o") for s in SOURCES]
+        with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+            list(pool.map(run, [[nvcc] + flags + ["-c", os.path.join(CSRC, s), "-o", o] for s, o in zip(SOURCES, objs)]))
+        run([nvcc] + flags + ["-shared", "-o", LIB] + objs)
     return LIB
 
 

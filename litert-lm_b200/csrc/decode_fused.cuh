@@ -282,7 +282,7 @@ __device__ __forceinline__ unsigned char* fu_slot(const FusedRing& r, unsigned f
 }
 // Records the first wait that gave up (kind 1: a poll of flag-carrying words, 2: a ring slot that never
 // filled, 3: the producer waiting for a free slot or for the previous step).
-__device__ __noinline__ void fu_gave_up(FusedCtx& c, int kind) {
+static __device__ __noinline__ void fu_gave_up(FusedCtx& c, int kind) {
   if (atomicCAS(c.gave_up + 3, 0, kind) == 0) {
     c.gave_up[0] = c.where / 1000;
     c.gave_up[1] = c.where % 1000;
@@ -306,7 +306,7 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 // The slot has not filled yet: bounded wait, with the development log of CTA 0.
-__device__ __noinline__ void fu_acquire_slow(FusedCtx& c, unsigned fill) {
+static __device__ __noinline__ void fu_acquire_slow(FusedCtx& c, unsigned fill) {
   if (*c.dead) return;
   const unsigned s = fill & (unsigned)(c.nslots - 1), par = (fill >> c.nslots_log2) & 1u;
   const bool log = c.fill_log && (threadIdx.x & 31) == 0 && fill < 4000u;
@@ -484,7 +484,7 @@ struct FusedOut {
 // the k range of a tile is split over several warps (latency), else a warp owns whole tiles and finalises
 // them on its own (throughput).  The caller acquires before and releases after.  One copy of this code
 // serves every GEMV phase: the step's instruction footprint matters more than a specialised inner loop.
-__device__ __noinline__ void fu_gemv_round(FusedCtx& c, unsigned fill0, int tpf, int ntiles, int ktn, const float* scales,
+static __device__ __noinline__ void fu_gemv_round(FusedCtx& c, unsigned fill0, int tpf, int ntiles, int ktn, const float* scales,
                                            bool kmajor, int ncols, int nterms, FusedOut o) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const FusedRing rg = fu_ring(c);
@@ -706,7 +706,7 @@ __device__ __forceinline__ ulonglong2 ll_wait2w(FusedCtx& c, const fu_u64* p, un
 
 // ------------------------------------------------------------------ prologues
 
-__device__ __noinline__ void fu_stamp(long long* pts, int bar, int k) {
+static __device__ __noinline__ void fu_stamp(long long* pts, int bar, int k) {
   pts[((size_t)bar * gridDim.x + blockIdx.x) * 8 + k] = clock64();
 }
 #define FU_TP(k)                                                                          \
@@ -1209,7 +1209,7 @@ __device__ __forceinline__ FusedCta fu_cta_share(const DecodeArgs& a, const Fuse
 // ------------------------------------------------------------------ producer warp
 
 // The slot of fill n is still in use: bounded wait.  False when it gave up (the CTA is then marked dead).
-__device__ __noinline__ bool fu_prod_wait_slow(FusedCtx& c, unsigned n) {
+static __device__ __noinline__ bool fu_prod_wait_slow(FusedCtx& c, unsigned n) {
   if (*c.dead) return false;
   const unsigned s = n & (unsigned)(c.nslots - 1);
   if (!mbar_wait(&c.empty[s], ((n >> c.nslots_log2) - 1u) & 1u, c.err)) {
@@ -1240,7 +1240,7 @@ __device__ __forceinline__ unsigned char* fu_prod_begin(const FusedRing& r, Fuse
 __device__ __forceinline__ uint64_t* fu_prod_bar(const FusedRing& r, unsigned n) { return &r.full[n & r.mask]; }
 
 template <typename T>
-__device__ __noinline__ void fused_producer(const DecodeArgs& a, const FusedPlan& pl, FusedCtx& c, const FusedCta& sh, int nsteps) {
+static __device__ __noinline__ void fused_producer(const DecodeArgs& a, const FusedPlan& pl, FusedCtx& c, const FusedCta& sh, int nsteps) {
   const ModelDims& dm = a.dims;
   const int lane = threadIdx.x & 31, cta = blockIdx.x;
   const int ktn = dm.d / 64;
@@ -1830,17 +1830,20 @@ decode_fused_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant_
   }
 }
 
-// Host-side selection of the instantiation for a model.
-inline const void* decode_fused_kernel_for(const ModelDims& d) {
+// Host-side selection of the instantiation for a model; the kernels of one cache type are a translation unit.
+template <typename T>
+inline const void* decode_fused_kernel_pick(const ModelDims& d) {
   const int G = d.hq / d.hkv;
-#define B2_PICK_G(T, HD)                                                                  \
+#define B2_PICK_G(HD)                                                                     \
   (G == 1 ? (const void*)decode_fused_kernel<T, HD, 1>                                    \
           : G == 2 ? (const void*)decode_fused_kernel<T, HD, 2> : (const void*)decode_fused_kernel<T, HD, 4>)
-#define B2_PICK_HD(T)                                                                     \
-  (d.hd == 32 ? B2_PICK_G(T, 32) : d.hd == 64 ? B2_PICK_G(T, 64) : d.hd == 128 ? B2_PICK_G(T, 128) : B2_PICK_G(T, 256))
-  return d.kv_dtype == 0 ? B2_PICK_HD(float) : B2_PICK_HD(__nv_bfloat16);
-#undef B2_PICK_HD
+  return d.hd == 32 ? B2_PICK_G(32) : d.hd == 64 ? B2_PICK_G(64) : d.hd == 128 ? B2_PICK_G(128) : B2_PICK_G(256);
 #undef B2_PICK_G
+}
+const void* decode_fused_kernel_f32(const ModelDims& d);
+const void* decode_fused_kernel_bf16(const ModelDims& d);
+inline const void* decode_fused_kernel_for(const ModelDims& d) {
+  return d.kv_dtype == 0 ? decode_fused_kernel_f32(d) : decode_fused_kernel_bf16(d);
 }
 
 }  // namespace b200lm

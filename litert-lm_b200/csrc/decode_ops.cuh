@@ -317,7 +317,7 @@ __device__ __forceinline__ void quantize_value(float r, int nterms, int8_t* q0, 
 }
 
 // Quantises xf[ncols][K] (shared) into xq with nterms int8 terms per column.
-__device__ __noinline__ void quantize_cols(const DecodeSmem& s, int K, int ncols, int nterms) {
+static __device__ __noinline__ void quantize_cols(const DecodeSmem& s, int K, int ncols, int nterms) {
   for (int col = 0; col < ncols; ++col) {
     const float* x = s.xf + (size_t)col * K;
     float m = 0.f;
@@ -964,7 +964,7 @@ __device__ inline void phase_head(const DecodeArgs& a, const DecodeSmem& s, int 
 }
 
 // Final arg-max over the per-CTA candidates; optionally feeds the token back.
-__device__ __noinline__ void phase_argmax(const DecodeArgs& a, int ncta_head) {
+static __device__ __noinline__ void phase_argmax(const DecodeArgs& a, int ncta_head) {
   if (threadIdx.x < 32) {
     // the state words are fetched up front, next to the first candidates: one L2 round trip, not a chain
     const int sd = threadIdx.x == 0 ? __ldcg(&a.st->steps_done) : 0;
@@ -1013,7 +1013,7 @@ __device__ __noinline__ void phase_argmax(const DecodeArgs& a, int ncta_head) {
 
 enum DecodePhase { kPhQkv = 0, kPhAttn, kPhOproj, kPhGateUp, kPhDown, kPhHead, kPhArgmax };
 
-__global__ void __launch_bounds__(kDecThreads, 1)
+static __global__ void __launch_bounds__(kDecThreads, 1)
 decode_phase_kernel(const __grid_constant__ DecodeArgs a, int phase, int layer) {
   extern __shared__ __align__(16) unsigned char dsm[];
   DecodeSmem s = carve_smem(dsm, a.dims, a.ncols);
@@ -1060,7 +1060,7 @@ __device__ __forceinline__ void grid_barrier(DecodeState* st, unsigned int* epoc
   dec_sync();
 }
 
-__global__ void __launch_bounds__(kDecThreads, 1)
+static __global__ void __launch_bounds__(kDecThreads, 1)
 decode_persistent_kernel(const __grid_constant__ DecodeArgs a, int nsteps, unsigned int epoch0) {
   extern __shared__ __align__(16) unsigned char dsm[];
   DecodeSmem s = carve_smem(dsm, a.dims, a.ncols);

@@ -163,7 +163,7 @@ __host__ inline bool stream_model_fits(const ModelDims& d, int o_slices, int dow
   return half_bytes >= 2 * d.hd * esz + 3 * d.hd * 4 + 64;   // at least one staged K/V row pair + RoPE row + gains
 }
 
-__device__ __noinline__ void stream_make_plans(const DecodeArgs& a, StreamCtx& c, int cta, int ncta) {
+static __device__ __noinline__ void stream_make_plans(const DecodeArgs& a, StreamCtx& c, int cta, int ncta) {
   const int phases[5] = {kSA, kSC, kSD, kSE, kSH};
   for (int i = 0; i < 5; ++i) {
     PhasePlan& p = c.plan[phases[i]];
@@ -190,7 +190,7 @@ __device__ __forceinline__ void stream_advance(StreamCursor& cur, const StreamCt
 
 // ------------------------------------------------------------ producer warp
 
-__device__ __noinline__ void stream_producer(const DecodeArgs& a, StreamCtx& c, int cta, int nsteps) {
+static __device__ __noinline__ void stream_producer(const DecodeArgs& a, StreamCtx& c, int cta, int nsteps) {
   const int lane = threadIdx.x & 31;
   const ModelDims& dm = a.dims;
   const int last = dm.n_layers - 1;
@@ -506,7 +506,7 @@ __device__ __forceinline__ void stream_prologue_resid(const DecodeArgs& a, Strea
   dec_sync();
 }
 
-__device__ __noinline__ void stream_prologue_embed(const DecodeArgs& a, StreamCtx& c, int cta, float* xout,
+static __device__ __noinline__ void stream_prologue_embed(const DecodeArgs& a, StreamCtx& c, int cta, float* xout,
                                                       const float* g_pre, float gmax_pre) {
   const int d = a.dims.d;
   const DecodeSmem& s = c.s;
@@ -1137,17 +1137,20 @@ decode_stream_kernel(const __grid_constant__ DecodeArgs a, int nsteps, unsigned 
   }
 }
 
-// Host-side selection of the instantiation for a model.
-inline const void* decode_stream_kernel_for(const ModelDims& d) {
+// Host-side selection of the instantiation for a model; the kernels of one cache type are a translation unit.
+template <typename T>
+inline const void* decode_stream_kernel_pick(const ModelDims& d) {
   const int G = d.hq / d.hkv;
-#define B2_PICK_G(T, HD)                                                                  \
-  (G == 1 ? (const void*)decode_stream_kernel<T, HD, 1>                                   \
+#define B2_PICK_G(HD)                                                                     \
+  (G == 1 ? (const void*)decode_stream_kernel<T, HD, 1>                                    \
           : G == 2 ? (const void*)decode_stream_kernel<T, HD, 2> : (const void*)decode_stream_kernel<T, HD, 4>)
-#define B2_PICK_HD(T)                                                                     \
-  (d.hd == 32 ? B2_PICK_G(T, 32) : d.hd == 64 ? B2_PICK_G(T, 64) : d.hd == 128 ? B2_PICK_G(T, 128) : B2_PICK_G(T, 256))
-  return d.kv_dtype == 0 ? B2_PICK_HD(float) : B2_PICK_HD(__nv_bfloat16);
-#undef B2_PICK_HD
+  return d.hd == 32 ? B2_PICK_G(32) : d.hd == 64 ? B2_PICK_G(64) : d.hd == 128 ? B2_PICK_G(128) : B2_PICK_G(256);
 #undef B2_PICK_G
+}
+const void* decode_stream_kernel_f32(const ModelDims& d);
+const void* decode_stream_kernel_bf16(const ModelDims& d);
+inline const void* decode_stream_kernel_for(const ModelDims& d) {
+  return d.kv_dtype == 0 ? decode_stream_kernel_f32(d) : decode_stream_kernel_bf16(d);
 }
 
 }  // namespace b200lm

@@ -27,7 +27,7 @@ struct WideState {
 
 // One CTA per session: arg-max of its logits row (lowest index among equal maxima, the rule of
 // runtime/components/sampling_cpu_util.cc:32-41), recorded as the step's id and as the next input.
-__global__ void __launch_bounds__(kWideArgThreads)
+static __global__ void __launch_bounds__(kWideArgThreads)
 wide_argmax_kernel(const float* __restrict__ logits, int vocab, int n, WideState st, int* __restrict__ step_tokens) {
   __shared__ float sv[kWideArgThreads / 32];
   __shared__ int si[kWideArgThreads / 32];
@@ -330,7 +330,7 @@ wide_attn_kernel(ModelDims dm, WideAttnArgs a) {
 
 // Sum of the key splits' partial states: one CTA per (session, query head).  The splits' (m, l) pairs are fetched
 // by one thread each and their weights exp(m_s - M) / L shared, so the element loop is independent loads only.
-__global__ void __launch_bounds__(128)
+static __global__ void __launch_bounds__(128)
 wide_attn_combine_kernel(const float* __restrict__ part, int nsplit, int hq, int hkv, int hd, __nv_bfloat16* __restrict__ out,
                          float* __restrict__ out_f32) {
   __shared__ float w_s[kMaxSplits];
@@ -413,13 +413,16 @@ inline void launch_wide_attn_h(cudaStream_t st, const ModelDims& d, int nb, size
     default: throw Error{kUnimplemented, "head size must be 32, 64, 128 or 256"};
   }
 }
+// The kernels of one cache type are a translation unit.
+void launch_wide_attn_f32(cudaStream_t st, const ModelDims& d, int nb, size_t smem_optin, const WideAttnArgs& a);
+void launch_wide_attn_bf16(cudaStream_t st, const ModelDims& d, int nb, size_t smem_optin, const WideAttnArgs& a);
 inline void launch_wide_attn(cudaStream_t st, const ModelDims& d, int nb, size_t smem_optin, const WideAttnArgs& a) {
-  if (d.kv_dtype == 0) launch_wide_attn_h<float>(st, d, nb, smem_optin, a);
-  else launch_wide_attn_h<__nv_bfloat16>(st, d, nb, smem_optin, a);
+  if (d.kv_dtype == 0) launch_wide_attn_f32(st, d, nb, smem_optin, a);
+  else launch_wide_attn_bf16(st, d, nb, smem_optin, a);
 }
 
 // out[t][:] = sum of the split-K partials parts[p][t][:], rows of `cols` floats.
-__global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(256)
 wide_sum_parts_kernel(const float* __restrict__ parts, int nparts, size_t part_stride, size_t count, float* __restrict__ out) {
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i * 4 >= count) return;

@@ -331,25 +331,6 @@ static CUtensorMap make_bf16_map(const void* base, int rank, const cuuint64_t* d
   return tm;
 }
 
-// Launch with programmatic stream serialisation: the kernel may be scheduled
-// while its predecessor in the stream is still running and does its set-up
-// (barrier init, TMEM allocation) there; it calls pdl_wait() before it touches
-// the predecessor's data.
-template <typename... KArgs, typename... Args>
-static void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  B2_CUDA(cudaLaunchKernelEx(&cfg, kernel, KArgs(std::forward<Args>(args))...));
-}
-
 // Split-K factor for a GEMM of `n_tiles` weight-row tiles over T tokens with KB
 // 64-wide k blocks: the smallest divisor of KB (at least 4 k blocks per split,
 // at most 8 splits) whose work units fill 90 % of the last round over the SMs,

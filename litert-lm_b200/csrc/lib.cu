@@ -1,5 +1,5 @@
-// Single translation unit of libb200lm.so: the kernels live in headers, so the
-// executor and the operator-level ABI are compiled together.
+// The executor, the prefill kernels and the operator-level ABI; the kernels with many instantiations are
+// translation units of their own.
 #include "executor.cu"
 #include "ops.cu"
 #include "ops_static.cu"

@@ -11,10 +11,12 @@
 // size.  Every GPU that loads this library carries that array until the
 // process exits.
 #include "../../include/b200lm_ops.h"
+#include "attn_mma.cuh"
 #include "common.cuh"
 #include "decode_ops.cuh"
 #include "prefill_ops.cuh"
 
+#include <atomic>
 #include <mutex>
 
 namespace b200lm {
@@ -28,6 +30,10 @@ constexpr int kStaticMaxQueries = (int)(kStaticHeaderBytes / 4) - 16;
 // device code may name the array directly.
 static __device__ __align__(256) unsigned char g_attn_static_scratch[kStaticScratchBytes];
 
+// Tickets of attn_shared_kernel: how many splits of a unit have arrived; the last one puts its ticket back to zero.
+constexpr int kStaticTickets = 256;
+static __device__ int g_attn_static_tickets[kStaticTickets];
+
 // Header layout: int[0] = error word, int[16 + i] = position of query i.
 __global__ void static_scratch_prepare_kernel(int nq, int pos) {
   int* hdr = reinterpret_cast<int*>(g_attn_static_scratch);
@@ -37,25 +43,34 @@ __global__ void static_scratch_prepare_kernel(int nq, int pos) {
 }
 
 constexpr int kMaxDevices = 64;
-static unsigned char* g_static_scratch_addr[kMaxDevices] = {nullptr};
+struct StaticScratch {
+  unsigned char* base;
+  int* tickets;
+  int sms;
+};
+static StaticScratch g_static_scratch[kMaxDevices] = {};
 static std::mutex g_static_scratch_mu;     // guards the per-device set-up below
 
 // Device address of the array on `device` (which must be current).  Looked up
 // once per device, under a lock: concurrent first calls do the set-up once.
-static unsigned char* static_scratch_for(int device) {
+static StaticScratch static_scratch_for(int device) {
   B2_CHECK(device >= 0 && device < kMaxDevices, kInvalidArgument, "device ordinal out of range");
   std::lock_guard<std::mutex> lock(g_static_scratch_mu);
-  if (!g_static_scratch_addr[device]) {
-    void* p = nullptr;
+  StaticScratch& s = g_static_scratch[device];
+  if (!s.base) {
+    void *p = nullptr, *t = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, g_attn_static_scratch);
-    if (e != cudaSuccess || p == nullptr)
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(&t, g_attn_static_tickets);
+    if (e != cudaSuccess || p == nullptr || t == nullptr)
       throw Error{kInternal, std::string("cudaGetSymbolAddress(static scratch): ") + cudaGetErrorString(e)};
     // attribute change, not an allocation; done with the set-up so later calls only launch.  The limit is
     // raised to the largest shape the entry point accepts and never lowered by any other caller.
     raise_dyn_smem(attn_decode_kernel, sizeof(float) * ((size_t)(4 + 2) * 256 + (size_t)kDecWarps * 4 * (256 + 2)));
-    g_static_scratch_addr[device] = reinterpret_cast<unsigned char*>(p);
+    B2_CUDA(cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, device));
+    s.tickets = reinterpret_cast<int*>(t);
+    s.base = reinterpret_cast<unsigned char*>(p);
   }
-  return g_static_scratch_addr[device];
+  return s;
 }
 
 // Makes `device` current for the duration of a call and puts the caller's device back afterwards.
@@ -63,7 +78,8 @@ struct DeviceScope {
   int prev = -1;
   explicit DeviceScope(int device) {
     if (cudaGetDevice(&prev) != cudaSuccess) { cudaGetLastError(); prev = -1; }
-    B2_CUDA(cudaSetDevice(device));
+    if (prev == device) prev = -1;            // already current: nothing to set, nothing to put back
+    else B2_CUDA(cudaSetDevice(device));
   }
   ~DeviceScope() {
     if (prev >= 0) cudaSetDevice(prev);
@@ -79,10 +95,14 @@ static int static_fail(char** err, int code, const std::string& msg) {
 }
 
 static void require_device(int device) {
-  int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) {
-    cudaGetLastError();
-    throw Error{kFailedPrecondition, "no CUDA device: this backend has no CPU fallback"};
+  static std::atomic<int> known{0};           // the count does not change while a process runs
+  int ndev = known.load(std::memory_order_relaxed);
+  if (ndev <= 0) {
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) {
+      cudaGetLastError();
+      throw Error{kFailedPrecondition, "no CUDA device: this backend has no CPU fallback"};
+    }
+    known.store(ndev, std::memory_order_relaxed);
   }
   B2_CHECK(device >= 0 && device < ndev, kInvalidArgument, "device ordinal out of range");
 }
@@ -113,11 +133,38 @@ extern "C" int B200LmOps_AttentionDecodeStatic(int32_t device, const float* q_de
                  std::to_string(kStaticScratchBytes - kStaticHeaderBytes) + " (lower batch or nsplit)");
     require_device(device);
     DeviceScope scope(device);                                  // the caller's current device is restored on return
-    unsigned char* scratch = static_scratch_for(device);        // first call on a device does the set-up
+    const StaticScratch sc = static_scratch_for(device);        // first call on a device does the set-up
+    unsigned char* scratch = sc.base;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     int* hdr = reinterpret_cast<int*>(scratch);
     float* part_o = reinterpret_cast<float*>(scratch + kStaticHeaderBytes);
     float* part_ml = reinterpret_cast<float*>(scratch + kStaticHeaderBytes + part_o_bytes);
+    // Bulk copies and 16-byte accesses need aligned rows; buffers that are not go through the plain-load kernel.
+    const uintptr_t align = (uintptr_t)q_dev | (uintptr_t)k_pages_dev | (uintptr_t)v_pages_dev | (uintptr_t)out_dev;
+    if (align % 16 == 0) {
+      AmArgs a{};
+      a.q = q_dev;
+      a.q_stride = (hq + 2 * hkv) * hd;
+      a.k = k_pages_dev;
+      a.v = v_pages_dev;
+      a.page_table = page_table_dev;
+      a.rows = batch * G;
+      a.G = G;
+      a.hkv = hkv;
+      a.lo = window > 0 && window < s ? s - window : 0;
+      a.k1 = s;
+      a.qscale = 1.4426950408889634f / sqrtf((float)hd);
+      a.out = out_dev;
+      a.part_o = part_o;
+      a.err = hdr;
+      // the caller's nsplit sized the check above; what fits the scratch is this kernel's own limit
+      const size_t per_split = (size_t)batch * hq * (hd + 2) * sizeof(float);
+      const int cap = (int)std::min<size_t>(256, (kStaticScratchBytes - kStaticHeaderBytes) / per_split);
+      a.part_ml = part_o + (size_t)batch * hq * cap * hd;
+      if (kv_bf16) launch_attn_shared_bf16(st, a, hd, device, sc.sms, cap, sc.tickets, kStaticTickets);
+      else launch_attn_shared_f32(st, a, hd, device, sc.sms, cap, sc.tickets, kStaticTickets);
+      return kOk;
+    }
     static_scratch_prepare_kernel<<<(batch + 255) / 256, 256, 0, st>>>(batch, s - 1);
     B2_CUDA(cudaGetLastError());
     ModelDims dm{};
@@ -142,11 +189,9 @@ extern "C" int B200LmOps_AttentionDecodeStatic(int32_t device, const float* q_de
     j.part_o = part_o;
     j.part_ml = part_ml;
     j.err = hdr;
-    int n_sms = 0;
-    B2_CUDA(cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, device));
     const size_t smem_dec = sizeof(float) * ((size_t)(G + 2) * hd + (size_t)kDecWarps * G * (hd + 2));
     const int items = batch * hkv * nsplit;
-    const int grid = items < n_sms ? items : n_sms;
+    const int grid = items < sc.sms ? items : sc.sms;
     attn_decode_kernel<<<grid, kDecThreads, smem_dec, st>>>(dm, j, batch);
     B2_CUDA(cudaGetLastError());         // a rejected launch must not be followed by a combine of stale partials
     const int total = batch * hq * hd;
@@ -173,6 +218,7 @@ extern "C" int B200LmOps_AttentionDecodeStaticStatus(int32_t device, void* strea
     B2_CUDA(cudaMemcpyFromSymbolAsync(&word, g_attn_static_scratch, sizeof(int), 0, cudaMemcpyDeviceToHost, st));
     B2_CUDA(cudaStreamSynchronize(st));
     if (device_error) *device_error = word;
+    if (word != kDevOk) B2_CUDA(cudaMemsetAsync(static_scratch_for(device).base, 0, sizeof(int), st));   // the next call starts clean
     if (word == kDevBadPosition) throw Error{kInvalidArgument, "a query position lay outside the cache"};
     if (word == kDevBarrierTimeout) throw Error{kDeadlineExceeded, "a bounded device-side wait gave up"};
     if (word != kDevOk) throw Error{kInternal, "device error word " + std::to_string(word)};

@@ -34,7 +34,7 @@ __device__ __forceinline__ float pf_block_sum(float v, float* scratch) {
 }
 
 // xres[t] = dequant(E[token]) * sqrt(d) ; h[t] = bf16(rmsnorm(x) * g)
-__global__ void __launch_bounds__(kPfThreads)
+static __global__ void __launch_bounds__(kPfThreads)
 pf_embed_norm_kernel(const int* __restrict__ tokens, const uint8_t* __restrict__ embed_rows,
                      const float* __restrict__ embed_scale, const float* __restrict__ g, int d,
                      int vocab, float eps, float* __restrict__ xres, __nv_bfloat16* __restrict__ h,
@@ -67,7 +67,7 @@ pf_embed_norm_kernel(const int* __restrict__ tokens, const uint8_t* __restrict__
 }
 
 // x[t] += rmsnorm(sum_p parts[p][t]) * g_post ; h[t] = bf16(rmsnorm(x[t]) * g_pre) (if g_pre)
-__global__ void __launch_bounds__(kPfThreads)
+static __global__ void __launch_bounds__(kPfThreads)
 pf_resid_norm_kernel(const float* __restrict__ parts, int nparts, size_t part_stride, int d,
                      float eps, const float* __restrict__ g_post, const float* __restrict__ g_pre,
                      float* __restrict__ xres, __nv_bfloat16* __restrict__ h) {
@@ -311,7 +311,7 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
 
 // Attention for T queries against the cache (keys already appended): one CTA
 // per (query, kv head), all G query heads of the group together.
-__global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(256)
 pf_attn_kernel(ModelDims dm, AttnJob job) {
   extern __shared__ __align__(16) float attn_sm[];
   int it = blockIdx.x;
@@ -323,7 +323,7 @@ pf_attn_kernel(ModelDims dm, AttnJob job) {
 // C[t][n] = scale[n] * sum_k W[n][k] * A[t][k] straight from the mma-tiled
 // weights, one thread per (row of a 16-row tile, token).  Slow; used for shapes
 // the tensor-core kernel does not take and as its on-device cross-check.
-__global__ void __launch_bounds__(128)
+static __global__ void __launch_bounds__(128)
 gemm_w4_simple_kernel(const __nv_bfloat16* __restrict__ A, const uint4* __restrict__ w,
                       const float* __restrict__ wscale, int T, int N, int K, int geglu,
                       float* __restrict__ outF, __nv_bfloat16* __restrict__ outB) {

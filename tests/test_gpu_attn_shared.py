@@ -1,0 +1,63 @@
+"""Decode attention of many queries over one cache (B200LmOps_AttentionDecodeStatic): every row-tile variant, edges of
+the 16-key chunks, pages and windows, one split and many, against fp64 softmax attention."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(q, k, v, table, s, window):
+    b, hq, hd = q.shape
+    hkv = k.shape[1]
+    lo = max(0, s - window) if window > 0 else 0
+    kk = k[table.long()].transpose(1, 2).reshape(-1, hkv, hd)[lo:s].double()
+    vv = v[table.long()].transpose(1, 2).reshape(-1, hkv, hd)[lo:s].double()
+    qq = q.double().reshape(b, hkv, hq // hkv, hd)
+    p = torch.softmax(torch.einsum("bkgd,skd->bkgs", qq, kk) / hd ** 0.5, dim=-1)
+    return torch.einsum("bkgs,skd->bkgd", p, vv).reshape(b, hq, hd)
+
+
+@pytest.mark.parametrize("hq,hkv,hd", [(4, 1, 256), (8, 4, 128), (2, 2, 64), (4, 2, 32)])
+@pytest.mark.parametrize("batch,s,window", [
+    (1, 1, 0), (1, 16, 0), (1, 1000, 0), (1, 5000, 512),       # at most four rows: packed terms
+    (3, 17, 0), (4, 777, 100), (7, 300, 0), (8, 2049, 0),      # 5 .. 32 rows
+    (9, 257, 0), (33, 1023, 256), (64, 3000, 0),               # row tiles with a remainder; more than one tile
+])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window, bf16):
+    gen = torch.Generator(device="cuda").manual_seed(batch * 1000 + s)
+    pages = -(-s // 256)
+    q = torch.randn(batch, (hq + 2 * hkv) * hd, device="cuda", generator=gen)
+    kv = torch.bfloat16 if bf16 else torch.float32
+    k = torch.randn(pages, hkv, 256, hd, device="cuda", generator=gen).to(kv)
+    v = torch.randn(pages, hkv, 256, hd, device="cuda", generator=gen).to(kv)
+    k[-1, :, s - (pages - 1) * 256:] = float("nan")            # slots past the last key are never read
+    v[-1, :, s - (pages - 1) * 256:] = float("nan")
+    k[-1], v[-1] = k[-1].clone(), v[-1].clone()
+    table = torch.randperm(pages, device="cuda", generator=gen).to(torch.int32)
+    inv = torch.empty_like(table)
+    inv[table.long()] = torch.arange(pages, device="cuda", dtype=torch.int32)
+    kp, vp = k[inv.long()].contiguous(), v[inv.long()].contiguous()       # logical page i lies at table[i]
+    out = torch.full((batch, hq, hd), float("nan"), device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    for _ in range(2):                                         # the second call finds the tickets of the first at zero
+        pkg.ops.attention_decode_static(q.data_ptr(), kp.data_ptr(), vp.data_ptr(), table.data_ptr(), out.data_ptr(), batch, s, hq, hkv,
+                                        hd, window=window, kv_bf16=bf16, nsplit=1, stream=stream)
+    assert pkg.ops.attention_decode_static_status(stream=stream) == 0
+    want = reference(q[:, :hq * hd].reshape(batch, hq, hd), kp, vp, table, s, window)
+    err = ((out.double() - want).norm() / want.norm()).item()
+    assert err < 2e-6, err
+
+
+def test_unaligned_cache_goes_through_the_plain_kernel(pkg):
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    s, hd = 300, 32
+    raw = [torch.randn(2 * 256 * hd + 1, device="cuda", generator=gen)[1:] for _ in range(2)]     # 4 bytes off
+    k, v = (r.reshape(2, 1, 256, hd) for r in raw)
+    q = torch.randn(3, 4 * hd + 2 * hd, device="cuda", generator=gen)
+    table = torch.arange(2, device="cuda", dtype=torch.int32)
+    out = torch.empty(3, 4, hd, device="cuda")
+    pkg.ops.attention_decode_static(q.data_ptr(), k.data_ptr(), v.data_ptr(), table.data_ptr(), out.data_ptr(), 3, s, 4, 1, hd, nsplit=2,
+                                    stream=torch.cuda.current_stream().cuda_stream)
+    want = reference(q[:, :4 * hd].reshape(3, 4, hd), k, v, table, s, 0)
+    assert ((out.double() - want).norm() / want.norm()).item() < 2e-6
