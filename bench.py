@@ -32,9 +32,9 @@ import __graft_entry__ as graft  # noqa: E402
 
 PREFILL_TOKENS = 1024
 DECODE_STEPS = 256
-# DRAM bytes per decode step: an ncu capture (2026-11-25) of one launch of two decode steps of the chained
-# kernel read 1079.5 MB and wrote 48.3 MB
-DECODE_DRAM_BYTES_PER_STEP = 563.9e6
+# DRAM bytes per decode step: an ncu capture (2026-12-01) of the 131 kernels of one step at context 1026 read
+# 541.8 MB and wrote 0.1 MB
+DECODE_DRAM_BYTES_PER_STEP = 541.9e6
 # The CPU arm's sample of the workload, used by `--impl reference` and by the in-line `cpu_baseline` alike:
 # the full 1024-token prefill once, then short runs of greedy decode steps that stay inside the protocol's
 # context range (1024 .. 1280 positions).
@@ -365,7 +365,7 @@ def run_cfg4(args, pkg, cfg, img, stream, rank: int, world: int, local_rank: int
         "config": {"workload": f"{cfg.name}: {args.sessions} sessions x ({PREFILL_TOKENS}-token prefill + {DECODE_STEPS} decode steps), "
                                f"sharded over {world} GPU(s), no collective", "seed": cfg.seed, "sessions_per_gpu": len(mine),
                    "lockstep_group": group, "decode_mode": {pkg.DECODE_WIDE: "wide (tensor-core GEMM per step, CUDA graph)",
-                                                            pkg.DECODE_CHAINED: "chained persistent kernel"}.get(decode_mode, str(decode_mode)),
+                                                            pkg.DECODE_CHAINED: "chain of step kernels (CUDA graph)"}.get(decode_mode, str(decode_mode)),
                    "kv_cache": "fp32" if cfg.kv_dtype == 0 else "bf16", "context": cfg.max_ctx,
                    "kv_capacity_per_session": cap},
         "prefill": {"value": world * n * len(mine) * PREFILL_TOKENS / (pf_ms / 1e3), "unit": "tok/s"},

@@ -30,16 +30,15 @@ extern "C" {
 
 typedef struct B200LmExecutor B200LmExecutor;
 
-/* decode_mode: AUTO picks the chained persistent kernel when the model fits its
- * shared-memory ring, else the streaming persistent kernel, else one kernel per
- * phase replayed from a CUDA graph. */
+/* decode_mode: AUTO picks the chain of step kernels, and B200LM_DECODE_WIDE for
+ * more than four sessions. */
 enum {
   B200LM_DECODE_AUTO = 0,
-  B200LM_DECODE_PHASE_KERNELS = 1,     /* one kernel per phase, CUDA graph per step */
+  B200LM_DECODE_PHASE_KERNELS = 1,     /* the same chain as B200LM_DECODE_CHAINED */
   B200LM_DECODE_PERSISTENT = 2,        /* one cooperative kernel, grid barrier per phase, weights streamed by bulk async copies */
   B200LM_DECODE_PERSISTENT_BASIC = 3,  /* one cooperative kernel, grid barrier per phase, plain loads (comparison) */
-  B200LM_DECODE_CHAINED = 4,           /* one cooperative kernel without grid barriers: phases hand results over in
-                                          flag-carrying words, gate/up + down fused */
+  B200LM_DECODE_CHAINED = 4,           /* a chain of kernels, one per phase, in a CUDA graph with programmatic edges:
+                                          each fetches its weights while its predecessor runs */
   B200LM_DECODE_WIDE = 5               /* lockstep groups of up to 128 sessions: the projections of a step run on the
                                           tensor-core int4 GEMM of the prefill path with the sessions as its token
                                           rows (bf16 activations), one attention CTA per (session, kv head), one CUDA
@@ -61,7 +60,7 @@ typedef struct B200LmConfig {
                               (page, slot) computation cannot pass the KV indexing checks by
                               accident.  Results do not depend on it. */
   void* stream;            /* cudaStream_t to run on, or NULL for an own stream */
-  int32_t n_sessions;      /* sessions held by this executor (0 = 1): 1..4 with the persistent decode
+  int32_t n_sessions;      /* sessions held by this executor (0 = 1): 1..4 with the chain and the persistent
                               kernels, up to 128 in B200LM_DECODE_WIDE; see B200Lm_DecodeTokensBatch */
   int32_t reserved1;
   /* Tensor parallelism.  tp_world > 1: this executor is rank tp_rank of tp_world and
@@ -182,8 +181,8 @@ int B200Lm_GetLastPrefillPlan(B200LmExecutor* e, int32_t* buckets, int32_t* leng
 int B200Lm_ReadKvRow(B200LmExecutor* e, int32_t layer, int32_t is_v, int32_t kv_head, int32_t pos,
                      float* out_row, int32_t* out_page, int32_t* out_slot, char** err);
 
-/* Device timeline of ONE greedy decode step run by a persistent decode mode
- * (equivalent to B200Lm_DecodeToken): for every grid barrier b and CTA c,
+/* Device timeline of ONE greedy decode step (any mode but B200LM_DECODE_WIDE;
+ * equivalent to B200Lm_DecodeToken): for every grid barrier b and CTA c,
  * stamps[(b * n_cta + c) * 2 + {0,1}] = that SM's cycle counter when the CTA
  * arrived at / was released from the barrier.  Within one CTA,
  * arrive[b] - release[b-1] is the time it worked in phase b and
@@ -191,7 +190,11 @@ int B200Lm_ReadKvRow(B200LmExecutor* e, int32_t layer, int32_t is_v, int32_t kv_
  * values come n_barriers * n_cta * 8 stamps taken inside the phase that ends
  * at barrier b (streaming mode: 0 phase start, 1 staged bytes arrived, 2 next
  * fill issued, 3 prologue done, 4 MMA done, 5 epilogue done, 6 phase end; 0
- * where a point was not reached).  The reference has no per-op
+ * where a point was not reached).  The chain of step kernels has a kernel where
+ * the others have a phase: its stamps are nanoseconds of one device-wide timer
+ * (sm_clock_khz = 1000000), "arrive" is the end of kernel b and "release" the
+ * moment kernel b + 1 saw it complete; inside a kernel 0 start, 1 predecessor
+ * complete, 2 activations ready, 3 products done, 4 end.  The reference has no per-op
  * profiler hook (only wall-clock BenchmarkInfo marks, runtime/engine/io_types.h:104-163).
  * capacity is in int64 elements; sm_clock_khz converts cycles to time. */
 int B200Lm_TraceDecodeStep(B200LmExecutor* e, int32_t* out_id, int64_t* stamps, int64_t capacity,

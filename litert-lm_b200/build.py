@@ -18,7 +18,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200lm.so")
 # one translation unit per kernel family and cache type, compiled side by side
-SOURCES = ["lib.cu"] + [f"{k}_{t}.cu" for k in ("decode_fused", "decode_stream", "decode_wide", "attn_mma") for t in ("f32", "bf16")]
+SOURCES = ["lib.cu", "decode_step.cu"] + [f"{k}_{t}.cu" for k in ("decode_stream", "decode_wide", "attn_mma") for t in ("f32", "bf16")]
 
 
 def _deps():

@@ -41,18 +41,6 @@ struct LayerWeights {
   float attn_bound;                    // |q.k| / sqrt(hd) <= attn_bound after QK-RMSNorm: sqrt(hd) max|g_q| max|g_k|
 };
 
-// Copies of a layer's decode weights in the layouts the chained kernel streams with ONE bulk copy per
-// ring slot (the barrier-per-phase kernels use the plain tile order of LayerWeights).
-struct ChainedLayer {
-  const unsigned char* wqkv_s;   // per 16-row tile: its KT 512-byte tiles, then its 16 scales (64 bytes)
-  const unsigned char* wgu_s;    // same for the gate / up tiles (alternating)
-  const uint4* wdown_k;          // tiles ordered [k_tile][row_tile]: a 64-feature K slice is contiguous
-  const uint4* wo_s;             // tiles ordered [head slice][row_tile][k_tile of the slice]
-  const float* gA;               // [g_pre_attn | g_post_ffn of the previous layer]
-  const float* gD;               // [g_pre_ffn | g_post_attn]
-  const float* qk;               // [g_q | g_k]
-};
-
 struct LayerKv {
   void* k;               // [pages][hkv][kPage][hd], fp32 or bf16
   void* v;
@@ -68,8 +56,6 @@ struct DecodeState {          // lives in device memory, one per executor
   int err;                    // DeviceError
   unsigned int barrier;       // grid barrier counter (persistent kernel)
   int steps_done;
-  int gave_up[8];             // first bounded wait that gave up (chained kernel): phase code, layer, CTA, kind of wait,
-                              // then for a poll: tag seen, tag wanted, word offset in the exchange area, thread
 };
 
 struct DecodeArgs {
@@ -102,13 +88,8 @@ struct DecodeArgs {
   int* step_tokens;     // [capacity][ncols] arg-max of every step since steps_done was reset
   int step_capacity;
   int advance;          // 1: feed arg-max back as next token and bump pos (device loop)
-  // chained kernel only
-  const ChainedLayer* chained;        // device array [n_layers]
-  const unsigned char* head_ws;       // tied embedding as row-tile records (tiles + scales)
-  const float* gH;                    // [g_final | g_post_ffn of the last layer]
-  const float* rope_cs[2];            // [max_ctx][cos(hd/2) | sin(hd/2)]; 0 local, 1 global
-  int* progress;                      // [n_cta] phase code * 1000 + layer each CTA has reached (diagnostics)
   long long* trace;     // optional [n_barriers][n_cta][2] SM-clock stamps (arrive, release), or null
+  int trace_ctas;       // CTAs per barrier in both arrays (chain of step kernels)
   long long* trace_pts; // optional [n_barriers][n_cta][8] stamps inside the phase that ends at that barrier
 };
 
@@ -1006,26 +987,6 @@ static __device__ __noinline__ void phase_argmax(const DecodeArgs& a, int ncta_h
       }
     }
     if (threadIdx.x == 0) a.st->steps_done = sd + 1;
-  }
-}
-
-// ------------------------------------------------------- one kernel per phase
-
-enum DecodePhase { kPhQkv = 0, kPhAttn, kPhOproj, kPhGateUp, kPhDown, kPhHead, kPhArgmax };
-
-static __global__ void __launch_bounds__(kDecThreads, 1)
-decode_phase_kernel(const __grid_constant__ DecodeArgs a, int phase, int layer) {
-  extern __shared__ __align__(16) unsigned char dsm[];
-  DecodeSmem s = carve_smem(dsm, a.dims, a.ncols);
-  const int cta = blockIdx.x, ncta = gridDim.x;
-  switch (phase) {
-    case kPhQkv: phase_qkv(a, s, layer, cta, ncta); break;
-    case kPhAttn: phase_attn(a, s, layer, cta, ncta); break;
-    case kPhOproj: phase_oproj(a, s, layer, cta, ncta); break;
-    case kPhGateUp: phase_gateup(a, s, layer, cta, ncta); break;
-    case kPhDown: phase_down(a, s, layer, cta, ncta); break;
-    case kPhHead: phase_head(a, s, cta, ncta); break;
-    case kPhArgmax: phase_argmax(a, layer /* = head grid size */); break;
   }
 }
 

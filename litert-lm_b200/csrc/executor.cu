@@ -17,7 +17,7 @@
 #include "common.cuh"
 #include "decode_ops.cuh"
 #include "decode_stream.cuh"
-#include "decode_fused.cuh"
+#include "decode_step.cuh"
 #include "model_host.h"
 #include "prefill_ops.cuh"
 #include "prefill_gemm_ts.cuh"
@@ -60,42 +60,6 @@ static std::vector<uint32_t> w4t_host(const uint8_t* packed, int64_t rows, int64
   repack_w4t(packed, rows, K, map, buf.data());
   return buf;
 }
-// Row-tile records: the KT tiles of a 16-row tile followed by its 16 scales.
-static const unsigned char* upload_w4ts(Model& m, const std::vector<uint32_t>& w4t, const float* scale_tile_order, int64_t rows,
-                                        int64_t K) {
-  const int64_t RT = rows / 16, KT = K / 64, rec = KT * 512 + 64;
-  std::vector<unsigned char> out((size_t)RT * rec);
-  const unsigned char* src = reinterpret_cast<const unsigned char*>(w4t.data());
-  for (int64_t rt = 0; rt < RT; ++rt) {
-    memcpy(out.data() + rt * rec, src + rt * KT * 512, (size_t)KT * 512);
-    memcpy(out.data() + rt * rec + KT * 512, scale_tile_order + rt * 16, 64);
-  }
-  return upload(m, out.data(), out.size());
-}
-// Tiles reordered [k_tile][row_tile].
-static const uint4* upload_w4t_kmajor(Model& m, const std::vector<uint32_t>& w4t, int64_t rows, int64_t K) {
-  const int64_t RT = rows / 16, KT = K / 64;
-  std::vector<uint32_t> out(w4t.size());
-  for (int64_t rt = 0; rt < RT; ++rt)
-    for (int64_t kt = 0; kt < KT; ++kt) memcpy(out.data() + (kt * RT + rt) * 128, w4t.data() + (rt * KT + kt) * 128, 512);
-  return reinterpret_cast<const uint4*>(upload(m, out.data(), out.size()));
-}
-// Tiles reordered [k slice][row_tile][k_tile within the slice].
-static const uint4* upload_w4t_sliced(Model& m, const std::vector<uint32_t>& w4t, int64_t rows, int64_t K, int slices) {
-  const int64_t RT = rows / 16, KT = K / 64, ktc = KT / slices;
-  std::vector<uint32_t> out(w4t.size());
-  for (int64_t sl = 0; sl < slices; ++sl)
-    for (int64_t rt = 0; rt < RT; ++rt)
-      memcpy(out.data() + ((sl * RT + rt) * ktc) * 128, w4t.data() + (rt * KT + sl * ktc) * 128, (size_t)ktc * 512);
-  return reinterpret_cast<const uint4*>(upload(m, out.data(), out.size()));
-}
-static const float* upload_pair(Model& m, const float* a, const float* b, size_t n) {
-  std::vector<float> v(2 * n, 0.f);
-  memcpy(v.data(), a, n * 4);
-  if (b) memcpy(v.data() + n, b, n * 4);
-  return upload(m, v.data(), v.size());
-}
-
 // W4G with rows padded to 128; scales padded with 1.0.
 static void upload_w4g(Model& m, const uint8_t* packed, const float* scale, int64_t rows, int64_t K,
                        const uint8_t** w_out, const float** s_out) {
@@ -138,12 +102,6 @@ std::shared_ptr<Model> Model::load(const uint8_t* image, size_t n, int device, b
     }
     auto ht = w4t_host(bytes(e), d.vocab, d.d, [](int64_t r) { return r; });
     m->head_w = reinterpret_cast<const uint4*>(upload(*m, ht.data(), ht.size()));
-    m->head_ws = upload_w4ts(*m, ht, reinterpret_cast<const float*>(bytes(rec.need("embed.scale", 1))), d.vocab, d.d);
-  }
-  {
-    int hps = 1;
-    while ((hps * d.hd) % 64 != 0) ++hps;
-    m->o_slices = d.hq % hps == 0 ? d.hq / hps : 1;
   }
   m->g_final = fvec("final_norm", d.d);
   {
@@ -153,7 +111,6 @@ std::shared_ptr<Model> Model::load(const uint8_t* image, size_t n, int device, b
   }
   m->layers_host.resize(d.n_layers);
   m->gemm_host.resize(d.n_layers);
-  m->chained_host.resize(d.n_layers);
   auto fptr = [&](const std::string& nm) { return reinterpret_cast<const float*>(bytes(rec.need(nm, 1))); };
   for (int i = 0; i < d.n_layers; ++i) {
     std::string p = "L" + std::to_string(i) + ".";
@@ -171,30 +128,22 @@ std::shared_ptr<Model> Model::load(const uint8_t* image, size_t n, int device, b
     const float* sg = reinterpret_cast<const float*>(bytes(rec.need(p + "wgate.scale", 1)));
     const float* su = reinterpret_cast<const float*>(bytes(rec.need(p + "wup.scale", 1)));
     const float* sd = reinterpret_cast<const float*>(bytes(rec.need(p + "wdown.scale", 1)));
-    ChainedLayer& Cl = m->chained_host[i];
-    memset(&Cl, 0, sizeof Cl);
     auto ident = [](int64_t r) { return r; };
     {
       auto t = w4t_host(bytes(eqkv), d.nqkv(), d.d, ident);
       L.wqkv = reinterpret_cast<const uint4*>(upload(*m, t.data(), t.size()));
-      Cl.wqkv_s = upload_w4ts(*m, t, sqkv, d.nqkv(), d.d);
     }
     L.sqkv = upload(*m, sqkv, d.nqkv());
     {
       auto t = w4t_host(bytes(eo), d.d, d.nq(), ident);
       L.wo = reinterpret_cast<const uint4*>(upload(*m, t.data(), t.size()));
-      Cl.wo_s = upload_w4t_sliced(*m, t, d.d, d.nq(), m->o_slices);
     }
     L.so = upload(*m, so, d.d);
     {
       auto t = w4t_host(bytes(ed), d.d, d.ffn, ident);
       L.wdown = reinterpret_cast<const uint4*>(upload(*m, t.data(), t.size()));
-      Cl.wdown_k = upload_w4t_kmajor(*m, t, d.d, d.ffn);
     }
     L.sdown = upload(*m, sd, d.d);
-    Cl.gA = upload_pair(*m, fptr(p + "pre_attn"), i > 0 ? fptr("L" + std::to_string(i - 1) + ".post_ffn") : nullptr, d.d);
-    Cl.gD = upload_pair(*m, fptr(p + "pre_ffn"), fptr(p + "post_attn"), d.d);
-    Cl.qk = upload_pair(*m, fptr(p + "q_norm"), fptr(p + "k_norm"), d.hd);
     // gate and up share one matrix: canonical rows [gate ; up]
     std::vector<uint8_t> gu((size_t)2 * d.ffn * d.d / 2);
     memcpy(gu.data(), bytes(eg), (size_t)eg.nbytes);
@@ -214,7 +163,6 @@ std::shared_ptr<Model> Model::load(const uint8_t* image, size_t n, int device, b
         sc[r] = src < ffn ? sg[src] : su[src - ffn];
       }
       L.sgu = upload(*m, sc.data(), sc.size());
-      Cl.wgu_s = upload_w4ts(*m, buf, sc.data(), 2 * ffn, d.d);
     }
     auto gmax = [&](const std::string& nm) {
       const float* g = reinterpret_cast<const float*>(bytes(rec.need(nm, 1)));
@@ -262,20 +210,11 @@ std::shared_ptr<Model> Model::load(const uint8_t* image, size_t n, int device, b
   }
   m->has_tc = want_tc;
   m->layers_dev = upload(*m, m->layers_host.data(), m->layers_host.size());
-  m->chained_dev = upload(*m, m->chained_host.data(), m->chained_host.size());
-  m->gH = upload_pair(*m, fptr("final_norm"), fptr("L" + std::to_string(d.n_layers - 1) + ".post_ffn"), d.d);
   for (int t = 0; t < 2; ++t) {
     std::vector<float> c, s;
     build_rope_table(t ? d.rope_global : d.rope_local, d.hd, d.max_ctx, c, s);
     m->rope_cos[t] = upload(*m, c.data(), c.size());
     m->rope_sin[t] = upload(*m, s.data(), s.size());
-    const int half = d.hd / 2;
-    std::vector<float> cs((size_t)d.max_ctx * d.hd);
-    for (int pz = 0; pz < d.max_ctx; ++pz) {
-      memcpy(cs.data() + (size_t)pz * d.hd, c.data() + (size_t)pz * half, (size_t)half * 4);
-      memcpy(cs.data() + (size_t)pz * d.hd + half, s.data() + (size_t)pz * half, (size_t)half * 4);
-    }
-    m->rope_cs[t] = upload(*m, cs.data(), cs.size());
   }
   return m;
 }
@@ -396,7 +335,7 @@ static int round_up(int v, int a) { return (v + a - 1) / a * a; }
 Executor::~Executor() {
   cudaSetDevice(device);
   if (stream) cudaStreamSynchronize(stream);
-  if (graph_exec) cudaGraphExecDestroy(graph_exec);
+  for (auto& g : step_graphs) cudaGraphExecDestroy(g.second);
   for (auto& g : wide_graphs) cudaGraphExecDestroy(g.second);
   if (tp_comm) {
     try { NcclApi::get().CommDestroy(tp_comm); } catch (...) {}
@@ -536,11 +475,6 @@ std::unique_ptr<Executor> Executor::create(std::shared_ptr<Model> model, const B
   a.g_final = model->g_final;
   a.gmax_final = model->gmax_final;
   for (int t = 0; t < 2; ++t) { a.rope_cos[t] = model->rope_cos[t]; a.rope_sin[t] = model->rope_sin[t]; }
-  a.chained = model->chained_dev;
-  a.head_ws = model->head_ws;
-  a.gH = model->gH;
-  for (int t = 0; t < 2; ++t) a.rope_cs[t] = model->rope_cs[t];
-  a.progress = reinterpret_cast<int*>(e->alloc(sizeof(int) * 2 * e->n_sms, true));   // live words, then a snapshot
   a.st = reinterpret_cast<DecodeState*>(e->alloc(sizeof(DecodeState), true));
   const int G = d.group();
   const int max_splits = std::max(a.n_attn_splits_local, a.n_attn_splits_global);
@@ -569,32 +503,11 @@ std::unique_ptr<Executor> Executor::create(std::shared_ptr<Model> model, const B
         e->alloc(sizeof(float) * (size_t)e->n_sessions * d.hkv * kWideMaxSplits * d.group() * (d.hd + 2), true));
   }
   a.advance = 1;
-  // the one-kernel-per-phase fallback drives one session; the persistent kernels carry all of them
-  e->dec_smem = dec_smem_bytes(d, e->decode_mode == B200LM_DECODE_PHASE_KERNELS || e->decode_mode == B200LM_DECODE_PERSISTENT_BASIC
-                                      ? e->n_sessions : 1);
-  B2_CHECK(e->dec_smem <= (size_t)prop.sharedMemPerBlockOptin, kUnimplemented,
-           "decode kernels need more shared memory than the device offers");
-  raise_dyn_smem(decode_phase_kernel, (size_t)(e->dec_smem));
-  raise_dyn_smem(decode_persistent_kernel, (size_t)(e->dec_smem));
-  if (e->decode_mode == B200LM_DECODE_CHAINED) {
-    // the chained kernel needs its ring to fit and the softmax shift of its attention to be usable;
-    // otherwise the barrier-per-phase streaming kernel takes over
-    FusedPlan pl;
-    size_t smem = 0;
-    const int nc = e->n_sessions, nt = nc * 3 <= kQCols ? 3 : kQCols / nc;
-    const int cap = std::max(1, e->n_sms / (nc * d.hkv));
-    bool ok = prop.cooperativeLaunch &&
-              fused_make_plan(d, nc, nt, e->n_sms, a.o_slices, std::min(a.n_attn_splits_local, cap),
-                              std::min(a.n_attn_splits_global, cap), (size_t)prop.sharedMemPerBlockOptin, &pl, &smem);
-    for (float b : model->attn_bound) ok = ok && b <= kFaMaxBound;
-    ok = ok && a.o_slices == model->o_slices;      // the sliced W_o copy was laid out for this split
-    if (ok) {
-      e->chained_ok = true;
-      e->ll_bytes = (size_t)2 * pl.ll_words * sizeof(fu_u64);
-      e->ll_dev = reinterpret_cast<fu_u64*>(e->alloc(e->ll_bytes, true));
-    } else {
-      e->decode_mode = B200LM_DECODE_PERSISTENT;
-    }
+  if (e->decode_mode == B200LM_DECODE_PERSISTENT_BASIC) {
+    e->dec_smem = dec_smem_bytes(d, e->n_sessions);
+    B2_CHECK(e->dec_smem <= (size_t)prop.sharedMemPerBlockOptin, kUnimplemented,
+             "the persistent decode kernel needs more shared memory than the device offers");
+    raise_dyn_smem(decode_persistent_kernel, (size_t)(e->dec_smem));
   }
   if (e->decode_mode == B200LM_DECODE_PERSISTENT) {
     // staging halves take what shared memory the activation staging leaves, up to 96 KiB each
@@ -613,14 +526,28 @@ std::unique_ptr<Executor> Executor::create(std::shared_ptr<Model> model, const B
       int occ = (size_t)fa.maxThreadsPerBlock >= (size_t)kStreamThreads ? 1 : 0;
       ok = occ >= 1;
     }
-    if (!ok) e->decode_mode = B200LM_DECODE_PHASE_KERNELS;
+    if (!ok) e->decode_mode = B200LM_DECODE_CHAINED;
   }
-  B2_CHECK(e->n_sessions == 1 || e->decode_mode != B200LM_DECODE_PHASE_KERNELS, kUnimplemented,
-           "several sessions per executor need a persistent decode kernel, which this model / device does not fit");
+  if (e->decode_mode == B200LM_DECODE_PHASE_KERNELS || e->decode_mode == B200LM_DECODE_CHAINED) {
+    StepPlan& sp = e->step;
+    B2_CHECK(step_plan(d, e->n_sms, e->smem_optin, e->max_num_tokens, &sp), kUnimplemented,
+             "the decode step's kernels do not take this model's geometry");
+    sp.part_o = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.hkv * sp.max_splits * G * d.hd, true));
+    sp.part_ml = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.hkv * sp.max_splits * G * 2, true));
+    sp.opart = reinterpret_cast<float*>(e->alloc(sizeof(float) * sp.o_slices * kMaxCols * d.d, true));
+    sp.fpart = reinterpret_cast<float*>(e->alloc(sizeof(float) * sp.down_slices * kMaxCols * d.d, true));
+    sp.ticket = reinterpret_cast<int*>(e->alloc(sizeof(int), true));
+    for (int nc : {1, e->n_sessions}) {
+      DecodeArgs p = a;
+      p.ncols = nc;
+      p.nterms = nc * 3 <= kQCols ? 3 : kQCols / nc;
+      step_prepare(p, sp, model->layers_host.data(), e->kv_host.data());
+    }
+  }
   if (e->decode_mode == B200LM_DECODE_PERSISTENT_BASIC) {
     int occ = 0;
     B2_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, decode_persistent_kernel, kDecThreads, e->dec_smem));
-    if (occ < 1 || !prop.cooperativeLaunch) e->decode_mode = B200LM_DECODE_PHASE_KERNELS;
+    B2_CHECK(occ >= 1 && prop.cooperativeLaunch, kUnimplemented, "the persistent decode kernel does not fit this device");
   }
   // ---- prefill buffers (rows padded to whole 128-token tiles, zero-filled)
   e->t_max = d.buckets[0];
@@ -685,7 +612,7 @@ void Executor::tp_allreduce(float* buf, size_t count) {
 
 void Executor::check_device_error(const char* where) {
   int err = 0;
-  // err, barrier, steps_done and gave_up[4] are adjacent
+  // err, barrier and steps_done are adjacent
   const size_t tail = sizeof(DecodeState) - offsetof(DecodeState, err);
   B2_CUDA(cudaMemcpyAsync(&pin_state->err, &dargs.st->err, tail, cudaMemcpyDeviceToHost, stream));
   B2_CUDA(cudaStreamSynchronize(stream));
@@ -697,54 +624,7 @@ void Executor::check_device_error(const char* where) {
   barrier_epoch = 0;
   std::string w(where);
   if (err == kDevBarrierTimeout) {
-    std::string detail;
-    const int* g = pin_state->gave_up;
-    if (g[3] != 0)
-      detail = " (first: " + std::string(g[3] == 1 ? "poll" : g[3] == 2 ? "ring slot" : "copy producer") + ", phase code " +
-               std::to_string(g[0]) + ", layer / fill " + std::to_string(g[1]) + ", CTA " + std::to_string(g[2]) +
-               (g[7] ? ", thread " + std::to_string(g[7] - 1) + " saw tag " + std::to_string((unsigned)g[4]) + " for " +
-                           std::to_string((unsigned)g[5]) + " at word " + std::to_string(g[6]) + " (tag0 " +
-                           std::to_string(last_plan_ll.tag0) + ", words per copy " + std::to_string(last_plan_ll.ll_words) +
-                           ", ffn out at " + std::to_string(last_plan_ll.ll_f) + ")"
-                     : std::string()) + ")";
-    if (decode_mode == B200LM_DECODE_CHAINED) {
-      std::vector<int> prog(n_sms);      // the snapshot taken by the first wait that gave up
-      B2_CUDA(cudaMemcpy(prog.data(), dargs.progress + n_sms, sizeof(int) * n_sms, cudaMemcpyDeviceToHost));
-      // a word is step * 10000 + phase code * 1000 + layer; order in time: step, layer, phase (the head phases 6, 7 last)
-      auto when = [&](int w) {
-        const int code = w / 1000 % 10, layer = code >= 6 ? model->dims.n_layers : w % 1000;
-        return (long)(w / 10000) * 1000000L + (long)layer * 10 + code;
-      };
-      int lo = 0;
-      for (int i = 1; i < n_sms; ++i)
-        if (when(prog[i]) < when(prog[lo])) lo = i;
-      // which words of the exchange area of that layer never received their tag
-      if (ll_dev && last_plan_ll.ll_words > 0) {
-        const FusedPlan& fp = last_plan_ll;
-        const int layer = prog[lo] % 1000, step = prog[lo] / 10000, code = prog[lo] / 1000 % 10;
-        const int L = model->dims.n_layers;
-        const int src_layer = code == 1 ? layer - 1 : layer;       // phase A waits for the previous layer's reduce
-        if (src_layer >= 0 && src_layer < L) {
-          const unsigned want = fp.tag0 + (unsigned)step * (unsigned)(L + 1) + (unsigned)src_layer + 1u;
-          std::vector<fu_u64> words((size_t)fp.ll_words);
-          B2_CUDA(cudaMemcpy(words.data(), ll_dev + (size_t)(src_layer & 1) * fp.ll_words, sizeof(fu_u64) * fp.ll_words,
-                             cudaMemcpyDeviceToHost));
-          auto count = [&](int off, int n) {
-            int bad = 0, first = -1;
-            for (int i = 0; i < n; ++i)
-              if ((unsigned)(words[off + i] >> 32) != want) { if (first < 0) first = i; ++bad; }
-            return std::to_string(bad) + "/" + std::to_string(n) + (bad ? " (first " + std::to_string(first) + ")" : "");
-          };
-          const int d = model->dims.d;
-          detail += "; untagged words of layer " + std::to_string(src_layer) + ": qkv " + count(fp.ll_qkv, last_ncols * model->dims.nqkv()) +
-                    ", o " + count(fp.ll_o, dargs.o_slices * last_ncols * d) + ", ffn partials " +
-                    count(fp.ll_fpart, fp.nprod * last_ncols * d) + ", ffn out " + count(fp.ll_f, last_ncols * d);
-        }
-      }
-      detail += "; least advanced CTA " + std::to_string(lo) + " at phase code " + std::to_string(prog[lo] / 1000 % 10) + ", layer " +
-                std::to_string(prog[lo] % 1000) + ", step " + std::to_string(prog[lo] / 10000);
-    }
-    throw Error{kDeadlineExceeded, w + ": a bounded device-side wait gave up" + detail};
+    throw Error{kDeadlineExceeded, w + ": a bounded device-side wait gave up"};
   }
   if (err == kDevBadToken) throw Error{kInvalidArgument, w + ": token id outside the vocabulary"};
   if (err == kDevBadPosition) throw Error{kInvalidArgument, w + ": position outside the KV capacity"};
@@ -942,49 +822,6 @@ void Executor::launch_decode_steps(int nsteps, int ncols, int first_session) {
     launch_wide_steps(nsteps, ncols, first_session);
     return;
   }
-  if (decode_mode == B200LM_DECODE_CHAINED) {
-    DecodeArgs a = dargs;
-    a.ncols = ncols;
-    a.nterms = ncols * 3 <= kQCols ? 3 : kQCols / ncols;
-    a.page_table = page_table_dev + (size_t)first_session * pages_per_seq;
-    const int cap = std::max(1, ncta / (ncols * d.hkv));
-    a.n_attn_splits_local = std::min(a.n_attn_splits_local, cap);
-    a.n_attn_splits_global = std::min(a.n_attn_splits_global, cap);
-    FusedPlan pl;
-    size_t smem = 0;
-    B2_CHECK(fused_make_plan(d, a.ncols, a.nterms, ncta, a.o_slices, a.n_attn_splits_local, a.n_attn_splits_global,
-                             smem_optin, &pl, &smem),
-             kInternal, "the chained decode kernel does not fit this launch");
-    B2_CHECK((size_t)2 * pl.ll_words * sizeof(fu_u64) <= ll_bytes, kInternal, "exchange area too small");
-    // tags grow by one per (step, layer) and once more per step; start over (area cleared) long before they wrap
-    const unsigned need = (unsigned)nsteps * (unsigned)(d.n_layers + 1) + 2u;
-    if (ll_tag > 0xF0000000u - need) {
-      B2_CUDA(cudaMemsetAsync(ll_dev, 0, ll_bytes, stream));
-      ll_tag = 0;
-    }
-    pl.tag0 = ll_tag;
-    ll_tag += need;
-    last_plan_ll = pl;
-    last_ncols = a.ncols;
-    const void* kfn = decode_fused_kernel_for(d);
-    raise_dyn_smem(kfn, smem);
-    fu_u64* ll = ll_dev;
-    void* params[] = {&a, &pl, &ll, &nsteps};
-    cudaError_t le = cudaLaunchCooperativeKernel(kfn, dim3(ncta), dim3(kFuThreads), params, smem, stream);
-    if (le != cudaSuccess) {
-      cudaGetLastError();
-      cudaFuncAttributes fa{};
-      cudaFuncGetAttributes(&fa, kfn);
-      int occ = -1;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, kFuThreads, smem);
-      throw Error{kInternal, std::string("chained decode kernel launch: ") + cudaGetErrorString(le) + " (registers " +
-                                 std::to_string(fa.numRegs) + ", static shared " + std::to_string(fa.sharedSizeBytes) +
-                                 ", dynamic shared " + std::to_string(smem) + ", max threads " +
-                                 std::to_string(fa.maxThreadsPerBlock) + ", blocks per SM " + std::to_string(occ) + ")"};
-    }
-    launches += 1;
-    return;
-  }
   if (decode_mode == B200LM_DECODE_PERSISTENT || decode_mode == B200LM_DECODE_PERSISTENT_BASIC) {
     DecodeArgs a = dargs;
     a.ncols = ncols;
@@ -1009,38 +846,47 @@ void Executor::launch_decode_steps(int nsteps, int ncols, int first_session) {
     launches += 1;
     return;
   }
-  B2_CHECK(ncols == 1, kFailedPrecondition, "batched decode needs a persistent decode mode");
-  B2_CHECK(n_sessions == 1, kFailedPrecondition, "several sessions per executor need a persistent decode mode");
+  launch_chain(nsteps, ncols, first_session);
+}
+
+// The chain of step kernels for sessions [first, first + ncols): one CUDA graph per step.  Under tensor parallelism
+// the ranks' partial O and down outputs are summed between the kernels, launch by launch.
+void Executor::launch_chain(int nsteps, int ncols, int first) {
+  DecodeArgs a = dargs;
+  a.ncols = ncols;
+  a.nterms = ncols * 3 <= kQCols ? 3 : kQCols / ncols;      // int8 terms per activation: 3, or 2 with 3-4 sessions
+  a.page_table = page_table_dev + (size_t)first * pages_per_seq;
+  const LayerWeights* L = model->layers_host.data();
   if (tp_world > 1) {
-    // the same phases, launched one by one, with the ranks' partial O and down outputs summed in between
-    for (int s = 0; s < nsteps; ++s) {
-      for (int li = 0; li < d.n_layers; ++li)
-        for (int ph = kPhQkv; ph <= kPhDown; ++ph) {
-          decode_phase_kernel<<<ncta, kDecThreads, dec_smem, stream>>>(dargs, ph, li);
-          if (ph == kPhOproj) tp_allreduce(dargs.opart, (size_t)dargs.o_slices * dargs.ncols * d.d);
-          if (ph == kPhDown) tp_allreduce(dargs.fpart, (size_t)dargs.down_slices * dargs.ncols * d.d);
-        }
-      decode_phase_kernel<<<ncta, kDecThreads, dec_smem, stream>>>(dargs, kPhHead, 0);
-      decode_phase_kernel<<<1, kDecThreads, dec_smem, stream>>>(dargs, kPhArgmax, ncta);
-    }
-    B2_CUDA(cudaGetLastError());
-    launches += (int64_t)nsteps * (5 * d.n_layers + 2);
+    auto reduce = [](void* self, float* buf, size_t count) { static_cast<Executor*>(self)->tp_allreduce(buf, count); };
+    for (int s = 0; s < nsteps; ++s) launches += step_launch(stream, a, step, L, kv_host.data(), reduce, this);
     return;
   }
-  if (!graph_exec) {
+  if (dargs.trace) {                          // a timeline is taken once: not worth a graph of its own
+    for (int s = 0; s < nsteps; ++s) launches += step_launch(stream, a, step, L, kv_host.data(), nullptr, nullptr);
+    return;
+  }
+  auto key = std::make_pair(ncols, first);
+  auto it = step_graphs.find(key);
+  if (it == step_graphs.end()) {
     cudaGraph_t graph;
     B2_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    for (int li = 0; li < d.n_layers; ++li)
-      for (int ph = kPhQkv; ph <= kPhDown; ++ph)
-        decode_phase_kernel<<<ncta, kDecThreads, dec_smem, stream>>>(dargs, ph, li);
-    decode_phase_kernel<<<ncta, kDecThreads, dec_smem, stream>>>(dargs, kPhHead, 0);
-    decode_phase_kernel<<<1, kDecThreads, dec_smem, stream>>>(dargs, kPhArgmax, ncta);
+    try {
+      step_launch(stream, a, step, L, kv_host.data(), nullptr, nullptr);
+    } catch (...) {
+      cudaGraph_t dead = nullptr;
+      cudaStreamEndCapture(stream, &dead);
+      if (dead) cudaGraphDestroy(dead);
+      throw;
+    }
     B2_CUDA(cudaStreamEndCapture(stream, &graph));
-    B2_CUDA(cudaGraphInstantiate(&graph_exec, graph, 0));
+    cudaGraphExec_t exec = nullptr;
+    B2_CUDA(cudaGraphInstantiate(&exec, graph, 0));
     cudaGraphDestroy(graph);
+    it = step_graphs.emplace(key, exec).first;
   }
-  for (int s = 0; s < nsteps; ++s) B2_CUDA(cudaGraphLaunch(graph_exec, stream));
-  launches += (int64_t)nsteps * (5 * d.n_layers + 2);
+  for (int s = 0; s < nsteps; ++s) B2_CUDA(cudaGraphLaunch(it->second, stream));
+  launches += (int64_t)nsteps * (5 * model->dims.n_layers + 1);
 }
 
 // One wide step for sessions [first, first + nb): the token rows of the GEMMs are the sessions.
@@ -1268,8 +1114,8 @@ void Executor::trace_decode_step(int* out_id, long long* stamps, long long capac
                                  int* khz) {
   const ModelDims& d = model->dims;
   B2_CHECK(decode_mode == B200LM_DECODE_PERSISTENT || decode_mode == B200LM_DECODE_PERSISTENT_BASIC ||
-               decode_mode == B200LM_DECODE_CHAINED,
-           kFailedPrecondition, "the decode timeline needs a persistent decode mode");
+               decode_mode == B200LM_DECODE_CHAINED || decode_mode == B200LM_DECODE_PHASE_KERNELS,
+           kFailedPrecondition, "the wide decode mode has no timeline");
   B2_CUDA(cudaSetDevice(device));
   const int nb = 5 * d.n_layers + 2;
   const long long need = (long long)nb * n_sms * 10;     // 2 barrier stamps + 8 in-phase stamps
@@ -1279,6 +1125,7 @@ void Executor::trace_decode_step(int* out_id, long long* stamps, long long capac
   B2_CUDA(cudaMemsetAsync(trace_dev, 0, sizeof(long long) * need, stream));
   dargs.trace = trace_dev;
   dargs.trace_pts = trace_dev + (size_t)nb * n_sms * 2;
+  dargs.trace_ctas = n_sms;
   try {
     decode_tokens(1, out_id);
   } catch (...) {
@@ -1293,7 +1140,8 @@ void Executor::trace_decode_step(int* out_id, long long* stamps, long long capac
   *n_cta = n_sms;
   int rate = 0;
   B2_CUDA(cudaDeviceGetAttribute(&rate, cudaDevAttrClockRate, device));
-  *khz = rate;
+  // the chain's kernels stamp nanoseconds: their CTAs move between SMs, whose cycle counters differ
+  *khz = decode_mode == B200LM_DECODE_PHASE_KERNELS || decode_mode == B200LM_DECODE_CHAINED ? 1000000 : rate;
 }
 
 void Executor::reset() {

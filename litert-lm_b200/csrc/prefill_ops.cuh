@@ -375,6 +375,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // Bounded wait: false (and the error word set) if the phase never completes.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err) {
   const uint32_t addr = smem_u32(bar);
+#pragma unroll 1
   for (int tries = 0; tries < (1 << 22); ++tries) {
     uint32_t done;
     asm volatile(

@@ -11,7 +11,7 @@
 #include "../../include/b200lm.h"
 #include "common.cuh"
 #include "decode_ops.cuh"
-#include "decode_fused.cuh"
+#include "decode_step.cuh"
 #include "decode_wide.cuh"
 #include "tp_nccl.h"
 
@@ -42,13 +42,6 @@ struct Model {
   std::vector<LayerGemmWeights> gemm_host;
   std::vector<float> attn_bound;     // per layer: sqrt(hd) max|g_q| max|g_k| >= any |q.k| / sqrt(hd)
   const LayerWeights* layers_dev = nullptr;
-  // layouts of the chained decode kernel (see ChainedLayer)
-  int o_slices = 1;                  // head slices of the o-proj (K split by whole heads, 64-wide at least)
-  std::vector<ChainedLayer> chained_host;
-  const ChainedLayer* chained_dev = nullptr;
-  const unsigned char* head_ws = nullptr;
-  const float* gH = nullptr;
-  const float* rope_cs[2] = {nullptr, nullptr};
   std::vector<void*> allocations;
 
   ~Model();
@@ -135,15 +128,10 @@ class Executor {
   // tensor parallelism: sum over the ranks of a buffer of partial projections, on the executor's stream
   NcclApi::Comm tp_comm = nullptr;
   unsigned barrier_epoch = 0;
-  // chained decode kernel: exchange area (two parity copies of flag-carrying words) and the next free tag
-  fu_u64* ll_dev = nullptr;
-  size_t ll_bytes = 0;
-  unsigned ll_tag = 0;
-  FusedPlan last_plan_ll{};         // plan of the last chained launch (diagnostics of a wait that gave up)
-  int last_ncols = 1;
-  bool chained_ok = false;          // the model fits the chained kernel (with n_sessions columns)
   long long* trace_dev = nullptr;
-  cudaGraphExec_t graph_exec = nullptr;
+  StepPlan step;                    // chain of step kernels (decode_step.cuh)
+  std::map<std::pair<int, int>, cudaGraphExec_t> step_graphs;   // one step, keyed by (sessions, first session)
+  void launch_chain(int nsteps, int ncols, int first);
   // wide lockstep decode (B200LM_DECODE_WIDE)
   WideState wide{nullptr, nullptr, nullptr};
   float* wide_part = nullptr;       // key-split partial states of the wide attention

@@ -1,0 +1,71 @@
+"""The chain of step kernels (default decode path) where it can go wrong: contexts of several key rounds per split,
+projections longer than their ring, two to four sessions against one at a time."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from conftest import seeded_ids
+
+pytestmark = pytest.mark.gpu
+
+
+def image(mio, cfg):
+    return mio.export_model_litertlm(cfg, mio.build_weights_record(cfg))
+
+
+@pytest.mark.parametrize("kv_dtype", [0, 1])
+@pytest.mark.parametrize("prompt", [33, 2048, 2049, 5003])       # one key, one round per split, one key more, several rounds
+def test_long_contexts_agree_with_the_streaming_kernel(pkg, mio, prompt, kv_dtype):
+    cfg = dataclasses.replace(mio.config_small(), max_ctx=6144, window=2500, kv_dtype=kv_dtype)
+    img = image(mio, cfg)
+    ids = seeded_ids(prompt, cfg.vocab, prompt)
+    chain, stream = (pkg.B200LlmExecutor(img, decode_mode=m) for m in (pkg.DECODE_CHAINED, pkg.DECODE_PERSISTENT))
+    assert stream.GetDecodeMode() == pkg.DECODE_PERSISTENT
+    for ex in (chain, stream):
+        ex.Prefill(ids)
+    for step in range(3):
+        a, b = (ex.DecodeLogits(None if step == 0 else 5 + step).ravel().astype(np.float64) for ex in (chain, stream))
+        assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(b), step
+
+
+@pytest.mark.parametrize("d_model,ffn,vocab", [(64, 64, 16), (448, 4096, 40000), (1152, 12800, 2048)])   # fewer tiles than CTAs .. streamed
+def test_odd_projections_agree_with_the_streaming_kernel(pkg, mio, d_model, ffn, vocab):
+    cfg = dataclasses.replace(mio.config_small(), n_layers=2, d_model=d_model, ffn=ffn, vocab=vocab, max_ctx=256)
+    img = image(mio, cfg)
+    ids = seeded_ids(3, cfg.vocab, 70)
+    out = []
+    for mode in (pkg.DECODE_CHAINED, pkg.DECODE_PERSISTENT_BASIC):
+        ex = pkg.B200LlmExecutor(img, decode_mode=mode)
+        ex.Prefill(ids)
+        out.append(ex.DecodeLogits().ravel().astype(np.float64))
+    assert np.linalg.norm(out[0] - out[1]) <= 1e-4 * np.linalg.norm(out[1])
+
+
+@pytest.mark.parametrize("sessions", [2, 3, 4])
+def test_sessions_in_lockstep_agree_with_one_at_a_time(pkg, models, sessions):
+    cfg, _, img = models("small")
+    prompts = [seeded_ids(40 + i, cfg.vocab, 30 + 41 * i) for i in range(sessions)]
+    ex = pkg.B200LlmExecutor(img, n_sessions=sessions)
+    for i, p in enumerate(prompts):
+        ex.PrefillSession(i, p)
+    got = ex.DecodeTokensBatch(6)
+    for i, p in enumerate(prompts):
+        solo = pkg.B200LlmExecutor(img)
+        solo.Prefill(p)
+        assert list(solo.DecodeTokens(6)) == list(got[:, i]), i
+        ex.SelectSession(i)
+        a, b = (e.DecodeLogits().ravel().astype(np.float64) for e in (ex, solo))
+        assert np.linalg.norm(a - b) <= 2e-3 * np.linalg.norm(b), i     # two int8 terms with three or four sessions
+
+
+def test_timeline_covers_every_kernel_of_the_step(pkg, models):
+    cfg, _, img = models("small")
+    ex = pkg.B200LlmExecutor(img)
+    ex.Prefill(seeded_ids(1, cfg.vocab, 20))
+    tok, stamps, khz = ex.TraceDecodeStep()
+    pts = ex.last_trace_points
+    assert stamps.shape[0] == 5 * cfg.n_layers + 2 and khz == 1000000 and 0 <= tok < cfg.vocab
+    for k in range(5 * cfg.n_layers + 1):
+        p = pts[k][pts[k][:, 4] > 0]
+        assert len(p) and (np.diff(p[:, :5], axis=1) >= 0).all(), k
