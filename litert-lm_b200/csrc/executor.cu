@@ -240,8 +240,7 @@ static EncodeTiledFn encode_tiled_fn() {
 // bf16 row-major [rows][cols]; box = 64 columns x 128 rows, 128-byte swizzle.
 ActMap make_activation_map(const __nv_bfloat16* base, int rows, int cols) {
   ActMap m;
-  m.box128 = make_activation_map_box(base, rows, cols, kGemmBM);
-  m.box64 = make_activation_map_box(base, rows, cols, 64);
+  for (int i = 0; i < 4; ++i) m.box[i] = make_activation_map_box(base, rows, cols, 16 << i);
   return m;
 }
 
@@ -290,8 +289,7 @@ int pick_ksplit(int T, int n_tiles, int KB, int sms) {
   return best;
 }
 
-// Launches one int4 GEMM.  a_map must describe `A` ([rows >= T][K] bf16); a GEMM of at most 64 token rows
-// uses a_map64, the same tensor with a 64-row box.
+// Launches one int4 GEMM.  a_map must describe `A` ([rows >= T][K] bf16).
 void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bfloat16* A,
                  const uint4* w4t, const float* s4t, const uint8_t* w4g, const float* s4g, int T, int N, int K,
                  int ksplit, bool geglu, float* outF, __nv_bfloat16* outB, int* err, int64_t* launches) {
@@ -308,6 +306,10 @@ void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bflo
       raise_dyn_smem(gemm_w4_ts_kernel<1, 128>, (size_t)ts_smem(128));
       raise_dyn_smem(gemm_w4_ts_kernel<0, 64>, (size_t)ts_smem(64));
       raise_dyn_smem(gemm_w4_ts_kernel<1, 64>, (size_t)ts_smem(64));
+      raise_dyn_smem(gemm_w4_ts_kernel<0, 32>, (size_t)ts_smem(32));
+      raise_dyn_smem(gemm_w4_ts_kernel<1, 32>, (size_t)ts_smem(32));
+      raise_dyn_smem(gemm_w4_ts_kernel<0, 16>, (size_t)ts_smem(16));
+      raise_dyn_smem(gemm_w4_ts_kernel<1, 16>, (size_t)ts_smem(16));
       B2_CUDA(cudaDeviceGetAttribute(&sms_of[dev], cudaDevAttrMultiProcessorCount, dev));
     }
     const int sms = sms_of[dev];
@@ -315,9 +317,15 @@ void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bflo
     const int total = ((N + kTsRows - 1) / kTsRows) * ((T + ntok - 1) / ntok) * ksplit;
     const int grid = total < sms ? total : sms;
 #define B2_TS(EPI_, NTOK_, MAP_) launch_pdl(gemm_w4_ts_kernel<EPI_, NTOK_>, dim3(grid), dim3(ts_threads(NTOK_)), ts_smem(NTOK_), st, MAP_, g)
-    if (ntok == 64) { if (geglu) B2_TS(1, 64, a_map.box64); else B2_TS(0, 64, a_map.box64); }
-    else if (ntok == 128) { if (geglu) B2_TS(1, 128, a_map.box128); else B2_TS(0, 128, a_map.box128); }
-    else { if (geglu) B2_TS(1, 256, a_map.box128); else B2_TS(0, 256, a_map.box128); }
+#define B2_TS2(NTOK_, MAP_) do { if (geglu) B2_TS(1, NTOK_, MAP_); else B2_TS(0, NTOK_, MAP_); } while (0)
+    switch (ntok) {
+      case 16: B2_TS2(16, a_map.box[0]); break;
+      case 32: B2_TS2(32, a_map.box[1]); break;
+      case 64: B2_TS2(64, a_map.box[2]); break;
+      case 128: B2_TS2(128, a_map.box[3]); break;
+      default: B2_TS2(256, a_map.box[3]); break;
+    }
+#undef B2_TS2
 #undef B2_TS
   } else {
     B2_CHECK(ksplit == 1, kInternal, "the check GEMM does not split K");

@@ -12,44 +12,55 @@
 // needs the full 128 B/clk of the SM by itself).
 //
 // The kernel is persistent: one CTA per SM walks a static list of output tiles
-// (128 weight rows x 256 tokens x one K split).  Lane i of the accumulator is
+// (128 weight rows x NTOK tokens x one K split).  Lane i of the accumulator is
 // weight row i, so the per-channel scale is one scalar per epilogue thread and
-// a warp's store covers 32 consecutive output features of one token.  The 16
-// epilogue warps first pull the whole accumulator into registers (64 values
-// per thread) and hand it back, so the scaling / GeGLU and the global stores
-// of one tile run under the main loop of the next.
+// a warp's store covers 32 consecutive output features of one token.  The
+// epilogue warps first pull the whole accumulator into registers (at most 64
+// values per thread) and hand it back, so the scaling / GeGLU and the global
+// stores of one tile run under the main loop of the next.
 //
-// Warp roles: 0 = TMA producer, 1 = TMEM owner + MMA issue, 2..5 = int4
-// expansion, 6..21 = epilogue.
+// Three rings, each with its own depth, move two k blocks (128 k) at a time: the
+// int4 blocks (from HBM, deep), the activation tiles (from L2, shallow) and the
+// expanded weights in tensor memory.  A hand-over between two roles costs a few
+// hundred cycles however little it covers; with one k block per hand-over and one
+// ring for all three, a k block took 780 - 990 cycles at any token width, where
+// the HBM time is 180 and the M128 N256 K64 product takes 512.
 //
-// TMEM columns: [0, NTOK) accumulator, then one slot of 32 columns per pipeline
-// stage holding one expanded 128 x 64 weight tile each.
+// The weights do not depend on the preceding kernel, so their stream and their
+// expansion start before griddepcontrol.wait; narrow tiles take half of an SM's
+// shared and tensor memory, which lets the next GEMM's CTA do that while this one
+// works.
+//
+// Warp roles: 0 = activation producer, 1 = TMEM owner + MMA issue, 2 = weight
+// producer, 4.. = int4 expansion, then epilogue.
+//
+// TMEM columns: [0, NTOK) accumulator, then slots of 64 columns holding one
+// expanded 128 x 128 weight tile each.
 #pragma once
 #include "prefill_ops.cuh"
 
 namespace b200lm {
 
-constexpr int kTsStages = 5;
 constexpr int kTsRows = 128;                        // weight rows per tile
-constexpr int kTsTok = 256;                         // tokens per tile
-constexpr int kTsAcols = 32;                        // TMEM columns of one expanded 128 x 64 weight tile
-// Warps per role and token width: narrow tiles give the warps their smaller epilogue does not need to the
-// int4 expansion (two warps per 32 accumulator lanes, half a weight row each).  The epilogue needs one warp
-// per 32 lanes x 64 token columns.
+constexpr int kTsKb = 2;                            // k blocks per stage
+constexpr int kTsAcols = 32;                        // TMEM columns of one expanded 128 x 64 weight block
+// Depth of the rings and warps per role by token width.  Narrow tiles: the bytes in flight that HBM wants sit in the
+// weight ring (8 KB a stage), everything together stays within half an SM.  256 tokens: tensor-bound, all of the SM.
+__host__ __device__ constexpr int ts_xs(int ntok) { return ntok >= 128 ? (ntok >= 256 ? 3 : 2) : 3; }
+__host__ __device__ constexpr int ts_qs(int ntok) { return ntok >= 256 ? 3 : ntok == 128 ? 5 : ntok == 64 ? 7 : 10; }
+__host__ __device__ constexpr int ts_ws(int ntok) { return ntok >= 256 ? 4 : ntok == 128 ? 2 : 3; }
+__host__ __device__ constexpr int ts_tmem(int ntok) { return ntok >= 256 ? 512 : 256; }
 __host__ __device__ constexpr int ts_deq_warps(int ntok) { return ntok >= 256 ? 4 : 8; }
-__host__ __device__ constexpr int ts_epi_warps(int ntok) { return 4 * (ntok / 64); }
-__host__ __device__ constexpr int ts_threads(int ntok) { return 64 + 32 * (ts_deq_warps(ntok) + ts_epi_warps(ntok)); }
-constexpr int kTsStageX = kTsTok * kGemmBK * 2;     // activation tile, 32 KB
-constexpr int kTsTmemCols = 512;
-// Pipeline depth per token width.  A stage holds one k block: NTOK x 64 activations and 4 KB of int4 weights.
-// The weights come from HBM, so what bounds a narrow tile is the bytes in flight per SM (stages x 4 KB over a
-// round trip of a few microseconds), not the MMA: narrow tiles spend the shared memory and the tensor-memory
-// columns the accumulator leaves on more stages.
-__host__ __device__ constexpr int ts_stages(int ntok) { return ntok >= 256 ? kTsStages : ntok == 128 ? 8 : 12; }
-__host__ __device__ constexpr int ts_smem(int ntok) { return ts_stages(ntok) * (ntok * kGemmBK * 2 + kGemmStageQ) + 1024 + 512; }
-static_assert(256 + ts_stages(256) * kTsAcols <= kTsTmemCols && 128 + ts_stages(128) * kTsAcols <= kTsTmemCols &&
-                  64 + ts_stages(64) * kTsAcols <= kTsTmemCols, "TMEM budget");
-static_assert(ts_smem(256) <= 227 * 1024 && ts_smem(128) <= 227 * 1024 && ts_smem(64) <= 227 * 1024, "shared memory budget");
+__host__ __device__ constexpr int ts_epi_cols(int ntok) { return ntok < 64 ? ntok : 64; }      // token columns per epilogue warp
+__host__ __device__ constexpr int ts_epi_warps(int ntok) { return 4 * (ntok / ts_epi_cols(ntok)); }
+__host__ __device__ constexpr int ts_threads(int ntok) { return 32 * (4 + ts_deq_warps(ntok) + ts_epi_warps(ntok)); }
+__host__ __device__ constexpr int ts_smem(int ntok) {
+  return ts_xs(ntok) * kTsKb * ntok * kGemmBK * 2 + ts_qs(ntok) * kTsKb * kGemmStageQ + 1024 + 512;
+}
+static_assert(ts_tmem(256) >= 256 + ts_ws(256) * kTsKb * kTsAcols && ts_tmem(128) >= 128 + ts_ws(128) * kTsKb * kTsAcols &&
+                  ts_tmem(64) >= 64 + ts_ws(64) * kTsKb * kTsAcols, "TMEM budget");
+static_assert(ts_smem(256) <= 227 * 1024 && 2 * (ts_smem(128) + 1024) <= 228 * 1024 && 2 * (ts_smem(64) + 1024) <= 228 * 1024 &&
+                  2 * (ts_smem(32) + 1024) <= 228 * 1024, "shared memory budget");
 
 // A operand in tensor memory, B through a shared-memory descriptor
 __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
@@ -92,76 +103,113 @@ __device__ __forceinline__ TsTile ts_tile(int tile, int n_tiles, int t_tiles) {
   return t;
 }
 
+// EC consecutive accumulator columns of this thread's lane
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+template <int EC>
+__device__ __forceinline__ void ts_load_acc(uint32_t taddr, uint32_t (&v)[EC]) {
+#pragma unroll
+  for (int c = 0; c < EC; c += 16) tmem_ld16(taddr + c, v + c);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 // EPI 0: fp32 partials outF[ks][T][N].  EPI 1: GeGLU; tile rows alternate
 // gate (even) and up (odd) rows of one ffn feature, output bf16 outB[T][N/2].
 //
-// NTOK is the token width of a tile (the N of the MMA): 256 for prefill; 128 or 64 when the whole GEMM has
+// NTOK is the token width of a tile (the N of the MMA): 256 for prefill; 128 .. 16 when the whole GEMM has
 // no more token rows than that (the wide decode step, short prompts), which cuts the activation bytes every
 // CTA re-reads per k block and the MMA time in proportion.  tmX must have a box of min(NTOK, 128) rows.
 template <int EPI, int NTOK>
-__global__ void __launch_bounds__(ts_threads(NTOK), 1)
+__global__ void __launch_bounds__(ts_threads(NTOK), NTOK <= 64 ? 2 : 1)
 gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
-  constexpr int kTsDeqWarps = ts_deq_warps(NTOK), kTsEpiWarps = ts_epi_warps(NTOK);
-  constexpr int S = ts_stages(NTOK);
-  constexpr int kStageX = NTOK * kGemmBK * 2;       // activation tile of one stage
-  constexpr uint32_t kStageTx = NTOK * kGemmBK * 2 + kGemmStageQ;
+  constexpr int D = ts_deq_warps(NTOK), E = ts_epi_warps(NTOK), EC = ts_epi_cols(NTOK);
+  constexpr int XS = ts_xs(NTOK), QS = ts_qs(NTOK), WS = ts_ws(NTOK);
+  constexpr int kXb = NTOK * kGemmBK * 2;           // activation bytes of a k block
   extern __shared__ unsigned char gsm_raw[];
   unsigned char* gsm = reinterpret_cast<unsigned char*>(((uintptr_t)gsm_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sX = gsm;
-  unsigned char* sQ = gsm + S * kStageX;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sQ + S * kGemmStageQ);
-  uint64_t* full_bar = bars;              // [S] TMA bytes landed
-  uint64_t* deq_bar = bars + S;           // [S] expanded weights are in TMEM
-  uint64_t* empty_bar = bars + 2 * S;     // [S] MMA finished with the stage (shared memory and TMEM slot)
-  uint64_t* acc_full = bars + 3 * S;      // accumulator complete
-  uint64_t* acc_empty = bars + 3 * S + 1; // accumulator read out by the epilogue warps
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * S + 2);
+  unsigned char* sQ = gsm + XS * kTsKb * kXb;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sQ + QS * kTsKb * kGemmStageQ);
+  uint64_t* x_full = bars;                          // [XS] activation tiles landed
+  uint64_t* x_empty = x_full + XS;                  // [XS] MMAs finished with them
+  uint64_t* q_full = x_empty + XS;                  // [QS] int4 blocks landed
+  uint64_t* q_empty = q_full + QS;                  // [QS] expansion has read them
+  uint64_t* w_full = q_empty + QS;                  // [WS] expanded weights are in TMEM
+  uint64_t* w_empty = w_full + WS;                  // [WS] MMAs finished with them
+  uint64_t* acc_full = w_empty + WS;                // accumulator complete
+  uint64_t* acc_empty = acc_full + 1;               // accumulator read out by the epilogue warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int KB = g.K / kGemmBK;
   const int nkb = KB / g.ksplit;
+  const int nst = (nkb + kTsKb - 1) / kTsKb;        // stages of a tile; the last may hold one k block
   const int n_tiles = (g.N + kTsRows - 1) / kTsRows;
   const int t_tiles = (g.T + NTOK - 1) / NTOK;
   const int total = n_tiles * t_tiles * g.ksplit;
   const int my_tiles = (int)blockIdx.x < total ? (total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
+  // weight producer: one lane's state, started ahead of everything else
+  int q_it = 0, q_li = 0, q_st = 0;
+  auto q_issue = [&]() {                            // warp 2, lane 0
+    const TsTile tl = ts_tile(blockIdx.x + q_li * gridDim.x, n_tiles, t_tiles);
+    const int kb = q_st * kTsKb, nk = min(kTsKb, nkb - kb), s = q_it % QS;
+    mbar_arrive_expect_tx(&q_full[s], (uint32_t)nk * kGemmStageQ);
+    bulk_load_1d(sQ + s * kTsKb * kGemmStageQ, g.w + ((size_t)tl.n_tile * KB + (size_t)tl.ks * nkb + kb) * kGemmStageQ,
+                 (uint32_t)nk * kGemmStageQ, &q_full[s]);
+    ++q_it;
+    if (++q_st == nst) { q_st = 0; ++q_li; }
+  };
+  if (threadIdx.x == 64) {
+#pragma unroll 1
+    for (int s = 0; s < QS; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], D); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+#pragma unroll 1
+    while (q_it < QS && q_li < my_tiles) q_issue();
+  }
   if (threadIdx.x == 0) {
-    for (int s = 0; s < S; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&deq_bar[s], kTsDeqWarps);
-      mbar_init(&empty_bar[s], 1);
-    }
+#pragma unroll 1
+    for (int s = 0; s < XS; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
+#pragma unroll 1
+    for (int s = 0; s < WS; ++s) { mbar_init(&w_full[s], D); mbar_init(&w_empty[s], 1); }
     mbar_init(acc_full, 1);
-    mbar_init(acc_empty, kTsEpiWarps);
+    mbar_init(acc_empty, E);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(tmem_slot, kTsTmemCols);
+  if (warp == 1) tmem_alloc(tmem_slot, ts_tmem(NTOK));
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_w = tmem_base + NTOK;         // weight slots follow the accumulator columns
-  // barriers and TMEM are set up: from here on the kernel reads what its predecessor wrote
-  pdl_wait();
   pdl_launch_dependents();
 
   if (warp == 0) {
-    // ---- producer: one elected lane issues the copies, the warp stays together
+    // ---- activation producer: what it reads comes from the preceding kernel
+    pdl_wait();
     int it = 0;
     bool ok = true;
+#pragma unroll 1
     for (int li = 0; li < my_tiles && ok; ++li) {
       const TsTile tl = ts_tile(blockIdx.x + li * gridDim.x, n_tiles, t_tiles);
-      const uint8_t* wtile = g.w + ((size_t)tl.n_tile * KB + (size_t)tl.ks * nkb) * kGemmStageQ;
-      for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
-        const int s = it % S, n = it / S;
-        if (n > 0) ok = mbar_wait(&empty_bar[s], (n - 1) & 1, g.err);
+#pragma unroll 1
+      for (int st = 0; st < nst && ok; ++st, ++it) {
+        const int s = it % XS, n = it / XS, kb = st * kTsKb, nk = min(kTsKb, nkb - kb);
+        if (n > 0) ok = mbar_wait(&x_empty[s], (n - 1) & 1, g.err);
         if (ok && lane == 0) {
-          mbar_arrive_expect_tx(&full_bar[s], kStageTx);
+          mbar_arrive_expect_tx(&x_full[s], (uint32_t)(nk * kXb));
+#pragma unroll 1
+          for (int k = 0; k < nk; ++k)
 #pragma unroll
-          for (int h = 0; h < (NTOK + 127) / 128; ++h)
-            tma_load_2d(sX + s * kStageX + h * 128 * 128, &tmX, (tl.ks * nkb + kb) * kGemmBK,
-                        tl.t_tile * NTOK + h * 128, &full_bar[s]);
-          bulk_load_1d(sQ + s * kGemmStageQ, wtile + (size_t)kb * kGemmStageQ, kGemmStageQ, &full_bar[s]);
+            for (int h = 0; h < (NTOK + 127) / 128; ++h)
+              tma_load_2d(sX + (s * kTsKb + k) * kXb + h * 128 * 128, &tmX, (tl.ks * nkb + kb + k) * kGemmBK, tl.t_tile * NTOK + h * 128,
+                          &x_full[s]);
         }
         __syncwarp();
       }
@@ -171,100 +219,122 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
     const uint32_t idesc = umma_idesc_bf16(kTsRows, NTOK);
     int it = 0;
     bool ok = true;
+#pragma unroll 1
     for (int li = 0; li < my_tiles && ok; ++li) {
       if (li > 0) ok = mbar_wait(acc_empty, (li - 1) & 1, g.err);
       tc_fence_after();
-      for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
-        const int s = it % S, n = it / S;
-        ok = mbar_wait(&full_bar[s], n & 1, g.err) && mbar_wait(&deq_bar[s], n & 1, g.err);
+#pragma unroll 1
+      for (int st = 0; st < nst && ok; ++st, ++it) {
+        const int sx = it % XS, sw = it % WS, nk = min(kTsKb, nkb - st * kTsKb);
+        ok = mbar_wait(&w_full[sw], (it / WS) & 1, g.err) && mbar_wait(&x_full[sx], (it / XS) & 1, g.err);
         if (!ok) break;
         tc_fence_after();
         if (lane == 0) {
-          const uint64_t xd = umma_desc_sw128(smem_u32(sX + s * kStageX));
+#pragma unroll 1
+          for (int kb = 0; kb < nk; ++kb) {
+            const uint64_t xd = umma_desc_sw128(smem_u32(sX + (sx * kTsKb + kb) * kXb));
 #pragma unroll
-          for (int k = 0; k < kGemmBK / 16; ++k)   // 16 bf16 along K per MMA: 8 TMEM columns, 32 bytes of X
-            umma_bf16_ts(tmem_base, tmem_w + s * kTsAcols + k * 8, xd + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
-          umma_commit(&empty_bar[s]);
+            for (int k = 0; k < kGemmBK / 16; ++k)   // 16 bf16 along K per MMA: 8 TMEM columns, 32 bytes of X
+              umma_bf16_ts(tmem_base, tmem_w + (sw * kTsKb + kb) * kTsAcols + k * 8, xd + (uint64_t)(k * 2), idesc, (st | kb | k) ? 1u : 0u);
+          }
+          umma_commit(&w_empty[sw]);
+          umma_commit(&x_empty[sx]);
         }
         __syncwarp();
       }
       if (ok && lane == 0) umma_commit(acc_full);
       __syncwarp();
     }
-  } else if (warp < 2 + kTsDeqWarps) {
-    // ---- int4 -> bf16 expansion into TMEM: this thread does the 64 k (32 columns) of its weight row, or one
-    // half of them when two warps share the 32 lanes
+  } else if (warp == 2) {
+    // ---- weight producer, behind the first fills
+    bool ok = true;
+    if (lane == 0) {
+#pragma unroll 1
+      while (q_li < my_tiles && ok) {
+        ok = mbar_wait(&q_empty[q_it % QS], (q_it / QS - 1) & 1, g.err);
+        if (ok) q_issue();
+      }
+    }
+  } else if (warp >= 4 && warp < 4 + D) {
+    // ---- int4 -> bf16 expansion into TMEM: this thread does the 64 k (32 columns) of its weight row in one k block of
+    // the stage, or in both when there is one warp per 32 lanes
     const int quarter = warp & 3;                  // TMEM lanes 32*quarter .. +31 belong to this warp
-    constexpr int kHalves = 8 / kTsDeqWarps;       // halves of a row per thread: 2 with four warps, 1 with eight
-    const int half0 = kTsDeqWarps == 8 ? (warp - 2) >> 2 : 0;
-    const int row = quarter * 32 + lane;
+    const int kb0 = D == 8 ? (warp - 4) >> 2 : 0;
+    constexpr int kPer = D == 8 ? 1 : kTsKb;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    const int iters = my_tiles * nkb;
+    const int iters = my_tiles * nst;
     const __nv_bfloat162 bias = __float2bfloat162_rn(136.0f);
     bool ok = true;
+    int st = 0;
+#pragma unroll 1
     for (int it = 0; it < iters && ok; ++it) {
-      const int s = it % S, n = it / S;
-      ok = mbar_wait(&full_bar[s], n & 1, g.err);
-      if (ok && n > 0) ok = mbar_wait(&empty_bar[s], (n - 1) & 1, g.err);
+      const int sq = it % QS, sw = it % WS, nk = min(kTsKb, nkb - st * kTsKb);
+      if (++st == nst) st = 0;
+      ok = mbar_wait(&q_full[sq], (it / QS) & 1, g.err);
+      if (ok && it >= WS) ok = mbar_wait(&w_empty[sw], (it / WS - 1) & 1, g.err);
       if (!ok) break;
       tc_fence_after();
 #pragma unroll
-      for (int hh = 0; hh < kHalves; ++hh) {
-        const int half = half0 + hh;
-        const uint4 q = *reinterpret_cast<const uint4*>(sQ + s * kGemmStageQ + row * 32 + half * 16);
-        const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
-        uint32_t r[16];
+      for (int u = 0; u < kPer; ++u) {
+        const int kb = kb0 + u;
+        if (kb < nk) {
+          const uint4* src = reinterpret_cast<const uint4*>(sQ + (sq * kTsKb + kb) * kGemmStageQ + (quarter * 32 + lane) * 32);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+          for (int half = 0; half < 2; ++half) {
+            const uint4 q = src[half];
+            const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+            uint32_t r[16];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint32_t v = ((qw[j] >> (4 * i)) & 0x000F000Fu) | 0x43004300u;   // bf16(128 + nibble) pairs
-            __nv_bfloat162 h = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&v), bias);
-            r[j * 4 + i] = *reinterpret_cast<uint32_t*>(&h);
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                uint32_t v = ((qw[j] >> (4 * i)) & 0x000F000Fu) | 0x43004300u;   // bf16(128 + nibble) pairs
+                __nv_bfloat162 h = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&v), bias);
+                r[j * 4 + i] = *reinterpret_cast<uint32_t*>(&h);
+              }
+            }
+            tmem_st16(tmem_w + lane_base + (sw * kTsKb + kb) * kTsAcols + half * 16, r);
           }
         }
-        tmem_st16(tmem_w + lane_base + s * kTsAcols + half * 16, r);
       }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&deq_bar[s]);
+      if (lane == 0) { mbar_arrive(&w_full[sw]); mbar_arrive(&q_empty[sq]); }
     }
-  } else {
-    // ---- epilogue: this warp takes 64 token columns of its 32 weight rows
+  } else if (warp >= 4 + D) {
+    // ---- epilogue: this warp takes EC token columns of its 32 weight rows
     const int quarter = warp & 3;
-    const int second = (warp - 2 - kTsDeqWarps) >> 2;      // 0..3
     const int row = quarter * 32 + lane;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    const int c0 = ((warp - 4 - D) >> 2) * EC;
     bool ok = true;
+    pdl_wait();                                     // the outputs may still be read by an earlier kernel
+#pragma unroll 1
     for (int li = 0; li < my_tiles && ok; ++li) {
       const TsTile tl = ts_tile(blockIdx.x + li * gridDim.x, n_tiles, t_tiles);
+      const float sc = g.wscale[tl.n_tile * kTsRows + row];
       ok = mbar_wait(acc_full, li & 1, g.err);
       if (!ok) break;
       tc_fence_after();
-      const int c0 = second * 64;
-      const int t0 = tl.t_tile * NTOK + c0;
-      uint32_t v0[32], v1[32];
-      if (c0 < NTOK) {
-        tmem_ld32(tmem_base + lane_base + c0, v0);
-        tmem_ld32(tmem_base + lane_base + c0 + 32, v1);
+      constexpr int EH = NTOK <= 64 && EC > 32 ? 32 : EC;   // columns in registers at a time
+#pragma unroll 1
+      for (int ch = 0; ch < EC; ch += EH) {
+      const int t0 = tl.t_tile * NTOK + c0 + ch;
+      uint32_t v[EH];
+      ts_load_acc<EH>(tmem_base + lane_base + c0 + ch, v);
+      if (ch + EH == EC) {                          // the accumulator is in registers: hand it back before the stores
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty);
       }
-      // the accumulator is in registers: hand it back before the stores
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty);
-      if (c0 >= NTOK) continue;                      // a narrow tile has no columns for this warp
-      const float sc = g.wscale[tl.n_tile * kTsRows + row];
       if constexpr (EPI == 0) {
         const int nrow = tl.n_tile * kTsRows + row;
         if (nrow < g.N) {
           float* dst = g.outF + ((size_t)tl.ks * g.T + t0) * g.N + nrow;
 #pragma unroll
-          for (int c = 0; c < 32; ++c)
-            if (t0 + c < g.T) dst[(size_t)c * g.N] = __uint_as_float(v0[c]) * sc;
-#pragma unroll
-          for (int c = 0; c < 32; ++c)
-            if (t0 + 32 + c < g.T) dst[(size_t)(32 + c) * g.N] = __uint_as_float(v1[c]) * sc;
+          for (int c = 0; c < EH; ++c)
+            if (t0 + c < g.T) dst[(size_t)c * g.N] = __uint_as_float(v[c]) * sc;
         }
       } else {
         const int F = g.N / 2;
@@ -273,19 +343,13 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
         __nv_bfloat16* dst = g.outB + (size_t)(t0 + (odd ? 1 : 0)) * F + f;
         const int tlim = g.T - t0 - (odd ? 1 : 0);          // columns c (even) with c < tlim are stored
 #pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-          float a = __uint_as_float(v0[c]) * sc, bb = __uint_as_float(v0[c + 1]) * sc;
+        for (int c = 0; c < EH; c += 2) {
+          float a = __uint_as_float(v[c]) * sc, bb = __uint_as_float(v[c + 1]) * sc;
           float got = __shfl_xor_sync(0xffffffffu, odd ? a : bb, 1);
           float gate = odd ? got : a, up = odd ? bb : got;
           if (c < tlim && f < F) dst[(size_t)c * F] = __float2bfloat16(gelu_tanh_fast(gate) * up);
         }
-#pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-          float a = __uint_as_float(v1[c]) * sc, bb = __uint_as_float(v1[c + 1]) * sc;
-          float got = __shfl_xor_sync(0xffffffffu, odd ? a : bb, 1);
-          float gate = odd ? got : a, up = odd ? bb : got;
-          if (32 + c < tlim && f < F) dst[(size_t)(32 + c) * F] = __float2bfloat16(gelu_tanh_fast(gate) * up);
-        }
+      }
       }
     }
   }
@@ -293,12 +357,13 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   __syncthreads();
   if (*reinterpret_cast<volatile int*>(g.err) == (int)kDevBarrierTimeout) {
     // a wait gave up: let any bulk copy still in flight land before the CTA retires
+#pragma unroll 1
     for (int i = 0; i < 2000; ++i) __nanosleep(100);
     __syncthreads();
   }
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTsTmemCols);
+    tmem_dealloc(tmem_base, ts_tmem(NTOK));
   }
 }
 

@@ -49,14 +49,13 @@ struct Model {
   static std::shared_ptr<Model> load(const uint8_t* image, size_t n, int device, bool want_tc);
 };
 
-// An activation matrix [rows][cols] bf16 as the GEMM's token operand: the same tensor with a 128-row and a
-// 64-row copy box (the kernel's token tile is 256 / 128 or 64 wide).
+// An activation matrix [rows][cols] bf16 as the GEMM's token operand: the same tensor with copy boxes of as many
+// rows as the kernel's token tile (256-token tiles take two 128-row boxes).
 struct ActMap {
-  CUtensorMap box128;
-  CUtensorMap box64;
+  CUtensorMap box[4];         // 16, 32, 64, 128 rows
 };
 // token width of the GEMM tile for T token rows
-inline int ts_tile_tokens(int T) { return T <= 64 ? 64 : T <= 128 ? 128 : 256; }
+inline int ts_tile_tokens(int T) { return T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256; }
 CUtensorMap make_activation_map_box(const __nv_bfloat16* base, int rows, int cols, int box_rows);
 ActMap make_activation_map(const __nv_bfloat16* base, int rows, int cols);
 int pick_ksplit(int T, int n_tiles, int KB, int sms);
