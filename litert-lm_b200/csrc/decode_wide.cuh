@@ -15,7 +15,7 @@ namespace b200lm {
 
 constexpr int kWideMax = 128;          // sessions of one wide step (half a token tile of the GEMM)
 constexpr int kWideArgThreads = 1024;
-constexpr int kWideMaxSplits = 8;     // key splits of one (session, kv head) in the wide attention
+constexpr int kWideMaxSplits = 16;    // key splits of one (session, kv head) in the wide attention
 
 // Per-session state of a wide run, device resident: [0, n) token of the next step, [kWideMax, +n)
 // its position, [2 kWideMax, +n) the position of the run's first step.
@@ -23,29 +23,40 @@ struct WideState {
   int* tok;
   int* pos;
   int* pos0;
+  float* part_val;            // arg-max of the parts of a row
+  int* part_idx;
+  int* ticket;                // parts of a row that are done; zero between launches
 };
 
-// One CTA per session: arg-max of its logits row (lowest index among equal maxima, the rule of
-// runtime/components/sampling_cpu_util.cc:32-41), recorded as the step's id and as the next input.
+// Arg-max of the sessions' logits rows (lowest index among equal maxima, the rule of
+// runtime/components/sampling_cpu_util.cc:32-41), recorded as the step's id and as the next input.  `parts` CTAs share
+// a row, so that a few rows (9 rows of 1 MB took one CTA each 17.4 us) draw on the whole chip; the last one to finish
+// joins them, and equal maxima go by index whatever the order.
+constexpr int kWideArgParts = 16;
 static __global__ void __launch_bounds__(kWideArgThreads)
-wide_argmax_kernel(const float* __restrict__ logits, int vocab, int n, WideState st, int* __restrict__ step_tokens) {
+wide_argmax_kernel(const float* __restrict__ logits, int vocab, int n, int parts, WideState st, int* __restrict__ step_tokens) {
   __shared__ float sv[kWideArgThreads / 32];
   __shared__ int si[kWideArgThreads / 32];
-  const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int row = blockIdx.x / parts, part = blockIdx.x % parts, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float4* src = reinterpret_cast<const float4*>(logits + (size_t)row * vocab);
   float bv = -INFINITY;
   int bi = 0x7fffffff;
-  for (int i = threadIdx.x; i < vocab / 4; i += kWideArgThreads) {     // ascending per thread: > keeps the first
+  const int v4 = vocab / 4, per = (v4 + parts - 1) / parts, beg = min(v4, part * per), end = min(v4, beg + per);
+#pragma unroll 4
+  for (int i = beg + threadIdx.x; i < end; i += kWideArgThreads) {     // ascending per thread: > keeps the first
     const float4 v = __ldcs(src + i);
     if (v.x > bv) { bv = v.x; bi = 4 * i; }
     if (v.y > bv) { bv = v.y; bi = 4 * i + 1; }
     if (v.z > bv) { bv = v.z; bi = 4 * i + 2; }
     if (v.w > bv) { bv = v.w; bi = 4 * i + 3; }
   }
-  for (int i = (vocab / 4) * 4 + threadIdx.x; i < vocab; i += kWideArgThreads) {
-    const float v = logits[(size_t)row * vocab + i];
-    if (v > bv) { bv = v; bi = i; }
-  }
+  if (part == parts - 1)
+    for (int i = v4 * 4 + threadIdx.x; i < vocab; i += kWideArgThreads) {
+      const float v = logits[(size_t)row * vocab + i];
+      if (v > bv) { bv = v; bi = i; }
+    }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
@@ -63,6 +74,28 @@ wide_argmax_kernel(const float* __restrict__ logits, int vocab, int n, WideState
       const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
+    if (parts > 1) {
+      float* pv = st.part_val + (size_t)row * kWideArgParts;
+      int* pi = st.part_idx + (size_t)row * kWideArgParts;
+      int last = 0;
+      if (lane == 0) {
+        pv[part] = bv;
+        pi[part] = bi;
+        __threadfence();
+        last = atomicAdd(st.ticket + row, 1) == parts - 1;
+        if (last) st.ticket[row] = 0;
+        __threadfence();
+      }
+      if (!__shfl_sync(0xffffffffu, last, 0)) return;
+      bv = lane < parts ? __ldcg(pv + lane) : -INFINITY;
+      bi = lane < parts ? __ldcg(pi + lane) : 0x7fffffff;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+      }
+    }
     if (lane == 0) {
       if (bi == 0x7fffffff) bi = 0;                 // a row of NaNs: id 0, as the host path casts
       const int p = st.pos[row];
@@ -74,13 +107,18 @@ wide_argmax_kernel(const float* __restrict__ logits, int vocab, int n, WideState
 }
 
 // ------------------------------------------------------------------ attention of a wide step
-// One CTA per (session, kv head, key split).  The session's K / V rows of this head are contiguous inside
-// a page ([page][kv head][slot][hd]), so the CTA streams them in blocks of kWaChunk consecutive positions
-// with one bulk async copy each for K and V into a ring of shared-memory stages, several blocks in flight;
-// the eight warps take two keys of a block each (online softmax per warp, all G query heads of the group
-// together) and the per-warp states are merged at the end.  Split 0 also norms, rotates and appends this
-// step's own K / V row; the current position's row is taken from shared memory, not from the cache.
-constexpr int kWaThreads = 256, kWaWarps = 8, kWaChunk = 2 * kWaWarps, kWaMaxStages = 6;
+// One CTA per (session, kv head, key split).  The session's K / V rows of this head are contiguous inside a page
+// ([page][kv head][slot][hd]), so a round's 16 or 32 keys are one or two bulk copies each for K and V, into a ring of
+// rounds that is requested ahead of griddepcontrol.wait.  Scores: a warp takes 2 or 4 keys of the round for all G query
+// heads, and the sums fold together, each exchange halving what a lane carries.  Softmax: a warp per head, a lane per
+// key.  P V: a thread per pair of elements.  So a round has one chain of exchanges and exponentials, where a warp that
+// owned its keys had one per key (9 sessions x 530 keys of 256 fp32: 17.5 us a layer and 6.1 for a kernel of its own
+// that joined the splits).  The last CTA of a (session, kv head) to finish joins the splits, in split order.  The CTA
+// whose keys end at the current position norms, rotates and appends the step's own K / V row.
+constexpr int kWaThreads = 256, kWaWarps = 8, kWaMaxStages = 6;
+// Keys of a round: 32 KB a stage for the largest rows, so that two CTAs of an SM hold three stages each.
+template <typename T, int HD>
+__host__ __device__ constexpr int wa_keys() { return HD * (int)sizeof(T) >= 1024 ? 16 : 32; }
 
 struct WideAttnArgs {
   const float* qkv;          // [sessions][nqkv] raw projections of this step
@@ -92,114 +130,133 @@ struct WideAttnArgs {
   int stages;                // ring depth (2 .. kWaMaxStages), sized by the host to the shared memory
   const float *g_q, *g_k, *cosT, *sinT;
   LayerKv kv;
-  float* part;               // nsplit > 1: [session][kv head][split][G][hd + 2] (o, then m and l)
-  __nv_bfloat16* out;        // nsplit == 1: [session][hq * hd]
+  float* part;               // nsplit > 1: [session][kv head] partial states, nsplit * G * (hd + 4) floats each (16-byte rows)
+  int* ticket;               // nsplit > 1: [session][kv head], zero before and after
+  __nv_bfloat16* out;        // [session][hq * hd], optional
   int* err;
   int seq_stride;            // 1: session i has row i of the page table; 0: every query reads sequence 0
   int appended;              // 1: q rows are final (no norm, no rotation) and every K / V row is already in the cache
-  float* out_f32;            // nsplit == 1: the same output in fp32 (operator-level callers), optional
+  float* out_f32;            // the same output in fp32 (operator-level callers), optional
   int ctas_per_sm;           // host-side hint: size the ring so that this many CTAs fit one SM (0 = 1)
   int qkv_parts;             // > 1: qkv is that many split-K partials, qkv_part_stride floats apart, summed on load
   size_t qkv_part_stride;
 };
 
 template <typename T, int HD>
-__host__ __device__ constexpr int wa_stage_bytes() { return 2 * kWaChunk * HD * (int)sizeof(T); }
+__host__ __device__ constexpr int wa_stage_bytes() { return 2 * wa_keys<T, HD>() * HD * (int)sizeof(T); }
 __host__ __device__ inline size_t wa_fixed_bytes(int hd, int G) {
-  return sizeof(float) * ((size_t)(G + 2) * hd + (size_t)kWaWarps * G * (hd + 2)) + 16 * kWaMaxStages + 128;
+  return sizeof(float) * ((size_t)(G + 2) * hd + 32 * G + 4 * G + 2 * kWaThreads * G) + 8 * kWaMaxStages + 128;
 }
 
 template <typename T, int HD, int G>
 __global__ void __launch_bounds__(kWaThreads, 2)
 wide_attn_kernel(ModelDims dm, WideAttnArgs a) {
-  constexpr int VEC = HD / 32, half = HD / 2;
+  constexpr int VEC = HD / 32, half = HD / 2, KEYS = wa_keys<T, HD>(), PARTS = kWaThreads / half;   // PARTS: key shares of P V
   constexpr int kStage = wa_stage_bytes<T, HD>();
   extern __shared__ __align__(128) unsigned char wa_sm[];
   const int S = a.stages;
-  unsigned char* ring = wa_sm;
-  float* q_s = reinterpret_cast<float*>(wa_sm + (size_t)S * kStage);   // [G][HD]
-  float* k_s = q_s + G * HD;                                           // [HD]
-  float* v_s = k_s + HD;                                               // [HD]
-  float* wm = v_s + HD;                                                // [warps][G]
-  float* wl = wm + kWaWarps * G;
-  float* wo = wl + kWaWarps * G;                                       // [warps][G][HD]
-  uint64_t* full = reinterpret_cast<uint64_t*>(wo + kWaWarps * G * HD);
-  uint64_t* empty = full + kWaMaxStages;
+  float* q_s = reinterpret_cast<float*>(wa_sm + (size_t)S * kStage);   // [G][HD], scaled by 1/sqrt(HD)
+  float* k_s = q_s + G * HD;
+  float* v_s = k_s + HD;
+  float* sc = v_s + HD;                        // [KEYS][G] scores, then probabilities
+  float* cr = sc + 32 * G;                     // [G] factor of the sums of earlier rounds, [G] running max, [G] running sum
+  float* ored = cr + 4 * G;                    // [PARTS][G][HD]
+  uint64_t* full = reinterpret_cast<uint64_t*>(ored + 2 * kWaThreads * G);
+  int* last = reinterpret_cast<int*>(full + kWaMaxStages);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int split = blockIdx.x % a.nsplit;
-  const int kvh = (blockIdx.x / a.nsplit) % dm.hkv;
-  const int qi = blockIdx.x / (a.nsplit * dm.hkv);
-  int pos = a.pos[qi];
+  const int split = blockIdx.x % a.nsplit, pair = blockIdx.x / a.nsplit, kvh = pair % dm.hkv, qi = pair / dm.hkv;
+  int pos = __ldcg(a.pos + qi);                // written two kernels back or earlier, as the cached rows are
   if (pos < 0 || pos >= dm.max_ctx) {
     if (threadIdx.x == 0) atomicExch(a.err, (int)kDevBadPosition);
     pos = 0;
   }
   const int* ptab = a.page_table + (size_t)(a.seq_stride ? qi : 0) * a.pages_per_seq;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], kWaWarps); }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
   const T* kbase = reinterpret_cast<const T*>(a.kv.k);
   const T* vbase = reinterpret_cast<const T*>(a.kv.v);
-  // ---- key range of this split; the current position is served from shared memory.  The first blocks are
-  // requested before the prologue below (they depend on the position only), so their latency hides behind it.
   int k0, k1;
   attn_split_range(dm, pos, a.is_global, a.nsplit, split, &k0, &k1);
-  const bool has_cur = !a.appended && k1 == pos + 1 && k1 > k0;
-  const int k1s = has_cur ? pos : k1;                  // streamed keys: [k0, k1s)
-  const int cb0 = k0 / kWaChunk;
-  const int nchunks = k1s > k0 ? (k1s + kWaChunk - 1) / kWaChunk - cb0 : 0;
-  auto issue = [&](int c) {                            // thread 0: block c of this split into its stage
-    const int s = c % S, key = (cb0 + c) * kWaChunk;
-    const size_t off = (((size_t)ptab[key / kPage] * dm.hkv + kvh) * kPage + (key % kPage)) * HD;
-    unsigned char* dst = ring + (size_t)s * kStage;
-    mbar_arrive_expect_tx(&full[s], (uint32_t)kStage);
-    bulk_load_1d(dst, kbase + off, kStage / 2, &full[s]);
-    bulk_load_1d(dst + kStage / 2, vbase + off, kStage / 2, &full[s]);
+  const bool has_new = !a.appended && k1 == pos + 1 && k1 > k0;
+  const int k1c = has_new ? pos : k1;          // cached keys [k0, k1c)
+  const int nrounds = k1 > k0 ? (k1 - k0 + KEYS - 1) / KEYS : 0;
+  auto issue = [&](int r) {                    // thread 0
+    const int b = r % S, ka = k0 + r * KEYS, n = min(KEYS, k1c - ka);
+    if (n <= 0) { mbar_arrive(&full[b]); return; }
+    unsigned char* dst = wa_sm + (size_t)b * kStage;
+    constexpr uint32_t rowb = HD * sizeof(T);
+    mbar_arrive_expect_tx(&full[b], 2u * (uint32_t)n * rowb);
+#pragma unroll 1
+    for (int done = 0; done < n;) {            // rows of one page are contiguous
+      const int key = ka + done, len = min(n - done, kPage - key % kPage);
+      const size_t off = (((size_t)__ldg(ptab + key / kPage) * dm.hkv + kvh) * kPage + key % kPage) * HD;
+      bulk_load_1d(dst + (size_t)done * rowb, kbase + off, (uint32_t)len * rowb, &full[b]);
+      bulk_load_1d(dst + (size_t)(KEYS + done) * rowb, vbase + off, (uint32_t)len * rowb, &full[b]);
+      done += len;
+    }
   };
-  if (threadIdx.x == 0)
-    for (int c = 0; c < nchunks && c < S - 1; ++c) issue(c);
-  // ---- this step's q heads (normed, rotated, scaled), k head and v head
-  const float* row = a.qkv + (size_t)qi * dm.nqkv();
-  const float att_scale = rsqrtf((float)HD);
-  const int nparts = a.qkv_parts > 1 ? a.qkv_parts : 1;
-  const size_t pstride = a.qkv_part_stride;
-  auto ld = [&](const float* p) {                      // one projection value: the sum of its split-K partials, in order
-    float v = p[0];
-    for (int q = 1; q < nparts; ++q) v += p[(size_t)q * pstride];
-    return v;
-  };
-  for (int h = warp; h < (a.appended ? G : G + 2); h += kWaWarps) {
-    if (a.appended) {                                  // final q rows: only the attention scale
-      const float* src = row + (size_t)(kvh * G + h) * HD;
-      for (int e = lane; e < HD; e += 32) q_s[h * HD + e] = ld(src + e) * att_scale;
-    } else if (h <= G) {
-      const float* src = h < G ? row + (size_t)(kvh * G + h) * HD : row + dm.nq() + (size_t)kvh * HD;
-      const float* gain = h < G ? a.g_q : a.g_k;
-      float* dst = h < G ? q_s + h * HD : k_s;
-      float ss = 0.f;
-      for (int e = lane; e < HD; e += 32) { const float v = ld(src + e); ss += v * v; }
-      ss = warp_sum(ss);
-      const float r = rsqrtf(ss / (float)HD + dm.eps);
-      const float post = h < G ? att_scale : 1.0f;
-      for (int e = lane; e < half; e += 32) {
-        const float a0 = ld(src + e) * r * gain[e], b0 = ld(src + e + half) * r * gain[e + half];
-        const float cs = a.cosT[(size_t)pos * half + e], sn = a.sinT[(size_t)pos * half + e];
-        dst[e] = (a0 * cs - b0 * sn) * post;
-        dst[e + half] = (b0 * cs + a0 * sn) * post;
-      }
-    } else {
-      const float* src = row + dm.nq() + dm.nkv() + (size_t)kvh * HD;
-      for (int e = lane; e < HD; e += 32) v_s[e] = ld(src + e);
+  if (threadIdx.x == 0) {
+#pragma unroll 1
+    for (int s = 0; s < S; ++s) mbar_init(&full[s], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+#pragma unroll 1
+    for (int r = 0; r < min(S, nrounds); ++r) issue(r);
+  }
+  // ---- q heads, k head and v head: a warp per head (or two), gains and RoPE rows requested before the wait
+  float ga[VEC], cs[(VEC + 1) / 2], sn[(VEC + 1) / 2];
+  if (warp <= G && !a.appended) {
+    const float* gain = warp < G ? a.g_q : a.g_k;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) ga[i] = __ldg(gain + lane + 32 * i);
+#pragma unroll
+    for (int i = 0; i < (VEC + 1) / 2; ++i) {  // HD 32: the pair of element e sits 16 lanes away
+      const int e = HD == 32 ? lane & 15 : lane + 32 * i;
+      cs[i] = __ldg(a.cosT + (size_t)pos * half + e);
+      sn[i] = __ldg(a.sinT + (size_t)pos * half + e);
     }
   }
+  pdl_wait();
+  pdl_launch_dependents();
+  if (warp < G || (warp < G + 2 && has_new)) {
+    const float* src = a.qkv + (size_t)qi * dm.nqkv() + (warp < G ? (kvh * G + warp) * HD : dm.nq() + (warp == G ? 0 : dm.nkv()) + kvh * HD);
+    float v[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) v[i] = __ldcg(src + lane + 32 * i);
+#pragma unroll 3
+    for (int p = 1; p < a.qkv_parts; ++p)      // a projection is the sum of its split-K partials, in order
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) v[i] += __ldcg(src + p * a.qkv_part_stride + lane + 32 * i);
+    float* dst = q_s + warp * HD;              // k_s and v_s follow the q heads
+    const float post = warp < G ? rsqrtf((float)HD) : 1.0f;
+    if (a.appended || warp > G) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) dst[lane + 32 * i] = v[i] * post;
+    } else {
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) ss += v[i] * v[i];
+      ss = warp_sum(ss);
+      const float r = rsqrtf(ss / (float)HD + dm.eps);
+      if constexpr (HD == 32) {
+        const float x = v[0] * r * ga[0], y = __shfl_xor_sync(0xffffffffu, x, 16);
+        dst[lane] = (lane < 16 ? x * cs[0] - y * sn[0] : x * cs[0] + y * sn[0]) * post;
+      } else {
+#pragma unroll
+        for (int i = 0; i < VEC / 2; ++i) {
+          const float a0 = v[i] * r * ga[i], b0 = v[i + VEC / 2] * r * ga[i + VEC / 2];
+          dst[lane + 32 * i] = (a0 * cs[i] - b0 * sn[i]) * post;
+          dst[lane + 32 * i + half] = (b0 * cs[i] + a0 * sn[i]) * post;
+        }
+      }
+    }
+  }
+  if (threadIdx.x < G) { cr[G + threadIdx.x] = -INFINITY; cr[2 * G + threadIdx.x] = 0.f; }
   __syncthreads();
-  if (split == 0 && !a.appended) {          // append: exactly one CTA per (session, kv head)
+  if (has_new) {                               // append: exactly one CTA per (session, kv head)
     const int page = ptab[pos / kPage], slot = pos % kPage;
     const size_t off = (((size_t)page * dm.hkv + kvh) * kPage + slot) * HD;
     T* kw = reinterpret_cast<T*>(a.kv.k);
     T* vw = reinterpret_cast<T*>(a.kv.v);
+#pragma unroll 1
     for (int e = threadIdx.x; e < HD; e += kWaThreads) {
       if constexpr (sizeof(T) == 4) {
         kw[off + e] = k_s[e];
@@ -213,162 +270,167 @@ wide_attn_kernel(ModelDims dm, WideAttnArgs a) {
     }
     asm volatile("fence.proxy.async.global;" ::: "memory");     // later steps fetch these rows with bulk copies
   }
-  float q[G][VEC], o[G][VEC], m[G], l[G];
+  float q[G][VEC];
 #pragma unroll
-  for (int g = 0; g < G; ++g) {
-    m[g] = -INFINITY;
-    l[g] = 0.f;
+  for (int h = 0; h < G; ++h)
 #pragma unroll
-    for (int c = 0; c < VEC; ++c) {
-      q[g][c] = q_s[g * HD + head_elem<HD>(lane, c)];
-      o[g][c] = 0.f;
-    }
-  }
+    for (int c = 0; c < VEC; ++c) q[h][c] = q_s[h * HD + head_elem<HD>(lane, c)];
+  const int e2 = 2 * (threadIdx.x % half), share = threadIdx.x / half;
+  float o[G][2];
+#pragma unroll
+  for (int h = 0; h < G; ++h) o[h][0] = o[h][1] = 0.f;
   bool ok = true;
-  for (int c = 0; c < nchunks && ok; ++c) {
-    const int s = c % S;
-    if (threadIdx.x == 0 && c + S - 1 < nchunks) {     // refill the stage that block c - 1 used
-      const int cn = c + S - 1;
-      if (cn >= S) ok = mbar_wait(&empty[cn % S], (uint32_t)((cn / S - 1) & 1), a.err);
-      if (ok) issue(cn);
+#pragma unroll 1
+  for (int r = 0; r < nrounds; ++r) {
+    const int b = r % S, n = min(KEYS, k1 - k0 - r * KEYS);
+    T* ks = reinterpret_cast<T*>(wa_sm + (size_t)b * kStage);
+    T* vs = ks + KEYS * HD;
+    ok = mbar_wait(&full[b], (uint32_t)((r / S) & 1), a.err) && ok;
+    if (has_new && r == nrounds - 1) {         // the step's own rows, as the cache will hand them back
+#pragma unroll 1
+      for (int e = threadIdx.x; e < HD; e += kWaThreads) {
+        if constexpr (sizeof(T) == 4) { ks[(n - 1) * HD + e] = k_s[e]; vs[(n - 1) * HD + e] = v_s[e]; }
+        else { ks[(n - 1) * HD + e] = __float2bfloat16(k_s[e]); vs[(n - 1) * HD + e] = __float2bfloat16(v_s[e]); }
+      }
+      __syncthreads();
     }
-    ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;    // warp 0 follows its producer lane; the others see the error word
-    if (!ok) break;
-    ok = mbar_wait(&full[s], (uint32_t)((c / S) & 1), a.err);
-    if (!ok) break;
-    const T* ks = reinterpret_cast<const T*>(ring + (size_t)s * kStage);
-    const T* vs = ks + kWaChunk * HD;
-    const int ka = (cb0 + c) * kWaChunk + warp, kb = ka + kWaWarps;
-    const bool hasa = ka >= k0 && ka < k1s, hasb = kb >= k0 && kb < k1s;
-    float kA[VEC], kB[VEC], vA[VEC], vB[VEC];
-    load_head_row_smem<T, HD>(ks + (size_t)warp * HD, lane, kA);
-    load_head_row_smem<T, HD>(ks + (size_t)(warp + kWaWarps) * HD, lane, kB);
-    load_head_row_smem<T, HD>(vs + (size_t)warp * HD, lane, vA);
-    load_head_row_smem<T, HD>(vs + (size_t)(warp + kWaWarps) * HD, lane, vB);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[s]);             // rows are in registers
-    if (hasa || hasb) {
+    constexpr int NK = KEYS / kWaWarps, NSUM = NK * G;
+    if (NK * warp < n) {
+      float s[NSUM];
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
-        float sa = 0.f, sb = 0.f;
+      for (int j = 0; j < NK; ++j) {
+        float x[VEC];
+        load_head_row_smem<T, HD>(ks + (size_t)min(NK * warp + j, n - 1) * HD, lane, x);
 #pragma unroll
-        for (int cc = 0; cc < VEC; ++cc) { sa += q[g][cc] * kA[cc]; sb += q[g][cc] * kB[cc]; }
-        sa = hasa ? warp_sum(sa) : -INFINITY;
-        sb = hasb ? warp_sum(sb) : -INFINITY;
-        const float mn = fmaxf(m[g], fmaxf(sa, sb));
-        const float corr = __expf(m[g] - mn);
-        const float pa = hasa ? __expf(sa - mn) : 0.f, pb = hasb ? __expf(sb - mn) : 0.f;
-        l[g] = l[g] * corr + pa + pb;
-        m[g] = mn;
+        for (int h = 0; h < G; ++h) {
+          float d = 0.f;
 #pragma unroll
-        for (int cc = 0; cc < VEC; ++cc) o[g][cc] = o[g][cc] * corr + (hasa ? pa * vA[cc] : 0.f) + (hasb ? pb * vB[cc] : 0.f);
+          for (int c = 0; c < VEC; ++c) d += q[h][c] * x[c];
+          s[j * G + h] = d;
+        }
+      }
+#pragma unroll
+      for (int w = NSUM / 2, bit = 16; w >= 1; w /= 2, bit /= 2) {
+        const bool up = lane & bit;
+#pragma unroll
+        for (int i = 0; i < w; ++i) {
+          const float give = up ? s[i] : s[i + w], keep = up ? s[i + w] : s[i];
+          s[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+        }
+      }
+#pragma unroll
+      for (int bit = 16 / NSUM; bit >= 1; bit /= 2) s[0] += __shfl_xor_sync(0xffffffffu, s[0], bit);
+      if (lane % (32 / NSUM) == 0) {
+        const int i = lane / (32 / NSUM), key = NK * warp + i / G;     // value i: key i / G, head i % G
+        if (key < n) sc[key * G + i % G] = s[0];
       }
     }
-  }
-  if (has_cur && warp == 0) {                          // this step's own key
-    float kA[VEC], vA[VEC];
+    __syncthreads();
+    if (warp < G) {                            // softmax: warp = head, lane = key
+      const float s = lane < n ? sc[lane * G + warp] : -INFINITY;
+      const float m0 = cr[G + warp], m1 = fmaxf(m0, warp_max(s)), f = __expf(m0 - m1);
+      const float p = __expf(s - m1), ps = warp_sum(p);
+      if (lane < n) sc[lane * G + warp] = p;
+      __syncwarp();
+      if (lane == 0) { cr[warp] = f; cr[G + warp] = m1; cr[2 * G + warp] = cr[2 * G + warp] * f + ps; }
+    }
+    __syncthreads();
 #pragma unroll
-    for (int cc = 0; cc < VEC; ++cc) {
-      kA[cc] = k_s[head_elem<HD>(lane, cc)];
-      vA[cc] = v_s[head_elem<HD>(lane, cc)];
-      if constexpr (sizeof(T) == 2) {                  // what a bf16 cache hands back
-        kA[cc] = __bfloat162float(__float2bfloat16(kA[cc]));
-        vA[cc] = __bfloat162float(__float2bfloat16(vA[cc]));
+    for (int h = 0; h < G; ++h) { o[h][0] *= cr[h]; o[h][1] *= cr[h]; }
+#pragma unroll 4
+    for (int kk = share; kk < n; kk += PARTS) {
+      float x0, x1;
+      if constexpr (sizeof(T) == 4) {
+        const float2 x = *reinterpret_cast<const float2*>(vs + (size_t)kk * HD + e2);
+        x0 = x.x; x1 = x.y;
+      } else {
+        const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(vs + (size_t)kk * HD + e2);
+        x0 = __low2float(x); x1 = __high2float(x);
+      }
+      float p[G];
+      ld_vec<G>(sc + kk * G, p);
+#pragma unroll
+      for (int h = 0; h < G; ++h) {
+        o[h][0] += p[h] * x0;
+        o[h][1] += p[h] * x1;
       }
     }
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      float sa = 0.f;
-#pragma unroll
-      for (int cc = 0; cc < VEC; ++cc) sa += q[g][cc] * kA[cc];
-      sa = warp_sum(sa);
-      const float mn = fmaxf(m[g], sa);
-      const float corr = __expf(m[g] - mn), pa = __expf(sa - mn);
-      l[g] = l[g] * corr + pa;
-      m[g] = mn;
-#pragma unroll
-      for (int cc = 0; cc < VEC; ++cc) o[g][cc] = o[g][cc] * corr + pa * vA[cc];
+    if (r + 1 < nrounds) {
+      __syncthreads();                         // everyone is done with the stage, the probabilities and cr
+      if (threadIdx.x == 0 && r + S < nrounds) issue(r + S);
     }
   }
-  // ---- merge the warps
+  // ---- the key shares meet
 #pragma unroll
-  for (int g = 0; g < G; ++g) {
-    if (lane == 0) { wm[warp * G + g] = m[g]; wl[warp * G + g] = l[g]; }
-#pragma unroll
-    for (int cc = 0; cc < VEC; ++cc) wo[((size_t)warp * G + g) * HD + head_elem<HD>(lane, cc)] = o[g][cc];
-  }
+  for (int h = 0; h < G; ++h) *reinterpret_cast<float2*>(ored + ((size_t)share * G + h) * HD + e2) = make_float2(o[h][0], o[h][1]);
   __syncthreads();
-  for (int i = threadIdx.x; i < G * HD; i += kWaThreads) {
-    const int g = i / HD, e = i - g * HD;
-    float M = -INFINITY;
-    for (int w = 0; w < kWaWarps; ++w) M = fmaxf(M, wm[w * G + g]);
-    float L = 0.f, O = 0.f;
-    if (M > -INFINITY) {
-      for (int w = 0; w < kWaWarps; ++w) {
-        const float f = __expf(wm[w * G + g] - M);
-        L += wl[w * G + g] * f;
-        O += wo[((size_t)w * G + g) * HD + e] * f;
-      }
+  // part: [split][G][HD] sums, then [split][G] maxima and [split][G] sums of the probabilities
+  constexpr int UNITS = G * HD / 4;
+  float* part = a.part + (size_t)pair * a.nsplit * G * (HD + 4);
+  float* part_m = part + (size_t)a.nsplit * G * HD;
+  float* part_l = part_m + a.nsplit * G;
+  auto put = [&](int i, float4 v, float f) {
+    v.x *= f; v.y *= f; v.z *= f; v.w *= f;
+    const size_t oi = ((size_t)qi * dm.hq + kvh * G) * HD + 4 * i;
+    if (a.out) {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+      *reinterpret_cast<uint2*>(a.out + oi) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+    if (a.out_f32) *reinterpret_cast<float4*>(a.out_f32 + oi) = v;
+  };
+  for (int i = threadIdx.x; i < UNITS; i += kWaThreads) {
+    float4 v = reinterpret_cast<const float4*>(ored)[i];
+#pragma unroll
+    for (int p = 1; p < PARTS; ++p) {
+      const float4 x = reinterpret_cast<const float4*>(ored)[p * UNITS + i];
+      v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
     }
     if (a.nsplit > 1) {
-      float* dst = a.part + ((((size_t)qi * dm.hkv + kvh) * a.nsplit + split) * G + g) * (HD + 2);
-      dst[e] = O;
-      if (e == 0) { dst[HD] = M; dst[HD + 1] = L; }
+      reinterpret_cast<float4*>(part)[split * UNITS + i] = v;
     } else {
-      const float val = L > 0.f ? O / L : 0.f;
-      const size_t oi = ((size_t)qi * dm.hq + kvh * G + g) * HD + e;
-      if (a.out) a.out[oi] = __float2bfloat16(val);
-      if (a.out_f32) a.out_f32[oi] = val;
+      const float L = cr[2 * G + i / (HD / 4)];
+      put(i, v, L > 0.f ? 1.0f / L : 0.f);
     }
   }
-  if (*reinterpret_cast<volatile int*>(a.err) == (int)kDevBarrierTimeout) {
-    // a wait gave up: let the bulk copies still in flight land before the CTA retires
-    for (int i = 0; i < 2000; ++i) __nanosleep(100);
+  if (a.nsplit > 1) {
+    if (threadIdx.x < G) { part_m[split * G + threadIdx.x] = cr[G + threadIdx.x]; part_l[split * G + threadIdx.x] = cr[2 * G + threadIdx.x]; }
+    __threadfence();
     __syncthreads();
-  }
-}
-
-// Sum of the key splits' partial states: one CTA per (session, query head).  The splits' (m, l) pairs are fetched
-// by one thread each and their weights exp(m_s - M) / L shared, so the element loop is independent loads only.
-static __global__ void __launch_bounds__(128)
-wide_attn_combine_kernel(const float* __restrict__ part, int nsplit, int hq, int hkv, int hd, __nv_bfloat16* __restrict__ out,
-                         float* __restrict__ out_f32) {
-  __shared__ float w_s[kMaxSplits];
-  const int G = hq / hkv;
-  const int qi = blockIdx.x / hq, h = blockIdx.x % hq, kvh = h / G, g = h % G;
-  const float* base = part + (((size_t)qi * hkv + kvh) * nsplit * G + g) * (hd + 2);
-  const size_t stride = (size_t)G * (hd + 2);
-  if (threadIdx.x < 32) {
-    float M = -INFINITY, L = 0.f;
-    float ms[(kMaxSplits + 31) / 32], ls[(kMaxSplits + 31) / 32];
-#pragma unroll
-    for (int r = 0; r < (kMaxSplits + 31) / 32; ++r) {
-      const int sp = threadIdx.x + 32 * r;
-      ms[r] = sp < nsplit ? base[sp * stride + hd] : -INFINITY;
-      ls[r] = sp < nsplit ? base[sp * stride + hd + 1] : 0.f;
-      M = fmaxf(M, ms[r]);
+    if (threadIdx.x == 0) {
+      *last = atomicAdd(a.ticket + pair, 1) == a.nsplit - 1;
+      if (*last) a.ticket[pair] = 0;
     }
-    M = warp_max(M);
-#pragma unroll
-    for (int r = 0; r < (kMaxSplits + 31) / 32; ++r) {
-      ms[r] = M > -INFINITY ? __expf(ms[r] - M) : 0.f;
-      L += ls[r] * ms[r];
-    }
-    L = warp_sum(L);
-    const float inv = L > 0.f ? 1.0f / L : 0.f;
-#pragma unroll
-    for (int r = 0; r < (kMaxSplits + 31) / 32; ++r) {
-      const int sp = threadIdx.x + 32 * r;
-      if (sp < nsplit) w_s[sp] = ms[r] * inv;
+    __syncthreads();
+    if (*last) {
+      __threadfence();
+      if (warp < G) {                          // weights of the splits, two to a lane: kMaxSplits in all
+        float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+        if (lane < a.nsplit) { m0 = __ldcg(part_m + lane * G + warp); l0 = __ldcg(part_l + lane * G + warp); }
+        if (lane + 32 < a.nsplit) { m1 = __ldcg(part_m + (lane + 32) * G + warp); l1 = __ldcg(part_l + (lane + 32) * G + warp); }
+        const float M = warp_max(fmaxf(m0, m1));
+        m0 = M > -INFINITY ? __expf(m0 - M) : 0.f;
+        m1 = M > -INFINITY ? __expf(m1 - M) : 0.f;
+        const float L = warp_sum(l0 * m0 + l1 * m1), inv = L > 0.f ? 1.0f / L : 0.f;
+        float* w = ored + warp * kMaxSplits;
+        w[lane] = m0 * inv;
+        w[lane + 32] = m1 * inv;
+      }
+      __syncthreads();
+      for (int i = threadIdx.x; i < UNITS; i += kWaThreads) {
+        const float* w = ored + i / (HD / 4) * kMaxSplits;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int s = 0; s < a.nsplit; ++s) {
+          const float4 x = __ldcg(reinterpret_cast<const float4*>(part) + s * UNITS + i);
+          v.x += x.x * w[s]; v.y += x.y * w[s]; v.z += x.z * w[s]; v.w += x.w * w[s];
+        }
+        put(i, v, 1.0f);
+      }
     }
   }
-  __syncthreads();
-  for (int e = threadIdx.x; e < hd; e += 128) {
-    float O = 0.f;
-    for (int s = 0; s < nsplit; ++s) O += base[s * stride + e] * w_s[s];
-    if (out) out[((size_t)qi * hq + h) * hd + e] = __float2bfloat16(O);
-    if (out_f32) out_f32[((size_t)qi * hq + h) * hd + e] = O;
-  }
+  if (!ok)                                     // a wait gave up: let the bulk copies still in flight land before the CTA retires
+#pragma unroll 1
+    for (int i = 0; i < 2000; ++i) __nanosleep(100);
 }
 
 // Host side: the kernel instantiated for the cache type, head size and group size.  nb <= 0 only sets the
@@ -377,9 +439,8 @@ template <typename T, int HD, int G>
 inline void launch_wide_attn_t(cudaStream_t st, const ModelDims& d, int nb, size_t smem_optin, WideAttnArgs a) {
   const size_t fixed = wa_fixed_bytes(HD, G);
   const int stage = wa_stage_bytes<T, HD>();
-  // The loop is a chain of dependent shuffles and exponentials on eight warps, so one CTA alone leaves the SM
-  // mostly idle (about 2 us per block of 16 keys, whatever its bytes): with two CTAs per SM the ring is shallower
-  // but twice as many chains run.
+  // A round is a chain of exchanges, exponentials and barriers: with two CTAs per SM the ring is shallower, but one
+  // CTA's chain runs beside the other's.
   int per_sm = std::max(1, a.ctas_per_sm);
   int stages = 0;
   for (; per_sm >= 1; --per_sm) {
@@ -392,7 +453,7 @@ inline void launch_wide_attn_t(cudaStream_t st, const ModelDims& d, int nb, size
   const size_t smem = fixed + (size_t)stages * stage;
   raise_dyn_smem(wide_attn_kernel<T, HD, G>, smem);
   if (nb <= 0) return;
-  wide_attn_kernel<T, HD, G><<<nb * d.hkv * a.nsplit, kWaThreads, smem, st>>>(d, a);
+  launch_pdl(wide_attn_kernel<T, HD, G>, dim3(nb * d.hkv * a.nsplit), dim3(kWaThreads), smem, st, d, a);
 }
 template <typename T, int HD>
 inline void launch_wide_attn_g(cudaStream_t st, const ModelDims& d, int nb, size_t smem_optin, const WideAttnArgs& a) {
@@ -419,19 +480,6 @@ void launch_wide_attn_bf16(cudaStream_t st, const ModelDims& d, int nb, size_t s
 inline void launch_wide_attn(cudaStream_t st, const ModelDims& d, int nb, size_t smem_optin, const WideAttnArgs& a) {
   if (d.kv_dtype == 0) launch_wide_attn_f32(st, d, nb, smem_optin, a);
   else launch_wide_attn_bf16(st, d, nb, smem_optin, a);
-}
-
-// out[t][:] = sum of the split-K partials parts[p][t][:], rows of `cols` floats.
-static __global__ void __launch_bounds__(256)
-wide_sum_parts_kernel(const float* __restrict__ parts, int nparts, size_t part_stride, size_t count, float* __restrict__ out) {
-  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
-  if (i * 4 >= count) return;
-  float4 a = reinterpret_cast<const float4*>(parts)[i];
-  for (int p = 1; p < nparts; ++p) {
-    const float4 b = reinterpret_cast<const float4*>(parts + (size_t)p * part_stride)[i];
-    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-  }
-  reinterpret_cast<float4*>(out)[i] = a;
 }
 
 }  // namespace b200lm

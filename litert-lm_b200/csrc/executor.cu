@@ -21,6 +21,7 @@
 #include "model_host.h"
 #include "prefill_ops.cuh"
 #include "prefill_gemm_ts.cuh"
+#include "gemm_small.cuh"
 #include "prefill_attn_tc.cuh"
 #include "runtime.h"
 
@@ -274,6 +275,7 @@ static CUtensorMap make_bf16_map(const void* base, int rank, const cuuint64_t* d
 // at most 8 splits) whose work units fill 90 % of the last round over the SMs,
 // else the divisor that fills it best.
 int pick_ksplit(int T, int n_tiles, int KB, int sms) {
+  if (const int s = gs_ksplit(T, n_tiles * 128, KB, sms)) return s;
   const int ntok = ts_tile_tokens(T);
   const int tiles = n_tiles * ((T + ntok - 1) / ntok);
   int best = 1;
@@ -313,6 +315,12 @@ void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bflo
       B2_CUDA(cudaDeviceGetAttribute(&sms_of[dev], cudaDevAttrMultiProcessorCount, dev));
     }
     const int sms = sms_of[dev];
+    if (gs_fits(T, N, K / 64, ksplit, geglu, sms)) {
+      launch_gemm_small(st, sms, dev, w4t, s4t, A, T, N, K, ksplit, geglu, outF, outB);
+      B2_CUDA(cudaGetLastError());
+      if (launches) ++*launches;
+      return;
+    }
     const int ntok = ts_tile_tokens(T);
     const int total = ((N + kTsRows - 1) / kTsRows) * ((T + ntok - 1) / ntok) * ksplit;
     const int grid = total < sms ? total : sms;
@@ -500,15 +508,17 @@ std::unique_ptr<Executor> Executor::create(std::shared_ptr<Model> model, const B
   a.step_capacity = d.max_ctx;
   a.step_tokens = reinterpret_cast<int*>(e->alloc(sizeof(int) * a.step_capacity * max_cols, true));
   if (e->decode_mode == B200LM_DECODE_WIDE) {
-    int* ws = reinterpret_cast<int*>(e->alloc(sizeof(int) * 3 * kWideMax, true));
-    e->wide = WideState{ws, ws + kWideMax, ws + 2 * kWideMax};
+    int* ws = reinterpret_cast<int*>(e->alloc(sizeof(int) * (4 + 2 * kWideArgParts) * kWideMax, true));
+    e->wide = WideState{ws, ws + kWideMax, ws + 2 * kWideMax, reinterpret_cast<float*>(ws + 4 * kWideMax), ws + (4 + kWideArgParts) * kWideMax,
+                        ws + 3 * kWideMax};
     {
       WideAttnArgs prep{};
       prep.ctas_per_sm = 2;
       launch_wide_attn(e->stream, d, 0, e->smem_optin, prep);
     }
     e->wide_part = reinterpret_cast<float*>(
-        e->alloc(sizeof(float) * (size_t)e->n_sessions * d.hkv * kWideMaxSplits * d.group() * (d.hd + 2), true));
+        e->alloc(sizeof(float) * (size_t)e->n_sessions * d.hkv * kWideMaxSplits * d.group() * (d.hd + 4), true));
+    e->wide_ticket = reinterpret_cast<int*>(e->alloc(sizeof(int) * (size_t)e->n_sessions * d.hkv, true));
   }
   a.advance = 1;
   if (e->decode_mode == B200LM_DECODE_PERSISTENT_BASIC) {
@@ -902,15 +912,10 @@ void Executor::wide_step(int nb, int first) {
   const ModelDims& d = model->dims;
   int* err = &dargs.st->err;
   const int mode = B200LM_GEMM_TCGEN05;
-  // key splits so that few sessions still fill the SMs: one CTA per (session, kv head, split)
-  const int nsplit = std::max(1, std::min(kWideMaxSplits, 2 * n_sms / std::max(1, nb * d.hkv)));   // two CTAs per SM
-  // The streaming kernel runs two CTAs per SM over key splits; with well over one (session, kv head) pair per SM
-  // the plain-load kernel, several CTAs resident per SM and no splits, was measured faster (64 sessions of the 4B shape).
-  const bool stream_attn = nb * d.hkv * 2 <= n_sms * 3;
-  const size_t attn_smem = sizeof(float) * ((size_t)(d.group() + 2) * d.hd + (size_t)8 * d.group() * (d.hd + 2));
-  pf_embed_norm_kernel<<<nb, kPfThreads, sizeof(float) * d.d, stream>>>(wide.tok, model->embed_rows, model->embed_scale,
-                                                                        model->layers_host[0].g_pre_attn, d.d, d.vocab, d.eps,
-                                                                        pf_xres, pf_h, err);
+  // key splits so that few sessions still fill the SMs with two CTAs each: one per (session, kv head, split)
+  const int nsplit = std::max(1, std::min(kWideMaxSplits, 2 * n_sms / std::max(1, nb * d.hkv)));
+  launch_pdl(pf_embed_norm_kernel, dim3(nb), dim3(kPfThreads), sizeof(float) * d.d, stream, wide.tok, model->embed_rows, model->embed_scale,
+             model->layers_host[0].g_pre_attn, d.d, d.vocab, d.eps, pf_xres, pf_h, err);
   int64_t* nl = &launches;
   ++*nl;
   for (int li = 0; li < d.n_layers; ++li) {
@@ -921,43 +926,11 @@ void Executor::wide_step(int nb, int first) {
     if ((size_t)ks_q * d.nqkv() > (size_t)8 * d.d) ks_q = 1;
     launch_gemm(stream, mode, tm_h, pf_h, L.wqkv, L.sqkv, Gm.wqkv, Gm.sqkv, nb, d.nqkv(), d.d, ks_q, false,
                 ks_q > 1 ? pf_parts : pf_qkv, nullptr, err, nl);
-    const bool fold_parts = ks_q > 1 && stream_attn;       // the streaming attention sums the partials as it reads them
-    if (ks_q > 1 && !fold_parts) {
-      const size_t count = (size_t)nb * d.nqkv();
-      wide_sum_parts_kernel<<<(unsigned)((count / 4 + 255) / 256), 256, 0, stream>>>(pf_parts, ks_q, count, count, pf_qkv);
-      ++*nl;
-    }
-    if (stream_attn) {
-    WideAttnArgs wa{fold_parts ? pf_parts : pf_qkv, wide.pos, page_table_dev + (size_t)first * pages_per_seq, pages_per_seq, L.is_global, nsplit, 0,
-                    L.g_q, L.g_k, model->rope_cos[L.is_global], model->rope_sin[L.is_global], kv_host[li], wide_part, pf_attn, err,
-                    1, 0, nullptr, 2, fold_parts ? ks_q : 1, (size_t)nb * d.nqkv()};
-    launch_wide_attn(stream, d, nb, smem_optin, wa);
+    WideAttnArgs wa{ks_q > 1 ? pf_parts : pf_qkv, wide.pos, page_table_dev + (size_t)first * pages_per_seq, pages_per_seq, L.is_global, nsplit, 0,
+                    L.g_q, L.g_k, model->rope_cos[L.is_global], model->rope_sin[L.is_global], kv_host[li], wide_part, wide_ticket, pf_attn, err,
+                    1, 0, nullptr, 2, ks_q, (size_t)nb * d.nqkv()};
+    launch_wide_attn(stream, d, nb, smem_optin, wa);         // sums the projections' partials as it reads them
     ++*nl;
-    if (nsplit > 1) {
-      wide_attn_combine_kernel<<<nb * d.hq, 128, 0, stream>>>(wide_part, nsplit, d.hq, d.hkv, d.hd, pf_attn, nullptr);
-      ++*nl;
-    }
-    } else {
-      AttnJob j;
-      memset(&j, 0, sizeof j);
-      j.qkv = pf_qkv;
-      j.pos = wide.pos;
-      j.page_table = page_table_dev + (size_t)first * pages_per_seq;
-      j.pages_per_seq = pages_per_seq;
-      j.seq_stride = 1;
-      j.is_global = L.is_global;
-      j.nsplit = 1;
-      j.appended = 0;                               // the kernel norms, rotates and appends this step's K / V rows
-      j.g_q = L.g_q;
-      j.g_k = L.g_k;
-      j.cosT = model->rope_cos[L.is_global];
-      j.sinT = model->rope_sin[L.is_global];
-      j.kv = kv_host[li];
-      j.out_bf16 = pf_attn;
-      j.err = err;
-      pf_attn_kernel<<<nb * d.hkv, 256, attn_smem, stream>>>(d, j);
-      ++*nl;
-    }
     const int ks_o = pick_ksplit(nb, (d.d + kTsRows - 1) / kTsRows, d.nq() / 64, n_sms);
     launch_gemm(stream, mode, tm_attn, pf_attn, L.wo, L.so, Gm.wo, Gm.so, nb, d.d, d.nq(), ks_o, false, pf_parts, nullptr, err, nl);
     launch_resid_norm(stream, pf_parts, ks_o, nb, d, L.g_post_attn, L.g_pre_ffn, pf_xres, pf_h);
@@ -970,9 +943,10 @@ void Executor::wide_step(int nb, int first) {
     launch_resid_norm(stream, pf_parts, ks_d, nb, d, L.g_post_ffn, g_next, pf_xres, pf_h);
     ++*nl;
   }
-  launch_gemm(stream, mode, tm_h, pf_h, nullptr, nullptr, model->head_g, model->head_gs, nb, d.vocab, d.d, 1, false, dargs.logits,
+  launch_gemm(stream, mode, tm_h, pf_h, model->head_w, model->embed_scale, model->head_g, model->head_gs, nb, d.vocab, d.d, 1, false, dargs.logits,
               nullptr, err, nl);
-  wide_argmax_kernel<<<nb, kWideArgThreads, 0, stream>>>(dargs.logits, d.vocab, nb, wide, dargs.step_tokens);
+  const int arg_parts = std::max(1, std::min(kWideArgParts, 2 * n_sms / nb));
+  launch_pdl(wide_argmax_kernel, dim3(nb * arg_parts), dim3(kWideArgThreads), 0, stream, dargs.logits, d.vocab, nb, arg_parts, wide, dargs.step_tokens);
   ++*nl;
   B2_CUDA(cudaGetLastError());
 }

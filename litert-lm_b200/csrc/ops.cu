@@ -413,16 +413,15 @@ int B200LmOps_Attention(int32_t device, const float* q, const float* k, const fl
   size_t smem_dec = sizeof(float) * ((size_t)(G + 2) * hd + (size_t)kDecWarps * G * (hd + 2));
   raise_dyn_smem(pf_attn_kernel, (size_t)(smem_pf));
   raise_dyn_smem(attn_decode_kernel, (size_t)(smem_dec));
-  // decode, on request: the streaming kernel (K / V blocks by bulk copies into a shared-memory ring) + its combine
-  DevBuf wpart((size_t)t * hkv * nsplit * G * (hd + 2) * 4, true);
+  // decode, on request: the streaming kernel (K / V blocks by bulk copies into a shared-memory ring)
+  DevBuf wpart((size_t)t * hkv * nsplit * G * (hd + 4) * 4, true), wticket(sizeof(int) * (size_t)t * hkv, true);
   WideAttnArgs wa{qd.as<float>(), posd.as<int>(), ptab.as<int>(), npages, window > 0 ? 0 : 1, nsplit, 0, nullptr, nullptr, nullptr,
-                  nullptr, LayerKv{kp.p, vp.p, nullptr, nullptr}, wpart.as<float>(), nullptr, errw.as<int>(), priv ? 1 : 0, 1,
-                  nullptr, 2};
+                  nullptr, LayerKv{kp.p, vp.p, nullptr, nullptr}, wpart.as<float>(), wticket.as<int>(), nullptr, errw.as<int>(), priv ? 1 : 0, 1,
+                  od.as<float>(), 2};
   const bool stream_decode = decode && (kv_bf16_flags & 4);
   auto run = [&]() {
     if (stream_decode) {
       launch_wide_attn(nullptr, dm, t, (size_t)prop.sharedMemPerBlockOptin, wa);
-      wide_attn_combine_kernel<<<t * hq, 128>>>(wpart.as<float>(), nsplit, hq, hkv, hd, nullptr, od.as<float>());
     } else if (decode) {
       j.part_o = po.as<float>();
       j.part_ml = pml.as<float>();

@@ -188,11 +188,11 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_w = tmem_base + NTOK;         // weight slots follow the accumulator columns
-  pdl_launch_dependents();
 
   if (warp == 0) {
     // ---- activation producer: what it reads comes from the preceding kernel
     pdl_wait();
+    pdl_launch_dependents();                        // not earlier: the next kernel may read what the kernels before this one wrote
     int it = 0;
     bool ok = true;
 #pragma unroll 1

@@ -52,13 +52,19 @@ pf_embed_norm_kernel(const int* __restrict__ tokens, const uint8_t* __restrict__
   const uint8_t* row = embed_rows + (size_t)tok * (d / 2);
   const float sc = embed_scale[tok] * sqrtf((float)d);
   float ss = 0.f;
-  for (int i = threadIdx.x; i < d; i += blockDim.x) {
-    int b = row[i >> 1];
-    int nib = (i & 1) ? (b >> 4) : (b & 0xF);
-    float v = (float)(nib >= 8 ? nib - 16 : nib) * sc;
-    pf_sm[i] = v;
-    xres[(size_t)t * d + i] = v;
-    ss += v * v;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < d / 8; i += kPfThreads) {            // rows of 64 k and more: whole words of eight
+    const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(row) + i);
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = (float)((int)(w << (28 - 4 * j)) >> 28) * sc;
+      ss += v[j] * v[j];
+    }
+    float4* xo = reinterpret_cast<float4*>(xres + (size_t)t * d) + 2 * i;
+    float4* so = reinterpret_cast<float4*>(pf_sm) + 2 * i;
+    so[0] = xo[0] = make_float4(v[0], v[1], v[2], v[3]);
+    so[1] = xo[1] = make_float4(v[4], v[5], v[6], v[7]);
   }
   ss = pf_block_sum(ss, scratch);
   float r = rsqrtf(ss / (float)d + eps);

@@ -132,8 +132,9 @@ class Executor {
   std::map<std::pair<int, int>, cudaGraphExec_t> step_graphs;   // one step, keyed by (sessions, first session)
   void launch_chain(int nsteps, int ncols, int first);
   // wide lockstep decode (B200LM_DECODE_WIDE)
-  WideState wide{nullptr, nullptr, nullptr};
+  WideState wide{};
   float* wide_part = nullptr;       // key-split partial states of the wide attention
+  int* wide_ticket = nullptr;       // splits of a (session, kv head) that are done
   int* pin_wide = nullptr;          // staging of the wide state words
   std::map<std::pair<int, int>, cudaGraphExec_t> wide_graphs;   // one step, keyed by (sessions, first session)
   int64_t wide_per_step = 0;        // kernel launches of one wide step
