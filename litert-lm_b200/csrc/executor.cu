@@ -272,19 +272,19 @@ static CUtensorMap make_bf16_map(const void* base, int rank, const cuuint64_t* d
 
 // Split-K factor for a GEMM of `n_tiles` weight-row tiles over T tokens with KB
 // 64-wide k blocks: the smallest divisor of KB (at least 4 k blocks per split,
-// at most 8 splits) whose work units fill 90 % of the last round over the SMs,
+// at most 8 splits) whose work units fill 90 % of the last round over the CTAs,
 // else the divisor that fills it best.
 int pick_ksplit(int T, int n_tiles, int KB, int sms) {
   if (const int s = gs_ksplit(T, n_tiles * 128, KB, sms)) return s;
   const int ntok = ts_tile_tokens(T);
-  const int tiles = n_tiles * ((T + ntok - 1) / ntok);
+  const int tiles = n_tiles * ((T + ntok - 1) / ntok), slots = ts_ctas_per_sm(ntok) * sms;
   int best = 1;
   double best_eff = 0.0;
   for (int s = 1; s <= 8; ++s) {
     if (KB % s) continue;
     if (s > 1 && KB / s < 4) break;
     const int units = tiles * s;
-    const double eff = (double)units / ((double)((units + sms - 1) / sms) * sms);
+    const double eff = (double)units / ((double)((units + slots - 1) / slots) * slots);
     if (eff > best_eff + 1e-9) { best_eff = eff; best = s; }
     if (eff >= 0.9) break;
   }
@@ -323,7 +323,7 @@ void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bflo
     }
     const int ntok = ts_tile_tokens(T);
     const int total = ((N + kTsRows - 1) / kTsRows) * ((T + ntok - 1) / ntok) * ksplit;
-    const int grid = total < sms ? total : sms;
+    const int slots = ts_ctas_per_sm(ntok) * sms, grid = total < slots ? total : slots;
 #define B2_TS(EPI_, NTOK_, MAP_) launch_pdl(gemm_w4_ts_kernel<EPI_, NTOK_>, dim3(grid), dim3(ts_threads(NTOK_)), ts_smem(NTOK_), st, MAP_, g)
 #define B2_TS2(NTOK_, MAP_) do { if (geglu) B2_TS(1, NTOK_, MAP_); else B2_TS(0, NTOK_, MAP_); } while (0)
     switch (ntok) {

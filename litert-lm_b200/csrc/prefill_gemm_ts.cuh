@@ -31,6 +31,9 @@
 // shared and tensor memory, which lets the next GEMM's CTA do that while this one
 // works.
 //
+// A narrow tile's k block still costs a CTA its hand-overs, so two CTAs share an SM and fill each other's gaps
+// (131072 x 2560, 64 tokens: 106 us with one, 87 with two; 20480 x 2560: 33 and 24).
+//
 // Warp roles: 0 = activation producer, 1 = TMEM owner + MMA issue, 2 = weight
 // producer, 4.. = int4 expansion, then epilogue.
 //
@@ -54,12 +57,13 @@ __host__ __device__ constexpr int ts_deq_warps(int ntok) { return ntok >= 256 ? 
 __host__ __device__ constexpr int ts_epi_cols(int ntok) { return ntok < 64 ? ntok : 64; }      // token columns per epilogue warp
 __host__ __device__ constexpr int ts_epi_warps(int ntok) { return 4 * (ntok / ts_epi_cols(ntok)); }
 __host__ __device__ constexpr int ts_threads(int ntok) { return 32 * (4 + ts_deq_warps(ntok) + ts_epi_warps(ntok)); }
+__host__ __device__ constexpr int ts_ctas_per_sm(int ntok) { return ntok <= 64 ? 2 : 1; }
 __host__ __device__ constexpr int ts_smem(int ntok) {
   return ts_xs(ntok) * kTsKb * ntok * kGemmBK * 2 + ts_qs(ntok) * kTsKb * kGemmStageQ + 1024 + 512;
 }
 static_assert(ts_tmem(256) >= 256 + ts_ws(256) * kTsKb * kTsAcols && ts_tmem(128) >= 128 + ts_ws(128) * kTsKb * kTsAcols &&
                   ts_tmem(64) >= 64 + ts_ws(64) * kTsKb * kTsAcols, "TMEM budget");
-static_assert(ts_smem(256) <= 227 * 1024 && 2 * (ts_smem(128) + 1024) <= 228 * 1024 && 2 * (ts_smem(64) + 1024) <= 228 * 1024 &&
+static_assert(ts_ctas_per_sm(64) * ts_tmem(64) <= 512 && ts_smem(256) <= 227 * 1024 && 2 * (ts_smem(128) + 1024) <= 228 * 1024 && 2 * (ts_smem(64) + 1024) <= 228 * 1024 &&
                   2 * (ts_smem(32) + 1024) <= 228 * 1024, "shared memory budget");
 
 // A operand in tensor memory, B through a shared-memory descriptor
@@ -126,7 +130,7 @@ __device__ __forceinline__ void ts_load_acc(uint32_t taddr, uint32_t (&v)[EC]) {
 // no more token rows than that (the wide decode step, short prompts), which cuts the activation bytes every
 // CTA re-reads per k block and the MMA time in proportion.  tmX must have a box of min(NTOK, 128) rows.
 template <int EPI, int NTOK>
-__global__ void __launch_bounds__(ts_threads(NTOK), NTOK <= 64 ? 2 : 1)
+__global__ void __launch_bounds__(ts_threads(NTOK), ts_ctas_per_sm(NTOK))
 gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   constexpr int D = ts_deq_warps(NTOK), E = ts_epi_warps(NTOK), EC = ts_epi_cols(NTOK);
   constexpr int XS = ts_xs(NTOK), QS = ts_qs(NTOK), WS = ts_ws(NTOK);
@@ -168,7 +172,7 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   };
   if (threadIdx.x == 64) {
 #pragma unroll 1
-    for (int s = 0; s < QS; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], D); }
+    for (int s = 0; s < QS; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 4); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 #pragma unroll 1
     while (q_it < QS && q_li < my_tiles) q_issue();
@@ -177,7 +181,7 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
 #pragma unroll 1
     for (int s = 0; s < XS; ++s) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
 #pragma unroll 1
-    for (int s = 0; s < WS; ++s) { mbar_init(&w_full[s], D); mbar_init(&w_empty[s], 1); }
+    for (int s = 0; s < WS; ++s) { mbar_init(&w_full[s], 4); mbar_init(&w_empty[s], 1); }
     mbar_init(acc_full, 1);
     mbar_init(acc_empty, E);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -256,27 +260,24 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
       }
     }
   } else if (warp >= 4 && warp < 4 + D) {
-    // ---- int4 -> bf16 expansion into TMEM: this thread does the 64 k (32 columns) of its weight row in one k block of
-    // the stage, or in both when there is one warp per 32 lanes
+    // ---- int4 -> bf16 expansion into TMEM: this thread does its weight row's part of a stage.  Eight warps take
+    // alternate stages in two groups of four, so that one group's waits run beside the other's expansion.
     const int quarter = warp & 3;                  // TMEM lanes 32*quarter .. +31 belong to this warp
-    const int kb0 = D == 8 ? (warp - 4) >> 2 : 0;
-    constexpr int kPer = D == 8 ? 1 : kTsKb;
+    constexpr int kGroups = D / 4;
+    const int group = (warp - 4) >> 2;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int iters = my_tiles * nst;
     const __nv_bfloat162 bias = __float2bfloat162_rn(136.0f);
     bool ok = true;
-    int st = 0;
 #pragma unroll 1
-    for (int it = 0; it < iters && ok; ++it) {
-      const int sq = it % QS, sw = it % WS, nk = min(kTsKb, nkb - st * kTsKb);
-      if (++st == nst) st = 0;
+    for (int it = group; it < iters && ok; it += kGroups) {
+      const int sq = it % QS, sw = it % WS, nk = min(kTsKb, nkb - it % nst * kTsKb);
       ok = mbar_wait(&q_full[sq], (it / QS) & 1, g.err);
       if (ok && it >= WS) ok = mbar_wait(&w_empty[sw], (it / WS - 1) & 1, g.err);
       if (!ok) break;
       tc_fence_after();
 #pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        const int kb = kb0 + u;
+      for (int kb = 0; kb < kTsKb; ++kb) {
         if (kb < nk) {
           const uint4* src = reinterpret_cast<const uint4*>(sQ + (sq * kTsKb + kb) * kGemmStageQ + (quarter * 32 + lane) * 32);
 #pragma unroll
