@@ -353,6 +353,8 @@ Executor::~Executor() {
   if (stream) cudaStreamSynchronize(stream);
   for (auto& g : step_graphs) cudaGraphExecDestroy(g.second);
   for (auto& g : wide_graphs) cudaGraphExecDestroy(g.second);
+  for (cudaEvent_t ev : logit_part)
+    if (ev) cudaEventDestroy(ev);
   if (tp_comm) {
     try { NcclApi::get().CommDestroy(tp_comm); } catch (...) {}
   }
@@ -628,16 +630,26 @@ void Executor::tp_allreduce(float* buf, size_t count) {
   nccl.check(nccl.AllReduce(buf, buf, count, kNcclFloat32, kNcclSum, tp_comm, stream), "ncclAllReduce");
 }
 
+// err, barrier and steps_done are adjacent
+constexpr size_t kErrTail = sizeof(DecodeState) - offsetof(DecodeState, err);
+
+void Executor::queue_device_error() {
+  B2_CUDA(cudaMemcpyAsync(&pin_state->err, &dargs.st->err, kErrTail, cudaMemcpyDeviceToHost, stream));
+}
+
 void Executor::check_device_error(const char* where) {
-  int err = 0;
-  // err, barrier and steps_done are adjacent
-  const size_t tail = sizeof(DecodeState) - offsetof(DecodeState, err);
-  B2_CUDA(cudaMemcpyAsync(&pin_state->err, &dargs.st->err, tail, cudaMemcpyDeviceToHost, stream));
+  queue_device_error();
   B2_CUDA(cudaStreamSynchronize(stream));
-  err = pin_state->err;
+  raise_device_error(where);
+}
+
+// The words queued by queue_device_error have arrived.
+void Executor::raise_device_error(const char* where) {
+  const int err = pin_state->err;
   if (err == kDevOk) return;
+  B2_CUDA(cudaStreamSynchronize(stream));
   // clear the words and the barrier count so the handle stays usable
-  B2_CUDA(cudaMemsetAsync(&dargs.st->err, 0, tail, stream));
+  B2_CUDA(cudaMemsetAsync(&dargs.st->err, 0, kErrTail, stream));
   B2_CUDA(cudaStreamSynchronize(stream));
   barrier_epoch = 0;
   std::string w(where);
@@ -1028,10 +1040,30 @@ void Executor::decode_logits(const int* id_or_null, float* host_logits) {
   cudaPointerAttributes pa{};
   const bool direct = cudaPointerGetAttributes(&pa, host_logits) == cudaSuccess && pa.type == cudaMemoryTypeHost;
   if (!direct) cudaGetLastError();
-  B2_CUDA(cudaMemcpyAsync(direct ? host_logits : pin_logits, dargs.logits, nb, cudaMemcpyDeviceToHost, stream));
   d2h_bytes += nb;
-  check_device_error("DecodeLogits");
-  if (!direct) memcpy(host_logits, pin_logits, nb);
+  if (direct) {
+    B2_CUDA(cudaMemcpyAsync(host_logits, dargs.logits, nb, cudaMemcpyDeviceToHost, stream));
+    check_device_error("DecodeLogits");
+  } else {
+    // In parts, so that one part's copy out of the staging runs under the next one's transfer: 1 MB is 20 us on the bus
+    // and as much again and more in the host's memory.  A part below 64 KB would cost more in calls than it hides.
+    const int parts = (int)std::min<size_t>(kLogitParts, std::max<size_t>(1, nb / (64 << 10)));
+    const size_t per = (nb / parts + 63) / 64 * 64;
+    queue_device_error();
+    for (int p = 0; p < parts; ++p) {
+      const size_t off = std::min(nb, p * per), len = p + 1 < parts ? std::min(per, nb - off) : nb - off;
+      B2_CUDA(cudaMemcpyAsync(reinterpret_cast<unsigned char*>(pin_logits) + off, reinterpret_cast<const unsigned char*>(dargs.logits) + off, len,
+                              cudaMemcpyDeviceToHost, stream));
+      if (!logit_part[p]) B2_CUDA(cudaEventCreateWithFlags(&logit_part[p], cudaEventDisableTiming));
+      B2_CUDA(cudaEventRecord(logit_part[p], stream));
+    }
+    for (int p = 0; p < parts; ++p) {
+      const size_t off = std::min(nb, p * per), len = p + 1 < parts ? std::min(per, nb - off) : nb - off;
+      B2_CUDA(cudaEventSynchronize(logit_part[p]));
+      if (p == 0) raise_device_error("DecodeLogits");
+      memcpy(reinterpret_cast<unsigned char*>(host_logits) + off, reinterpret_cast<const unsigned char*>(pin_logits) + off, len);
+    }
+  }
   ++current_step;
 }
 

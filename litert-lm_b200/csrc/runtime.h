@@ -77,6 +77,8 @@ class Executor {
   void select_session(int session);                 // the calls above then act on that session
   void decode_tokens_batch(int nsteps, int* out_ids /* [nsteps][n_sessions] */);
   void check_device_error(const char* where);
+  void queue_device_error();
+  void raise_device_error(const char* where);
   void trace_decode_step(int* out_id, long long* stamps, long long capacity, int* n_barriers, int* n_cta, int* khz);
   void read_kv_row(int layer, int is_v, int kv_head, int pos, float* out, int* page, int* slot);
   void tp_allreduce(float* buf, size_t count);      // sum over the tensor-parallel ranks, in place, on `stream`
@@ -158,6 +160,8 @@ class Executor {
   static constexpr int kTokRing = 4;    // prompt-id slices that may be queued for upload at once
   void* pinned = nullptr;
   float* pin_logits = nullptr;
+  static constexpr int kLogitParts = 4;
+  cudaEvent_t logit_part[kLogitParts] = {};      // parts of a logits row that are in the staging
   int* pin_ints = nullptr;          // kTokRing slices of t_pad ids
   int* pin_steps = nullptr;         // ids sampled by a multi-step decode call
   cudaEvent_t tok_ring_done[kTokRing] = {nullptr, nullptr, nullptr, nullptr};
