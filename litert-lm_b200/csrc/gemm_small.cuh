@@ -111,8 +111,8 @@ gemm_w4_small_kernel(const GsArgs g) {
   __syncthreads();
   const int nshared = nmet;
   for (int i = threadIdx.x; i < nshared * 16; i += kGsThreads) scales[i] = __ldg(g.wscale + (t0 + (met[i >> 4] >> 16)) * 16 + (i & 15));
+  pdl_launch_dependents();                         // ahead of the wait, as in the tcgen05 kernel
   pdl_wait();
-  pdl_launch_dependents();                         // not earlier: the next kernel may read what the kernels before this one wrote
   // ---- X of the slice
   for (int row = warp; row < g.T; row += kGsWarps) {
     const uint4* from = reinterpret_cast<const uint4*>(g.x + (size_t)row * (g.KT * 64) + split * KTs * 64);

@@ -192,11 +192,13 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_w = tmem_base + NTOK;         // weight slots follow the accumulator columns
+  // Ahead of the wait below: the next GEMM may fill its weight ring while this one still waits.  A kernel behind this one
+  // that reads ahead of its own wait must read nothing that the two kernels before it write.
+  pdl_launch_dependents();
 
   if (warp == 0) {
     // ---- activation producer: what it reads comes from the preceding kernel
     pdl_wait();
-    pdl_launch_dependents();                        // not earlier: the next kernel may read what the kernels before this one wrote
     int it = 0;
     bool ok = true;
 #pragma unroll 1
@@ -270,8 +272,10 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
     const __nv_bfloat162 bias = __float2bfloat162_rn(136.0f);
     bool ok = true;
 #pragma unroll 1
-    for (int it = group; it < iters && ok; it += kGroups) {
-      const int sq = it % QS, sw = it % WS, nk = min(kTsKb, nkb - it % nst * kTsKb);
+    for (int it = group, st = group; it < iters && ok; it += kGroups, st += kGroups) {
+#pragma unroll 1
+      while (st >= nst) st -= nst;
+      const int sq = it % QS, sw = it % WS, nk = min(kTsKb, nkb - st * kTsKb);
       ok = mbar_wait(&q_full[sq], (it / QS) & 1, g.err);
       if (ok && it >= WS) ok = mbar_wait(&w_empty[sw], (it / WS - 1) & 1, g.err);
       if (!ok) break;
