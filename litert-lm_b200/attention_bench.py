@@ -75,13 +75,13 @@ def main() -> None:
         v = rng.standard_normal((s, HKV, HD), dtype=np.float32)
         q = rng.standard_normal((batch, HQ, HD), dtype=np.float32)
         nsplit = max(2, min(64, s // 256))
-        if args.streaming_kernel:       # one CTA per SM there: about two (sequence, kv head, split) items per SM
+        if args.streaming_kernel:       # about two (sequence, kv head, split) items per SM
             nsplit = max(2, min(nsplit, -(-2 * 148 // (batch * HKV))))
         _, ms = pkg.ops.attention(q, k, v, nsplit=nsplit, repeat=args.repeat, kv_bf16=True, private_caches=True,
                                   streaming_kernel=args.streaming_kernel)
         nbytes = 2.0 * s * HKV * HD * 2 * batch
         gbs = nbytes / (ms * 1e-3) / 1e9
-        print(json.dumps({"op": "decode_attention", "kernel": ("wide_attn_kernel + wide_attn_combine_kernel" if args.streaming_kernel else
+        print(json.dumps({"op": "decode_attention", "kernel": ("wide_attn_kernel" if args.streaming_kernel else
                                                             "attn_decode_kernel + attn_combine_kernel"), "kv_len": s,
                           "batch": batch, "nsplit": nsplit, "page": 256, "kv_dtype": "bf16", "ms": ms, "bytes": nbytes,
                           "roofline": {"bound": "hbm", "achieved": gbs, "peak": hbm, "unit": "GB/s",

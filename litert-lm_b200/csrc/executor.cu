@@ -686,9 +686,8 @@ template <typename T>
 static void launch_kv_append(cudaStream_t st, const ModelDims& d, int T_, const float* qkv, int nparts, int pos0, const int* pt,
                              const LayerWeights& L, const float* c, const float* s, const LayerKv& kv,
                              __nv_bfloat16* qout) {
-  const int jobs = T_ * (d.hkv + (qout ? d.hq : 0));
-  const int per = kKvaThreads / 32;
-  const int grid = (jobs + per - 1) / per;
+  const int groups = (T_ + pos0 % kKvaTok + kKvaTok - 1) / kKvaTok;
+  const int grid = groups * d.hkv + (qout ? (T_ * d.hq + kKvaTok - 1) / kKvaTok : 0);
   const size_t stride = (size_t)T_ * d.nqkv();
 #define B2_KVA(HD_) launch_pdl(pf_kv_append_kernel<T, HD_>, dim3(grid), dim3(kKvaThreads), 0, st, d, qkv, nparts, stride, T_, pos0, pt, L.g_k, c, s, kv, L.g_q, qout)
   switch (d.hd) {

@@ -218,13 +218,16 @@ __device__ __forceinline__ void st_vec(__nv_bfloat16* p, const float (&o)[V]) {
 // K-RMSNorm + RoPE on the new keys, then K and V rows into the paged cache (and
 // the bf16 operands of the tensor-core attention); with qout, also Q-RMSNorm +
 // RoPE + 1/sqrt(hd) on the query heads into a bf16 [T][hq][hd] buffer.  One
-// warp per (token, head): job = token * nheads + head, kv heads first.  Lane l
+// warp per (token, head).  The first CTAs take a kv head and the eight tokens
+// of an aligned group of positions each, so that the transposed V rows go out
+// through shared memory as 16 bytes an element, where a warp's own stores were
+// two bytes a line; the others take the query heads in token order.  Lane l
 // holds V consecutive elements of each half of the head (V = HD / 64, or one
 // element on the low lanes for HD 32).  The QKV row may arrive as `nparts`
 // split-K partial sums `part_stride` floats apart; they are added on load.
-constexpr int kKvaThreads = 128;
+constexpr int kKvaThreads = 256, kKvaTok = kKvaThreads / 32;
 template <typename T, int HD>
-__global__ void __launch_bounds__(kKvaThreads, HD == 256 ? 8 : 10)
+__global__ void __launch_bounds__(kKvaThreads, HD == 256 ? 4 : 5)
 pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, size_t part_stride, int ntok, int pos0,
                     const int* __restrict__ page_table, const float* __restrict__ g_k,
                     const float* __restrict__ cosT, const float* __restrict__ sinT, LayerKv kv,
@@ -234,16 +237,18 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
   constexpr int V = HD >= 64 ? HD / 64 : 1;
   constexpr int half = HD / 2;
   const int lane = threadIdx.x & 31;
-  const int nheads = dm.hkv + (qout ? dm.hq : 0);
-  const int job = blockIdx.x * (kKvaThreads / 32) + (threadIdx.x >> 5);
-  if (job >= ntok * nheads) return;
-  const int t = job / nheads, h = job - t * nheads, pos = pos0 + t;
-  const bool is_q = h >= dm.hkv;
-  const int e0 = lane * V;
-  const bool act = e0 < half;                                   // HD 32: lanes 16..31 idle
+  const int warp = threadIdx.x >> 5, skew = pos0 % kKvaTok, groups = (ntok + skew + kKvaTok - 1) / kKvaTok;
+  const bool is_q = (int)blockIdx.x >= groups * dm.hkv;
+  const int job = (blockIdx.x - groups * dm.hkv) * kKvaTok + warp;
+  const int t = is_q ? job / dm.hq : (int)(blockIdx.x % groups) * kKvaTok + warp - skew;
+  const int h = is_q ? job % dm.hq : blockIdx.x / groups;       // of the query or of the kv heads
+  const bool has = t >= 0 && t < ntok;
+  if (is_q && !has) return;
+  const int pos = pos0 + t, e0 = lane * V;
+  const bool act = has && e0 < half;                            // HD 32: lanes 16..31 idle
   // head offset within the QKV row: [q heads | k heads | v heads]
-  const int col = is_q ? (h - dm.hkv) * HD : dm.nq() + h * HD;
-  const float* row = qkv + (size_t)t * dm.nqkv() + col;
+  const int col = is_q ? h * HD : dm.nq() + h * HD;
+  const float* row = qkv + (ptrdiff_t)t * dm.nqkv() + col;
   float a[V], b[V], va[V], vb[V];
 #pragma unroll
   for (int i = 0; i < V; ++i) a[i] = b[i] = va[i] = vb[i] = 0.f;
@@ -269,10 +274,9 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
   ss = warp_sum(ss);
   float r = rsqrtf(ss / (float)HD + dm.eps);
   if (is_q) r *= rsqrtf((float)HD);
-  if (!act) return;
   const float* gain = is_q ? g_q : g_k;
   float k0[V], k1[V];
-  {
+  if (act) {
     float ga[V], gb[V], cs[V], sn[V];
     ld_vec<V>(gain + e0, ga);
     ld_vec<V>(gain + e0 + half, gb);
@@ -286,11 +290,15 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
     }
   }
   if (is_q) {
-    __nv_bfloat16* dst = qout + ((size_t)t * dm.hq + (h - dm.hkv)) * HD;
-    st_vec<V>(dst + e0, k0);
-    st_vec<V>(dst + e0 + half, k1);
+    if (act) {
+      __nv_bfloat16* dst = qout + ((size_t)t * dm.hq + h) * HD;
+      st_vec<V>(dst + e0, k0);
+      st_vec<V>(dst + e0 + half, k1);
+    }
     return;
   }
+  __shared__ __align__(16) __nv_bfloat16 vt_s[HD][kKvaTok];
+  if (act) {
   const int page = page_table[pos / kPage], slot = pos % kPage;
   const size_t off = (((size_t)page * dm.hkv + h) * kPage + slot) * HD;
   T* kbase = reinterpret_cast<T*>(kv.k);
@@ -305,13 +313,21 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
       st_vec<V>(kv.k16 + off + e0 + half, k1);
     }
   }
-  if (kv.v16) {
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      const size_t vt = (((size_t)page * dm.hkv + h) * HD + e0 + i) * kPage + slot;
-      kv.v16[vt] = __float2bfloat16(va[i]);
-      kv.v16[vt + (size_t)half * kPage] = __float2bfloat16(vb[i]);
-    }
+  for (int i = 0; i < V; ++i) {
+    vt_s[e0 + i][warp] = __float2bfloat16(va[i]);
+    vt_s[e0 + half + i][warp] = __float2bfloat16(vb[i]);
+  }
+  }
+  if (kv.v16 == nullptr) return;
+  __syncthreads();
+  const int first = pos - warp;                                 // position of the group's first token
+  const int w0 = max(0, pos0 - first), w1 = min(kKvaTok, pos0 + ntok - first);
+  __nv_bfloat16* vt = kv.v16 + ((size_t)page_table[first / kPage] * dm.hkv + h) * HD * kPage + first % kPage;
+  for (int e = threadIdx.x; e < HD; e += kKvaThreads) {
+    if (w1 - w0 == kKvaTok) *reinterpret_cast<uint4*>(vt + (size_t)e * kPage) = *reinterpret_cast<const uint4*>(vt_s[e]);
+    else
+      for (int w = w0; w < w1; ++w) vt[(size_t)e * kPage + w] = vt_s[e][w];
   }
 }
 
