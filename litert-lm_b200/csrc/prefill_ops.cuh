@@ -245,6 +245,7 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
   const bool has = t >= 0 && t < ntok;
   if (is_q && !has) return;
   const int pos = pos0 + t, e0 = lane * V;
+  const int page = is_q ? 0 : page_table[pos / kPage];          // one of the whole group; asked for early
   const bool act = has && e0 < half;                            // HD 32: lanes 16..31 idle
   // head offset within the QKV row: [q heads | k heads | v heads]
   const int col = is_q ? h * HD : dm.nq() + h * HD;
@@ -299,7 +300,7 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
   }
   __shared__ __align__(16) __nv_bfloat16 vt_s[HD][kKvaTok];
   if (act) {
-  const int page = page_table[pos / kPage], slot = pos % kPage;
+  const int slot = pos % kPage;
   const size_t off = (((size_t)page * dm.hkv + h) * kPage + slot) * HD;
   T* kbase = reinterpret_cast<T*>(kv.k);
   T* vbase = reinterpret_cast<T*>(kv.v);
@@ -323,7 +324,7 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
   __syncthreads();
   const int first = pos - warp;                                 // position of the group's first token
   const int w0 = max(0, pos0 - first), w1 = min(kKvaTok, pos0 + ntok - first);
-  __nv_bfloat16* vt = kv.v16 + ((size_t)page_table[first / kPage] * dm.hkv + h) * HD * kPage + first % kPage;
+  __nv_bfloat16* vt = kv.v16 + ((size_t)page * dm.hkv + h) * HD * kPage + first % kPage;
   for (int e = threadIdx.x; e < HD; e += kKvaThreads) {
     if (w1 - w0 == kKvaTok) *reinterpret_cast<uint4*>(vt + (size_t)e * kPage) = *reinterpret_cast<const uint4*>(vt_s[e]);
     else
