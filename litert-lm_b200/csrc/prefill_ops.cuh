@@ -298,7 +298,7 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
     }
     return;
   }
-  __shared__ __align__(16) __nv_bfloat16 vt_s[HD][kKvaTok];
+  __shared__ __align__(16) __nv_bfloat16 v_s[kKvaTok][HD];
   if (act) {
   const int slot = pos % kPage;
   const size_t off = (((size_t)page * dm.hkv + h) * kPage + slot) * HD;
@@ -314,11 +314,8 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
       st_vec<V>(kv.k16 + off + e0 + half, k1);
     }
   }
-#pragma unroll
-  for (int i = 0; i < V; ++i) {
-    vt_s[e0 + i][warp] = __float2bfloat16(va[i]);
-    vt_s[e0 + half + i][warp] = __float2bfloat16(vb[i]);
-  }
+  st_vec<V>(&v_s[warp][e0], va);
+  st_vec<V>(&v_s[warp][e0 + half], vb);
   }
   if (kv.v16 == nullptr) return;
   __syncthreads();
@@ -326,9 +323,17 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
   const int w0 = max(0, pos0 - first), w1 = min(kKvaTok, pos0 + ntok - first);
   __nv_bfloat16* vt = kv.v16 + ((size_t)page * dm.hkv + h) * HD * kPage + first % kPage;
   for (int e = threadIdx.x; e < HD; e += kKvaThreads) {
-    if (w1 - w0 == kKvaTok) *reinterpret_cast<uint4*>(vt + (size_t)e * kPage) = *reinterpret_cast<const uint4*>(vt_s[e]);
-    else
-      for (int w = w0; w < w1; ++w) vt[(size_t)e * kPage + w] = vt_s[e][w];
+    if (w1 - w0 == kKvaTok) {
+      uint32_t x[kKvaTok / 2];
+#pragma unroll
+      for (int w = 0; w < kKvaTok; w += 2) {
+        const __nv_bfloat162 two(v_s[w][e], v_s[w + 1][e]);
+        x[w / 2] = *reinterpret_cast<const uint32_t*>(&two);
+      }
+      *reinterpret_cast<uint4*>(vt + (size_t)e * kPage) = make_uint4(x[0], x[1], x[2], x[3]);
+    } else {
+      for (int w = w0; w < w1; ++w) vt[(size_t)e * kPage + w] = v_s[w][e];
+    }
   }
 }
 
