@@ -25,6 +25,7 @@
 #include "common.cuh"
 #include "decode_ops.cuh"
 #include "prefill_ops.cuh"
+#include "split_ticket.h"
 
 namespace b200lm {
 
@@ -106,7 +107,7 @@ struct AmArgs {
   float* out;               // [batch][hkv * G][hd]
   float* part_o;            // [hkv][rows][nsplit][hd]   (nsplit > 1)
   float* part_ml;           // [hkv][rows][nsplit][2]
-  int* tickets;             // one per (kv head, row tile): the last split to arrive sums up; null: a second kernel does
+  unsigned* tickets;        // (kv head, row tile) by split count: the last split to arrive sums up; null: a second kernel does
   int* err;
 };
 
@@ -490,10 +491,10 @@ attn_shared_kernel(const AmArgs a) {
     }
   }
   if (a.nsplit > 1 && a.tickets) {
-    // ---- the split that arrives last sums up this unit's rows and leaves the ticket at zero for the next call
+    // ---- the split that arrives last sums up this unit's rows
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) *last_s = atomicAdd(a.tickets + unit, 1) == a.nsplit - 1;
+    if (threadIdx.x == 0) *last_s = ticket_last(a.tickets, unit, a.nsplit, [](unsigned* t, unsigned top) { return atomicInc(t, top); });
     __syncthreads();
     if (*last_s) {
       __threadfence();
@@ -527,7 +528,6 @@ attn_shared_kernel(const AmArgs a) {
         }
         *reinterpret_cast<float4*>(a.out + am_out_row(a, kvh, r0 + r) * HD + e) = s;
       }
-      if (threadIdx.x == 0) a.tickets[unit] = 0;
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");       // only a wait that gave up leaves copies behind
@@ -589,14 +589,14 @@ attn_shared_sum_kernel(const AmArgs a, int hd) {
 // The shape and split count of one call: as many splits as fill the SMs, no fewer than one chunk of 16 keys per key
 // group of a split, no more partials than `cap` splits' worth of scratch.
 template <typename T, int HD, int MT, bool PACK>
-inline void launch_attn_shared_t(cudaStream_t st, AmArgs a, int device, int sms, int cap, int* tickets, int n_tickets) {
+inline void launch_attn_shared_t(cudaStream_t st, AmArgs a, int device, int sms, int cap, unsigned* tickets) {
   using S = AmShape<T, HD, MT, PACK>;
   const int units = a.hkv * ((a.rows + S::kRows - 1) / S::kRows);
   const int nchunks = (a.k1 + 15) / 16 - a.lo / 16;
-  a.nsplit = std::max(1, std::min(std::min(sms / units, cap), std::min(256, (nchunks + S::KG - 1) / S::KG)));
+  a.nsplit = std::max(1, std::min(std::min(sms / units, cap), std::min(kTicketSplits, (nchunks + S::KG - 1) / S::KG)));
   // One CTA sums up to 128 KB of partials in about the time that a second launch costs; more is spread over a grid.
   const size_t part = (size_t)a.nsplit * std::min(a.rows, S::kRows) * HD * 4;
-  a.tickets = part <= 128 * 1024 && units <= n_tickets ? tickets : nullptr;
+  a.tickets = part <= 128 * 1024 && units <= kTicketUnits ? tickets : nullptr;
   static unsigned char ready[64] = {};                                // per device; a race only repeats the call
   if (!ready[device]) {
     raise_dyn_smem(attn_shared_kernel<T, HD, MT, PACK>, (size_t)S::kSmem);
@@ -607,23 +607,23 @@ inline void launch_attn_shared_t(cudaStream_t st, AmArgs a, int device, int sms,
     launch_pdl(attn_shared_sum_kernel, dim3(a.hkv * a.rows * (HD < 64 ? 1 : HD / 64)), dim3(kAmSumThreads), (size_t)0, st, a, (int)HD);
 }
 template <typename T, int HD>
-inline void launch_attn_shared_r(cudaStream_t st, const AmArgs& a, int device, int sms, int cap, int* tickets, int n_tickets) {
-  if (a.rows <= 4) launch_attn_shared_t<T, HD, 1, true>(st, a, device, sms, cap, tickets, n_tickets);
-  else if (a.rows <= 16) launch_attn_shared_t<T, HD, 1, false>(st, a, device, sms, cap, tickets, n_tickets);
-  else if (a.rows <= 32) launch_attn_shared_t<T, HD, 2, false>(st, a, device, sms, cap, tickets, n_tickets);
-  else launch_attn_shared_t<T, HD, 4, false>(st, a, device, sms, cap, tickets, n_tickets);
+inline void launch_attn_shared_r(cudaStream_t st, const AmArgs& a, int device, int sms, int cap, unsigned* tickets) {
+  if (a.rows <= 4) launch_attn_shared_t<T, HD, 1, true>(st, a, device, sms, cap, tickets);
+  else if (a.rows <= 16) launch_attn_shared_t<T, HD, 1, false>(st, a, device, sms, cap, tickets);
+  else if (a.rows <= 32) launch_attn_shared_t<T, HD, 2, false>(st, a, device, sms, cap, tickets);
+  else launch_attn_shared_t<T, HD, 4, false>(st, a, device, sms, cap, tickets);
 }
 template <typename T>
-inline void launch_attn_shared(cudaStream_t st, const AmArgs& a, int hd, int device, int sms, int cap, int* tickets, int n_tickets) {
+inline void launch_attn_shared(cudaStream_t st, const AmArgs& a, int hd, int device, int sms, int cap, unsigned* tickets) {
   switch (hd) {
-    case 32: launch_attn_shared_r<T, 32>(st, a, device, sms, cap, tickets, n_tickets); break;
-    case 64: launch_attn_shared_r<T, 64>(st, a, device, sms, cap, tickets, n_tickets); break;
-    case 128: launch_attn_shared_r<T, 128>(st, a, device, sms, cap, tickets, n_tickets); break;
-    default: launch_attn_shared_r<T, 256>(st, a, device, sms, cap, tickets, n_tickets); break;
+    case 32: launch_attn_shared_r<T, 32>(st, a, device, sms, cap, tickets); break;
+    case 64: launch_attn_shared_r<T, 64>(st, a, device, sms, cap, tickets); break;
+    case 128: launch_attn_shared_r<T, 128>(st, a, device, sms, cap, tickets); break;
+    default: launch_attn_shared_r<T, 256>(st, a, device, sms, cap, tickets); break;
   }
 }
 // The kernels of one cache type are a translation unit.
-void launch_attn_shared_f32(cudaStream_t st, const AmArgs& a, int hd, int device, int sms, int cap, int* tickets, int n_tickets);
-void launch_attn_shared_bf16(cudaStream_t st, const AmArgs& a, int hd, int device, int sms, int cap, int* tickets, int n_tickets);
+void launch_attn_shared_f32(cudaStream_t st, const AmArgs& a, int hd, int device, int sms, int cap, unsigned* tickets);
+void launch_attn_shared_bf16(cudaStream_t st, const AmArgs& a, int hd, int device, int sms, int cap, unsigned* tickets);
 
 }  // namespace b200lm

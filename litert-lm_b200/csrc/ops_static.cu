@@ -30,9 +30,8 @@ constexpr int kStaticMaxQueries = (int)(kStaticHeaderBytes / 4) - 16;
 // device code may name the array directly.
 static __device__ __align__(256) unsigned char g_attn_static_scratch[kStaticScratchBytes];
 
-// Tickets of attn_shared_kernel: how many splits of a unit have arrived; the last one puts its ticket back to zero.
-constexpr int kStaticTickets = 256;
-static __device__ int g_attn_static_tickets[kStaticTickets];
+// Tickets of attn_shared_kernel (split_ticket.h), 128 KiB; zero whenever no call is on the GPU.
+static __device__ unsigned g_attn_static_tickets[kTicketWords];
 
 // Header layout: int[0] = error word, int[16 + i] = position of query i.
 __global__ void static_scratch_prepare_kernel(int nq, int pos) {
@@ -45,7 +44,7 @@ __global__ void static_scratch_prepare_kernel(int nq, int pos) {
 constexpr int kMaxDevices = 64;
 struct StaticScratch {
   unsigned char* base;
-  int* tickets;
+  unsigned* tickets;
   int sms;
 };
 static StaticScratch g_static_scratch[kMaxDevices] = {};
@@ -67,7 +66,7 @@ static StaticScratch static_scratch_for(int device) {
     // raised to the largest shape the entry point accepts and never lowered by any other caller.
     raise_dyn_smem(attn_decode_kernel, sizeof(float) * ((size_t)(4 + 2) * 256 + (size_t)kDecWarps * 4 * (256 + 2)));
     B2_CUDA(cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, device));
-    s.tickets = reinterpret_cast<int*>(t);
+    s.tickets = reinterpret_cast<unsigned*>(t);
     s.base = reinterpret_cast<unsigned char*>(p);
   }
   return s;
@@ -159,10 +158,10 @@ extern "C" int B200LmOps_AttentionDecodeStatic(int32_t device, const float* q_de
       a.err = hdr;
       // the caller's nsplit sized the check above; what fits the scratch is this kernel's own limit
       const size_t per_split = (size_t)batch * hq * (hd + 2) * sizeof(float);
-      const int cap = (int)std::min<size_t>(256, (kStaticScratchBytes - kStaticHeaderBytes) / per_split);
+      const int cap = (int)std::min<size_t>(kTicketSplits, (kStaticScratchBytes - kStaticHeaderBytes) / per_split);
       a.part_ml = part_o + (size_t)batch * hq * cap * hd;
-      if (kv_bf16) launch_attn_shared_bf16(st, a, hd, device, sc.sms, cap, sc.tickets, kStaticTickets);
-      else launch_attn_shared_f32(st, a, hd, device, sc.sms, cap, sc.tickets, kStaticTickets);
+      if (kv_bf16) launch_attn_shared_bf16(st, a, hd, device, sc.sms, cap, sc.tickets);
+      else launch_attn_shared_f32(st, a, hd, device, sc.sms, cap, sc.tickets);
       return kOk;
     }
     static_scratch_prepare_kernel<<<(batch + 255) / 256, 256, 0, st>>>(batch, s - 1);
