@@ -31,10 +31,16 @@ extern "C" {
 typedef struct B200LmExecutor B200LmExecutor;
 
 /* decode_mode: AUTO picks the chain of step kernels, and B200LM_DECODE_WIDE for
- * more than four sessions. */
+ * more than four sessions.  Kernels that do not take the model's geometry give way
+ * to others.  The chain does not take a vector of a projection above 24576 values
+ * (6144 with two to four sessions), nor one that shared memory does not hold; then
+ * PERSISTENT carries the steps, else the chain with the sessions of a group one
+ * after another, else one kernel per phase.  PERSISTENT gives way to the chain.
+ * B200Lm_GetDecodeMode tells what runs. */
 enum {
   B200LM_DECODE_AUTO = 0,
-  B200LM_DECODE_PHASE_KERNELS = 1,     /* the same chain as B200LM_DECODE_CHAINED */
+  B200LM_DECODE_PHASE_KERNELS = 1,     /* the same chain as B200LM_DECODE_CHAINED; where that does not fit, one kernel
+                                          per phase of PERSISTENT_BASIC, the last fallback of all modes */
   B200LM_DECODE_PERSISTENT = 2,        /* one cooperative kernel, grid barrier per phase, weights streamed by bulk async copies */
   B200LM_DECODE_PERSISTENT_BASIC = 3,  /* one cooperative kernel, grid barrier per phase, plain loads (comparison) */
   B200LM_DECODE_CHAINED = 4,           /* a chain of kernels, one per phase, in a CUDA graph with programmatic edges:

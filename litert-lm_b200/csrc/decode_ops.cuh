@@ -990,6 +990,28 @@ static __device__ __noinline__ void phase_argmax(const DecodeArgs& a, int ncta_h
   }
 }
 
+// ------------------------------------------------------- one kernel per phase
+// The last resort of the decode modes: any geometry whose vectors fit shared memory, and the only one beside the chain
+// that can run a collective between two phases.
+
+enum DecodePhase { kPhQkv = 0, kPhAttn, kPhOproj, kPhGateUp, kPhDown, kPhHead, kPhArgmax };
+
+static __global__ void __launch_bounds__(kDecThreads, 1)
+decode_phase_kernel(const __grid_constant__ DecodeArgs a, int phase, int layer) {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  DecodeSmem s = carve_smem(dsm, a.dims, a.ncols);
+  const int cta = blockIdx.x, ncta = gridDim.x;
+  switch (phase) {
+    case kPhQkv: phase_qkv(a, s, layer, cta, ncta); break;
+    case kPhAttn: phase_attn(a, s, layer, cta, ncta); break;
+    case kPhOproj: phase_oproj(a, s, layer, cta, ncta); break;
+    case kPhGateUp: phase_gateup(a, s, layer, cta, ncta); break;
+    case kPhDown: phase_down(a, s, layer, cta, ncta); break;
+    case kPhHead: phase_head(a, s, cta, ncta); break;
+    case kPhArgmax: phase_argmax(a, layer /* = head grid size */); break;
+  }
+}
+
 // ------------------------------------------ persistent kernel: whole step(s)
 
 // Sense-free counting barrier: every CTA adds one and waits for the count to

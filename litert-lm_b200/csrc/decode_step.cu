@@ -33,13 +33,13 @@ constexpr int kStSmemTarget = 112 * 1024;
 
 struct Launch {
   cudaStream_t st;
-  bool dry;                                    // only raise the shared-memory limits
+  bool* fits = nullptr;                        // dry run: raise the shared-memory limits, note what does not fit
   bool pdl = true;
 };
 
 template <typename... KArgs, typename... Args>
 void go(const Launch& l, void (*kernel)(KArgs...), int grid, int block, size_t smem, Args&&... args) {
-  if (l.dry) { raise_dyn_smem(kernel, smem); return; }
+  if (l.fits) { raise_dyn_smem(kernel, smem); return; }
   if (l.pdl) launch_pdl(kernel, dim3(grid), dim3(block), smem, l.st, std::forward<Args>(args)...);
   else kernel<<<grid, block, smem, l.st>>>(std::forward<Args>(args)...);
 }
@@ -88,10 +88,13 @@ void launch_gemv(const Launch& l, const DecodeArgs& a, const StepPlan& pl, StepG
     g.nslots = 2;
   }
   g.sm = st_smem(g, a.ncols, a.nterms);
-  B2_CHECK((size_t)g.sm.total <= pl.smem_optin, kUnimplemented, "the decode step needs more shared memory than the device offers");
   const int T = kStThreads / st_cols(a.ncols);
-  const int nv = (g.kmax / 4 + T - 1) / T;
-  B2_CHECK(nv <= 12, kUnimplemented, "the decode step does not take vectors this long with so many sessions");
+  const int nv = (g.kmax / 4 + T - 1) / T;                               // float4 of a vector per thread
+  if ((size_t)g.sm.total > pl.smem_optin || nv > 12) {
+    B2_CHECK(l.fits != nullptr, kInternal, "the decode step does not fit, but was planned");
+    *l.fits = false;
+    return;
+  }
   if (nv <= 1) launch_gemv_cp<PRO, EPI, 1>(l, a, g);
   else if (nv <= 4) launch_gemv_cp<PRO, EPI, 4>(l, a, g);
   else launch_gemv_cp<PRO, EPI, 12>(l, a, g);
@@ -125,7 +128,7 @@ int run(Launch l, const DecodeArgs& a, const StepPlan& pl, const LayerWeights* l
   const ModelDims& d = a.dims;
   const int KTd = d.d / 64, KTo = d.nq() / 64, KTf = d.ffn / 64;
   int n = 0;
-  const int nl = l.dry ? 1 : d.n_layers;
+  const int nl = l.fits ? 1 : d.n_layers;
   auto resid = [&](StepGemv& g, const float* parts, int nparts, int from, const float* g_post, const float* g_pre) {
     g.parts = parts;
     g.nparts = nparts;
@@ -145,7 +148,7 @@ int run(Launch l, const DecodeArgs& a, const StepPlan& pl, const LayerWeights* l
     q.bar = 5 * i;
     launch_gemv<kStResid, kStPlain>(l, a, pl, q);
     l.pdl = true;
-    for (int glob = l.dry ? 0 : L.is_global; glob <= (l.dry ? 1 : L.is_global); ++glob) {
+    for (int glob = l.fits ? 0 : L.is_global; glob <= (l.fits ? 1 : L.is_global); ++glob) {
       StepAttn t{};
       t.qkv = a.qkv; t.g_q = L.g_q; t.g_k = L.g_k; t.cosT = a.rope_cos[glob]; t.sinT = a.rope_sin[glob]; t.kv = kv[i];
       t.is_global = glob; t.nsplit = pl.nsplit[glob]; t.part_o = pl.part_o; t.part_ml = pl.part_ml;
@@ -158,7 +161,7 @@ int run(Launch l, const DecodeArgs& a, const StepPlan& pl, const LayerWeights* l
     o.part_o = pl.part_o; o.part_ml = pl.part_ml; o.nsplit = pl.nsplit[L.is_global ? 1 : 0]; o.is_global = L.is_global;
     o.bar = 5 * i + 2;
     launch_gemv<kStCombine, kStPlain>(l, a, pl, o);
-    if (reduce && !l.dry) reduce(ctx, pl.opart, (size_t)pl.o_slices * a.ncols * d.d);
+    if (reduce) reduce(ctx, pl.opart, (size_t)pl.o_slices * a.ncols * d.d);
     StepGemv gu{};
     gu.w = L.wgu; gu.wscale = L.sgu; gu.tiles = 2 * d.ffn / 16; gu.KT = KTd; gu.slices = 1; gu.y = a.act;
     resid(gu, pl.opart, pl.o_slices, x, L.g_post_attn, L.g_pre_ffn);
@@ -171,7 +174,7 @@ int run(Launch l, const DecodeArgs& a, const StepPlan& pl, const LayerWeights* l
     dn.w = L.wdown; dn.wscale = L.sdown; dn.tiles = d.d / 16; dn.KT = KTf; dn.slices = pl.down_slices; dn.y = pl.fpart; dn.act = a.act;
     dn.bar = 5 * i + 4;
     launch_gemv<kStAct, kStPlain>(l, a, pl, dn);
-    if (reduce && !l.dry) reduce(ctx, pl.fpart, (size_t)pl.down_slices * a.ncols * d.d);
+    if (reduce) reduce(ctx, pl.fpart, (size_t)pl.down_slices * a.ncols * d.d);
     n += 5;
   }
   StepGemv h{};
@@ -180,19 +183,23 @@ int run(Launch l, const DecodeArgs& a, const StepPlan& pl, const LayerWeights* l
   l.pdl = !reduce;
   h.bar = 5 * d.n_layers;
   launch_gemv<kStResid, kStHead>(l, a, pl, h);
-  if (!l.dry) B2_CUDA(cudaGetLastError());
+  if (!l.fits) B2_CUDA(cudaGetLastError());
   return n + 1;
 }
 
 }  // namespace
 
-void step_prepare(const DecodeArgs& a, const StepPlan& pl, const LayerWeights* layers, const LayerKv* kv) {
-  run(Launch{nullptr, true}, a, pl, layers, kv, nullptr, nullptr);
+bool step_prepare(const DecodeArgs& a, const StepPlan& pl, const LayerWeights* layers, const LayerKv* kv) {
+  bool fits = true;
+  Launch l{nullptr};
+  l.fits = &fits;
+  run(l, a, pl, layers, kv, nullptr, nullptr);
+  return fits;
 }
 
 int step_launch(cudaStream_t st, const DecodeArgs& a, const StepPlan& pl, const LayerWeights* layers, const LayerKv* kv, StepReduceFn reduce,
                 void* reduce_ctx) {
-  return run(Launch{st, false}, a, pl, layers, kv, reduce, reduce_ctx);
+  return run(Launch{st}, a, pl, layers, kv, reduce, reduce_ctx);
 }
 
 }  // namespace b200lm

@@ -947,8 +947,9 @@ typedef void (*StepReduceFn)(void* ctx, float* buf, size_t count);
 
 // Fills in the splits; false when the model's geometry does not fit the kernels.
 bool step_plan(const ModelDims& d, int sms, size_t smem_optin, int max_tokens, StepPlan* pl);
-// Raises the kernels' shared-memory limits (outside any capture).
-void step_prepare(const DecodeArgs& a, const StepPlan& pl, const LayerWeights* layers, const LayerKv* kv);
+// Raises the kernels' shared-memory limits (outside any capture); false when a projection of a.ncols sessions does not
+// fit: a vector longer than twelve float4 per thread, or too long for shared memory.
+bool step_prepare(const DecodeArgs& a, const StepPlan& pl, const LayerWeights* layers, const LayerKv* kv);
 // Queues one step of a.ncols sessions; returns the number of launches.
 int step_launch(cudaStream_t st, const DecodeArgs& a, const StepPlan& pl, const LayerWeights* layers, const LayerKv* kv, StepReduceFn reduce,
                 void* reduce_ctx);

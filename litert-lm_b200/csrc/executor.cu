@@ -525,51 +525,46 @@ std::unique_ptr<Executor> Executor::create(std::shared_ptr<Model> model, const B
     e->wide_ticket = reinterpret_cast<int*>(e->alloc(sizeof(int) * (size_t)e->n_sessions * d.hkv, true));
   }
   a.advance = 1;
-  if (e->decode_mode == B200LM_DECODE_PERSISTENT_BASIC) {
-    e->dec_smem = dec_smem_bytes(d, e->n_sessions);
-    B2_CHECK(e->dec_smem <= (size_t)prop.sharedMemPerBlockOptin, kUnimplemented,
-             "the persistent decode kernel needs more shared memory than the device offers");
-    raise_dyn_smem(decode_persistent_kernel, (size_t)(e->dec_smem));
-  }
-  if (e->decode_mode == B200LM_DECODE_PERSISTENT) {
-    // staging halves take what shared memory the activation staging leaves, up to 96 KiB each
-    size_t fixed = stream_fixed_bytes(d, e->n_sessions);
-    long room = ((long)prop.sharedMemPerBlockOptin - (long)fixed - 2048) / 2;   // margin: static shared memory
-    int half = (int)std::min<long>(room, 96 * 1024) / 1024 * 1024;
-    bool ok = half > 0 && stream_model_fits(d, a.o_slices, a.down_slices, half) && prop.cooperativeLaunch;
-    for (float b : model->attn_bound) ok = ok && b <= kFaMaxBound;   // its attention shifts the softmax by the bound
-    if (ok) {
-      e->stream_half = half;
-      e->stream_smem = fixed + 2 * (size_t)half;
-      const void* kfn = decode_stream_kernel_for(d);
-      raise_dyn_smem(kfn, (size_t)(e->stream_smem));
-      cudaFuncAttributes fa;
-      B2_CUDA(cudaFuncGetAttributes(&fa, kfn));
-      int occ = (size_t)fa.maxThreadsPerBlock >= (size_t)kStreamThreads ? 1 : 0;
-      ok = occ >= 1;
+  // Which kernels carry a step, and how many sessions at once.  The chain gives way to the persistent kernel, that to the
+  // chain with the sessions of a group one after another, that to one kernel per phase; the persistent kernels give way
+  // to the chain.  No persistent kernel under tensor parallelism, whose collectives run between the phases.
+  e->step_cols = e->n_sessions;
+  if (e->decode_mode != B200LM_DECODE_WIDE) {
+    const bool coop = prop.cooperativeLaunch && cfg.tp_world <= 1;
+    bool placed = false;
+    if (e->decode_mode == B200LM_DECODE_PERSISTENT) placed = e->plan_persistent(coop);
+    if (e->decode_mode == B200LM_DECODE_PERSISTENT_BASIC) {
+      e->dec_smem = dec_smem_bytes(d, e->n_sessions);
+      B2_CHECK(e->dec_smem <= e->smem_optin, kUnimplemented, "the persistent decode kernel needs more shared memory than the device offers");
+      raise_dyn_smem(decode_persistent_kernel, e->dec_smem);
+      int occ = 0;
+      B2_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, decode_persistent_kernel, kDecThreads, e->dec_smem));
+      placed = occ >= 1 && coop;
     }
-    if (!ok) e->decode_mode = B200LM_DECODE_CHAINED;
+    if (!placed) placed = e->chain = e->plan_chain();
+    if (!placed && e->decode_mode == B200LM_DECODE_CHAINED && e->plan_persistent(coop)) {
+      placed = true;
+      e->decode_mode = B200LM_DECODE_PERSISTENT;
+    }
+    if (!placed && e->n_sessions > 1) {
+      e->step_cols = 1;
+      placed = e->chain = e->plan_chain();
+    }
+    if (e->chain && e->decode_mode != B200LM_DECODE_PHASE_KERNELS) e->decode_mode = B200LM_DECODE_CHAINED;
+    if (!placed) {
+      e->dec_smem = dec_smem_bytes(d, 1);
+      B2_CHECK(e->dec_smem <= e->smem_optin, kUnimplemented, "decode kernels need more shared memory than the device offers");
+      raise_dyn_smem(decode_phase_kernel, e->dec_smem);
+      e->decode_mode = B200LM_DECODE_PHASE_KERNELS;
+    }
   }
-  if (e->decode_mode == B200LM_DECODE_PHASE_KERNELS || e->decode_mode == B200LM_DECODE_CHAINED) {
+  if (e->chain) {
     StepPlan& sp = e->step;
-    B2_CHECK(step_plan(d, e->n_sms, e->smem_optin, e->max_num_tokens, &sp), kUnimplemented,
-             "the decode step's kernels do not take this model's geometry");
     sp.part_o = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.hkv * sp.max_splits * G * d.hd, true));
     sp.part_ml = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.hkv * sp.max_splits * G * 2, true));
     sp.opart = reinterpret_cast<float*>(e->alloc(sizeof(float) * sp.o_slices * kMaxCols * d.d, true));
     sp.fpart = reinterpret_cast<float*>(e->alloc(sizeof(float) * sp.down_slices * kMaxCols * d.d, true));
     sp.ticket = reinterpret_cast<int*>(e->alloc(sizeof(int), true));
-    for (int nc : {1, e->n_sessions}) {
-      DecodeArgs p = a;
-      p.ncols = nc;
-      p.nterms = nc * 3 <= kQCols ? 3 : kQCols / nc;
-      step_prepare(p, sp, model->layers_host.data(), e->kv_host.data());
-    }
-  }
-  if (e->decode_mode == B200LM_DECODE_PERSISTENT_BASIC) {
-    int occ = 0;
-    B2_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, decode_persistent_kernel, kDecThreads, e->dec_smem));
-    B2_CHECK(occ >= 1 && prop.cooperativeLaunch, kUnimplemented, "the persistent decode kernel does not fit this device");
   }
   // ---- prefill buffers (rows padded to whole 128-token tiles, zero-filled)
   e->t_max = d.buckets[0];
@@ -625,6 +620,36 @@ std::unique_ptr<Executor> Executor::create(std::shared_ptr<Model> model, const B
   for (int i = 0; i < kTokRing; ++i) B2_CUDA(cudaEventCreateWithFlags(&e->tok_ring_done[i], cudaEventDisableTiming));
   B2_CUDA(cudaDeviceSynchronize());
   return e;
+}
+
+bool Executor::plan_chain() {
+  if (!step_plan(model->dims, n_sms, smem_optin, max_num_tokens, &step)) return false;
+  for (int nc : {1, step_cols}) {
+    DecodeArgs p = dargs;
+    p.ncols = nc;
+    p.nterms = nc * 3 <= kQCols ? 3 : kQCols / nc;
+    if (!step_prepare(p, step, model->layers_host.data(), kv_host.data())) return false;
+  }
+  return true;
+}
+
+bool Executor::plan_persistent(bool cooperative) {
+  const ModelDims& d = model->dims;
+  if (!cooperative) return false;
+  for (float b : model->attn_bound)
+    if (b > kFaMaxBound) return false;              // its attention shifts the softmax by the bound
+  // staging halves take what shared memory the activation staging leaves, up to 96 KiB each
+  const size_t fixed = stream_fixed_bytes(d, n_sessions);
+  const long room = ((long)smem_optin - (long)fixed - 2048) / 2;   // margin: static shared memory
+  const int half = (int)std::min<long>(room, 96 * 1024) / 1024 * 1024;
+  if (half <= 0 || !stream_model_fits(d, dargs.o_slices, dargs.down_slices, half)) return false;
+  const void* kfn = decode_stream_kernel_for(d);
+  stream_half = half;
+  stream_smem = fixed + 2 * (size_t)half;
+  raise_dyn_smem(kfn, stream_smem);
+  cudaFuncAttributes fa;
+  B2_CUDA(cudaFuncGetAttributes(&fa, kfn));
+  return fa.maxThreadsPerBlock >= kStreamThreads;
 }
 
 void Executor::tp_allreduce(float* buf, size_t count) {
@@ -851,7 +876,7 @@ void Executor::launch_decode_steps(int nsteps, int ncols, int first_session) {
     launch_wide_steps(nsteps, ncols, first_session);
     return;
   }
-  if (decode_mode == B200LM_DECODE_PERSISTENT || decode_mode == B200LM_DECODE_PERSISTENT_BASIC) {
+  if (!chain) {
     DecodeArgs a = dargs;
     a.ncols = ncols;
     a.nterms = ncols * 3 <= kQCols ? 3 : kQCols / ncols;      // int8 terms per activation: 3, or 2 with 3-4 sessions
@@ -860,6 +885,10 @@ void Executor::launch_decode_steps(int nsteps, int ncols, int first_session) {
     const int cap = std::max(1, ncta / (ncols * d.hkv));
     a.n_attn_splits_local = std::min(a.n_attn_splits_local, cap);
     a.n_attn_splits_global = std::min(a.n_attn_splits_global, cap);
+    if (decode_mode == B200LM_DECODE_PHASE_KERNELS) {
+      launch_phases(nsteps, a);
+      return;
+    }
     unsigned epoch0 = barrier_epoch;
     if (decode_mode == B200LM_DECODE_PERSISTENT) {
       int half = stream_half;
@@ -876,6 +905,23 @@ void Executor::launch_decode_steps(int nsteps, int ncols, int first_session) {
     return;
   }
   launch_chain(nsteps, ncols, first_session);
+}
+
+// The phases of the persistent kernel launched one by one, with the ranks' partial O and down outputs summed in between.
+void Executor::launch_phases(int nsteps, const DecodeArgs& a) {
+  const ModelDims& d = model->dims;
+  for (int s = 0; s < nsteps; ++s) {
+    for (int li = 0; li < d.n_layers; ++li)
+      for (int ph = kPhQkv; ph <= kPhDown; ++ph) {
+        decode_phase_kernel<<<n_sms, kDecThreads, dec_smem, stream>>>(a, ph, li);
+        if (tp_world > 1 && ph == kPhOproj) tp_allreduce(a.opart, (size_t)a.o_slices * a.ncols * d.d);
+        if (tp_world > 1 && ph == kPhDown) tp_allreduce(a.fpart, (size_t)a.down_slices * a.ncols * d.d);
+      }
+    decode_phase_kernel<<<n_sms, kDecThreads, dec_smem, stream>>>(a, kPhHead, 0);
+    decode_phase_kernel<<<1, kDecThreads, dec_smem, stream>>>(a, kPhArgmax, n_sms);
+  }
+  B2_CUDA(cudaGetLastError());
+  launches += (int64_t)nsteps * (5 * d.n_layers + 2);
 }
 
 // The chain of step kernels for sessions [first, first + ncols): one CUDA graph per step.  Under tensor parallelism
@@ -1098,6 +1144,16 @@ void Executor::decode_tokens_batch(int nsteps, int* out_ids) {
     B2_CHECK(pending != -1, kInvalidArgument, "No id available to be decoded (session " + std::to_string(sn) + ").");
     B2_CHECK(step + nsteps <= max_num_tokens, kInvalidArgument, "Maximum kv-cache size reached.");
   }
+  if (step_cols < n_sessions) {                    // the step's kernels carry one session of this geometry at a time
+    std::vector<int> ids(nsteps);
+    for (int sn = 0; sn < n_sessions; ++sn) {
+      select_session(sn);
+      decode_tokens(nsteps, ids.data());
+      for (int s = 0; out_ids && s < nsteps; ++s) out_ids[(size_t)s * n_sessions + sn] = ids[s];
+    }
+    select_session(keep);
+    return;
+  }
   for (int sn = 0; sn < n_sessions; ++sn) {
     select_session(sn);
     tok[sn] = take_decode_id(nullptr);
@@ -1126,9 +1182,8 @@ void Executor::decode_tokens_batch(int nsteps, int* out_ids) {
 void Executor::trace_decode_step(int* out_id, long long* stamps, long long capacity, int* n_barriers, int* n_cta,
                                  int* khz) {
   const ModelDims& d = model->dims;
-  B2_CHECK(decode_mode == B200LM_DECODE_PERSISTENT || decode_mode == B200LM_DECODE_PERSISTENT_BASIC ||
-               decode_mode == B200LM_DECODE_CHAINED || decode_mode == B200LM_DECODE_PHASE_KERNELS,
-           kFailedPrecondition, "the wide decode mode has no timeline");
+  B2_CHECK(chain || decode_mode == B200LM_DECODE_PERSISTENT || decode_mode == B200LM_DECODE_PERSISTENT_BASIC, kFailedPrecondition,
+           "the wide decode mode and one kernel per phase have no timeline");
   B2_CUDA(cudaSetDevice(device));
   const int nb = 5 * d.n_layers + 2;
   const long long need = (long long)nb * n_sms * 10;     // 2 barrier stamps + 8 in-phase stamps
@@ -1154,7 +1209,7 @@ void Executor::trace_decode_step(int* out_id, long long* stamps, long long capac
   int rate = 0;
   B2_CUDA(cudaDeviceGetAttribute(&rate, cudaDevAttrClockRate, device));
   // the chain's kernels stamp nanoseconds: their CTAs move between SMs, whose cycle counters differ
-  *khz = decode_mode == B200LM_DECODE_PHASE_KERNELS || decode_mode == B200LM_DECODE_CHAINED ? 1000000 : rate;
+  *khz = chain ? 1000000 : rate;
 }
 
 void Executor::reset() {

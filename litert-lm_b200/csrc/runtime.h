@@ -130,9 +130,14 @@ class Executor {
   NcclApi::Comm tp_comm = nullptr;
   unsigned barrier_epoch = 0;
   long long* trace_dev = nullptr;
+  bool chain = false;               // the chain of step kernels carries the steps
   StepPlan step;                    // chain of step kernels (decode_step.cuh)
   std::map<std::pair<int, int>, cudaGraphExec_t> step_graphs;   // one step, keyed by (sessions, first session)
   void launch_chain(int nsteps, int ncols, int first);
+  int step_cols = 1;                // sessions that one step carries: all of them, or one
+  bool plan_chain();                                // false: it does not take the model's geometry with step_cols sessions
+  bool plan_persistent(bool cooperative);           // likewise, the streaming persistent kernel, with all sessions
+  void launch_phases(int nsteps, const DecodeArgs& a);
   // wide lockstep decode (B200LM_DECODE_WIDE)
   WideState wide{};
   float* wide_part = nullptr;       // key-split partial states of the wide attention

@@ -5,7 +5,7 @@ import dataclasses
 import numpy as np
 import pytest
 
-from conftest import seeded_ids
+from conftest import logits_close, seeded_ids
 
 pytestmark = pytest.mark.gpu
 
@@ -69,3 +69,44 @@ def test_timeline_covers_every_kernel_of_the_step(pkg, models):
     for k in range(5 * cfg.n_layers + 1):
         p = pts[k][pts[k][:, 4] > 0]
         assert len(p) and (np.diff(p[:, :5], axis=1) >= 0).all(), k
+
+
+@pytest.mark.parametrize("d_model,ffn,heads,sessions,mode", [
+    (64, 6208, (4, 1, 256), 2, 2),      # ffn = 64 * 97 has no K split: too long for two sessions, the persistent kernel
+    (64, 6208, (4, 1, 256), 4, 4),      # too much staging for that with four: the chain, one session after another
+    (6208, 64, (4, 1, 256), 2, 4),      # a residual that the persistent kernel does not take either
+    (64, 24896, (2, 2, 32), 1, 1),      # 64 * 389, too long for one session: one kernel per phase
+])
+def test_geometries_beyond_the_chain_have_a_fallback(pkg, orc, mio, d_model, ffn, heads, sessions, mode):
+    cfg = dataclasses.replace(mio.config_small(), n_layers=2, d_model=d_model, ffn=ffn, n_q_heads=heads[0], n_kv_heads=heads[1],
+                              head_dim=heads[2], vocab=512, max_ctx=256)
+    record = mio.build_weights_record(cfg)
+    ex = pkg.B200LlmExecutor(mio.export_model_litertlm(cfg, record), n_sessions=sessions)
+    assert ex.GetDecodeMode() == mode
+    prompts = [seeded_ids(60 + i, cfg.vocab, 20 + 9 * i) for i in range(sessions)]
+    for i, p in enumerate(prompts):
+        ex.PrefillSession(i, p)
+    got = ex.DecodeTokensBatch(3)
+    model = orc.OracleModel(record)
+    for i, p in enumerate(prompts):
+        ref = orc.OracleExecutor(model)
+        assert ref.prefill(p) == 0
+        for step in range(3):                # teacher-forced: the device's id is one the oracle puts at its best, within the prefill's tolerance
+            rc, want = ref.decode_logits()
+            assert rc == 0 and want[got[step, i]] >= want.max() - 2e-2 * (want.max() - want.min()), (i, step)
+            assert ref.prefill(got[step:step + 1, i].copy()) == 0
+        ex.SelectSession(i)
+        rc, want = ref.decode_logits()
+        cos, err = logits_close(ex.DecodeLogits(), want)
+        assert rc == 0 and cos >= 0.999 and err <= 2e-2, (i, cos, err)
+
+
+def test_every_requested_mode_finds_kernels(pkg, mio):
+    cfg = dataclasses.replace(mio.config_small(), n_layers=1, d_model=64, ffn=6208, vocab=512, max_ctx=256)
+    img = image(mio, cfg)
+    want = {(pkg.DECODE_PHASE_KERNELS, 4): 1, (pkg.DECODE_PERSISTENT, 1): 2, (pkg.DECODE_PERSISTENT, 4): 4, (pkg.DECODE_PERSISTENT_BASIC, 2): 3,
+            (pkg.DECODE_CHAINED, 1): 4, (pkg.DECODE_CHAINED, 2): 2}
+    for (mode, n), runs in want.items():
+        assert pkg.B200LlmExecutor(img, n_sessions=n, decode_mode=mode).GetDecodeMode() == runs, (mode, n)
+    with pytest.raises(Exception, match="shared memory"):
+        pkg.B200LlmExecutor(img, n_sessions=4, decode_mode=pkg.DECODE_PERSISTENT_BASIC)
