@@ -353,7 +353,10 @@ static int round_up(int v, int a) { return (v + a - 1) / a * a; }
 Executor::~Executor() {
   cudaSetDevice(device);
   if (stream) cudaStreamSynchronize(stream);
-  for (auto& g : step_graphs) cudaGraphExecDestroy(g.second);
+  for (auto& g : step_graphs) {
+    if (g.second.graph) cudaGraphDestroy(g.second.graph);
+    if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
+  }
   for (auto& g : wide_graphs) cudaGraphExecDestroy(g.second);
   for (cudaEvent_t ev : logit_part)
     if (ev) cudaEventDestroy(ev);
@@ -924,7 +927,7 @@ void Executor::launch_phases(int nsteps, const DecodeArgs& a) {
   launches += (int64_t)nsteps * (5 * d.n_layers + 2);
 }
 
-// The chain of step kernels for sessions [first, first + ncols): one CUDA graph per step.  Under tensor parallelism
+// The chain of step kernels for sessions [first, first + ncols).  Under tensor parallelism
 // the ranks' partial O and down outputs are summed between the kernels, launch by launch.
 void Executor::launch_chain(int nsteps, int ncols, int first) {
   DecodeArgs a = dargs;
@@ -941,27 +944,38 @@ void Executor::launch_chain(int nsteps, int ncols, int first) {
     for (int s = 0; s < nsteps; ++s) launches += step_launch(stream, a, step, L, kv_host.data(), nullptr, nullptr);
     return;
   }
-  auto key = std::make_pair(ncols, first);
-  auto it = step_graphs.find(key);
-  if (it == step_graphs.end()) {
-    cudaGraph_t graph;
-    B2_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    try {
-      step_launch(stream, a, step, L, kv_host.data(), nullptr, nullptr);
-    } catch (...) {
-      cudaGraph_t dead = nullptr;
-      cudaStreamEndCapture(stream, &dead);
-      if (dead) cudaGraphDestroy(dead);
-      throw;
+  // Replaying the step as one graph saves 45 of 640 us (131 launches of the 1B model), but the host takes 75 us to capture
+  // it, 270 to instantiate it and 220 to upload it, and the first call of every executor used to wait for all of that
+  // (1102 us for the first DecodeLogits against 652 now).  So the steps start as plain launches, which take the host 430
+  // us, and each part is done while the GPU runs one of them: an executor that decodes one step never makes a graph.
+  StepGraph& g = step_graphs[std::make_pair(ncols, first)];
+  for (int s = 0; s < nsteps; ++s) {
+    if (g.steps >= 4 && g.exec) {
+      B2_CUDA(cudaGraphLaunch(g.exec, stream));
+      launches += 5 * model->dims.n_layers + 1;
+      continue;
     }
-    B2_CUDA(cudaStreamEndCapture(stream, &graph));
-    cudaGraphExec_t exec = nullptr;
-    B2_CUDA(cudaGraphInstantiate(&exec, graph, 0));
-    cudaGraphDestroy(graph);
-    it = step_graphs.emplace(key, exec).first;
+    launches += step_launch(stream, a, step, L, kv_host.data(), nullptr, nullptr);
+    ++g.steps;
+    if (g.steps == 2) {
+      B2_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+      try {
+        step_launch(stream, a, step, L, kv_host.data(), nullptr, nullptr);
+      } catch (...) {
+        cudaGraph_t dead = nullptr;
+        cudaStreamEndCapture(stream, &dead);
+        if (dead) cudaGraphDestroy(dead);
+        throw;
+      }
+      B2_CUDA(cudaStreamEndCapture(stream, &g.graph));
+    } else if (g.steps == 3 && g.graph) {
+      B2_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
+      cudaGraphDestroy(g.graph);
+      g.graph = nullptr;
+    } else if (g.steps == 4 && g.exec) {
+      B2_CUDA(cudaGraphUpload(g.exec, stream));
+    }
   }
-  for (int s = 0; s < nsteps; ++s) B2_CUDA(cudaGraphLaunch(it->second, stream));
-  launches += (int64_t)nsteps * (5 * model->dims.n_layers + 1);
 }
 
 // One wide step for sessions [first, first + nb): the token rows of the GEMMs are the sessions.

@@ -132,7 +132,12 @@ class Executor {
   long long* trace_dev = nullptr;
   bool chain = false;               // the chain of step kernels carries the steps
   StepPlan step;                    // chain of step kernels (decode_step.cuh)
-  std::map<std::pair<int, int>, cudaGraphExec_t> step_graphs;   // one step, keyed by (sessions, first session)
+  struct StepGraph {
+    int steps = 0;                  // taken by plain launches so far
+    cudaGraph_t graph = nullptr;    // captured, not yet instantiated
+    cudaGraphExec_t exec = nullptr;
+  };
+  std::map<std::pair<int, int>, StepGraph> step_graphs;         // one step, keyed by (sessions, first session)
   void launch_chain(int nsteps, int ncols, int first);
   int step_cols = 1;                // sessions that one step carries: all of them, or one
   bool plan_chain();                                // false: it does not take the model's geometry with step_cols sessions
