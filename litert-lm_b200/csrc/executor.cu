@@ -927,6 +927,36 @@ void Executor::launch_phases(int nsteps, const DecodeArgs& a) {
   launches += (int64_t)nsteps * (5 * d.n_layers + 2);
 }
 
+// What `body` queues on `stream`, as a graph.  It is recorded on a stream made for that: the caller's may be the legacy
+// default stream, which cannot be captured, or a blocking one, whose capture would make other threads' work on the
+// default stream fail.
+template <typename Body>
+cudaGraph_t Executor::capture(const Body& body) {
+  cudaStream_t rec = nullptr;
+  cudaGraph_t graph = nullptr;
+  B2_CUDA(cudaStreamCreateWithFlags(&rec, cudaStreamNonBlocking));
+  std::swap(stream, rec);
+  auto done = [&]() {
+    std::swap(stream, rec);
+    cudaStreamDestroy(rec);
+  };
+  try {
+    B2_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+    try {
+      body();
+    } catch (...) {
+      if (cudaStreamEndCapture(stream, &graph) == cudaSuccess && graph) cudaGraphDestroy(graph);
+      throw;
+    }
+    B2_CUDA(cudaStreamEndCapture(stream, &graph));
+  } catch (...) {
+    done();
+    throw;
+  }
+  done();
+  return graph;
+}
+
 // The chain of step kernels for sessions [first, first + ncols).  Under tensor parallelism
 // the ranks' partial O and down outputs are summed between the kernels, launch by launch.
 void Executor::launch_chain(int nsteps, int ncols, int first) {
@@ -958,16 +988,7 @@ void Executor::launch_chain(int nsteps, int ncols, int first) {
     launches += step_launch(stream, a, step, L, kv_host.data(), nullptr, nullptr);
     ++g.steps;
     if (g.steps == 2) {
-      B2_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-      try {
-        step_launch(stream, a, step, L, kv_host.data(), nullptr, nullptr);
-      } catch (...) {
-        cudaGraph_t dead = nullptr;
-        cudaStreamEndCapture(stream, &dead);
-        if (dead) cudaGraphDestroy(dead);
-        throw;
-      }
-      B2_CUDA(cudaStreamEndCapture(stream, &g.graph));
+      g.graph = capture([&] { step_launch(stream, a, step, L, kv_host.data(), nullptr, nullptr); });
     } else if (g.steps == 3 && g.graph) {
       B2_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
       cudaGraphDestroy(g.graph);
@@ -1033,17 +1054,7 @@ void Executor::launch_wide_steps(int nsteps, int nb, int first) {
   auto it = wide_graphs.find(key);
   if (it == wide_graphs.end()) {
     const int64_t before = launches;
-    cudaGraph_t graph;
-    B2_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    try {
-      wide_step(nb, first);
-    } catch (...) {
-      cudaGraph_t dead = nullptr;
-      cudaStreamEndCapture(stream, &dead);
-      if (dead) cudaGraphDestroy(dead);
-      throw;
-    }
-    B2_CUDA(cudaStreamEndCapture(stream, &graph));
+    cudaGraph_t graph = capture([&] { wide_step(nb, first); });
     cudaGraphExec_t exec = nullptr;
     B2_CUDA(cudaGraphInstantiate(&exec, graph, 0));
     cudaGraphDestroy(graph);

@@ -138,6 +138,8 @@ class Executor {
     cudaGraphExec_t exec = nullptr;
   };
   std::map<std::pair<int, int>, StepGraph> step_graphs;         // one step, keyed by (sessions, first session)
+  template <typename Body>
+  cudaGraph_t capture(const Body& body);
   void launch_chain(int nsteps, int ncols, int first);
   int step_cols = 1;                // sessions that one step carries: all of them, or one
   bool plan_chain();                                // false: it does not take the model's geometry with step_cols sessions

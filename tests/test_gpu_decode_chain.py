@@ -134,3 +134,15 @@ def test_the_first_decode_call_does_not_wait_for_a_graph(pkg, mio):
     least = np.min(times, axis=0)
     assert least[0] <= 1.5 * least[4:].min(), (least * 1e6).round().tolist()
     assert all(np.array_equal(x, logits[0]) for x in logits)
+
+
+@pytest.mark.parametrize("sessions", [1, 3, 6])               # the chain, and the wide step
+def test_the_callers_stream_may_be_the_default_stream(pkg, models, sessions):
+    cfg, _, img = models("small")
+    out = []
+    for stream in (0, 1):                                     # an own stream; cudaStreamLegacy, which cannot be captured
+        ex = pkg.B200LlmExecutor(img, n_sessions=sessions, stream=stream)
+        for i in range(sessions):
+            ex.PrefillSession(i, seeded_ids(70 + i, cfg.vocab, 25 + 7 * i))
+        out.append((ex.DecodeTokensBatch(8), ex.DecodeLogits().copy()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
