@@ -86,8 +86,9 @@ int B200LmOps_AttentionPrefillTc(int32_t device, const float* q, const float* k,
  * GPU memory was handed out completely at start-up.  The ordinary entry point
  * above allocates scratch for the per-split partial results on every call;
  * this one keeps them (with the query positions and an error word) in one
- * fixed 8 MiB device array that is part of the library image, so every GPU
- * that loads the library holds those 8 MiB until the process ends.
+ * fixed 8 MiB device array that is part of the library image (and 129 KiB of
+ * counters beside it), so every GPU that loads the library holds those until
+ * the process ends.
  *
  * All pointers are DEVICE memory owned by the caller:
  *   q_dev          [batch] rows of (hq + 2*hkv)*hd floats, the layout of a fused
@@ -100,25 +101,32 @@ int B200LmOps_AttentionPrefillTc(int32_t device, const float* q, const float* k,
  * queued on `stream` (NULL: the default stream) and the call returns without
  * waiting.
  *
+ * With all four data pointers on 16-byte boundaries the kernel of
+ * csrc/attn_mma.cuh runs, which reads the cache once for the whole batch and
+ * picks its own number of splits; nsplit then only enters the size check below.
+ * Otherwise the split kernel of csrc/decode_ops.cuh runs with nsplit splits.
+ *
  * Limits: batch <= 16368 and batch*hq*nsplit*(hd+2)*4 bytes <= 8 MiB - 64 KiB;
  * larger requests are rejected with InvalidArgument.  The first call on a
  * device looks up the array's address and sets a kernel attribute; make that
  * first call before starting any stream capture.  All calls on a device share
- * the array, which keeps what the last call left in it (the call itself resets
- * the one word that must start at zero); two calls whose kernels overlap on
- * the GPU -- different streams, no ordering between them -- race on it.  The
- * caller's current device is left as it was.  The per-device set-up is done
- * under a lock, so first calls from several threads are safe. */
+ * the array, which keeps what the last call left in it; two calls whose kernels
+ * overlap on the GPU -- different streams, no ordering between them -- race on
+ * it, which spoils the results of those calls and of no others.  The error word
+ * is only written by a call that fails and stays until the status call below has
+ * reported it.  The caller's current device is left as it was.  The per-device
+ * set-up is done under a lock, so first calls from several threads are safe. */
 int B200LmOps_AttentionDecodeStatic(int32_t device, const float* q_dev, const void* k_pages_dev,
                                     const void* v_pages_dev, const int32_t* page_table_dev, int32_t batch, int32_t s,
                                     int32_t hq, int32_t hkv, int32_t hd, int32_t window, int32_t kv_bf16,
                                     int32_t nsplit, float* out_dev, void* stream, char** err);
 
 /* Status of the work queued by B200LmOps_AttentionDecodeStatic on `stream`:
- * waits for the stream, then reads the error word its kernels keep in the
- * static array (no allocation either).  Returns OK, or InvalidArgument when a
- * query position lay outside the cache; *device_error (optional) receives the
- * raw word.  No counterpart in the reference. */
+ * waits for the stream, then reads and clears the error word of the static
+ * array (no allocation either).  Returns OK when no call since the last status
+ * call failed, InvalidArgument when a query position lay outside the cache,
+ * DeadlineExceeded when a bounded device-side wait gave up; *device_error
+ * (optional) receives the raw word.  No counterpart in the reference. */
 int B200LmOps_AttentionDecodeStaticStatus(int32_t device, void* stream, int32_t* device_error, char** err);
 
 #ifdef __cplusplus

@@ -33,11 +33,11 @@ static __device__ __align__(256) unsigned char g_attn_static_scratch[kStaticScra
 // Tickets of attn_shared_kernel (split_ticket.h), 128 KiB; zero whenever no call is on the GPU.
 static __device__ unsigned g_attn_static_tickets[kTicketWords];
 
-// Header layout: int[0] = error word, int[16 + i] = position of query i.
+// Header layout: int[0] = error word (zero in the image, cleared by the status call that reports it), int[16 + i] =
+// position of query i.
 __global__ void static_scratch_prepare_kernel(int nq, int pos) {
   int* hdr = reinterpret_cast<int*>(g_attn_static_scratch);
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) hdr[0] = 0;                   // the error word must start at zero
   if (i < nq) hdr[16 + i] = pos;
 }
 
