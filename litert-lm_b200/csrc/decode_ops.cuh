@@ -87,7 +87,6 @@ struct DecodeArgs {
   int* amax_idx;        // [n_cta][ncols]
   int* step_tokens;     // [capacity][ncols] arg-max of every step since steps_done was reset
   int step_capacity;
-  int advance;          // 1: feed arg-max back as next token and bump pos (device loop)
   long long* trace;     // optional [n_barriers][n_cta][2] SM-clock stamps (arrive, release), or null
   int trace_ctas;       // CTAs per barrier in both arrays (chain of step kernels)
   long long* trace_pts; // optional [n_barriers][n_cta][8] stamps inside the phase that ends at that barrier
@@ -944,7 +943,7 @@ __device__ inline void phase_head(const DecodeArgs& a, const DecodeSmem& s, int 
   }
 }
 
-// Final arg-max over the per-CTA candidates; optionally feeds the token back.
+// Final arg-max over the per-CTA candidates, fed back as the next token.
 static __device__ __noinline__ void phase_argmax(const DecodeArgs& a, int ncta_head) {
   if (threadIdx.x < 32) {
     // the state words are fetched up front, next to the first candidates: one L2 round trip, not a chain
@@ -980,10 +979,8 @@ static __device__ __noinline__ void phase_argmax(const DecodeArgs& a, int ncta_h
         if (bi == 0x7fffffff) bi = 0;
         a.st->out_token[col] = bi;
         if (a.step_tokens && sd < a.step_capacity) a.step_tokens[(size_t)sd * a.ncols + col] = bi;
-        if (a.advance) {
-          a.st->token[col] = bi;
-          a.st->pos[col] = pos_now + 1;
-        }
+        a.st->token[col] = bi;
+        a.st->pos[col] = pos_now + 1;
       }
     }
     if (threadIdx.x == 0) a.st->steps_done = sd + 1;

@@ -85,7 +85,7 @@ void launch_gemv(const Launch& l, const DecodeArgs& a, const StepPlan& pl, StepG
     g.nslots = 1;
   } else {
     g.slot_tiles = 8;
-    g.nslots = 2;
+    g.nslots = kStMaxSlots;
   }
   g.sm = st_smem(g, a.ncols, a.nterms);
   const int T = kStThreads / st_cols(a.ncols);

@@ -29,7 +29,7 @@
 namespace b200lm {
 
 constexpr int kStThreads = 512, kStWarps = kStThreads / 32;
-constexpr int kStMaxSlots = 8;            // ring slots of a warp
+constexpr int kStMaxSlots = 2;            // ring slots of a warp
 constexpr int kStKeys = 32;               // keys of one attention round (one per lane of the softmax warps)
 constexpr int kStMaxSplits = 64;
 constexpr int kAtThreads = 256;
@@ -649,10 +649,8 @@ step_gemv_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
             if (ix == 0x7fffffff) ix = 0;
             a.st->out_token[c] = ix;
             if (a.step_tokens && sd < a.step_capacity) a.step_tokens[(size_t)sd * ncols + c] = ix;
-            if (a.advance) {
-              a.st->token[c] = ix;
-              a.st->pos[c] = __ldcg(&a.st->pos[c]) + 1;
-            }
+            a.st->token[c] = ix;
+            a.st->pos[c] = __ldcg(&a.st->pos[c]) + 1;
           }
         }
         if (lane == 0) a.st->steps_done = sd + 1;

@@ -500,15 +500,10 @@ std::unique_ptr<Executor> Executor::create(std::shared_ptr<Model> model, const B
   for (int t = 0; t < 2; ++t) { a.rope_cos[t] = model->rope_cos[t]; a.rope_sin[t] = model->rope_sin[t]; }
   a.st = reinterpret_cast<DecodeState*>(e->alloc(sizeof(DecodeState), true));
   const int G = d.group();
-  const int max_splits = std::max(a.n_attn_splits_local, a.n_attn_splits_global);
   a.xres[0] = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.d, true));
   a.xres[1] = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.d, true));
   a.qkv = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.nqkv(), true));
-  a.part_o = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.hkv * max_splits * G * d.hd, true));
-  a.part_ml = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.hkv * max_splits * G * 2, true));
-  a.opart = reinterpret_cast<float*>(e->alloc(sizeof(float) * a.o_slices * kMaxCols * d.d, true));
   a.act = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.ffn, true));
-  a.fpart = reinterpret_cast<float*>(e->alloc(sizeof(float) * a.down_slices * kMaxCols * d.d, true));
   a.logits = reinterpret_cast<float*>(e->alloc(sizeof(float) * max_cols * d.vocab, true));
   a.amax_val = reinterpret_cast<float*>(e->alloc(sizeof(float) * e->n_sms * kMaxCols, true));
   a.amax_idx = reinterpret_cast<int*>(e->alloc(sizeof(int) * e->n_sms * kMaxCols, true));
@@ -527,7 +522,6 @@ std::unique_ptr<Executor> Executor::create(std::shared_ptr<Model> model, const B
         e->alloc(sizeof(float) * (size_t)e->n_sessions * d.hkv * kWideMaxSplits * d.group() * (d.hd + 4), true));
     e->wide_ticket = reinterpret_cast<int*>(e->alloc(sizeof(int) * (size_t)e->n_sessions * d.hkv, true));
   }
-  a.advance = 1;
   // Which kernels carry a step, and how many sessions at once.  The chain gives way to the persistent kernel, that to the
   // chain with the sessions of a group one after another, that to one kernel per phase; the persistent kernels give way
   // to the chain.  No persistent kernel under tensor parallelism, whose collectives run between the phases.
@@ -561,13 +555,16 @@ std::unique_ptr<Executor> Executor::create(std::shared_ptr<Model> model, const B
       e->decode_mode = B200LM_DECODE_PHASE_KERNELS;
     }
   }
-  if (e->chain) {
+  // split partials of the kernels that run (the wide step has its own)
+  if (e->decode_mode != B200LM_DECODE_WIDE) {
+    auto floats = [&](size_t n) { return reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * n, true)); };
     StepPlan& sp = e->step;
-    sp.part_o = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.hkv * sp.max_splits * G * d.hd, true));
-    sp.part_ml = reinterpret_cast<float*>(e->alloc(sizeof(float) * kMaxCols * d.hkv * sp.max_splits * G * 2, true));
-    sp.opart = reinterpret_cast<float*>(e->alloc(sizeof(float) * sp.o_slices * kMaxCols * d.d, true));
-    sp.fpart = reinterpret_cast<float*>(e->alloc(sizeof(float) * sp.down_slices * kMaxCols * d.d, true));
-    sp.ticket = reinterpret_cast<int*>(e->alloc(sizeof(int), true));
+    const size_t splits = e->chain ? sp.max_splits : std::max(a.n_attn_splits_local, a.n_attn_splits_global);
+    (e->chain ? sp.part_o : a.part_o) = floats(d.hkv * splits * G * d.hd);
+    (e->chain ? sp.part_ml : a.part_ml) = floats(d.hkv * splits * G * 2);
+    (e->chain ? sp.opart : a.opart) = floats((size_t)(e->chain ? sp.o_slices : a.o_slices) * d.d);
+    (e->chain ? sp.fpart : a.fpart) = floats((size_t)(e->chain ? sp.down_slices : a.down_slices) * d.d);
+    if (e->chain) sp.ticket = reinterpret_cast<int*>(e->alloc(sizeof(int), true));
   }
   // ---- prefill buffers (rows padded to whole 128-token tiles, zero-filled)
   e->t_max = d.buckets[0];
