@@ -107,7 +107,7 @@ struct AmArgs {
   float* out;               // [batch][hkv * G][hd]
   float* part_o;            // [hkv][rows][nsplit][hd]   (nsplit > 1)
   float* part_ml;           // [hkv][rows][nsplit][2]
-  unsigned* tickets;        // (kv head, row tile) by split count: the last split to arrive sums up; null: a second kernel does
+  unsigned* tickets;        // one per (kv head, row tile): the last split to arrive sums up; null: a second kernel does
   int* err;
 };
 
@@ -494,7 +494,7 @@ attn_shared_kernel(const AmArgs a) {
     // ---- the split that arrives last sums up this unit's rows
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) *last_s = ticket_last(a.tickets, unit, a.nsplit, [](unsigned* t, unsigned top) { return atomicInc(t, top); });
+    if (threadIdx.x == 0) *last_s = ticket_last(a.tickets + unit, a.nsplit, [](unsigned* t, unsigned top) { return atomicInc(t, top); });
     __syncthreads();
     if (*last_s) {
       __threadfence();
@@ -596,7 +596,7 @@ inline void launch_attn_shared_t(cudaStream_t st, AmArgs a, int device, int sms,
   a.nsplit = std::max(1, std::min(std::min(sms / units, cap), std::min(kTicketSplits, (nchunks + S::KG - 1) / S::KG)));
   // One CTA sums up to 128 KB of partials in about the time that a second launch costs; more is spread over a grid.
   const size_t part = (size_t)a.nsplit * std::min(a.rows, S::kRows) * HD * 4;
-  a.tickets = part <= 128 * 1024 && units <= kTicketUnits ? tickets : nullptr;
+  a.tickets = part <= 128 * 1024 && units <= kTicketUnits ? ticket_row(tickets, a.nsplit) : nullptr;
   static unsigned char ready[64] = {};                                // per device; a race only repeats the call
   if (!ready[device]) {
     raise_dyn_smem(attn_shared_kernel<T, HD, MT, PACK>, (size_t)S::kSmem);

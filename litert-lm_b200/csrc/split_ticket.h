@@ -17,14 +17,14 @@ namespace b200lm {
 constexpr int kTicketSplits = 256;         // most splits of a unit
 constexpr int kTicketUnits = 128;          // most units of a call with splits: two splits each fill 256 SMs
 
-B2_TICKET_FN int ticket_slot(int unit, int nsplit) { return nsplit * kTicketUnits + unit; }
 constexpr int kTicketWords = (kTicketSplits + 1) * kTicketUnits;
+// The tickets of a call, one per unit.
+B2_TICKET_FN unsigned* ticket_row(unsigned* tickets, int nsplit) { return tickets + nsplit * kTicketUnits; }
 
 // Arrival of one split; true for the last one.  `inc` is atomicInc: returns the old value v and stores v >= top ? 0 : v + 1.
 template <typename Inc>
-B2_TICKET_FN bool ticket_last(unsigned* tickets, int unit, int nsplit, const Inc& inc) {
-  const unsigned top = (unsigned)nsplit - 1u;
-  return inc(tickets + ticket_slot(unit, nsplit), top) == top;
+B2_TICKET_FN bool ticket_last(unsigned* ticket, int nsplit, const Inc& inc) {
+  return (int)inc(ticket, (unsigned)(nsplit - 1)) == nsplit - 1;
 }
 
 }  // namespace b200lm

@@ -25,7 +25,7 @@ static bool clean(const std::vector<unsigned>& t) {
 static bool alone(std::vector<unsigned>& t, Call c) {
   for (int u = 0; u < c.units; ++u)
     for (int s = 0; s < c.nsplit; ++s)
-      if (ticket_last(t.data(), u, c.nsplit, inc) != (s == c.nsplit - 1)) return false;
+      if (ticket_last(ticket_row(t.data(), c.nsplit) + u, c.nsplit, inc) != (s == c.nsplit - 1)) return false;
   return clean(t);
 }
 
@@ -44,7 +44,7 @@ int main() {
           const bool first = all ? order >> i & 1 : (int)(rng() % (unsigned)(na - ia + nb - ib)) < na - ia;
           int& at = first ? ia : ib;
           const Call& c = first ? a : b;
-          ticket_last(t.data(), at / c.nsplit, c.nsplit, inc);
+          ticket_last(ticket_row(t.data(), c.nsplit) + at / c.nsplit, c.nsplit, inc);
           ++at;
         }
         if (!clean(t)) { printf("off zero after %dx%d and %dx%d\n", a.units, a.nsplit, b.units, b.nsplit); return 1; }
