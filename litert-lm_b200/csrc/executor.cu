@@ -423,7 +423,7 @@ std::unique_ptr<Executor> Executor::create(std::shared_ptr<Model> model, const B
   if (e->decode_mode == B200LM_DECODE_WIDE)
     B2_CHECK(e->prefill_gemm == B200LM_GEMM_TCGEN05 && cfg.tp_world <= 1, kFailedPrecondition,
              "the wide decode mode needs the tensor-core GEMM weights and no tensor parallelism");
-  // a collective cannot run inside a persistent kernel: tensor-parallel decode is one kernel per phase
+  // a collective cannot run inside a persistent kernel: tensor-parallel decode launches its kernels one by one
   if (cfg.tp_world > 1) e->decode_mode = B200LM_DECODE_PHASE_KERNELS;
   const int esz = d.kv_dtype == 0 ? 4 : 2;
   // ---- paged KV cache
@@ -924,18 +924,18 @@ void Executor::launch_phases(int nsteps, const DecodeArgs& a) {
   launches += (int64_t)nsteps * (5 * d.n_layers + 2);
 }
 
-// What `body` queues on `stream`, as a graph.  It is recorded on a stream made for that: the caller's may be the legacy
-// default stream, which cannot be captured, or a blocking one, whose capture would make other threads' work on the
-// default stream fail.
+// What `body` queues on `stream`, as a graph.  A caller's stream is not captured, but one made for that: the caller's may
+// be the legacy default stream, which cannot be captured, or a blocking one, whose capture would make other threads' work
+// on the default stream fail.  (Not for the executor's own stream: making and destroying one takes about 200 us.)
 template <typename Body>
 cudaGraph_t Executor::capture(const Body& body) {
-  cudaStream_t rec = nullptr;
+  cudaStream_t rec = stream;
   cudaGraph_t graph = nullptr;
-  B2_CUDA(cudaStreamCreateWithFlags(&rec, cudaStreamNonBlocking));
+  if (!own_stream) B2_CUDA(cudaStreamCreateWithFlags(&rec, cudaStreamNonBlocking));
   std::swap(stream, rec);
   auto done = [&]() {
     std::swap(stream, rec);
-    cudaStreamDestroy(rec);
+    if (!own_stream) cudaStreamDestroy(rec);
   };
   try {
     B2_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
