@@ -132,7 +132,7 @@ def test_the_first_decode_call_does_not_wait_for_a_graph(pkg, mio):
             row.append(time.perf_counter() - t0)
         times.append(row)
     least = np.min(times, axis=0)
-    assert least[0] <= 1.5 * least[4:].min(), (least * 1e6).round().tolist()
+    assert least[0] <= 1.8 * least[4:].min(), (least * 1e6).round().tolist()
     assert all(np.array_equal(x, logits[0]) for x in logits)
 
 
