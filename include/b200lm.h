@@ -47,8 +47,8 @@ enum {
                                           each fetches its weights while its predecessor runs */
   B200LM_DECODE_WIDE = 5               /* lockstep groups of up to 128 sessions: the projections of a step run on the
                                           tensor-core int4 GEMM of the prefill path with the sessions as its token
-                                          rows (bf16 activations), one attention CTA per (session, kv head), one CUDA
-                                          graph per step.  AUTO picks it when n_sessions > 4.  Needs the tensor-core
+                                          rows (bf16 activations), attention CTAs per (session, kv head, key split),
+                                          one CUDA graph per step.  AUTO picks it when n_sessions > 4.  Needs the tensor-core
                                           GEMM weights; no tensor parallelism. */
 };
 enum { B200LM_GEMM_AUTO = 0, B200LM_GEMM_CHECK = 1, B200LM_GEMM_TCGEN05 = 2 };

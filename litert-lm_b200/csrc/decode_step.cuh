@@ -71,7 +71,10 @@ struct StepGemv {
   int bar;                    // index of this kernel in the step (timeline)
 };
 
-__host__ __device__ inline int st_cols(int ncols) { return ncols <= 1 ? 1 : 4; }    // session groups of a CTA
+// Session groups of a CTA.  Two and three sessions take the instantiation of four: half or a quarter of the warps have no
+// vector in the prologue.  A step of the 1B model at 300 keys is 554 / 744 / 779 / 838 us with 1 / 2 / 3 / 4 sessions; an
+// instantiation for two has not been built.
+__host__ __device__ inline int st_cols(int ncols) { return ncols <= 1 ? 1 : 4; }
 __host__ __device__ inline int st_xstride(int kmax) { return (kmax + 127) / 128 * 128 + 64; }
 
 inline StepSmem st_smem(const StepGemv& g, int ncols, int nterms) {
@@ -666,7 +669,7 @@ step_gemv_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
 
 // Attention of one (session, kv head, key split): the split's cached rows arrive by bulk copies issued before the wait
 // on the QKV projection, in rounds of kStKeys keys over `nbuf` buffers; the step's own key joins the last split in
-// shared memory and is appended to the cache by it.  A round is: scores (a warp takes two keys, the G * 2 sums of a
+// shared memory and is appended to the cache by it.  A round is: scores (a warp takes four keys, the G * 4 sums of a
 // warp fold together), softmax (one warp per head, one lane per key), P V (two elements and a share of the keys per
 // thread).
 struct StepAttn {

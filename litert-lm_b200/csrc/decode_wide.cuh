@@ -1,11 +1,11 @@
 // Wide lockstep decode: one greedy step for MANY sessions at once, with the projections on the
 // tensor-core int4 GEMM of the prefill path (the sessions' current tokens are the GEMM's token rows)
-// and one attention CTA per (session, kv head) over that session's own pages.  The weights stream
+// and attention CTAs per (session, kv head, key split) over that session's own pages.  The weights stream
 // once per step for the whole group, which is what a group of more sessions than the GEMV kernels
 // carry (kMaxCols) needs.  Activations are bf16 as in prefill.
 //
-// This file holds the two small kernels the step adds to the prefill kernels; the step itself is
-// Executor::launch_wide_steps.
+// This file holds the two kernels the step adds to the prefill kernels, its attention and its arg-max; the
+// step itself is Executor::wide_step.
 #pragma once
 #include <algorithm>
 #include "decode_ops.cuh"

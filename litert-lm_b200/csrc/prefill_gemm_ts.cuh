@@ -11,8 +11,8 @@
 // variant (an M128 N128 K16 MMA reading both operands from shared memory
 // needs the full 128 B/clk of the SM by itself).
 //
-// The kernel is persistent: one CTA per SM walks a static list of output tiles
-// (128 weight rows x NTOK tokens x one K split).  Lane i of the accumulator is
+// The kernel is persistent: one CTA per SM (two with tiles of up to 64 tokens)
+// walks a static list of output tiles (128 weight rows x NTOK tokens x one K split).  Lane i of the accumulator is
 // weight row i, so the per-channel scale is one scalar per epilogue thread and
 // a warp's store covers 32 consecutive output features of one token.  The
 // epilogue warps first pull the whole accumulator into registers (at most 64
@@ -32,7 +32,8 @@
 // works.
 //
 // A narrow tile's k block still costs a CTA its hand-overs, so two CTAs share an SM and fill each other's gaps
-// (131072 x 2560, 64 tokens: 106 us with one, 87 with two; 20480 x 2560: 33 and 24).
+// (131072 x 2560, 64 tokens: 106 us with one, 83 with two; 20480 x 2560: 33 and 22.5).  The expansion's reads of the
+// int4 block (16 bytes a lane at a stride of 32) take 8.2 shared-memory wavefronts each, where 4 are the least.
 //
 // Warp roles: 0 = activation producer, 1 = TMEM owner + MMA issue, 2 = weight
 // producer, 4.. = int4 expansion, then epilogue.
