@@ -7,7 +7,7 @@
 // long sum stays in its accumulators: scores leave them every 64 elements, P V every 16 keys (left in them over 32768
 // keys, the result was off by 2e-6 where fp32 adds are off by 3e-7).  tcgen05 would want the three query terms of a 128-row tile
 // (192 KB at head size 256) next to the K / V stages; they do not fit, mma.sync takes them from shared memory
-// in 16-row pieces.
+// in 16-row pieces.  (About 40 rows with their three terms in ONE 128-row tile would fit; that has not been built.)
 //
 // A warp owns (row tile of 16 query rows) x (every KG-th chunk of 16 keys): scores, online softmax and P V of a
 // chunk stay in its registers, so warps meet only at the end.  The warps of a key group stream the chunks' K
