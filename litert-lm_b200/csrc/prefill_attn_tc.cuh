@@ -85,7 +85,7 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   volatile int* sm_fail = reinterpret_cast<volatile int*>(bars + 15);   // a softmax thread's wait gave up
   float* l_part = reinterpret_cast<float*>(bars + 16);     // [128] row sums of the upper 32 keys
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int G = g.hq / g.hkv;
   const int TT = 128 / G;                       // tokens per tile
   // later query tiles see more keys: they are scheduled first so the longest CTAs do not start last
@@ -119,14 +119,15 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   pdl_wait();                 // set-up done; Q, K, V below come from the preceding kernel
   pdl_launch_dependents();
 
   if (warp == 0) {
     // ---- producer
     bool ok = true;
-    if (lane == 0) {
+    const bool leader = elect_one();
+    if (leader) {
       // Q tile: KB boxes of 64 columns x (G heads x TT tokens) rows
       mbar_arrive_expect_tx(q_full, L::kQ);
       for (int kb = 0; kb < KB; ++kb) {
@@ -140,15 +141,15 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       const int s = j & 1, n = j >> 1;
       const int key0 = (tile_lo + j) * kFaBN;
       const int page = g.page_table[key0 / kPage], slot0 = key0 % kPage;
-      if (n > 0) ok = mbar_wait(&k_empty[s], (n - 1) & 1, g.err);
-      if (ok && lane == 0) {
+      if (n > 0) ok = __all_sync(0xffffffffu, mbar_wait(&k_empty[s], (n - 1) & 1, g.err));
+      if (ok && leader) {
         mbar_arrive_expect_tx(&k_full[s], L::kK);
         const int krow = (page * g.hkv + kvh) * kPage + slot0;
         for (int kb = 0; kb < KB; ++kb)
           tma_load_2d(sK + s * L::kK + kb * kFaBN * 128, &tmK, kb * 64, krow, &k_full[s]);
       }
-      if (ok && n > 0) ok = mbar_wait(&v_empty[s], (n - 1) & 1, g.err);
-      if (ok && lane == 0) {
+      if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(&v_empty[s], (n - 1) & 1, g.err));
+      if (ok && leader) {
         mbar_arrive_expect_tx(&v_full[s], L::kV);
         tma_load_2d(sV + s * L::kV, &tmVt, slot0, (page * g.hkv + kvh) * HD, &v_full[s]);
       }
@@ -171,25 +172,26 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       umma_commit(&s_full[s]);
       umma_commit(&k_empty[s]);
     };
-    bool ok = mbar_wait(q_full, 0, g.err) && mbar_wait(&k_full[0], 0, g.err);
+    const bool leader = elect_one();
+    bool ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0, g.err) && mbar_wait(&k_full[0], 0, g.err));
     if (ok) {
       tc_fence_after();
-      if (lane == 0) issue_s(0);
+      if (leader) issue_s(0);
       __syncwarp();
     }
     for (int j = 0; j < ntiles && ok; ++j) {
       const int s = j & 1, n = j >> 1;
       if (j + 1 < ntiles) {
-        ok = mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, g.err);
+        ok = __all_sync(0xffffffffu, mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, g.err));
         if (!ok) break;
         tc_fence_after();
-        if (lane == 0) issue_s(j + 1);
+        if (leader) issue_s(j + 1);
         __syncwarp();
       }
-      ok = mbar_wait(&v_full[s], n & 1, g.err) && mbar_wait(&p_full[s], n & 1, g.err);
+      ok = __all_sync(0xffffffffu, mbar_wait(&v_full[s], n & 1, g.err) && mbar_wait(&p_full[s], n & 1, g.err));
       if (!ok) break;
       tc_fence_after();
-      if (lane == 0) {
+      if (leader) {
         const uint64_t vd = umma_desc_sw128(smem_u32(sV + s * L::kV));
 #pragma unroll
         for (int k = 0; k < kFaBN / 16; ++k)      // P: 8 TMEM columns per 16 keys
@@ -198,7 +200,7 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       }
       __syncwarp();
     }
-    if (ok && lane == 0) umma_commit(o_full);
+    if (ok && leader) umma_commit(o_full);
     __syncwarp();
   } else {
     // ---- softmax warps: two threads per query row (TMEM lane), 32 keys each

@@ -22,18 +22,20 @@
 // Three rings, each with its own depth, move two k blocks (128 k) at a time: the
 // int4 blocks (from HBM, deep), the activation tiles (from L2, shallow) and the
 // expanded weights in tensor memory.  A hand-over between two roles costs a few
-// hundred cycles however little it covers; with one k block per hand-over and one
-// ring for all three, a k block took 780 - 990 cycles at any token width, where
-// the HBM time is 180 and the M128 N256 K64 product takes 512.
+// hundred cycles however little it covers.  A stage of two k blocks takes 1020
+// cycles at 256 tokens, of which the products are 1024: tensor-bound.  It takes
+// 720 at 64 tokens: the expansion's chain of waits, loads and stores.  (While the
+// MMA role issued behind `lane == 0`, its 8 instructions took 810 cycles and a
+// stage 1260 at any width: elect_one in prefill_ops.cuh.)
 //
 // The weights do not depend on the preceding kernel, so their stream and their
 // expansion start before griddepcontrol.wait; narrow tiles take half of an SM's
 // shared and tensor memory, which lets the next GEMM's CTA do that while this one
 // works.
 //
-// A narrow tile's k block still costs a CTA its hand-overs, so two CTAs share an SM and fill each other's gaps
-// (131072 x 2560, 64 tokens: 106 us with one, 83 with two; 20480 x 2560: 33 and 22.5).  The expansion's reads of the
-// int4 block (16 bytes a lane at a stride of 32) take 8.2 shared-memory wavefronts each, where 4 are the least.
+// A narrow tile's k block still costs a CTA its hand-overs, so two CTAs share an SM and fill each other's gaps.
+// The expansion's reads of the int4 block (16 bytes a lane at a stride of 32) take 8.2 shared-memory wavefronts
+// each, where 4 are the least.
 //
 // Warp roles: 0 = activation producer, 1 = TMEM owner + MMA issue, 2 = weight
 // producer, 4.. = int4 expansion, then epilogue.
@@ -151,7 +153,7 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   uint64_t* acc_empty = acc_full + 1;               // accumulator read out by the epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int KB = g.K / kGemmBK;
   const int nkb = KB / g.ksplit;
   const int nst = (nkb + kTsKb - 1) / kTsKb;        // stages of a tile; the last may hold one k block
@@ -191,7 +193,7 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const uint32_t tmem_w = tmem_base + NTOK;         // weight slots follow the accumulator columns
   // Ahead of the wait below: the next GEMM may fill its weight ring while this one still waits.  A kernel behind this one
   // that reads ahead of its own wait must read nothing that the two kernels before it write.
@@ -202,14 +204,15 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
     pdl_wait();
     int it = 0;
     bool ok = true;
+    const bool leader = elect_one();
 #pragma unroll 1
     for (int li = 0; li < my_tiles && ok; ++li) {
       const TsTile tl = ts_tile(blockIdx.x + li * gridDim.x, n_tiles, t_tiles);
 #pragma unroll 1
       for (int st = 0; st < nst && ok; ++st, ++it) {
         const int s = it % XS, n = it / XS, kb = st * kTsKb, nk = min(kTsKb, nkb - kb);
-        if (n > 0) ok = mbar_wait(&x_empty[s], (n - 1) & 1, g.err);
-        if (ok && lane == 0) {
+        if (n > 0) ok = __all_sync(0xffffffffu, mbar_wait(&x_empty[s], (n - 1) & 1, g.err));
+        if (ok && leader) {
           mbar_arrive_expect_tx(&x_full[s], (uint32_t)(nk * kXb));
 #pragma unroll 1
           for (int k = 0; k < nk; ++k)
@@ -226,19 +229,21 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
     const uint32_t idesc = umma_idesc_bf16(kTsRows, NTOK);
     int it = 0;
     bool ok = true;
+    const bool leader = elect_one();
 #pragma unroll 1
     for (int li = 0; li < my_tiles && ok; ++li) {
-      if (li > 0) ok = mbar_wait(acc_empty, (li - 1) & 1, g.err);
+      if (li > 0) ok = __all_sync(0xffffffffu, mbar_wait(acc_empty, (li - 1) & 1, g.err));
       tc_fence_after();
 #pragma unroll 1
       for (int st = 0; st < nst && ok; ++st, ++it) {
         const int sx = it % XS, sw = it % WS, nk = min(kTsKb, nkb - st * kTsKb);
-        ok = mbar_wait(&w_full[sw], (it / WS) & 1, g.err) && mbar_wait(&x_full[sx], (it / XS) & 1, g.err);
+        ok = __all_sync(0xffffffffu, mbar_wait(&w_full[sw], (it / WS) & 1, g.err) && mbar_wait(&x_full[sx], (it / XS) & 1, g.err));
         if (!ok) break;
         tc_fence_after();
-        if (lane == 0) {
-#pragma unroll 1
-          for (int kb = 0; kb < nk; ++kb) {
+        if (leader) {
+#pragma unroll
+          for (int kb = 0; kb < kTsKb; ++kb) {
+            if (kb >= nk) break;
             const uint64_t xd = umma_desc_sw128(smem_u32(sX + (sx * kTsKb + kb) * kXb));
 #pragma unroll
             for (int k = 0; k < kGemmBK / 16; ++k)   // 16 bf16 along K per MMA: 8 TMEM columns, 32 bytes of X
@@ -249,7 +254,7 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
         }
         __syncwarp();
       }
-      if (ok && lane == 0) umma_commit(acc_full);
+      if (ok && leader) umma_commit(acc_full);
       __syncwarp();
     }
   } else if (warp == 2) {
@@ -281,27 +286,25 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
       if (ok && it >= WS) ok = mbar_wait(&w_empty[sw], (it / WS - 1) & 1, g.err);
       if (!ok) break;
       tc_fence_after();
+      uint4 q[2 * kTsKb];                            // all of the row's part first: the stores below order what follows them
 #pragma unroll
-      for (int kb = 0; kb < kTsKb; ++kb) {
-        if (kb < nk) {
-          const uint4* src = reinterpret_cast<const uint4*>(sQ + (sq * kTsKb + kb) * kGemmStageQ + (quarter * 32 + lane) * 32);
+      for (int i = 0; i < 2 * kTsKb; ++i)
+        if (i / 2 < nk) q[i] = reinterpret_cast<const uint4*>(sQ + (sq * kTsKb + i / 2) * kGemmStageQ + (quarter * 32 + lane) * 32)[i % 2];
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const uint4 q = src[half];
-            const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
-            uint32_t r[16];
+      for (int i = 0; i < 2 * kTsKb; ++i) {
+        if (i / 2 >= nk) break;
+        const uint32_t qw[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
+        uint32_t r[16];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < 4; ++j) {
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                uint32_t v = ((qw[j] >> (4 * i)) & 0x000F000Fu) | 0x43004300u;   // bf16(128 + nibble) pairs
-                __nv_bfloat162 h = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&v), bias);
-                r[j * 4 + i] = *reinterpret_cast<uint32_t*>(&h);
-              }
-            }
-            tmem_st16(tmem_w + lane_base + (sw * kTsKb + kb) * kTsAcols + half * 16, r);
+          for (int k = 0; k < 4; ++k) {
+            uint32_t v = ((qw[j] >> (4 * k)) & 0x000F000Fu) | 0x43004300u;   // bf16(128 + nibble) pairs
+            __nv_bfloat162 h = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&v), bias);
+            r[j * 4 + k] = *reinterpret_cast<uint32_t*>(&h);
           }
         }
+        tmem_st16(tmem_w + lane_base + (sw * kTsKb + i / 2) * kTsAcols + i % 2 * 16, r);
       }
       tmem_st_wait();
       tc_fence_before();

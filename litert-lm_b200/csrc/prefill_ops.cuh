@@ -390,6 +390,16 @@ gemm_w4_simple_kernel(const __nv_bfloat16* __restrict__ A, const uint4* __restri
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
+// One lane of a converged warp, chosen by elect.sync.  tcgen05.mma / commit and the TMA copies take their operands from
+// uniform registers: behind `lane == 0` the compiler cannot know that one thread is left and serialises every such
+// instruction over the lanes (100 cycles per tcgen05.mma, measured), behind elect.sync it does not.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t is;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}" : "=r"(is));
+  return is != 0;
+}
+// The warp's index as a value the compiler knows to be the same in all lanes.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
