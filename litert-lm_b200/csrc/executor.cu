@@ -270,23 +270,47 @@ static CUtensorMap make_bf16_map(const void* base, int rank, const cuuint64_t* d
   return tm;
 }
 
-// Split-K factor for a GEMM of `n_tiles` weight-row tiles over T tokens with KB
-// 64-wide k blocks: the smallest divisor of KB (at least 4 k blocks per split,
-// at most 8 splits) whose work units fill 90 % of the last round over the CTAs,
-// else the divisor that fills it best.
-int pick_ksplit(int T, int n_tiles, int KB, int sms) {
-  if (const int s = gs_ksplit(T, n_tiles * 128, KB, sms)) return s;
-  const int ntok = ts_tile_tokens(T);
-  const int tiles = n_tiles * ((T + ntok - 1) / ntok), slots = ts_ctas_per_sm(ntok) * sms;
+// What a GEMM of the tcgen05 kernel and its consumer's pass over the partial sums take, in us, for one choice of token
+// tile and K split.  The terms are what the kernel spends its time on: rounds of tiles over the CTA slots, each a row of k
+// blocks whose price depends on the tile's width (tensor-bound at 256 tokens, the expansion's chain of waits below; dearer
+// where two CTAs share an SM), then the accumulators' stores, then the partials once more out of L2.  The constants are a
+// least-squares fit to 2600 timed pairs of GEMM and residual norm (14 projections of four models, 20 - 1023 tokens): it is
+// off by 8 % on average and its choice costs 1.3 % more than the best one, where filling 90 % of the last round with the
+// widest tile cost 15 % (2560 x 2048 at 1023 tokens: 45.6 us with eight splits, 22.5 with one).
+static double ts_cost(int T, int N, int K, bool geglu, int ntok, int ks, int sms) {
+  struct Width { int ntok; double kb, kb_shared, round; };
+  static const Width widths[] = {{16, 0.172, 0.325, 0.0}, {32, 0.188, 0.312, 0.0}, {64, 0.209, 0.317, 0.0}, {128, 0.281, 0.281, 0.0}, {256, 0.331, 0.331, 0.6}};
+  const Width* w = widths;
+  while (w->ntok != ntok) ++w;
+  const int tiles = ((N + kTsRows - 1) / kTsRows) * ((T + ntok - 1) / ntok) * ks, slots = ts_ctas_per_sm(ntok) * sms;
+  const double mb = 1e-6 * 4, rounds = (tiles + slots - 1) / slots;
+  double us = rounds * ((double)(K / kGemmBK / ks) * (tiles > sms ? w->kb_shared : w->kb) + w->round);
+  us += 0.126 * mb * std::min(tiles, slots) * ntok * kTsRows * (geglu ? 0.5 : 1.0);
+  if (!geglu) us += 0.25 * mb * ks * T * N + 0.15 * ks;
+  return us;
+}
+// Token tile of the tcgen05 kernel for a given K split.
+static int ts_tile_tokens(int T, int N, int K, bool geglu, int ks, int sms) {
+  int best = 16;
+  double best_us = ts_cost(T, N, K, geglu, best, ks, sms);
+  for (int ntok : {32, 64, 128, 256}) {
+    const double us = ts_cost(T, N, K, geglu, ntok, ks, sms);
+    if (us < best_us) { best_us = us; best = ntok; }
+  }
+  return best;
+}
+
+// Split-K factor of a GEMM: a divisor of the 64-wide k blocks, at most `most` (what the partials buffer holds) and eight,
+// two blocks a split and more.
+int pick_ksplit(int T, int N, int K, int sms, int most) {
+  const int KB = K / kGemmBK;
+  if (const int s = gs_ksplit(T, N, KB, sms, most)) return s;
   int best = 1;
-  double best_eff = 0.0;
-  for (int s = 1; s <= 8; ++s) {
-    if (KB % s) continue;
-    if (s > 1 && KB / s < 4) break;
-    const int units = tiles * s;
-    const double eff = (double)units / ((double)((units + slots - 1) / slots) * slots);
-    if (eff > best_eff + 1e-9) { best_eff = eff; best = s; }
-    if (eff >= 0.9) break;
+  double best_us = 1e30;
+  for (int s = 1; s <= std::min(8, most); ++s) {
+    if (KB % s || (s > 1 && KB / s < 2)) continue;
+    const double us = ts_cost(T, N, K, false, ts_tile_tokens(T, N, K, false, s, sms), s, sms);
+    if (us < best_us) { best_us = us; best = s; }
   }
   return best;
 }
@@ -323,7 +347,7 @@ void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bflo
       if (launches) ++*launches;
       return;
     }
-    const int ntok = ts_tile_tokens(T);
+    const int ntok = ts_tile_tokens(T, N, K, geglu, ksplit, sms);
     const int total = ((N + kTsRows - 1) / kTsRows) * ((T + ntok - 1) / ntok) * ksplit;
     const int slots = ts_ctas_per_sm(ntok) * sms, grid = total < slots ? total : slots;
 #define B2_TS(EPI_, NTOK_, MAP_) launch_pdl(gemm_w4_ts_kernel<EPI_, NTOK_>, dim3(grid), dim3(ts_threads(NTOK_)), ts_smem(NTOK_), st, MAP_, g)
@@ -756,18 +780,19 @@ void Executor::run_prefill_chunk(const int* tokens, int T, int start) {
   ++launches;
   const int mode = prefill_gemm;
   const size_t attn_smem = sizeof(float) * ((size_t)(d.group() + 2) * d.hd + (size_t)8 * d.group() * (d.hd + 2));
+  // split-K partials go to the partials buffer (8 x d floats per token); those of the QKV rows are summed by the append
+  // kernel, but the CUDA-core attention reads whole rows, so it keeps one split
+  int ks_q = 1, ks_o = 1, ks_d = 1;
+  if (mode == B200LM_GEMM_TCGEN05) {
+    if (attn_tc) ks_q = pick_ksplit(T, d.nqkv(), d.d, n_sms, std::max(1, 8 * d.d / d.nqkv()));
+    ks_o = pick_ksplit(T, d.d, d.nq(), n_sms);
+    ks_d = pick_ksplit(T, d.d, d.ffn, n_sms);
+  }
   for (int li = 0; li < d.n_layers; ++li) {
     const LayerWeights& L = model->layers_host[li];
     const LayerGemmWeights& Gm = model->gemm_host[li];
     const float* cosT = model->rope_cos[L.is_global];
     const float* sinT = model->rope_sin[L.is_global];
-    // split-K partials of the QKV rows go to the partials buffer (8 x d floats per token) and are summed by
-    // the append kernel; the CUDA-core attention reads whole rows, so it keeps one split
-    int ks_q = 1;
-    if (mode == B200LM_GEMM_TCGEN05 && attn_tc) {
-      ks_q = pick_ksplit(T, (d.nqkv() + kTsRows - 1) / kTsRows, d.d / 64, n_sms);
-      if ((size_t)ks_q * d.nqkv() > (size_t)8 * d.d) ks_q = 1;
-    }
     float* qkv_buf = ks_q > 1 ? pf_parts : pf_qkv;
     launch_gemm(stream, mode, tm_h, pf_h, L.wqkv, L.sqkv, Gm.wqkv, Gm.sqkv, T, d.nqkv(), d.d, ks_q, false, qkv_buf,
                 nullptr, err, &launches);
@@ -804,7 +829,6 @@ void Executor::run_prefill_chunk(const int* tokens, int T, int start) {
     pf_attn_kernel<<<T * d.hkv, 256, attn_smem, stream>>>(d, j);
     ++launches;
     }
-    int ks_o = mode == B200LM_GEMM_TCGEN05 ? pick_ksplit(T, (d.d + kTsRows - 1) / kTsRows, d.nq() / 64, n_sms) : 1;
     launch_gemm(stream, mode, tm_attn, pf_attn, L.wo, L.so, Gm.wo, Gm.so, T, d.d, d.nq(), ks_o, false, pf_parts,
                 nullptr, err, &launches);
     if (tp_world > 1) tp_allreduce(pf_parts, (size_t)ks_o * T * d.d);
@@ -812,7 +836,6 @@ void Executor::run_prefill_chunk(const int* tokens, int T, int start) {
     ++launches;
     launch_gemm(stream, mode, tm_h, pf_h, L.wgu, L.sgu, Gm.wgu, Gm.sgu, T, 2 * d.ffn, d.d, 1, true, nullptr, pf_act,
                 err, &launches);
-    int ks_d = mode == B200LM_GEMM_TCGEN05 ? pick_ksplit(T, (d.d + kTsRows - 1) / kTsRows, d.ffn / 64, n_sms) : 1;
     launch_gemm(stream, mode, tm_act, pf_act, L.wdown, L.sdown, Gm.wdown, Gm.sdown, T, d.d, d.ffn, ks_d, false,
                 pf_parts, nullptr, err, &launches);
     if (tp_world > 1) tp_allreduce(pf_parts, (size_t)ks_d * T * d.d);
@@ -1007,12 +1030,12 @@ void Executor::wide_step(int nb, int first) {
              model->layers_host[0].g_pre_attn, d.d, d.vocab, d.eps, pf_xres, pf_h, err);
   int64_t* nl = &launches;
   ++*nl;
+  // split K so that the few token rows still spread the weight tiles over the SMs; the attention adds the QKV rows' parts
+  const int ks_q = pick_ksplit(nb, d.nqkv(), d.d, n_sms, std::max(1, 8 * d.d / d.nqkv()));
+  const int ks_o = pick_ksplit(nb, d.d, d.nq(), n_sms), ks_d = pick_ksplit(nb, d.d, d.ffn, n_sms);
   for (int li = 0; li < d.n_layers; ++li) {
     const LayerWeights& L = model->layers_host[li];
     const LayerGemmWeights& Gm = model->gemm_host[li];
-    // split K so that the few token rows still spread the weight tiles over the SMs; the attention reads whole rows
-    int ks_q = pick_ksplit(nb, (d.nqkv() + kTsRows - 1) / kTsRows, d.d / 64, n_sms);
-    if ((size_t)ks_q * d.nqkv() > (size_t)8 * d.d) ks_q = 1;
     launch_gemm(stream, mode, tm_h, pf_h, L.wqkv, L.sqkv, Gm.wqkv, Gm.sqkv, nb, d.nqkv(), d.d, ks_q, false,
                 ks_q > 1 ? pf_parts : pf_qkv, nullptr, err, nl);
     WideAttnArgs wa{ks_q > 1 ? pf_parts : pf_qkv, wide.pos, page_table_dev + (size_t)first * pages_per_seq, pages_per_seq, L.is_global, nsplit, 0,
@@ -1020,12 +1043,10 @@ void Executor::wide_step(int nb, int first) {
                     1, 0, nullptr, 2, ks_q, (size_t)nb * d.nqkv()};
     launch_wide_attn(stream, d, nb, smem_optin, wa);         // sums the projections' partials as it reads them
     ++*nl;
-    const int ks_o = pick_ksplit(nb, (d.d + kTsRows - 1) / kTsRows, d.nq() / 64, n_sms);
     launch_gemm(stream, mode, tm_attn, pf_attn, L.wo, L.so, Gm.wo, Gm.so, nb, d.d, d.nq(), ks_o, false, pf_parts, nullptr, err, nl);
     launch_resid_norm(stream, pf_parts, ks_o, nb, d, L.g_post_attn, L.g_pre_ffn, pf_xres, pf_h);
     ++*nl;
     launch_gemm(stream, mode, tm_h, pf_h, L.wgu, L.sgu, Gm.wgu, Gm.sgu, nb, 2 * d.ffn, d.d, 1, true, nullptr, pf_act, err, nl);
-    const int ks_d = pick_ksplit(nb, (d.d + kTsRows - 1) / kTsRows, d.ffn / 64, n_sms);
     launch_gemm(stream, mode, tm_act, pf_act, L.wdown, L.sdown, Gm.wdown, Gm.sdown, nb, d.d, d.ffn, ks_d, false, pf_parts, nullptr,
                 err, nl);
     const float* g_next = li + 1 < d.n_layers ? model->layers_host[li + 1].g_pre_attn : model->g_final;

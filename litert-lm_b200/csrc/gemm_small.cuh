@@ -224,10 +224,10 @@ inline bool gs_fits(int T, int N, int KT, int ksplit, bool geglu, int sms) {
 }
 
 // K splits: tiles of the busiest CTA, plus what each part costs its consumer.
-inline int gs_ksplit(int T, int N, int KT, int sms) {
+inline int gs_ksplit(int T, int N, int KT, int sms, int most) {
   int best = 0;
   double best_cost = 1e30;
-  for (int s = 1; s <= 8; ++s) {
+  for (int s = 1; s <= 8 && s <= most; ++s) {
     if (KT % s || (s > 1 && KT / s < 4) || !gs_fits(T, N, KT, s, false, sms)) continue;
     const double cost = (double)gs_tiles(0, N, s, sms) * (KT / s) + 6.0 * s;
     if (cost < best_cost - 1e-9) { best_cost = cost; best = s; }

@@ -54,11 +54,9 @@ struct Model {
 struct ActMap {
   CUtensorMap box[4];         // 16, 32, 64, 128 rows
 };
-// token width of the GEMM tile for T token rows
-inline int ts_tile_tokens(int T) { return T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256; }
 CUtensorMap make_activation_map_box(const __nv_bfloat16* base, int rows, int cols, int box_rows);
 ActMap make_activation_map(const __nv_bfloat16* base, int rows, int cols);
-int pick_ksplit(int T, int n_tiles, int KB, int sms);
+int pick_ksplit(int T, int N, int K, int sms, int most = 8);
 void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bfloat16* A, const uint4* w4t,
                  const float* s4t, const uint8_t* w4g, const float* s4g, int T, int N, int K, int ksplit, bool geglu,
                  float* outF, __nv_bfloat16* outB, int* err, int64_t* launches);

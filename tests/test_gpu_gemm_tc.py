@@ -20,6 +20,19 @@ def test_tcgen05_gemm_matches_oracle(pkg, orc, mio, t, n, k, ksplit):
     assert np.abs(got - want).max() / np.abs(want).max() < 2e-5, np.abs(got - want).max() / np.abs(want).max()
 
 
+@pytest.mark.parametrize("t,n,k,ksplit", [
+    (17, 128, 512, 4), (33, 1152, 1024, 2), (49, 384, 128, 1), (65, 2560, 512, 2), (100, 1536, 1152, 2), (129, 1152, 1024, 1),
+    (203, 1152, 1024, 2), (511, 1152, 1024, 2), (1023, 512, 1536, 4),
+])
+def test_tcgen05_gemm_of_several_narrow_token_tiles(pkg, orc, mio, t, n, k, ksplit):
+    """Sizes at which the cheapest tile is narrower than the token rows: several token tiles, the last one ragged."""
+    packed, scale = make_matrix(mio, n, k, 3 * n + k)
+    a = bf16_round(np.random.Generator(np.random.PCG64(t + 2)).standard_normal((t, k), dtype=np.float32))
+    want = orc.matmul_w4(packed, scale, a)
+    got, _ = pkg.ops.gemm_w4(packed, scale, a, mode=pkg.GEMM_TCGEN05, ksplit=ksplit)
+    assert np.abs(got - want).max() / np.abs(want).max() < 2e-5      # exact products, fp32 sums in another order
+
+
 def test_tcgen05_gemm_agrees_with_check_gemm(pkg, mio):
     packed, scale = make_matrix(mio, 768, 384, 77)
     a = bf16_round(np.random.Generator(np.random.PCG64(6)).standard_normal((150, 384), dtype=np.float32))
