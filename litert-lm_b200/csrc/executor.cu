@@ -719,15 +719,12 @@ static void launch_resid_norm(cudaStream_t st, const float* parts, int nparts, i
                               const float* g_post, const float* g_pre, float* xres, __nv_bfloat16* h) {
   const int d4 = d.d / 4;
   const size_t stride = (size_t)T * d.d;
-  const bool few = T <= 128;       // long rows: too few CTAs to hide the partial loads behind one another
   if (d4 <= 128 * 3)
     launch_pdl(pf_resid_norm_reg_kernel<128, 3, 4>, dim3(T), dim3(128), 0, st, parts, nparts, stride, d.d, d.eps, g_post, g_pre, xres, h);
   else if (d4 <= 256 * 3)
     launch_pdl(pf_resid_norm_reg_kernel<256, 3, 4>, dim3(T), dim3(256), 0, st, parts, nparts, stride, d.d, d.eps, g_post, g_pre, xres, h);
-  else if (d4 <= 256 * 6 && few)
-    launch_pdl(pf_resid_norm_reg_kernel<256, 6, 4>, dim3(T), dim3(256), 0, st, parts, nparts, stride, d.d, d.eps, g_post, g_pre, xres, h);
-  else if (d4 <= 256 * 6)
-    launch_pdl(pf_resid_norm_reg_kernel<256, 6>, dim3(T), dim3(256), 0, st, parts, nparts, stride, d.d, d.eps, g_post, g_pre, xres, h);
+  else if (d4 <= 512 * 3)
+    launch_pdl(pf_resid_norm_reg_kernel<512, 3, 4>, dim3(T), dim3(512), 0, st, parts, nparts, stride, d.d, d.eps, g_post, g_pre, xres, h);
   else
     pf_resid_norm_kernel<<<T, kPfThreads, sizeof(float) * d.d, st>>>(parts, nparts, stride, d.d, d.eps, g_post, g_pre,
                                                                     xres, h);

@@ -113,12 +113,24 @@ __global__ void __launch_bounds__(THREADS)
 pf_resid_norm_reg_kernel(const float* __restrict__ parts, int nparts, size_t part_stride, int d, float eps,
                          const float* __restrict__ g_post, const float* __restrict__ g_pre,
                          float* __restrict__ xres, __nv_bfloat16* __restrict__ h) {
-  pdl_wait();
-  pdl_launch_dependents();
   __shared__ float red[2][THREADS / 32];
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int d4 = d / 4;
-  float4 f[MAXV], x[MAXV];
+  constexpr bool kAhead = MAXV <= 3;           // as far as the registers go
+  float4 f[MAXV], x[MAXV], gp[MAXV], gq[MAXV];
+  if (kAhead) {
+#pragma unroll
+    for (int u = 0; u < MAXV; ++u) {
+      const int i = threadIdx.x + THREADS * u;
+      gp[u] = gq[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < d4) {
+        gp[u] = __ldg(reinterpret_cast<const float4*>(g_post) + i);
+        if (g_pre) gq[u] = __ldg(reinterpret_cast<const float4*>(g_pre) + i);
+      }
+    }
+  }
+  pdl_wait();
+  pdl_launch_dependents();
   float4* xr = reinterpret_cast<float4*>(xres + (size_t)t * d);
 #pragma unroll
   for (int u = 0; u < MAXV; ++u) {
@@ -158,8 +170,8 @@ pf_resid_norm_reg_kernel(const float* __restrict__ parts, int nparts, size_t par
   for (int u = 0; u < MAXV; ++u) {
     const int i = threadIdx.x + THREADS * u;
     if (i < d4) {
-      float4 gp = reinterpret_cast<const float4*>(g_post)[i];
-      x[u].x += f[u].x * r * gp.x; x[u].y += f[u].y * r * gp.y; x[u].z += f[u].z * r * gp.z; x[u].w += f[u].w * r * gp.w;
+      if (!kAhead) gp[u] = __ldg(reinterpret_cast<const float4*>(g_post) + i);
+      x[u].x += f[u].x * r * gp[u].x; x[u].y += f[u].y * r * gp[u].y; x[u].z += f[u].z * r * gp[u].z; x[u].w += f[u].w * r * gp[u].w;
       xr[i] = x[u];
       ss2 += x[u].x * x[u].x + x[u].y * x[u].y + x[u].z * x[u].z + x[u].w * x[u].w;
     }
@@ -176,9 +188,9 @@ pf_resid_norm_reg_kernel(const float* __restrict__ parts, int nparts, size_t par
   for (int u = 0; u < MAXV; ++u) {
     const int i = threadIdx.x + THREADS * u;
     if (i < d4) {
-      float4 gq = reinterpret_cast<const float4*>(g_pre)[i];
-      __nv_bfloat162 a = __floats2bfloat162_rn(x[u].x * r2 * gq.x, x[u].y * r2 * gq.y);
-      __nv_bfloat162 b = __floats2bfloat162_rn(x[u].z * r2 * gq.z, x[u].w * r2 * gq.w);
+      if (!kAhead) gq[u] = __ldg(reinterpret_cast<const float4*>(g_pre) + i);
+      __nv_bfloat162 a = __floats2bfloat162_rn(x[u].x * r2 * gq[u].x, x[u].y * r2 * gq[u].y);
+      __nv_bfloat162 b = __floats2bfloat162_rn(x[u].z * r2 * gq[u].z, x[u].w * r2 * gq[u].w);
       uint2 w;
       w.x = *reinterpret_cast<uint32_t*>(&a);
       w.y = *reinterpret_cast<uint32_t*>(&b);
@@ -232,8 +244,6 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
                     const int* __restrict__ page_table, const float* __restrict__ g_k,
                     const float* __restrict__ cosT, const float* __restrict__ sinT, LayerKv kv,
                     const float* __restrict__ g_q, __nv_bfloat16* __restrict__ qout) {
-  pdl_wait();
-  pdl_launch_dependents();
   constexpr int V = HD >= 64 ? HD / 64 : 1;
   constexpr int half = HD / 2;
   const int lane = threadIdx.x & 31;
@@ -243,10 +253,22 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
   const int t = is_q ? job / dm.hq : (int)(blockIdx.x % groups) * kKvaTok + warp - skew;
   const int h = is_q ? job % dm.hq : blockIdx.x / groups;       // of the query or of the kv heads
   const bool has = t >= 0 && t < ntok;
-  if (is_q && !has) return;
   const int pos = pos0 + t, e0 = lane * V;
-  const int page = is_q ? 0 : page_table[pos / kPage];          // one of the whole group; asked for early
   const bool act = has && e0 < half;                            // HD 32: lanes 16..31 idle
+  // what no kernel writes is asked for ahead of the wait
+  int page = 0;                                                 // one of the whole group
+  if (!is_q) page = __ldg(page_table + pos / kPage);
+  const float* gain = is_q ? g_q : g_k;
+  float ga[V], gb[V], cs[V], sn[V];
+  if (act) {
+    ld_vec<V>(gain + e0, ga);
+    ld_vec<V>(gain + e0 + half, gb);
+    ld_vec<V>(cosT + (size_t)pos * half + e0, cs);
+    ld_vec<V>(sinT + (size_t)pos * half + e0, sn);
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  if (is_q && !has) return;
   // head offset within the QKV row: [q heads | k heads | v heads]
   const int col = is_q ? h * HD : dm.nq() + h * HD;
   const float* row = qkv + (ptrdiff_t)t * dm.nqkv() + col;
@@ -275,14 +297,8 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
   ss = warp_sum(ss);
   float r = rsqrtf(ss / (float)HD + dm.eps);
   if (is_q) r *= rsqrtf((float)HD);
-  const float* gain = is_q ? g_q : g_k;
   float k0[V], k1[V];
   if (act) {
-    float ga[V], gb[V], cs[V], sn[V];
-    ld_vec<V>(gain + e0, ga);
-    ld_vec<V>(gain + e0 + half, gb);
-    ld_vec<V>(cosT + (size_t)pos * half + e0, cs);
-    ld_vec<V>(sinT + (size_t)pos * half + e0, sn);
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const float a0 = a[i] * r * ga[i], b0 = b[i] * r * gb[i];
