@@ -266,8 +266,8 @@ pf_kv_append_kernel(ModelDims dm, const float* __restrict__ qkv, int nparts, siz
     ld_vec<V>(cosT + (size_t)pos * half + e0, cs);
     ld_vec<V>(sinT + (size_t)pos * half + e0, sn);
   }
+  pdl_launch_dependents();                                      // ahead of the wait: what follows waits for this kernel
   pdl_wait();
-  pdl_launch_dependents();
   if (is_q && !has) return;
   // head offset within the QKV row: [q heads | k heads | v heads]
   const int col = is_q ? h * HD : dm.nq() + h * HD;
