@@ -183,7 +183,7 @@ step_gemv_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
   constexpr int W = kStWarps / CP, T = W * 32;                          // warps, threads of a session group
   extern __shared__ __align__(128) unsigned char st_sm[];
   const int ncols = CP == 1 ? 1 : a.ncols, nterms = CP == 1 ? 3 : a.nterms;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   st_stamp(a, g.bar, 0);
   uint64_t* bars = reinterpret_cast<uint64_t*>(st_sm + g.sm.bars) + warp * kStMaxSlots;
   int8_t* xq = reinterpret_cast<int8_t*>(st_sm + g.sm.xq);
@@ -217,6 +217,7 @@ step_gemv_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
   const int nslots = STREAM ? g.nslots : 1, slot_tiles = g.slot_tiles;
   unsigned char* wring = st_sm + g.sm.ring + (size_t)warp * nslots * slot_tiles * 512;
   int ps = 0;                                                            // slot of the next fill
+  const bool leader = elect_one();
   auto issue = [&]() {
     if (STREAM) {
 #pragma unroll 1
@@ -225,14 +226,14 @@ step_gemv_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
     if (pc.left <= 0) return;
     int n = STREAM ? min(slot_tiles, pc.left) : pc.left;
     uint64_t* bar = &bars[ps];
-    if (lane == 0) mbar_arrive_expect_tx(bar, (uint32_t)n * 512u);
+    if (leader) mbar_arrive_expect_tx(bar, (uint32_t)n * 512u);
     unsigned char* dst = wring + (size_t)ps * slot_tiles * 512;
     const uint4* src = g.w + ((size_t)(t0 + pc.tile) * g.KT + kt0 + pc.kt) * 32;
     pc.left -= n;
 #pragma unroll 1
     while (n > 0) {                                                      // one copy per row tile (one in all when K is not split)
       const int len = g.slices == 1 ? n : min(n, KTs - pc.kt);
-      if (lane == 0) bulk_load_1d(dst, src, (uint32_t)len * 512u, bar);
+      if (leader) bulk_load_1d(dst, src, (uint32_t)len * 512u, bar);
       dst += len * 512;
       n -= len;
       pc.kt += len;
@@ -247,7 +248,7 @@ step_gemv_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
       if (++ps == nslots) ps = 0;
     }
   };
-  if (lane == 0) {
+  if (leader) {
 #pragma unroll 1
     for (int s = 0; s < nslots; ++s) mbar_init(&bars[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -695,7 +696,7 @@ step_attn_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
   constexpr int half = HD / 2, VEC = HD / 32, PARTS = kAtThreads / half;      // key shares of the P V stage
   extern __shared__ __align__(128) unsigned char st_sm[];
   const ModelDims& dm = a.dims;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   unsigned char* kvbuf = st_sm;
   float* q_s = reinterpret_cast<float*>(st_sm + (size_t)g.nbuf * st_kv_bytes<T, HD>());   // [G][HD], scaled by 1/sqrt(HD)
   float* k_s = q_s + G * HD;
@@ -723,7 +724,7 @@ step_attn_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
   const bool has_new = k1 == pos + 1;
   const int k1c = has_new ? pos : k1;          // cached keys [k0, k1c)
   const int nrounds = (k1 - k0 + kStKeys - 1) / kStKeys;
-  auto issue = [&](int r) {                    // thread 0
+  auto issue = [&](int r) {                    // one thread
     const int b = r % g.nbuf, ka = k0 + r * kStKeys, n = min(kStKeys, k1c - ka);
     if (n <= 0) { mbar_arrive(&bars[b]); return; }
     constexpr uint32_t rowb = HD * sizeof(T);
@@ -738,7 +739,7 @@ step_attn_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
       done += len;
     }
   };
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
 #pragma unroll 1
     for (int b = 0; b < g.nbuf; ++b) mbar_init(&bars[b], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -884,7 +885,7 @@ step_attn_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
     }
     if (r + 1 < nrounds) {
       __syncthreads();                         // everyone is done with the buffer, the probabilities and cr
-      if (threadIdx.x == 0 && r + g.nbuf < nrounds) issue(r + g.nbuf);
+      if (warp == 0 && r + g.nbuf < nrounds && elect_one()) issue(r + g.nbuf);
     }
   }
   // ---- the key shares meet, the split's state goes out
