@@ -63,6 +63,18 @@ inline void raise_dyn_smem(void (*kernel)(KArgs...), size_t bytes) {
   raise_dyn_smem(reinterpret_cast<const void*>(kernel), bytes);
 }
 
+// Asks for the largest share of an SM's memory as shared memory, whatever the kernel uses of it.  An SM changes its split
+// only when it is empty: a kernel that leaves most of it to L1 keeps its successor's CTAs, which a programmatic edge
+// launches ahead of its end, off the SM.  Said of every kernel of the chains that those edges connect, where the setup is
+// done (the gate / up CTAs of a decode step started 2 us late behind an O projection that needs 20 KB).
+inline void share_memory(const void* kernel) {
+  B2_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+}
+template <typename... KArgs>
+inline void share_memory(void (*kernel)(KArgs...)) {
+  share_memory(reinterpret_cast<const void*>(kernel));
+}
+
 constexpr int kPage = 256;       // KV positions per page
 constexpr int kMaxBuckets = 8;
 

@@ -39,7 +39,7 @@ struct Launch {
 
 template <typename... KArgs, typename... Args>
 void go(const Launch& l, void (*kernel)(KArgs...), int grid, int block, size_t smem, Args&&... args) {
-  if (l.fits) { raise_dyn_smem(kernel, smem); return; }
+  if (l.fits) { raise_dyn_smem(kernel, smem); share_memory(kernel); return; }
   if (l.pdl) launch_pdl(kernel, dim3(grid), dim3(block), smem, l.st, std::forward<Args>(args)...);
   else kernel<<<grid, block, smem, l.st>>>(std::forward<Args>(args)...);
 }

@@ -434,7 +434,7 @@ wide_attn_kernel(ModelDims dm, WideAttnArgs a) {
 }
 
 // Host side: the kernel instantiated for the cache type, head size and group size.  nb <= 0 only sets the
-// kernel's shared-memory attribute (executor creation, outside any stream capture).
+// kernel's shared-memory attributes (executor creation, outside any stream capture).
 template <typename T, int HD, int G>
 inline void launch_wide_attn_t(cudaStream_t st, const ModelDims& d, int nb, size_t smem_optin, WideAttnArgs a) {
   const size_t fixed = wa_fixed_bytes(HD, G);
@@ -452,7 +452,7 @@ inline void launch_wide_attn_t(cudaStream_t st, const ModelDims& d, int nb, size
   a.stages = stages;
   const size_t smem = fixed + (size_t)stages * stage;
   raise_dyn_smem(wide_attn_kernel<T, HD, G>, smem);
-  if (nb <= 0) return;
+  if (nb <= 0) { share_memory(wide_attn_kernel<T, HD, G>); return; }
   launch_pdl(wide_attn_kernel<T, HD, G>, dim3(nb * d.hkv * a.nsplit), dim3(kWaThreads), smem, st, d, a);
 }
 template <typename T, int HD>

@@ -326,16 +326,17 @@ void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bflo
     B2_CUDA(cudaGetDevice(&dev));
     B2_CHECK(dev >= 0 && dev < 64, kInternal, "device ordinal out of range");
     if (!sms_of[dev]) {
-      raise_dyn_smem(gemm_w4_ts_kernel<0, 256>, (size_t)ts_smem(256));
-      raise_dyn_smem(gemm_w4_ts_kernel<1, 256>, (size_t)ts_smem(256));
-      raise_dyn_smem(gemm_w4_ts_kernel<0, 128>, (size_t)ts_smem(128));
-      raise_dyn_smem(gemm_w4_ts_kernel<1, 128>, (size_t)ts_smem(128));
-      raise_dyn_smem(gemm_w4_ts_kernel<0, 64>, (size_t)ts_smem(64));
-      raise_dyn_smem(gemm_w4_ts_kernel<1, 64>, (size_t)ts_smem(64));
-      raise_dyn_smem(gemm_w4_ts_kernel<0, 32>, (size_t)ts_smem(32));
-      raise_dyn_smem(gemm_w4_ts_kernel<1, 32>, (size_t)ts_smem(32));
-      raise_dyn_smem(gemm_w4_ts_kernel<0, 16>, (size_t)ts_smem(16));
-      raise_dyn_smem(gemm_w4_ts_kernel<1, 16>, (size_t)ts_smem(16));
+#define B2_TS_PREP(NTOK_)                                              \
+  raise_dyn_smem(gemm_w4_ts_kernel<0, NTOK_>, (size_t)ts_smem(NTOK_)); \
+  raise_dyn_smem(gemm_w4_ts_kernel<1, NTOK_>, (size_t)ts_smem(NTOK_)); \
+  share_memory(gemm_w4_ts_kernel<0, NTOK_>);                           \
+  share_memory(gemm_w4_ts_kernel<1, NTOK_>)
+      B2_TS_PREP(16);
+      B2_TS_PREP(32);
+      B2_TS_PREP(64);
+      B2_TS_PREP(128);
+      B2_TS_PREP(256);
+#undef B2_TS_PREP
       B2_CUDA(cudaDeviceGetAttribute(&sms_of[dev], cudaDevAttrMultiProcessorCount, dev));
     }
     const int sms = sms_of[dev];
@@ -371,6 +372,16 @@ void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bflo
 }
 
 // --------------------------------------------------------------- the executor
+
+template <typename T>
+static auto kv_append_kernel(const ModelDims& d) {
+  switch (d.hd) {
+    case 32: return pf_kv_append_kernel<T, 32>;
+    case 64: return pf_kv_append_kernel<T, 64>;
+    case 128: return pf_kv_append_kernel<T, 128>;
+    default: return pf_kv_append_kernel<T, 256>;
+  }
+}
 
 static int round_up(int v, int a) { return (v + a - 1) / a * a; }
 
@@ -622,11 +633,21 @@ std::unique_ptr<Executor> Executor::create(std::shared_ptr<Model> model, const B
       cuuint32_t vb[2] = {(cuuint32_t)kFaBN, (cuuint32_t)d.hd};
       e->tm_vt.push_back(make_bf16_map(e->kv_host[i].v16, 2, vd, vs, vb));
     }
-    if (d.hd == 256)
+    if (d.hd == 256) {
       raise_dyn_smem(flash_prefill_tc_kernel<256>, (size_t)(FaSmem<256>::kTotal));
-    else
+      share_memory(flash_prefill_tc_kernel<256>);
+    } else {
       raise_dyn_smem(flash_prefill_tc_kernel<128>, (size_t)(FaSmem<128>::kTotal));
+      share_memory(flash_prefill_tc_kernel<128>);
+    }
   }
+  share_memory(pf_embed_norm_kernel);
+  share_memory(pf_resid_norm_reg_kernel<128, 3, 4>);
+  share_memory(pf_resid_norm_reg_kernel<256, 3, 4>);
+  share_memory(pf_resid_norm_reg_kernel<512, 3, 4>);
+  if (d.kv_dtype == 0) share_memory(kv_append_kernel<float>(d));
+  else share_memory(kv_append_kernel<__nv_bfloat16>(d));
+  share_memory(wide_argmax_kernel);
   raise_dyn_smem(pf_attn_kernel, sizeof(float) * ((size_t)(d.group() + 2) * d.hd + (size_t)8 * d.group() * (d.hd + 2)));
   if (e->prefill_gemm == B200LM_GEMM_TCGEN05) {
     e->tm_h = make_activation_map(e->pf_h, (int)tp, d.d);
@@ -737,14 +758,7 @@ static void launch_kv_append(cudaStream_t st, const ModelDims& d, int T_, const 
   const int groups = (T_ + pos0 % kKvaTok + kKvaTok - 1) / kKvaTok;
   const int grid = groups * d.hkv + (qout ? (T_ * d.hq + kKvaTok - 1) / kKvaTok : 0);
   const size_t stride = (size_t)T_ * d.nqkv();
-#define B2_KVA(HD_) launch_pdl(pf_kv_append_kernel<T, HD_>, dim3(grid), dim3(kKvaThreads), 0, st, d, qkv, nparts, stride, T_, pos0, pt, L.g_k, c, s, kv, L.g_q, qout)
-  switch (d.hd) {
-    case 32: B2_KVA(32); break;
-    case 64: B2_KVA(64); break;
-    case 128: B2_KVA(128); break;
-    default: B2_KVA(256); break;
-  }
-#undef B2_KVA
+  launch_pdl(kv_append_kernel<T>(d), dim3(grid), dim3(kKvaThreads), 0, st, d, qkv, nparts, stride, T_, pos0, pt, L.g_k, c, s, kv, L.g_q, qout);
 }
 
 void Executor::run_prefill_chunk(const int* tokens, int T, int start) {

@@ -250,6 +250,10 @@ inline void launch_gemm_small(cudaStream_t st, int sms, int device, const uint4*
     raise_dyn_smem(gemm_w4_small_kernel<1, 1>, (size_t)kGsMaxSmem);
     raise_dyn_smem(gemm_w4_small_kernel<0, 2>, (size_t)kGsMaxSmem);
     raise_dyn_smem(gemm_w4_small_kernel<1, 2>, (size_t)kGsMaxSmem);
+    share_memory(gemm_w4_small_kernel<0, 1>);
+    share_memory(gemm_w4_small_kernel<1, 1>);
+    share_memory(gemm_w4_small_kernel<0, 2>);
+    share_memory(gemm_w4_small_kernel<1, 2>);
     ready[device] = 1;
   }
   const dim3 grid(g.cps * ksplit), block(kGsThreads);
