@@ -68,7 +68,7 @@ void launch_gemv(const Launch& l, const DecodeArgs& a, const StepPlan& pl, StepG
   g.kmax = g.KTs * 64;
   g.xstride = st_xstride(g.kmax);
   g.inv_k = 1.0f / (float)g.kmax;
-  g.heads = PRO == kStCombine ? g.kmax / a.dims.hd : 0;
+  g.heads = PRO == kStCombine || PRO == kStCombineShort ? g.kmax / a.dims.hd : 0;
   for (g.hd_log2 = 0; (1 << g.hd_log2) < a.dims.hd;) ++g.hd_log2;
   // sums of a head CTA's tiles are held in two goes, so that the ring keeps most of the shared memory
   g.round_tiles = std::min(most, 64);
@@ -160,7 +160,9 @@ int run(Launch l, const DecodeArgs& a, const StepPlan& pl, const LayerWeights* l
     o.w = L.wo; o.wscale = L.so; o.tiles = d.d / 16; o.KT = KTo; o.slices = pl.o_slices; o.y = pl.opart;
     o.part_o = pl.part_o; o.part_ml = pl.part_ml; o.nsplit = pl.nsplit[L.is_global ? 1 : 0]; o.is_global = L.is_global;
     o.bar = 5 * i + 2;
-    launch_gemv<kStCombine, kStPlain>(l, a, pl, o);
+    // one head of 256 or two of 128 in a slice of K, and sessions that have the warps for it
+    if (d.hd >= 128 && d.nq() / pl.o_slices <= 256) launch_gemv<kStCombineShort, kStPlain>(l, a, pl, o);
+    else launch_gemv<kStCombine, kStPlain>(l, a, pl, o);
     if (reduce) reduce(ctx, pl.opart, (size_t)pl.o_slices * a.ncols * d.d);
     StepGemv gu{};
     gu.w = L.wgu; gu.wscale = L.sgu; gu.tiles = 2 * d.ffn / 16; gu.KT = KTd; gu.slices = 1; gu.y = a.act;

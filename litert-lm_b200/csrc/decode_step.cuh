@@ -34,7 +34,7 @@ constexpr int kStKeys = 32;               // keys of one attention round (one pe
 constexpr int kStMaxSplits = 64;
 constexpr int kAtThreads = 256;
 
-enum StepPrologue { kStResid = 0, kStAct = 1, kStCombine = 2 };
+enum StepPrologue { kStResid = 0, kStAct = 1, kStCombine = 2, kStCombineShort = 3 };
 enum StepEpilogue { kStPlain = 0, kStGeglu = 1, kStHead = 2 };
 
 // Byte offsets of a projection's shared-memory areas (made on the host).
@@ -143,6 +143,12 @@ __device__ __forceinline__ void st_stamp(const DecodeArgs& a, int bar, int k) {
 
 __device__ __forceinline__ float4 st_ld4(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
 
+// Maximum over the warp in one instruction: of floats that are not negative (their bits order as they do), and of any.
+__device__ __forceinline__ float st_warp_absmax(float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v))); }
+__device__ __forceinline__ float st_warp_max(float v) {
+  const int b = __float_as_int(v), k = __reduce_max_sync(0xffffffffu, b ^ ((b >> 31) & 0x7fffffff));
+  return __int_as_float(k ^ ((k >> 31) & 0x7fffffff));
+}
 __device__ __forceinline__ float st_absmax(float4 v) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))); }
 __device__ __forceinline__ float st_sq(float4 v) { return (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w); }
 
@@ -369,11 +375,77 @@ step_gemv_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
     }
     // sum and maximum share one pass through shared memory
     ss2 = warp_sum(ss2);
-    m = warp_max(m);
+    m = st_warp_absmax(m);
     if (lane == 0) { scratch[16 + slot_r] = ss2; scratch[32 + slot_r] = m; }
     __syncthreads();
     m = st_max_row<W>(scratch + 32 + col * W);
     post = rsqrtf(st_sum_row<W>(scratch + 16 + col * W) * g.inv_k + a.dims.eps);   // the row factor leaves with the column scale
+  } else if constexpr (PRO == kStCombineShort) {
+    // The combine below for a slice of at most 256 values and heads of 128 and more: a warp's 128 values belong to one
+    // head, so it makes the weights of that head's splits itself and takes them out of its lanes; one warp of the session
+    // then adds the split groups, and the vector's maximum is a maximum over its lanes.  Two barriers of the CTA instead of
+    // four: the prologue of the 1B model's O projection takes 2.2 us, 2.6 with the general form.
+    const int k4 = g.kmax / 4, wide = k4 > 32, sg = W >> wide, sgi = gw >> wide, c4 = (wide ? (gw & 1) * 32 : 0) + lane;
+    const int hd = 1 << g.hd_log2, G = a.dims.hq / a.dims.hkv, h = slice * g.heads + ((4 * c4) >> g.hd_log2), kvh = h / G;
+    const int pos = colok ? __ldcg(&a.st->pos[col]) : 0;                 // has not changed since the step began
+    const int nkeys = st_visible(a.dims, min(max(pos, 0), a.dims.max_ctx - 1), g.is_global);
+    const int chunk = st_chunk(nkeys, g.nsplit), na = colok ? (nkeys + chunk - 1) / chunk : 0;      // splits that hold keys
+    const size_t base = (((size_t)col * a.dims.hkv + kvh) * g.nsplit) * G + (h - kvh * G), sstride = (size_t)G << g.hd_log2;
+    const float* p = g.part_o + (base << g.hd_log2) + ((4 * c4) & (hd - 1));
+    const float* ml = g.part_ml + base * 2;
+    float4* part = reinterpret_cast<float4*>(st_sm + g.sm.vals);         // [split groups][ncols][k4]
+    pdl_wait();
+    pdl_launch_dependents();
+    st_stamp(a, g.bar, 1);
+    float2 x[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int s = lane + 32 * q;
+      x[q] = s < na ? __ldcg(reinterpret_cast<const float2*>(ml + (size_t)s * G * 2)) : make_float2(-INFINITY, 0.f);
+    }
+    constexpr int kAhead = 4;
+    float4 pre[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) pre[u] = sgi + u * sg < na ? st_ld4(p + (sgi + u * sg) * sstride) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float M = st_warp_max(fmaxf(x[0].x, x[1].x));
+    float w0 = __expf(x[0].x - M), w1 = __expf(x[1].x - M);
+    const float Lsum = warp_sum(x[0].y * w0 + x[1].y * w1), inv = Lsum > 0.f ? __fdividef(1.0f, Lsum) : 0.f;
+    w0 *= inv;
+    w1 *= inv;
+    auto weight = [&](int s) { return __shfl_sync(0xffffffffu, s < 32 ? w0 : w1, s & 31); };
+    float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](const float4& o, float w) { s4.x += w * o.x; s4.y += w * o.y; s4.z += w * o.z; s4.w += w * o.w; };
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const float w = weight(sgi + u * sg);                              // zero past the last split, or read as zero
+      add(pre[u], sgi + u * sg < na ? w : 0.f);
+    }
+#pragma unroll 2
+    for (int s = sgi + kAhead * sg; s < na; s += sg) add(st_ld4(p + s * sstride), weight(s));
+    if (colok) part[(sgi * ncols + col) * k4 + c4] = s4;
+    __syncthreads();
+    if (gw == 0 && colok) {
+      float4 y[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        y[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c <= wide) {
+#pragma unroll
+          for (int q = 0; q < W; ++q)
+            if (q < sg && c * 32 + lane < k4) {
+              const float4 o = part[(q * ncols + col) * k4 + c * 32 + lane];
+              y[c].x += o.x; y[c].y += o.y; y[c].z += o.z; y[c].w += o.w;
+            }
+        }
+        m = fmaxf(m, st_absmax(y[c]));
+      }
+      m = st_warp_absmax(m);
+      const float k = m > 0.f ? __fdividef(127.0f, m) * 0.9999999f : 0.f;
+      if (lane == 0) colscale[col] = k > 0.f ? __fdividef(post, k) : 0.f;
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        if (c * 32 + lane < k4) st_quantize4(make_float4(y[c].x * k, y[c].y * k, y[c].z * k, y[c].w * k), nterms, q0, 4 * (c * 32 + lane), xstride);
+    }
   } else {
     const int K = g.kmax, k4 = K / 4;
 #pragma unroll
@@ -471,12 +543,12 @@ step_gemv_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
     }
 #pragma unroll
     for (int u = 0; u < NV; ++u) m = fmaxf(m, st_absmax(v[u]));
-    m = warp_max(m);
+    m = st_warp_absmax(m);
     if (lane == 0) scratch[warp] = m;
     __syncthreads();
     m = st_max_row<W>(scratch + col * W);
   }
-  {
+  if constexpr (PRO != kStCombineShort) {
     const float k = m > 0.f ? __fdividef(127.0f, m) * 0.9999999f : 0.f;    // never above 127, whatever the quotient's last bit
     if (tl == 0 && colok) colscale[col] = k > 0.f ? __fdividef(post, k) : 0.f;
 #pragma unroll
