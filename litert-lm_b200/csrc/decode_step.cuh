@@ -876,6 +876,25 @@ step_attn_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
   float o[G][2];
 #pragma unroll
   for (int h = 0; h < G; ++h) o[h][0] = o[h][1] = 0.f;
+  auto append = [&](int first, int step) {
+    T* kbase = reinterpret_cast<T*>(g.kv.k);
+    T* vbase = reinterpret_cast<T*>(g.kv.v);
+    const int page = ptab[pos / kPage], slot = pos % kPage;
+    const size_t off = (((size_t)page * dm.hkv + kvh) * kPage + slot) * HD;
+#pragma unroll 1
+    for (int e = first; e < HD; e += step) {
+      if constexpr (sizeof(T) == 4) {
+        kbase[off + e] = k_s[e];
+        vbase[off + e] = v_s[e];
+        if (g.kv.k16) g.kv.k16[off + e] = __float2bfloat16(k_s[e]);
+      } else {
+        kbase[off + e] = __float2bfloat16(k_s[e]);
+        vbase[off + e] = __float2bfloat16(v_s[e]);
+      }
+      if (g.kv.v16) g.kv.v16[(((size_t)page * dm.hkv + kvh) * HD + e) * kPage + slot] = __float2bfloat16(v_s[e]);
+    }
+    asm volatile("fence.proxy.async.global;" ::: "memory");     // later steps fetch these rows with bulk copies
+  };
   bool ok = true;
 #pragma unroll 1
   for (int r = 0; r < nrounds; ++r) {
@@ -932,6 +951,8 @@ step_attn_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
       if (lane < n) sc[lane * G + warp] = p;
       __syncwarp();
       if (lane == 0) { cr[warp] = f; cr[G + warp] = m1; cr[2 * G + warp] = cr[2 * G + warp] * f + ps; }
+    } else if (has_new && r == 0) {            // the other warps append meanwhile: at the end, the stores held up the kernel's completion
+      append(threadIdx.x - 32 * G, kAtThreads - 32 * G);
     }
     __syncthreads();
     // ---- P V: elements e2, e2 + 1, keys part, part + PARTS, ...
@@ -976,25 +997,6 @@ step_attn_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
   if (threadIdx.x < G) {
     g.part_ml[(pi + threadIdx.x) * 2] = cr[G + threadIdx.x];
     g.part_ml[(pi + threadIdx.x) * 2 + 1] = cr[2 * G + threadIdx.x];
-  }
-  if (has_new) {                               // append
-    T* kbase = reinterpret_cast<T*>(g.kv.k);
-    T* vbase = reinterpret_cast<T*>(g.kv.v);
-    const int page = ptab[pos / kPage], slot = pos % kPage;
-    const size_t off = (((size_t)page * dm.hkv + kvh) * kPage + slot) * HD;
-#pragma unroll 1
-    for (int e = threadIdx.x; e < HD; e += kAtThreads) {
-      if constexpr (sizeof(T) == 4) {
-        kbase[off + e] = k_s[e];
-        vbase[off + e] = v_s[e];
-        if (g.kv.k16) g.kv.k16[off + e] = __float2bfloat16(k_s[e]);
-      } else {
-        kbase[off + e] = __float2bfloat16(k_s[e]);
-        vbase[off + e] = __float2bfloat16(v_s[e]);
-      }
-      if (g.kv.v16) g.kv.v16[(((size_t)page * dm.hkv + kvh) * HD + e) * kPage + slot] = __float2bfloat16(v_s[e]);
-    }
-    asm volatile("fence.proxy.async.global;" ::: "memory");     // later steps fetch these rows with bulk copies
   }
   st_stamp(a, g.bar, 4);
   if (!ok)
