@@ -18,6 +18,9 @@
 // overflow, and the O accumulator in tensor memory never has to be rescaled.
 // (Layers whose bound is too large for fp32 exponents use the CUDA-core kernel.)
 //
+// At head size 256 the queries are copied to tensor memory and enter S = Q K^T from there: an M128 N64 K16 product takes 32
+// cycles, but reading its 4 KB of Q from shared memory about 60.
+//
 // S is double buffered in tensor memory and the MMA warp issues S(j+1) before
 // P(j) V(j), so the tensor pipe works on the next scores while the softmax
 // warps turn the current ones into probabilities.  K and V tiles have their
@@ -84,6 +87,7 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
   volatile int* sm_fail = reinterpret_cast<volatile int*>(bars + 15);   // a softmax thread's wait gave up
   float* l_part = reinterpret_cast<float*>(bars + 16);     // [128] row sums of the upper 32 keys
+  uint64_t* q_tmem = bars + 80;       // Q copied to tensor memory
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int G = g.hq / g.hkv;
@@ -92,7 +96,9 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   const int t0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * TT, kvh = blockIdx.y;
   constexpr int KB = HD / 64;                   // 64-column blocks of the head dimension
   constexpr uint32_t kTmemCols = HD + 2 * kFaBN <= 256 ? 256 : 512;
-  constexpr uint32_t kOCol = 0, kSCol = HD;     // O, then two S buffers of 64 columns
+  constexpr uint32_t kOCol = 0, kSCol = HD;     // O, then two S buffers of 64 columns, then Q where it fits
+  constexpr bool kQTmem = HD == 256;            // with head size 128, two CTAs share an SM's tensor memory
+  constexpr uint32_t kQCol = HD + 2 * kFaBN;
 
   // key range of this query tile
   const int qpos_min = g.start + t0;
@@ -112,6 +118,7 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       mbar_init(&p_full[s], 8);
     }
     mbar_init(o_full, 1);
+    mbar_init(q_tmem, 8);
     *sm_fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -167,13 +174,14 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         const uint64_t kd = umma_desc_sw128(smem_u32(sK + s * L::kK + kb * kFaBN * 128));
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          umma_bf16(tmem + kSCol + s * kFaBN, qd + (uint64_t)(k * 2), kd + (uint64_t)(k * 2), idesc_s, (kb | k) ? 1u : 0u);
+          if constexpr (kQTmem) umma_bf16_ts(tmem + kSCol + s * kFaBN, tmem + kQCol + (kb * 4 + k) * 8, kd + (uint64_t)(k * 2), idesc_s, (kb | k) ? 1u : 0u);
+          else umma_bf16(tmem + kSCol + s * kFaBN, qd + (uint64_t)(k * 2), kd + (uint64_t)(k * 2), idesc_s, (kb | k) ? 1u : 0u);
       }
       umma_commit(&s_full[s]);
       umma_commit(&k_empty[s]);
     };
     const bool leader = elect_one();
-    bool ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0, g.err) && mbar_wait(&k_full[0], 0, g.err));
+    bool ok = __all_sync(0xffffffffu, mbar_wait2(kQTmem ? q_tmem : q_full, 0, &k_full[0], 0, g.err));
     if (ok) {
       tc_fence_after();
       if (leader) issue_s(0);
@@ -214,6 +222,25 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     const float shift = g.bound * log2e;
     float lsum = 0.f;
     bool ok = true;
+    if constexpr (kQTmem) {                            // half of the row's queries into tensor memory
+      if (mbar_wait(q_full, 0, g.err)) {
+#pragma unroll
+        for (int c = 0; c < HD / 2; c += 32) {
+          uint32_t q[16];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int col = khalf * (HD / 2) + c + 8 * i;
+            const uint4 w = *reinterpret_cast<const uint4*>(sQ + col / 64 * 128 * 128 + r * 128 + (((col % 64 / 8) ^ (r & 7)) << 4));
+            q[4 * i] = w.x; q[4 * i + 1] = w.y; q[4 * i + 2] = w.z; q[4 * i + 3] = w.w;
+          }
+          tmem_st16(lane_addr + kQCol + (khalf * (HD / 2) + c) / 2, q);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(q_tmem);
+      }
+    }
     // The eight warps leave this loop together: a thread whose wait gave up raises
     // sm_fail before the named barrier, everyone reads it after.
     for (int j = 0; j < ntiles; ++j) {

@@ -445,6 +445,27 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   atomicExch(err, (int)kDevBarrierTimeout);
   return false;
 }
+// The same for two barriers at once: one round trip where both are complete.
+__device__ __forceinline__ bool mbar_wait2(uint64_t* bar0, uint32_t parity0, uint64_t* bar1, uint32_t parity1, int* err) {
+  const uint32_t addr0 = smem_u32(bar0), addr1 = smem_u32(bar1);
+#pragma unroll 1
+  for (int tries = 0; tries < (1 << 22); ++tries) {
+    uint32_t done;
+    asm volatile(
+        "{\n.reg .pred p, q;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n"
+        "and.pred p, p, q;\n"
+        "selp.b32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(addr0), "r"(parity0), "r"(addr1), "r"(parity1)
+        : "memory");
+    if (done) return true;
+    if ((tries & 1023) == 1023 && *reinterpret_cast<volatile int*>(err) == (int)kDevBarrierTimeout) return false;
+  }
+  atomicExch(err, (int)kDevBarrierTimeout);
+  return false;
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
