@@ -164,7 +164,7 @@ wide_attn_kernel(ModelDims dm, WideAttnArgs a) {
   uint64_t* full = reinterpret_cast<uint64_t*>(ored + 2 * kWaThreads * G);
   int* last = reinterpret_cast<int*>(full + kWaMaxStages);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int split = blockIdx.x % a.nsplit, pair = blockIdx.x / a.nsplit, kvh = pair % dm.hkv, qi = pair / dm.hkv;
   int pos = __ldcg(a.pos + qi);                // written two kernels back or earlier, as the cached rows are
   if (pos < 0 || pos >= dm.max_ctx) {
@@ -179,7 +179,7 @@ wide_attn_kernel(ModelDims dm, WideAttnArgs a) {
   const bool has_new = !a.appended && k1 == pos + 1 && k1 > k0;
   const int k1c = has_new ? pos : k1;          // cached keys [k0, k1c)
   const int nrounds = k1 > k0 ? (k1 - k0 + KEYS - 1) / KEYS : 0;
-  auto issue = [&](int r) {                    // thread 0
+  auto issue = [&](int r) {                    // one thread
     const int b = r % S, ka = k0 + r * KEYS, n = min(KEYS, k1c - ka);
     if (n <= 0) { mbar_arrive(&full[b]); return; }
     unsigned char* dst = wa_sm + (size_t)b * kStage;
@@ -194,7 +194,7 @@ wide_attn_kernel(ModelDims dm, WideAttnArgs a) {
       done += len;
     }
   };
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
 #pragma unroll 1
     for (int s = 0; s < S; ++s) mbar_init(&full[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -357,7 +357,7 @@ wide_attn_kernel(ModelDims dm, WideAttnArgs a) {
     }
     if (r + 1 < nrounds) {
       __syncthreads();                         // everyone is done with the stage, the probabilities and cr
-      if (threadIdx.x == 0 && r + S < nrounds) issue(r + S);
+      if (warp == 0 && r + S < nrounds && elect_one()) issue(r + S);
     }
   }
   // ---- the key shares meet
