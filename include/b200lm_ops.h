@@ -102,8 +102,9 @@ int B200LmOps_AttentionPrefillTc(int32_t device, const float* q, const float* k,
  * waiting.
  *
  * With all four data pointers on 16-byte boundaries the kernel of
- * csrc/attn_mma.cuh runs, which reads the cache once for the whole batch and
- * picks its own number of splits; nsplit then only enters the size check below.
+ * csrc/attn_mma.cuh runs, or that of csrc/attn_tc.cuh for many queries over a
+ * long bf16 cache; they read the cache once for the whole batch and pick their
+ * own number of splits; nsplit then only enters the size check below.
  * Otherwise the split kernel of csrc/decode_ops.cuh runs with nsplit splits.
  *
  * Limits: batch <= 16368 and batch*hq*nsplit*(hd+2)*4 bytes <= 8 MiB - 64 KiB;

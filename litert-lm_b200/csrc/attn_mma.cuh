@@ -5,9 +5,8 @@
 // tensor-core products as up to three bf16 terms each (x = hi + mid + lo, 24 bits) and the products whose
 // weight is above 2^-24 are accumulated in fp32.  The tensor core cuts its sums off rather than rounding them, so no
 // long sum stays in its accumulators: scores leave them every 64 elements, P V every 16 keys (left in them over 32768
-// keys, the result was off by 2e-6 where fp32 adds are off by 3e-7).  tcgen05 would want the three query terms of a 128-row tile
-// (192 KB at head size 256) next to the K / V stages; they do not fit, mma.sync takes them from shared memory
-// in 16-row pieces.  (About 40 rows with their three terms in ONE 128-row tile would fit; that has not been built.)
+// keys, the result was off by 2e-6 where fp32 adds are off by 3e-7).  Many rows over a long
+// bf16 cache run on tcgen05 instead (attn_tc.cuh), with an O accumulator per tile of keys for the same reason.
 //
 // A warp owns (row tile of 16 query rows) x (every KG-th chunk of 16 keys): scores, online softmax and P V of a
 // chunk stay in its registers, so warps meet only at the end.  The warps of a key group stream the chunks' K
@@ -17,8 +16,8 @@
 //   PACK: at most four rows: the three query terms share ONE 16-row tile (row 4 * term + r), which takes a third
 //   of the products; that is the shape bound by the cache bytes.
 //
-// What bounds it: 64 queries x 4 heads over 32768 bf16 keys of 256 are 6.3 M m16n8k16 products (the mma.sync
-// pipe); few rows over a long cache run at the cache's bytes; short caches at the launch.
+// What bounds it: the mma.sync pipe for many rows (54 % busy), the cache's bytes for few rows over a long cache, and for
+// short caches one chain of latencies.
 #pragma once
 #include <algorithm>
 

@@ -12,6 +12,7 @@
 // process exits.
 #include "../../include/b200lm_ops.h"
 #include "attn_mma.cuh"
+#include "attn_tc.cuh"
 #include "common.cuh"
 #include "decode_ops.cuh"
 #include "prefill_ops.cuh"
@@ -46,6 +47,7 @@ struct StaticScratch {
   unsigned char* base;
   unsigned* tickets;
   int sms;
+  int clusters[2];            // of attn_tc_kernel at head size 128 and 256
 };
 static StaticScratch g_static_scratch[kMaxDevices] = {};
 static std::mutex g_static_scratch_mu;     // guards the per-device set-up below
@@ -66,6 +68,9 @@ static StaticScratch static_scratch_for(int device) {
     // raised to the largest shape the entry point accepts and never lowered by any other caller.
     raise_dyn_smem(attn_decode_kernel, sizeof(float) * ((size_t)(4 + 2) * 256 + (size_t)kDecWarps * 4 * (256 + 2)));
     B2_CUDA(cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, device));
+    s.clusters[0] = atc_prepare<128>();
+    s.clusters[1] = atc_prepare<256>();
+    (void)encode_tiled_fn();
     s.tickets = reinterpret_cast<unsigned*>(t);
     s.base = reinterpret_cast<unsigned char*>(p);
   }
@@ -160,7 +165,15 @@ extern "C" int B200LmOps_AttentionDecodeStatic(int32_t device, const float* q_de
       const size_t per_split = (size_t)batch * hq * (hd + 2) * sizeof(float);
       const int cap = (int)std::min<size_t>(kTicketSplits, (kStaticScratchBytes - kStaticHeaderBytes) / per_split);
       a.part_ml = part_o + (size_t)batch * hq * cap * hd;
-      if (kv_bf16) launch_attn_shared_bf16(st, a, hd, device, sc.sms, cap, sc.tickets);
+      if (const int ns = kv_bf16 ? atc_splits(a, hd, sc.clusters[hd == 256], cap) : 0) {
+        // the pages of a cache as [page][kv head x slot][hd]; how many there are, only the caller knows
+        const cuuint64_t dims[3] = {(cuuint64_t)hd, (cuuint64_t)hkv * kPage, 1ull << 24};
+        const cuuint64_t strides[2] = {(cuuint64_t)hd * 2, (cuuint64_t)hkv * kPage * hd * 2};
+        const cuuint32_t box[3] = {64, kAtcKeys, 1};
+        const CUtensorMap tm_k = make_bf16_map(k_pages_dev, 3, dims, strides, box), tm_v = make_bf16_map(v_pages_dev, 3, dims, strides, box);
+        if (hd == 256) launch_attn_tc<256>(st, tm_k, tm_v, a, ns);
+        else launch_attn_tc<128>(st, tm_k, tm_v, a, ns);
+      } else if (kv_bf16) launch_attn_shared_bf16(st, a, hd, device, sc.sms, cap, sc.tickets);
       else launch_attn_shared_f32(st, a, hd, device, sc.sms, cap, sc.tickets);
       return kOk;
     }

@@ -49,6 +49,17 @@ def test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window,
     assert err < 2e-6, err
 
 
+@pytest.mark.parametrize("batch,s,window,hq,hkv,hd", [
+    (16, 1000, 0, 4, 1, 256), (33, 1023, 1001, 4, 1, 256),      # the shortest, a row tile and four rows, both ends inside a tile
+    (64, 4097, 0, 4, 1, 256), (32, 1281, 0, 4, 1, 128),
+    (10, 8001, 0, 4, 1, 256), (20, 2500, 0, 8, 4, 128),         # at most 48 rows
+    (49, 3000, 1500, 2, 2, 128), (64, 1700, 0, 32, 16, 128),    # a group of one; 16 units
+    (64, 1100, 0, 32, 32, 128),                                 # as many units as leave one split each
+])
+def test_many_rows_on_tcgen05(pkg, batch, s, window, hq, hkv, hd):
+    test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window, True)
+
+
 def test_unaligned_cache_goes_through_the_plain_kernel(pkg):
     gen = torch.Generator(device="cuda").manual_seed(5)
     s, hd = 300, 32
