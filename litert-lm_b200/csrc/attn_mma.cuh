@@ -157,6 +157,19 @@ attn_shared_kernel(const AmArgs a) {
     if (c < c1) asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(page) : "l"(a.page_table + c * 16 / kPage));
   };
   next_page(c0 + kg);
+  // a short query tile is asked for ahead of the cache rows, whose copies wait for the page number
+  constexpr int NQ = S::kRows * (HD / 2) / S::kThreads;
+  constexpr bool kQAhead = NQ <= 8 && NQ * S::kThreads == S::kRows * (HD / 2);
+  auto q_pair = [&](int i) {
+    const int r = i / (HD / 2), e = 2 * (i % (HD / 2));
+    return r0 + r < a.rows ? *reinterpret_cast<const float2*>(a.q + (size_t)((r0 + r) / a.G) * a.q_stride + (kvh * a.G + (r0 + r) % a.G) * HD + e)
+                           : make_float2(0.f, 0.f);
+  };
+  float2 qa[kQAhead ? NQ : 1];
+  if constexpr (kQAhead) {
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) qa[u] = q_pair(threadIdx.x + u * S::kThreads);
+  }
   int is_slot = 0, is_round = 0;               // slot and use of the slot of the next entry to issue
   auto issue = [&](int n) {
     const int isv = n & 1, c = c0 + kg + (n >> 1) * KG, slot = is_slot, round = is_round;
@@ -188,12 +201,8 @@ attn_shared_kernel(const AmArgs a) {
   for (int n = 0; n < NS - 1; ++n) issue(n);
   {
     // ---- query rows, scaled, as bf16 planes
-#pragma unroll 8
-    for (int i = threadIdx.x; i < S::kRows * (HD / 2); i += S::kThreads) {
+    auto place = [&](int i, float2 x) {
       const int r = i / (HD / 2), e = 2 * (i % (HD / 2));
-      float2 x = make_float2(0.f, 0.f);
-      if (r0 + r < a.rows)
-        x = *reinterpret_cast<const float2*>(a.q + (size_t)((r0 + r) / a.G) * a.q_stride + (kvh * a.G + (r0 + r) % a.G) * HD + e);
       uint32_t s3[3];
       am_split3(x.x * a.qscale, x.y * a.qscale, s3);
 #pragma unroll
@@ -202,6 +211,13 @@ attn_shared_kernel(const AmArgs a) {
         *reinterpret_cast<uint32_t*>(am_sm + row * S::kQRow + e * 2) = s3[p];
       }
       if (PACK) *reinterpret_cast<uint32_t*>(am_sm + (12 + r) * S::kQRow + e * 2) = 0u;
+    };
+    if constexpr (kQAhead) {
+#pragma unroll
+      for (int u = 0; u < NQ; ++u) place(threadIdx.x + u * S::kThreads, qa[u]);
+    } else {
+#pragma unroll 8
+      for (int i = threadIdx.x; i < S::kRows * (HD / 2); i += S::kThreads) place(i, q_pair(i));
     }
     __syncthreads();
     const uint32_t q_addr = smem_u32(am_sm) + (uint32_t)((mt * 16 + (lane & 15)) * S::kQRow + (lane >> 4) * 16);
@@ -500,30 +516,45 @@ attn_shared_kernel(const AmArgs a) {
       const int nr = min(S::kRows, a.rows - r0);
       float* w_s = reinterpret_cast<float*>(am_sm);                    // [row][nsplit]: exp2(m - M) / L
       const float2* ml = reinterpret_cast<const float2*>(a.part_ml) + ((size_t)kvh * a.rows + r0) * a.nsplit;
+      // A chain of round trips to L2 if written so: sixteen partials are in flight at once, the first of them ahead of the
+      // weights, and the (m, l) pairs of up to 32 splits are read once.
+      constexpr int P = 16;
+      const int items = nr * (HD / 4);
+      float4 x[P];
+      auto request = [&](int i, int p0) {
+        const float* po = a.part_o + ((size_t)kvh * a.rows + r0 + i / (HD / 4)) * a.nsplit * HD + 4 * (i % (HD / 4));
+#pragma unroll
+        for (int u = 0; u < P; ++u)
+          if (i < items && p0 + u < a.nsplit) x[u] = __ldcg(reinterpret_cast<const float4*>(po + (size_t)(p0 + u) * HD));
+      };
+      request(threadIdx.x, 0);
       for (int r = warp; r < nr; r += S::kThreads / 32) {
-        float M = -INFINITY, L = 0.f;
-        for (int s = lane; s < a.nsplit; s += 32) M = fmaxf(M, __ldcg(ml + (size_t)r * a.nsplit + s).x);
+        const float2 own = lane < a.nsplit ? __ldcg(ml + (size_t)r * a.nsplit + lane) : make_float2(-INFINITY, 0.f);
+        float M = own.x, L = 0.f;
+        for (int s = lane + 32; s < a.nsplit; s += 32) M = fmaxf(M, __ldcg(ml + (size_t)r * a.nsplit + s).x);
         M = warp_max(M);
         for (int s = lane; s < a.nsplit; s += 32) {
-          const float2 x = __ldcg(ml + (size_t)r * a.nsplit + s);
-          const float w = M > -INFINITY ? am_ex2(x.x - M) : 0.f;
+          const float2 y = s < 32 ? own : __ldcg(ml + (size_t)r * a.nsplit + s);
+          const float w = M > -INFINITY ? am_ex2(y.x - M) : 0.f;
           w_s[r * a.nsplit + s] = w;
-          L += w * x.y;
+          L += w * y.y;
         }
         L = warp_sum(L);
         const float inv = L > 0.f ? 1.0f / L : 0.f;
         for (int s = lane; s < a.nsplit; s += 32) w_s[r * a.nsplit + s] *= inv;
       }
       __syncthreads();
-      for (int i = threadIdx.x; i < nr * (HD / 4); i += S::kThreads) {
+      for (int i = threadIdx.x; i < items; i += S::kThreads) {
         const int r = i / (HD / 4), e = 4 * (i % (HD / 4));
-        const float* po = a.part_o + ((size_t)kvh * a.rows + r0 + r) * a.nsplit * HD + e;
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-        for (int p = 0; p < a.nsplit; ++p) {
-          const float4 x = __ldcg(reinterpret_cast<const float4*>(po + (size_t)p * HD));
-          const float w = w_s[r * a.nsplit + p];
-          s.x += w * x.x; s.y += w * x.y; s.z += w * x.z; s.w += w * x.w;
+        for (int p0 = 0; p0 < a.nsplit; p0 += P) {
+          if (i != (int)threadIdx.x || p0 > 0) request(i, p0);
+#pragma unroll
+          for (int u = 0; u < P; ++u)
+            if (p0 + u < a.nsplit) {
+              const float w = w_s[r * a.nsplit + p0 + u];
+              s.x += w * x[u].x; s.y += w * x[u].y; s.z += w * x[u].z; s.w += w * x[u].w;
+            }
         }
         *reinterpret_cast<float4*>(a.out + am_out_row(a, kvh, r0 + r) * HD + e) = s;
       }
