@@ -96,6 +96,7 @@ void launch_gemv(const Launch& l, const DecodeArgs& a, const StepPlan& pl, StepG
     return;
   }
   if (nv <= 1) launch_gemv_cp<PRO, EPI, 1>(l, a, g);
+  else if (nv <= 3) launch_gemv_cp<PRO, EPI, 3>(l, a, g);
   else if (nv <= 4) launch_gemv_cp<PRO, EPI, 4>(l, a, g);
   else launch_gemv_cp<PRO, EPI, 12>(l, a, g);
 }

@@ -141,6 +141,11 @@ __device__ __forceinline__ void st_stamp(const DecodeArgs& a, int bar, int k) {
   if (k == 1 && bar > 0) a.trace[(i - a.trace_ctas) * 2 + 1] = t;
 }
 
+// Asks for a line ahead of its use, without waiting for it or keeping the value.
+__device__ __forceinline__ void st_touch(const float* p) {
+  float x;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(x) : "l"(p));
+}
 __device__ __forceinline__ float4 st_ld4(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
 
 // Maximum over the warp in one instruction: of floats that are not negative (their bits order as they do), and of any.
@@ -313,6 +318,9 @@ step_gemv_kernel(const __grid_constant__ DecodeArgs a, const __grid_constant__ S
       if (kGainsAhead && vi[u] >= 0) {
         if (g.parts) gp[u] = __ldg(reinterpret_cast<const float4*>(g.g_post) + vi[u]);
         gq[u] = __ldg(reinterpret_cast<const float4*>(g.g_pre) + vi[u]);
+      } else if (vi[u] >= 0) {                                           // else into L1: they come from HBM in every step
+        if (g.parts) st_touch(g.g_post + 4 * vi[u]);
+        st_touch(g.g_pre + 4 * vi[u]);
       }
     }
     pdl_wait();
