@@ -53,6 +53,7 @@ void launch_gemv_s(const Launch& l, const DecodeArgs& a, const StepGemv& g) {
 template <int PRO, int EPI, int NV>
 void launch_gemv_cp(const Launch& l, const DecodeArgs& a, const StepGemv& g) {
   if (st_cols(a.ncols) == 1) launch_gemv_s<PRO, EPI, NV, 1>(l, a, g);
+  else if (st_cols(a.ncols) == 2) launch_gemv_s<PRO, EPI, NV, 2>(l, a, g);
   else launch_gemv_s<PRO, EPI, NV, 4>(l, a, g);
 }
 
@@ -90,7 +91,9 @@ void launch_gemv(const Launch& l, const DecodeArgs& a, const StepPlan& pl, StepG
   g.sm = st_smem(g, a.ncols, a.nterms);
   const int T = kStThreads / st_cols(a.ncols);
   const int nv = (g.kmax / 4 + T - 1) / T;                               // float4 of a vector per thread
-  if ((size_t)g.sm.total > pl.smem_optin || nv > 12) {
+  // one limit for every group: what the instantiation of four holds (two sessions alone would hold twice as much)
+  const int widest = 12 * (a.ncols <= 1 ? kStThreads : kStThreads / 4);
+  if ((size_t)g.sm.total > pl.smem_optin || g.kmax / 4 > widest) {
     B2_CHECK(l.fits != nullptr, kInternal, "the decode step does not fit, but was planned");
     *l.fits = false;
     return;

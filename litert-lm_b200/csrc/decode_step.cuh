@@ -71,10 +71,10 @@ struct StepGemv {
   int bar;                    // index of this kernel in the step (timeline)
 };
 
-// Session groups of a CTA.  Two and three sessions take the instantiation of four: half or a quarter of the warps have no
-// vector in the prologue.  A step of the 1B model at 300 keys is 554 / 744 / 779 / 838 us with 1 / 2 / 3 / 4 sessions; an
-// instantiation for two has not been built.
-__host__ __device__ inline int st_cols(int ncols) { return ncols <= 1 ? 1 : 4; }
+// Session groups of a CTA: three sessions take the instantiation of four, a quarter of whose warps then have no vector in the
+// prologue.  A step of the 1B model at 300 keys is 485 / 621 / 688 / 732 us with 1 / 2 / 3 / 4 sessions; two took 658 with the
+// instantiation of four.
+__host__ __device__ inline int st_cols(int ncols) { return ncols <= 2 ? (ncols <= 1 ? 1 : 2) : 4; }
 __host__ __device__ inline int st_xstride(int kmax) { return (kmax + 127) / 128 * 128 + 64; }
 
 inline StepSmem st_smem(const StepGemv& g, int ncols, int nterms) {
@@ -157,7 +157,7 @@ __device__ __forceinline__ float st_warp_max(float v) {
 __device__ __forceinline__ float st_absmax(float4 v) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))); }
 __device__ __forceinline__ float st_sq(float4 v) { return (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w); }
 
-// Sum or maximum of N floats in shared memory (N = 4 or 16, 16-byte aligned): wide loads, a tree.
+// Sum or maximum of N floats in shared memory (N = 4, 8 or 16, 16-byte aligned): wide loads, a tree.
 template <int N>
 __device__ __forceinline__ float st_sum_row(const float* p) {
   float4 v[N / 4];
@@ -184,7 +184,7 @@ __device__ __forceinline__ float st_max_row(const float* p) {
 }
 
 // One projection.  NV: float4 of a session's vector per thread; CP: session groups (one session: three terms and all
-// 16 warps on its vector; up to four: four warps each).
+// 16 warps on its vector; two: eight warps each; up to four: four).
 // STREAM: the warps' runs are longer than the ring (else a run is one slot, requested ahead of the wait and awaited
 // once).  A kernel runs its code once, so the code is kept short: nothing with a run-time count is unrolled (with the
 // compiler's unrolling these kernels were 60 - 120 KB each, and five of them in turn waited for instructions).

@@ -340,8 +340,9 @@ void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bflo
       B2_CUDA(cudaDeviceGetAttribute(&sms_of[dev], cudaDevAttrMultiProcessorCount, dev));
     }
     const int sms = sms_of[dev];
-    // At most 16 rows whose slice of X fits beside the weight ring: mma.sync (131072 x 2560, 16 rows: 48 us against 77 on
-    // tcgen05).  From 17 rows on it loses (13824 x 1152: 10.2 against 9.8 us at 20 rows, 12.8 against 9.9 at 32).
+    // At most 16 rows whose slice of X fits beside the weight ring: mma.sync (20480 x 2560 with GeGLU, 16 rows: 11.9 us against
+    // 13.2 on tcgen05; 4096 x 2560 and what follows it 7.0 against 7.3; of the 1B model's only gate/up loses, 6.8 against 6.1).
+    // From 17 rows on it loses (13824 x 1152: 10.2 against 6.9 us at 20 rows, 12.8 against 8.2 at 36).
     if (gs_fits(T, N, K / 64, ksplit, geglu, sms)) {
       launch_gemm_small(st, sms, dev, w4t, s4t, A, T, N, K, ksplit, geglu, outF, outB);
       B2_CUDA(cudaGetLastError());

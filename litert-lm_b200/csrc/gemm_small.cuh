@@ -3,8 +3,8 @@
 //   out[token][n] = scale[n] * sum_k W[n][k] X[token][k],  X bf16, W the 16 x 64 tiles of decode_ops.cuh
 //
 // With few token rows the work is streaming the weights.  The tcgen05 kernel passes every weight block through four
-// roles (copy, expand, tensor memory, MMA), whose hand-overs cost a block as much at 16 tokens as at 64 (2.0 - 2.2 TB/s
-// with two CTAs an SM, 1.8 with one; here 3.5 - 4.3 at 16 - 5 rows).  Here a warp expands a tile from its own 16 bytes per lane straight into the A operand: a
+// roles (copy, expand, tensor memory, MMA), whose hand-overs cost a block as much at 16 tokens as at 64 (2560 x 10240 and the
+// norm behind it, 5 rows: 11.1 us there, 9.4 here; 2560 x 2048: 6.3 and 5.7).  Here a warp expands a tile from its own 16 bytes per lane straight into the A operand: a
 // shift and a mask turn two of the tile's nibbles into bf16(136 + q), one packed subtract takes the bias off.  The k
 // order inside a 16-wide step is the tile's own (lane t holds k = 4t .. 4t + 3, even ones first), and X follows it.
 //
