@@ -105,10 +105,11 @@ pf_resid_norm_kernel(const float* __restrict__ parts, int nparts, size_t part_st
 
 // Same as pf_resid_norm_kernel with the token's row in registers: one CTA of
 // THREADS threads per token, MAXV float4 per thread, 16-byte loads, two block
-// reductions.  Latency of the partial-sum loads bounds it: small CTAs keep many tokens in flight per SM, and
-// PU > 1 fetches PU partials per round of loads, the sums taken in the same order (1023 rows of 2560: 20.0 us with
-// MAXV 6, PU 1; a prefill of the 4B slice goes from 1702 to 1630 us with MAXV 3, PU 4).
-template <int THREADS, int MAXV, int PU = 1>
+// reductions.  Latency of the loads bounds it: small CTAs keep many tokens in flight per SM, PU partials are
+// fetched per round of loads, the sums taken in order (a prefill of the 4B slice went from 1702 to 1630 us with
+// MAXV 3, PU 4 against MAXV 6, PU 1), and the gains are asked for ahead of the wait on the projection (with the
+// same in the KV append, a prompt of 37 tokens of the 1B model went from 1686 to 1616 us).
+template <int THREADS, int MAXV, int PU>
 __global__ void __launch_bounds__(THREADS)
 pf_resid_norm_reg_kernel(const float* __restrict__ parts, int nparts, size_t part_stride, int d, float eps,
                          const float* __restrict__ g_post, const float* __restrict__ g_pre,
@@ -116,17 +117,14 @@ pf_resid_norm_reg_kernel(const float* __restrict__ parts, int nparts, size_t par
   __shared__ float red[2][THREADS / 32];
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int d4 = d / 4;
-  constexpr bool kAhead = MAXV <= 3;           // as far as the registers go
   float4 f[MAXV], x[MAXV], gp[MAXV], gq[MAXV];
-  if (kAhead) {
 #pragma unroll
-    for (int u = 0; u < MAXV; ++u) {
-      const int i = threadIdx.x + THREADS * u;
-      gp[u] = gq[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (i < d4) {
-        gp[u] = __ldg(reinterpret_cast<const float4*>(g_post) + i);
-        if (g_pre) gq[u] = __ldg(reinterpret_cast<const float4*>(g_pre) + i);
-      }
+  for (int u = 0; u < MAXV; ++u) {
+    const int i = threadIdx.x + THREADS * u;
+    gp[u] = gq[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < d4) {
+      gp[u] = __ldg(reinterpret_cast<const float4*>(g_post) + i);
+      if (g_pre) gq[u] = __ldg(reinterpret_cast<const float4*>(g_pre) + i);
     }
   }
   pdl_wait();
@@ -170,7 +168,6 @@ pf_resid_norm_reg_kernel(const float* __restrict__ parts, int nparts, size_t par
   for (int u = 0; u < MAXV; ++u) {
     const int i = threadIdx.x + THREADS * u;
     if (i < d4) {
-      if (!kAhead) gp[u] = __ldg(reinterpret_cast<const float4*>(g_post) + i);
       x[u].x += f[u].x * r * gp[u].x; x[u].y += f[u].y * r * gp[u].y; x[u].z += f[u].z * r * gp[u].z; x[u].w += f[u].w * r * gp[u].w;
       xr[i] = x[u];
       ss2 += x[u].x * x[u].x + x[u].y * x[u].y + x[u].z * x[u].z + x[u].w * x[u].w;
@@ -188,7 +185,6 @@ pf_resid_norm_reg_kernel(const float* __restrict__ parts, int nparts, size_t par
   for (int u = 0; u < MAXV; ++u) {
     const int i = threadIdx.x + THREADS * u;
     if (i < d4) {
-      if (!kAhead) gq[u] = __ldg(reinterpret_cast<const float4*>(g_pre) + i);
       __nv_bfloat162 a = __floats2bfloat162_rn(x[u].x * r2 * gq[u].x, x[u].y * r2 * gq[u].y);
       __nv_bfloat162 b = __floats2bfloat162_rn(x[u].z * r2 * gq[u].z, x[u].w * r2 * gq[u].w);
       uint2 w;
