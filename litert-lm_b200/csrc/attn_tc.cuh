@@ -24,7 +24,8 @@
 //
 // Warps: 0 copies (TMA, no multicast), 1 issues the products and owns tensor memory, 4 - 11 softmax and sums (two threads
 // per row: half of the tile's keys, then half of the head).  The latter take the registers that the first four give up
-// (launched with 168: 4 warps x 56 + 8 warps x 224 = 12 x 168).  All waits are bounded.
+// (launched with 168: 4 warps x 56 + 8 warps x 224 = 12 x 168).  All waits on mbarriers are bounded; the cluster's barriers
+// wait for CTAs whose every path comes to them.
 #pragma once
 #include <cuda.h>
 
@@ -165,17 +166,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   const int nsub = a.nsplit * kAtcCluster, sub = split * kAtcCluster + rank;
   const int c0 = tfirst + (int)((long long)ntiles * sub / nsub), n = tfirst + (int)((long long)ntiles * (sub + 1) / nsub) - c0;
 
-
-  // The two kinds of warps do not meet in common code again (it would have the fewer registers): each has its own tail.
-  auto all_done = [&]() {
-    tc_fence_before();
-    __syncthreads();
-    if (*reinterpret_cast<volatile int*>(a.err) == (int)kDevBarrierTimeout) {
-#pragma unroll 1
-      for (int i = 0; i < 2000; ++i) __nanosleep(100);                // a wait gave up: let copies in flight land
-      __syncthreads();
-    }
-  };
+  // The two kinds of warps do not meet in common code again (it would have the fewer registers): each has its own tail, of
+  // sync_after_waits and the two cluster barriers.  Nobody leaves it early: a CTA whose wait gave up, or that saw the word of
+  // another, comes to the cluster's barriers like the rest.
   if (warp < 4) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
@@ -280,7 +273,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       __syncwarp();
     }
   }
-  all_done();
+  tc_fence_before();
+  sync_after_waits(a.err);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
@@ -417,7 +411,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       add_tile();
     }
   }
-  all_done();
+  tc_fence_before();
+  sync_after_waits(a.err);
   // ---- the cluster's four ranges meet: CTA q adds quarter q of the head, out of all four CTAs' shared memory
   {                                                                   // the CTA's products and copies are done: over the planes and the ring
     float* at = reinterpret_cast<float*>(atc_sm) + row * S::kMRow;

@@ -324,11 +324,7 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     }
   }
   tc_fence_before();
-  __syncthreads();
-  if (*reinterpret_cast<volatile int*>(g.err) == (int)kDevBarrierTimeout) {
-    for (int i = 0; i < 2000; ++i) __nanosleep(100);   // let copies in flight land before the CTA retires
-    __syncthreads();
-  }
+  sync_after_waits(g.err);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, kTmemCols);

@@ -363,13 +363,7 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
     }
   }
   tc_fence_before();
-  __syncthreads();
-  if (*reinterpret_cast<volatile int*>(g.err) == (int)kDevBarrierTimeout) {
-    // a wait gave up: let any bulk copy still in flight land before the CTA retires
-#pragma unroll 1
-    for (int i = 0; i < 2000; ++i) __nanosleep(100);
-    __syncthreads();
-  }
+  sync_after_waits(g.err);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, ts_tmem(NTOK));

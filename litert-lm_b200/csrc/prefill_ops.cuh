@@ -14,6 +14,7 @@
 #pragma once
 #include <cuda.h>
 
+#include "block_vote.h"
 #include "common.cuh"
 #include "decode_ops.cuh"
 
@@ -461,6 +462,16 @@ __device__ __forceinline__ bool mbar_wait2(uint64_t* bar0, uint32_t parity0, uin
   }
   atomicExch(err, (int)kDevBarrierTimeout);
   return false;
+}
+// The block's last barrier ahead of handing tensor memory back: where a wait gave up, in this block or any other, copies still
+// in flight land first.  All threads of the block take the same branch.
+__device__ __forceinline__ void sync_after_waits(int* err) {
+  if (block_gave_up([&] { return *reinterpret_cast<volatile int*>(err) == (int)kDevBarrierTimeout; },
+                    [](bool seen) { return __syncthreads_or(seen) != 0; })) {
+#pragma unroll 1
+    for (int i = 0; i < 2000; ++i) __nanosleep(100);
+    __syncthreads();
+  }
 }
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
