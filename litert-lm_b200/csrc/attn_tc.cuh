@@ -131,7 +131,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   uint64_t* p_full = b_empty + 1;                                     // probabilities written, O of the tile before read
   uint64_t* o_full = p_full + 1;                                      // P V of a tile complete
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 1);
-  volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int rank = blockIdx.x % kAtcCluster, group = blockIdx.x / kAtcCluster;      // of the cluster; key range, then unit
   const int split = group % a.nsplit, unit = group / a.nsplit;
@@ -151,7 +150,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     mbar_init(b_empty, 8);
     mbar_init(p_full, 8);
     mbar_init(o_full, 1);
-    *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
@@ -167,12 +165,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   const int c0 = tfirst + (int)((long long)ntiles * sub / nsub), n = tfirst + (int)((long long)ntiles * (sub + 1) / nsub) - c0;
 
   // The two kinds of warps do not meet in common code again (it would have the fewer registers): each has its own tail, of
-  // sync_after_waits and the two cluster barriers.  Nobody leaves it early: a CTA whose wait gave up, or that saw the word of
-  // another, comes to the cluster's barriers like the rest.
+  // sync_after_waits and the two cluster barriers.  Nobody leaves it early: a CTA whose wait gave up comes to the
+  // cluster's barriers like the rest.
+  bool ok = true;                                                     // none of this thread's waits has given up
   if (warp < 4) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
-    bool ok = true;
     const bool leader = elect_one();
 #pragma unroll 1
     for (int j = 0; j < n && ok; ++j) {
@@ -219,7 +217,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       umma_commit(b_full);
       umma_commit(&k_empty[s]);
     };
-    bool ok = __all_sync(0xffffffffu, mbar_wait2(q_ready, 0, &k_full[0], 0, a.err));
+    ok = __all_sync(0xffffffffu, mbar_wait2(q_ready, 0, &k_full[0], 0, a.err));
     if (ok) {
       tc_fence_after();
       if (leader) part_a(0);
@@ -274,7 +272,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     }
   }
   tc_fence_before();
-  sync_after_waits(a.err);
+  sync_after_waits(ok);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
@@ -355,17 +353,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       for (int i = 0; i < 16; ++i) s[i] = (add ? s[i] : 0.f) + (__uint_as_float(x[i]) + __uint_as_float(y[i]));
       return true;
     };
-    bool ok = true, late = false;
+    bool late = false;
 #pragma unroll 1
     for (int j = 0; j < n; ++j) {
-      // 16 keys of the row.  The eight warps leave the loop together: one whose wait gave up says so ahead of the barrier.
+      // 16 keys of the row.  The eight warps leave the loop together: the barrier tells them whether a wait of one gave up.
       const int key0 = (c0 + j) * kAtcKeys + half * 16;
       bool got = true;
       if (j == 0) got = read_scores(a_full, a_empty, 0, false);       // the later ones are read ahead, below
       got = got && !late && read_scores(b_full, b_empty, j, true);
-      if (!got) {
-        *failed = 1;
-      } else {
+      if (got) {
         const bool inside = key0 >= a.lo && key0 + 16 <= a.k1;
         float mx = -INFINITY;
 #pragma unroll
@@ -375,8 +371,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         }
         row_max[((j & 1) * 2 + half) * 128 + row] = mx;
       }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (*failed) { ok = false; break; }
+      ok = !block_gave_up([&] { return !got; }, bar_or<1, 256>);
+      if (!ok) break;
       const float mn = fmaxf(m, fmaxf(row_max[(j & 1) * 256 + row], row_max[(j & 1) * 256 + 128 + row]));
       const float f = am_ex2(m - mn);
       m = mn;
@@ -406,13 +402,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
     }
-    if (ok && __all_sync(0xffffffffu, mbar_wait(o_full, (n - 1) & 1, a.err))) {
+    ok = ok && !late && __all_sync(0xffffffffu, mbar_wait(o_full, (n - 1) & 1, a.err));
+    if (ok) {
       tc_fence_after();
       add_tile();
     }
   }
   tc_fence_before();
-  sync_after_waits(a.err);
+  sync_after_waits(ok);
   // ---- the cluster's four ranges meet: CTA q adds quarter q of the head, out of all four CTAs' shared memory
   {                                                                   // the CTA's products and copies are done: over the planes and the ring
     float* at = reinterpret_cast<float*>(atc_sm) + row * S::kMRow;

@@ -1,7 +1,7 @@
-// How the threads of a block part where a bounded wait may have given up.  The sign of it (a device-wide error word, a wait
-// of one's own) can appear while the threads look: one that saw it and one that did not would go on to different barriers
-// and wait there for each other.  So every thread looks ahead of the barrier and takes the barrier's answer, which is the
-// same for all: whether anyone had seen it.  A sign that appears later is the next vote's.
+// How the threads of a block part where a bounded wait may have given up.  Not every thread's wait does, and a word that all
+// of them read can change while they read it: one that saw the sign and one that did not would go on to different barriers
+// and wait there for each other.  So every thread brings what it knows to the barrier and takes the barrier's answer, which
+// is the same for all: whether anyone had seen it.  A sign that appears later is the next vote's.
 #pragma once
 
 #ifdef __CUDACC__

@@ -85,7 +85,6 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   uint64_t* p_full = bars + 11;       // [2] probabilities written over the scores
   uint64_t* o_full = bars + 13;       // all MMAs complete
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
-  volatile int* sm_fail = reinterpret_cast<volatile int*>(bars + 15);   // a softmax thread's wait gave up
   float* l_part = reinterpret_cast<float*>(bars + 16);     // [128] row sums of the upper 32 keys
   uint64_t* q_tmem = bars + 80;       // Q copied to tensor memory
 
@@ -119,7 +118,6 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     }
     mbar_init(o_full, 1);
     mbar_init(q_tmem, 8);
-    *sm_fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
@@ -130,9 +128,9 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   pdl_wait();                 // set-up done; Q, K, V below come from the preceding kernel
   pdl_launch_dependents();
 
+  bool ok = true;             // none of this thread's waits has given up
   if (warp == 0) {
     // ---- producer
-    bool ok = true;
     const bool leader = elect_one();
     if (leader) {
       // Q tile: KB boxes of 64 columns x (G heads x TT tokens) rows
@@ -181,7 +179,7 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       umma_commit(&k_empty[s]);
     };
     const bool leader = elect_one();
-    bool ok = __all_sync(0xffffffffu, mbar_wait2(kQTmem ? q_tmem : q_full, 0, &k_full[0], 0, g.err));
+    ok = __all_sync(0xffffffffu, mbar_wait2(kQTmem ? q_tmem : q_full, 0, &k_full[0], 0, g.err));
     if (ok) {
       tc_fence_after();
       if (leader) issue_s(0);
@@ -221,9 +219,8 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     const float log2e = 1.4426950408889634f;
     const float shift = g.bound * log2e;
     float lsum = 0.f;
-    bool ok = true;
     if constexpr (kQTmem) {                            // half of the row's queries into tensor memory
-      if (mbar_wait(q_full, 0, g.err)) {
+      if (__all_sync(0xffffffffu, mbar_wait(q_full, 0, g.err))) {
 #pragma unroll
         for (int c = 0; c < HD / 2; c += 32) {
           uint32_t q[16];
@@ -241,14 +238,13 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         if (lane == 0) mbar_arrive(q_tmem);
       }
     }
-    // The eight warps leave this loop together: a thread whose wait gave up raises
-    // sm_fail before the named barrier, everyone reads it after.
+    // The eight warps leave this loop together: the named barrier tells all of them
+    // whether a wait of one gave up.
     for (int j = 0; j < ntiles; ++j) {
       const int s = j & 1, n = j >> 1;
       uint32_t packed[16];
-      if (!mbar_wait(&s_full[s], n & 1, g.err)) {
-        *sm_fail = 1;
-      } else {
+      const bool got = __all_sync(0xffffffffu, mbar_wait(&s_full[s], n & 1, g.err));
+      if (got) {
         tc_fence_after();
         uint32_t v[32];
         tmem_ld32(lane_addr + kSCol + s * kFaBN + khalf * 32, v);
@@ -282,8 +278,8 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       }
       // The 16 columns a thread writes lie inside the 32 that it or the other thread
       // of its row has just read, so all eight warps meet before anyone overwrites.
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (*sm_fail) { ok = false; break; }
+      ok = !block_gave_up([&] { return !got; }, bar_or<1, 256>);
+      if (!ok) break;
       tmem_st16(lane_addr + kSCol + s * kFaBN + khalf * 16, packed);
       tmem_st_wait();
       tc_fence_before();
@@ -298,7 +294,8 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     if (khalf == 0) l_part[r] = lsum;
     asm volatile("bar.sync 1, 256;" ::: "memory");
     lsum = l_part[r];
-    if (ok && mbar_wait(o_full, 0, g.err)) {
+    ok = ok && __all_sync(0xffffffffu, mbar_wait(o_full, 0, g.err));
+    if (ok) {
       tc_fence_after();
       const float inv = lsum > 0.f ? 1.0f / lsum : 0.f;
       const int head = kvh * G + (r % G);
@@ -324,7 +321,7 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     }
   }
   tc_fence_before();
-  sync_after_waits(g.err);
+  sync_after_waits(ok);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, kTmemCols);

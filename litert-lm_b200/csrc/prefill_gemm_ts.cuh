@@ -199,11 +199,11 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   // that reads ahead of its own wait must read nothing that the two kernels before it write.
   pdl_launch_dependents();
 
+  bool ok = true;                                   // none of this thread's waits has given up
   if (warp == 0) {
     // ---- activation producer: what it reads comes from the preceding kernel
     pdl_wait();
     int it = 0;
-    bool ok = true;
     const bool leader = elect_one();
 #pragma unroll 1
     for (int li = 0; li < my_tiles && ok; ++li) {
@@ -228,7 +228,6 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
     // ---- MMA issue
     const uint32_t idesc = umma_idesc_bf16(kTsRows, NTOK);
     int it = 0;
-    bool ok = true;
     const bool leader = elect_one();
 #pragma unroll 1
     for (int li = 0; li < my_tiles && ok; ++li) {
@@ -259,7 +258,6 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
     }
   } else if (warp == 2) {
     // ---- weight producer, behind the first fills
-    bool ok = true;
     if (lane == 0) {
 #pragma unroll 1
       while (q_li < my_tiles && ok) {
@@ -276,14 +274,12 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int iters = my_tiles * nst;
     const __nv_bfloat162 bias = __float2bfloat162_rn(136.0f);
-    bool ok = true;
 #pragma unroll 1
     for (int it = group, st = group; it < iters && ok; it += kGroups, st += kGroups) {
 #pragma unroll 1
       while (st >= nst) st -= nst;
       const int sq = it % QS, sw = it % WS, nk = min(kTsKb, nkb - st * kTsKb);
-      ok = mbar_wait(&q_full[sq], (it / QS) & 1, g.err);
-      if (ok && it >= WS) ok = mbar_wait(&w_empty[sw], (it / WS - 1) & 1, g.err);
+      ok = __all_sync(0xffffffffu, mbar_wait(&q_full[sq], (it / QS) & 1, g.err) && (it < WS || mbar_wait(&w_empty[sw], (it / WS - 1) & 1, g.err)));
       if (!ok) break;
       tc_fence_after();
       uint4 q[2 * kTsKb];                            // all of the row's part first: the stores below order what follows them
@@ -317,13 +313,12 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
     const int row = quarter * 32 + lane;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int c0 = ((warp - 4 - D) >> 2) * EC;
-    bool ok = true;
     pdl_wait();                                     // the outputs may still be read by an earlier kernel
 #pragma unroll 1
     for (int li = 0; li < my_tiles && ok; ++li) {
       const TsTile tl = ts_tile(blockIdx.x + li * gridDim.x, n_tiles, t_tiles);
       const float sc = g.wscale[tl.n_tile * kTsRows + row];
-      ok = mbar_wait(acc_full, li & 1, g.err);
+      ok = __all_sync(0xffffffffu, mbar_wait(acc_full, li & 1, g.err));
       if (!ok) break;
       tc_fence_after();
       constexpr int EH = NTOK <= 64 && EC > 32 ? 32 : EC;   // columns in registers at a time
@@ -363,7 +358,7 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
     }
   }
   tc_fence_before();
-  sync_after_waits(g.err);
+  sync_after_waits(ok);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, ts_tmem(NTOK));

@@ -463,11 +463,19 @@ __device__ __forceinline__ bool mbar_wait2(uint64_t* bar0, uint32_t parity0, uin
   atomicExch(err, (int)kDevBarrierTimeout);
   return false;
 }
-// The block's last barrier ahead of handing tensor memory back: where a wait gave up, in this block or any other, copies still
-// in flight land first.  All threads of the block take the same branch.
-__device__ __forceinline__ void sync_after_waits(int* err) {
-  if (block_gave_up([&] { return *reinterpret_cast<volatile int*>(err) == (int)kDevBarrierTimeout; },
-                    [](bool seen) { return __syncthreads_or(seen) != 0; })) {
+// Barrier `id` of `n` threads, whole warps; true for all where it is for one (barrier 0 of all threads: __syncthreads_or).
+template <int id, int n>
+__device__ __forceinline__ bool bar_or(bool x) {
+  uint32_t any;
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.or.pred q, %2, %3, p;\nselp.b32 %0, 1, 0, q;\n}"
+               : "=r"(any) : "r"((uint32_t)x), "n"(id), "n"(n) : "memory");
+  return any != 0;
+}
+// The block's last barrier ahead of handing tensor memory back.  `ok`: none of this thread's waits gave up.  Where one of the
+// block's did, copies and products may still be in flight: they get time to land.  Where none did, all of them have been
+// waited for, whatever other blocks say in the error word.
+__device__ __forceinline__ void sync_after_waits(bool ok) {
+  if (block_gave_up([&] { return !ok; }, [](bool seen) { return __syncthreads_or(seen) != 0; })) {
 #pragma unroll 1
     for (int i = 0; i < 2000; ++i) __nanosleep(100);
     __syncthreads();
