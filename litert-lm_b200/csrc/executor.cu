@@ -300,15 +300,27 @@ static int ts_tile_tokens(int T, int N, int K, bool geglu, int ks, int sms) {
   return best;
 }
 
+// K that one accumulator of the tcgen05 GEMM takes, by what its rows are.  Short chains lose less in the accumulators,
+// which cut off, long ones less in rounding the sums of their parts.  Which of the two counts depends on the rows: products of
+// two values (GeGLU) spread over more binades than normed rows, and attention's rows, whose heads differ in size, lie between.
+// 2-norm errors against 64 bits: GeGLU rows, K = 6912 in 1 / 2 / 4 / 6 chains 1.2e-6 / 5.0e-7 / 2.3e-7 / 1.6e-7; normed rows,
+// K = 5376 in 1 / 2 / 4 / 6 / 9 chains 1.5e-7 / 8.6e-8 / 6.5e-8 / 6.4e-8 / 7.0e-8; attention's, K = 2048 in 1 / 2 / 4 / 8 chains
+// 1.1e-7 / 6.7e-8 / 5.6e-8 / 6.2e-8.
+int gemm_chain(GemmRows rows, int K) {
+  if (rows == GemmRows::kNormed) return 1024;
+  if (rows == GemmRows::kAttention) return std::min(512, K / 2);
+  return std::max(256, K / 8);
+}
+
 // Split-K factor of a GEMM: a divisor of the 64-wide k blocks, at most `most` (what the partials buffer holds) and eight,
-// two blocks a split and more.
+// four blocks a split and more.
 int pick_ksplit(int T, int N, int K, int sms, int most) {
   const int KB = K / kGemmBK;
   if (const int s = gs_ksplit(T, N, KB, sms, most)) return s;
   int best = 1;
   double best_us = 1e30;
   for (int s = 1; s <= std::min(8, most); ++s) {
-    if (KB % s || (s > 1 && KB / s < 2)) continue;
+    if (KB % s || (s > 1 && KB / s < 4)) continue;
     const double us = ts_cost(T, N, K, false, ts_tile_tokens(T, N, K, false, s, sms), s, sms);
     if (us < best_us) { best_us = us; best = s; }
   }
@@ -318,9 +330,11 @@ int pick_ksplit(int T, int N, int K, int sms, int most) {
 // Launches one int4 GEMM.  a_map must describe `A` ([rows >= T][K] bf16).
 void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bfloat16* A,
                  const uint4* w4t, const float* s4t, const uint8_t* w4g, const float* s4g, int T, int N, int K,
-                 int ksplit, bool geglu, float* outF, __nv_bfloat16* outB, int* err, int64_t* launches) {
+                 int ksplit, int chain, bool geglu, float* outF, __nv_bfloat16* outB, int* err, int64_t* launches) {
   if (mode == B200LM_GEMM_TCGEN05) {
-    GemmArgs g{w4g, s4g, T, N, K, ksplit, outF, outB, err};
+    const int stages = (K / kGemmBK / ksplit + kTsKb - 1) / kTsKb, most = std::max(1, (chain + kTsKb * kGemmBK - 1) / (kTsKb * kGemmBK));
+    const int chains = (stages + most - 1) / most;
+    GemmArgs g{w4g, s4g, T, N, K, ksplit, (stages + chains - 1) / chains, outF, outB, err};
     static int sms_of[64] = {0};              // per device: SM count, set once together with the kernel attributes
     int dev = 0;
     B2_CUDA(cudaGetDevice(&dev));
@@ -337,6 +351,14 @@ void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bflo
       B2_TS_PREP(128);
       B2_TS_PREP(256);
 #undef B2_TS_PREP
+#define B2_TS_REGS(NTOK_)                                                    \
+  B2_CUDA(cudaFuncGetAttributes(&fa, gemm_w4_ts_kernel<0, NTOK_>));          \
+  B2_CHECK(fa.numRegs == ts_regs(NTOK_).launch, kInternal, "GEMM kernel: not the registers that its warps share out")
+      cudaFuncAttributes fa;                  // a warp would wait for ever for registers that the block does not have
+      B2_TS_REGS(64);
+      B2_TS_REGS(128);
+      B2_TS_REGS(256);
+#undef B2_TS_REGS
       B2_CUDA(cudaDeviceGetAttribute(&sms_of[dev], cudaDevAttrMultiProcessorCount, dev));
     }
     const int sms = sms_of[dev];
@@ -795,6 +817,7 @@ void Executor::run_prefill_chunk(const int* tokens, int T, int start) {
   // split-K partials go to the partials buffer (8 x d floats per token); those of the QKV rows are summed by the append
   // kernel, but the CUDA-core attention reads whole rows, so it keeps one split
   int ks_q = 1, ks_o = 1, ks_d = 1;
+  const int ch_q = gemm_chain(GemmRows::kNormed, d.d), ch_o = gemm_chain(GemmRows::kAttention, d.nq()), ch_d = gemm_chain(GemmRows::kGeglu, d.ffn);
   if (mode == B200LM_GEMM_TCGEN05) {
     if (attn_tc) ks_q = pick_ksplit(T, d.nqkv(), d.d, n_sms, std::max(1, 8 * d.d / d.nqkv()));
     ks_o = pick_ksplit(T, d.d, d.nq(), n_sms);
@@ -806,7 +829,7 @@ void Executor::run_prefill_chunk(const int* tokens, int T, int start) {
     const float* cosT = model->rope_cos[L.is_global];
     const float* sinT = model->rope_sin[L.is_global];
     float* qkv_buf = ks_q > 1 ? pf_parts : pf_qkv;
-    launch_gemm(stream, mode, tm_h, pf_h, L.wqkv, L.sqkv, Gm.wqkv, Gm.sqkv, T, d.nqkv(), d.d, ks_q, false, qkv_buf,
+    launch_gemm(stream, mode, tm_h, pf_h, L.wqkv, L.sqkv, Gm.wqkv, Gm.sqkv, T, d.nqkv(), d.d, ks_q, ch_q, false, qkv_buf,
                 nullptr, err, &launches);
     __nv_bfloat16* qout = attn_tc ? pf_q : nullptr;
     if (d.kv_dtype == 0) launch_kv_append<float>(stream, d, T, qkv_buf, ks_q, start, ptab, L, cosT, sinT, kv_host[li], qout);
@@ -841,14 +864,14 @@ void Executor::run_prefill_chunk(const int* tokens, int T, int start) {
     pf_attn_kernel<<<T * d.hkv, 256, attn_smem, stream>>>(d, j);
     ++launches;
     }
-    launch_gemm(stream, mode, tm_attn, pf_attn, L.wo, L.so, Gm.wo, Gm.so, T, d.d, d.nq(), ks_o, false, pf_parts,
+    launch_gemm(stream, mode, tm_attn, pf_attn, L.wo, L.so, Gm.wo, Gm.so, T, d.d, d.nq(), ks_o, ch_o, false, pf_parts,
                 nullptr, err, &launches);
     if (tp_world > 1) tp_allreduce(pf_parts, (size_t)ks_o * T * d.d);
     launch_resid_norm(stream, pf_parts, ks_o, T, d, L.g_post_attn, L.g_pre_ffn, pf_xres, pf_h);
     ++launches;
-    launch_gemm(stream, mode, tm_h, pf_h, L.wgu, L.sgu, Gm.wgu, Gm.sgu, T, 2 * d.ffn, d.d, 1, true, nullptr, pf_act,
+    launch_gemm(stream, mode, tm_h, pf_h, L.wgu, L.sgu, Gm.wgu, Gm.sgu, T, 2 * d.ffn, d.d, 1, d.d, true, nullptr, pf_act,
                 err, &launches);
-    launch_gemm(stream, mode, tm_act, pf_act, L.wdown, L.sdown, Gm.wdown, Gm.sdown, T, d.d, d.ffn, ks_d, false,
+    launch_gemm(stream, mode, tm_act, pf_act, L.wdown, L.sdown, Gm.wdown, Gm.sdown, T, d.d, d.ffn, ks_d, ch_d, false,
                 pf_parts, nullptr, err, &launches);
     if (tp_world > 1) tp_allreduce(pf_parts, (size_t)ks_d * T * d.d);
     const float* g_next = li + 1 < d.n_layers ? model->layers_host[li + 1].g_pre_attn : nullptr;
@@ -1045,27 +1068,28 @@ void Executor::wide_step(int nb, int first) {
   // split K so that the few token rows still spread the weight tiles over the SMs; the attention adds the QKV rows' parts
   const int ks_q = pick_ksplit(nb, d.nqkv(), d.d, n_sms, std::max(1, 8 * d.d / d.nqkv()));
   const int ks_o = pick_ksplit(nb, d.d, d.nq(), n_sms), ks_d = pick_ksplit(nb, d.d, d.ffn, n_sms);
+  const int ch_q = gemm_chain(GemmRows::kNormed, d.d), ch_o = gemm_chain(GemmRows::kAttention, d.nq()), ch_d = gemm_chain(GemmRows::kGeglu, d.ffn);
   for (int li = 0; li < d.n_layers; ++li) {
     const LayerWeights& L = model->layers_host[li];
     const LayerGemmWeights& Gm = model->gemm_host[li];
-    launch_gemm(stream, mode, tm_h, pf_h, L.wqkv, L.sqkv, Gm.wqkv, Gm.sqkv, nb, d.nqkv(), d.d, ks_q, false,
+    launch_gemm(stream, mode, tm_h, pf_h, L.wqkv, L.sqkv, Gm.wqkv, Gm.sqkv, nb, d.nqkv(), d.d, ks_q, ch_q, false,
                 ks_q > 1 ? pf_parts : pf_qkv, nullptr, err, nl);
     WideAttnArgs wa{ks_q > 1 ? pf_parts : pf_qkv, wide.pos, page_table_dev + (size_t)first * pages_per_seq, pages_per_seq, L.is_global, nsplit, 0,
                     L.g_q, L.g_k, model->rope_cos[L.is_global], model->rope_sin[L.is_global], kv_host[li], wide_part, wide_ticket, pf_attn, err,
                     1, 0, nullptr, 2, ks_q, (size_t)nb * d.nqkv()};
     launch_wide_attn(stream, d, nb, smem_optin, wa);         // sums the projections' partials as it reads them
     ++*nl;
-    launch_gemm(stream, mode, tm_attn, pf_attn, L.wo, L.so, Gm.wo, Gm.so, nb, d.d, d.nq(), ks_o, false, pf_parts, nullptr, err, nl);
+    launch_gemm(stream, mode, tm_attn, pf_attn, L.wo, L.so, Gm.wo, Gm.so, nb, d.d, d.nq(), ks_o, ch_o, false, pf_parts, nullptr, err, nl);
     launch_resid_norm(stream, pf_parts, ks_o, nb, d, L.g_post_attn, L.g_pre_ffn, pf_xres, pf_h);
     ++*nl;
-    launch_gemm(stream, mode, tm_h, pf_h, L.wgu, L.sgu, Gm.wgu, Gm.sgu, nb, 2 * d.ffn, d.d, 1, true, nullptr, pf_act, err, nl);
-    launch_gemm(stream, mode, tm_act, pf_act, L.wdown, L.sdown, Gm.wdown, Gm.sdown, nb, d.d, d.ffn, ks_d, false, pf_parts, nullptr,
+    launch_gemm(stream, mode, tm_h, pf_h, L.wgu, L.sgu, Gm.wgu, Gm.sgu, nb, 2 * d.ffn, d.d, 1, d.d, true, nullptr, pf_act, err, nl);
+    launch_gemm(stream, mode, tm_act, pf_act, L.wdown, L.sdown, Gm.wdown, Gm.sdown, nb, d.d, d.ffn, ks_d, ch_d, false, pf_parts, nullptr,
                 err, nl);
     const float* g_next = li + 1 < d.n_layers ? model->layers_host[li + 1].g_pre_attn : model->g_final;
     launch_resid_norm(stream, pf_parts, ks_d, nb, d, L.g_post_ffn, g_next, pf_xres, pf_h);
     ++*nl;
   }
-  launch_gemm(stream, mode, tm_h, pf_h, model->head_w, model->embed_scale, model->head_g, model->head_gs, nb, d.vocab, d.d, 1, false, dargs.logits,
+  launch_gemm(stream, mode, tm_h, pf_h, model->head_w, model->embed_scale, model->head_g, model->head_gs, nb, d.vocab, d.d, 1, d.d, false, dargs.logits,
               nullptr, err, nl);
   const int arg_parts = std::max(1, std::min(kWideArgParts, 2 * n_sms / nb));
   launch_pdl(wide_argmax_kernel, dim3(nb * arg_parts), dim3(kWideArgThreads), 0, stream, dargs.logits, d.vocab, nb, arg_parts, wide, dargs.step_tokens);

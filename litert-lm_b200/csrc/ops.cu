@@ -271,7 +271,7 @@ static void run_gemm_common(int device, int mode, const uint8_t* packed_rows, co
   B2_CUDA(cudaEventCreate(&e1));
   auto run = [&]() {
     launch_gemm(nullptr, mode, tm, a16.as<__nv_bfloat16>(), wt.as<uint4>(), dst.as<float>(), wg.as<uint8_t>(),
-                dsg.as<float>(), t, (int)n, (int)k, ksplit, geglu, of.as<float>(), ob.as<__nv_bfloat16>(),
+                dsg.as<float>(), t, (int)n, (int)k, ksplit, gemm_chain(GemmRows::kGeglu, (int)k), geglu, of.as<float>(), ob.as<__nv_bfloat16>(),
                 errw.as<int>(), nullptr);
   };
   run();

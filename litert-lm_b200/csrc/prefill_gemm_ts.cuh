@@ -16,8 +16,15 @@
 // weight row i, so the per-channel scale is one scalar per epilogue thread and
 // a warp's store covers 32 consecutive output features of one token.  The
 // epilogue warps first pull the whole accumulator into registers (at most 64
-// values per thread) and hand it back, so the scaling / GeGLU and the global
+// values per thread, added to those of the tile's chains before) and hand it back, so the scaling / GeGLU and the global
 // stores of one tile run under the main loop of the next.
+//
+// The accumulator cuts off what it adds instead of rounding it, so its error grows with the products it takes: 5.1e-6 of
+// the result over K = 21504 in one (GeGLU rows, 2-norm against 64 bits), 3.6e-7 over eight of 2688.  So EPI 0 hands its
+// accumulator over every `chain` stages and adds the parts in fp32 in the epilogue's registers.  With narrower tiles the other
+// CTA or the expansion's slack fills the gap (1152 x 1024 over 1023 tokens in four chains 7.4 us, in one 7.2); at 256 tokens the
+// tensor cores stand still for 0.45 us (2560 x 10240 over 1023 tokens in eight chains 59.5, in one 56.5).  Handing the
+// accumulator over in two halves cost more: M128 N128 products take 106 cycles, not 64.  gemm_chain in executor.cu has the lengths.
 //
 // Three rings, each with its own depth, move two k blocks (128 k) at a time: the
 // int4 blocks (from HBM, deep), the activation tiles (from L2, shallow) and the
@@ -64,6 +71,15 @@ __host__ __device__ constexpr int ts_ctas_per_sm(int ntok) { return ntok <= 64 ?
 __host__ __device__ constexpr int ts_smem(int ntok) {
   return ts_xs(ntok) * kTsKb * ntok * kGemmBK * 2 + ts_qs(ntok) * kTsKb * kGemmStageQ + 1024 + 512;
 }
+// EPI 0 adds its chains in registers, a sum per column and thread of the epilogue.  From 64 tokens on that is more than
+// an even share of the registers, and the other warps give up some of theirs.
+struct TsRegs { int launch, issue, expand, sum; };
+__host__ __device__ constexpr TsRegs ts_regs(int ntok) { return ntok >= 256 ? TsRegs{80, 56, 72, 88} : ntok == 128 ? TsRegs{96, 56, 80, 128} : ntok == 64 ? TsRegs{64, 56, 56, 88} : TsRegs{}; }
+__host__ __device__ constexpr bool ts_shares_add_up(int ntok) {
+  const TsRegs r = ts_regs(ntok);
+  return 4 * r.issue + ts_deq_warps(ntok) * r.expand + ts_epi_warps(ntok) * r.sum <= ts_threads(ntok) / 32 * r.launch;
+}
+static_assert(ts_shares_add_up(256) && ts_shares_add_up(128) && ts_shares_add_up(64), "a warp that asks for more registers than the block has waits for ever");
 static_assert(ts_tmem(256) >= 256 + ts_ws(256) * kTsKb * kTsAcols && ts_tmem(128) >= 128 + ts_ws(128) * kTsKb * kTsAcols &&
                   ts_tmem(64) >= 64 + ts_ws(64) * kTsKb * kTsAcols, "TMEM budget");
 static_assert(ts_ctas_per_sm(64) * ts_tmem(64) <= 512 && ts_smem(256) <= 227 * 1024 && 2 * (ts_smem(128) + 1024) <= 228 * 1024 && 2 * (ts_smem(64) + 1024) <= 228 * 1024 &&
@@ -126,7 +142,7 @@ __device__ __forceinline__ void ts_load_acc(uint32_t taddr, uint32_t (&v)[EC]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// EPI 0: fp32 partials outF[ks][T][N].  EPI 1: GeGLU; tile rows alternate
+// EPI 0: fp32 partials outF[ks][T][N], each the sum of its chains.  EPI 1: GeGLU; tile rows alternate
 // gate (even) and up (odd) rows of one ffn feature, output bf16 outB[T][N/2].
 //
 // NTOK is the token width of a tile (the N of the MMA): 256 for prefill; 128 .. 16 when the whole GEMM has
@@ -138,6 +154,7 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   constexpr int D = ts_deq_warps(NTOK), E = ts_epi_warps(NTOK), EC = ts_epi_cols(NTOK);
   constexpr int XS = ts_xs(NTOK), QS = ts_qs(NTOK), WS = ts_ws(NTOK);
   constexpr int kXb = NTOK * kGemmBK * 2;           // activation bytes of a k block
+  constexpr bool kShare = EPI == 0 && ts_regs(NTOK).launch > 0;
   extern __shared__ unsigned char gsm_raw[];
   unsigned char* gsm = reinterpret_cast<unsigned char*>(((uintptr_t)gsm_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sX = gsm;
@@ -149,7 +166,7 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   uint64_t* q_empty = q_full + QS;                  // [QS] expansion has read them
   uint64_t* w_full = q_empty + QS;                  // [WS] expanded weights are in TMEM
   uint64_t* w_empty = w_full + WS;                  // [WS] MMAs finished with them
-  uint64_t* acc_full = w_empty + WS;                // accumulator complete
+  uint64_t* acc_full = w_empty + WS;                // accumulator of a chain complete
   uint64_t* acc_empty = acc_full + 1;               // accumulator read out by the epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 2);
 
@@ -200,6 +217,10 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   pdl_launch_dependents();
 
   bool ok = true;                                   // none of this thread's waits has given up
+  if constexpr (kShare) {
+    if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ts_regs(NTOK).issue));
+    else if (warp < 4 + D) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ts_regs(NTOK).expand));
+  }
   if (warp == 0) {
     // ---- activation producer: what it reads comes from the preceding kernel
     pdl_wait();
@@ -227,14 +248,19 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
   } else if (warp == 1) {
     // ---- MMA issue
     const uint32_t idesc = umma_idesc_bf16(kTsRows, NTOK);
-    int it = 0;
+    int it = 0, nacc = 0;                            // stages, accumulators begun
     const bool leader = elect_one();
 #pragma unroll 1
     for (int li = 0; li < my_tiles && ok; ++li) {
-      if (li > 0) ok = __all_sync(0xffffffffu, mbar_wait(acc_empty, (li - 1) & 1, g.err));
-      tc_fence_after();
 #pragma unroll 1
-      for (int st = 0; st < nst && ok; ++st, ++it) {
+      for (int st = 0, left = 0; st < nst && ok; ++st, ++it, --left) {
+        const bool first = left == 0;                // stage of a chain
+        if (first) {
+          left = EPI == 0 ? g.chain : nst;
+          if (nacc > 0) ok = __all_sync(0xffffffffu, mbar_wait(acc_empty, (nacc - 1) & 1, g.err));
+          ++nacc;
+          if (!ok) break;
+        }
         const int sx = it % XS, sw = it % WS, nk = min(kTsKb, nkb - st * kTsKb);
         ok = __all_sync(0xffffffffu, mbar_wait(&w_full[sw], (it / WS) & 1, g.err) && mbar_wait(&x_full[sx], (it / XS) & 1, g.err));
         if (!ok) break;
@@ -246,15 +272,14 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
             const uint64_t xd = umma_desc_sw128(smem_u32(sX + (sx * kTsKb + kb) * kXb));
 #pragma unroll
             for (int k = 0; k < kGemmBK / 16; ++k)   // 16 bf16 along K per MMA: 8 TMEM columns, 32 bytes of X
-              umma_bf16_ts(tmem_base, tmem_w + (sw * kTsKb + kb) * kTsAcols + k * 8, xd + (uint64_t)(k * 2), idesc, (st | kb | k) ? 1u : 0u);
+              umma_bf16_ts(tmem_base, tmem_w + (sw * kTsKb + kb) * kTsAcols + k * 8, xd + (uint64_t)(k * 2), idesc, first && !(kb | k) ? 0u : 1u);
           }
           umma_commit(&w_empty[sw]);
           umma_commit(&x_empty[sx]);
+          if (left == 1 || st + 1 == nst) umma_commit(acc_full);
         }
         __syncwarp();
       }
-      if (ok && leader) umma_commit(acc_full);
-      __syncwarp();
     }
   } else if (warp == 2) {
     // ---- weight producer, behind the first fills
@@ -313,47 +338,68 @@ gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
     const int row = quarter * 32 + lane;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int c0 = ((warp - 4 - D) >> 2) * EC;
+    if constexpr (kShare) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(ts_regs(NTOK).sum));
+    int nacc = 0;
     pdl_wait();                                     // the outputs may still be read by an earlier kernel
 #pragma unroll 1
     for (int li = 0; li < my_tiles && ok; ++li) {
       const TsTile tl = ts_tile(blockIdx.x + li * gridDim.x, n_tiles, t_tiles);
       const float sc = g.wscale[tl.n_tile * kTsRows + row];
-      ok = __all_sync(0xffffffffu, mbar_wait(acc_full, li & 1, g.err));
-      if (!ok) break;
-      tc_fence_after();
-      constexpr int EH = NTOK <= 64 && EC > 32 ? 32 : EC;   // columns in registers at a time
-#pragma unroll 1
-      for (int ch = 0; ch < EC; ch += EH) {
-      const int t0 = tl.t_tile * NTOK + c0 + ch;
-      uint32_t v[EH];
-      ts_load_acc<EH>(tmem_base + lane_base + c0 + ch, v);
-      if (ch + EH == EC) {                          // the accumulator is in registers: hand it back before the stores
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty);
-      }
       if constexpr (EPI == 0) {
-        const int nrow = tl.n_tile * kTsRows + row;
-        if (nrow < g.N) {
+        float sum[EC];
+#pragma unroll
+        for (int c = 0; c < EC; ++c) sum[c] = 0.f;
+#pragma unroll 1
+        for (int st = 0; st < nst; st += g.chain, ++nacc) {
+          ok = __all_sync(0xffffffffu, mbar_wait(acc_full, nacc & 1, g.err));
+          if (!ok) break;
+          tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < EC; c += 16) {
+            uint32_t v[16];
+            ts_load_acc<16>(tmem_base + lane_base + c0 + c, v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) sum[c + i] += __uint_as_float(v[i]);
+          }
+          tc_fence_before();                        // the accumulator is in registers: hand it back before the stores
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_empty);
+        }
+        const int nrow = tl.n_tile * kTsRows + row, t0 = tl.t_tile * NTOK + c0;
+        if (ok && nrow < g.N) {
           float* dst = g.outF + ((size_t)tl.ks * g.T + t0) * g.N + nrow;
 #pragma unroll
-          for (int c = 0; c < EH; ++c)
-            if (t0 + c < g.T) dst[(size_t)c * g.N] = __uint_as_float(v[c]) * sc;
+          for (int c = 0; c < EC; ++c, dst += g.N)
+            if (t0 + c < g.T) *dst = sum[c] * sc;
         }
       } else {
-        const int F = g.N / 2;
-        const int f = tl.n_tile * (kTsRows / 2) + (row >> 1);
-        const bool odd = lane & 1;
-        __nv_bfloat16* dst = g.outB + (size_t)(t0 + (odd ? 1 : 0)) * F + f;
-        const int tlim = g.T - t0 - (odd ? 1 : 0);          // columns c (even) with c < tlim are stored
+        ok = __all_sync(0xffffffffu, mbar_wait(acc_full, li & 1, g.err));
+        if (!ok) break;
+        tc_fence_after();
+        constexpr int EH = NTOK <= 64 && EC > 32 ? 32 : EC;   // columns in registers at a time
+#pragma unroll 1
+        for (int ch = 0; ch < EC; ch += EH) {
+          const int t0 = tl.t_tile * NTOK + c0 + ch;
+          uint32_t v[EH];
+          ts_load_acc<EH>(tmem_base + lane_base + c0 + ch, v);
+          if (ch + EH == EC) {                      // the accumulator is in registers: hand it back before the stores
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty);
+          }
+          const int F = g.N / 2;
+          const int f = tl.n_tile * (kTsRows / 2) + (row >> 1);
+          const bool odd = lane & 1;
+          __nv_bfloat16* dst = g.outB + (size_t)(t0 + (odd ? 1 : 0)) * F + f;
+          const int tlim = g.T - t0 - (odd ? 1 : 0);          // columns c (even) with c < tlim are stored
 #pragma unroll
-        for (int c = 0; c < EH; c += 2) {
-          float a = __uint_as_float(v[c]) * sc, bb = __uint_as_float(v[c + 1]) * sc;
-          float got = __shfl_xor_sync(0xffffffffu, odd ? a : bb, 1);
-          float gate = odd ? got : a, up = odd ? bb : got;
-          if (c < tlim && f < F) dst[(size_t)c * F] = __float2bfloat16(gelu_tanh_fast(gate) * up);
+          for (int c = 0; c < EH; c += 2) {
+            float a = __uint_as_float(v[c]) * sc, bb = __uint_as_float(v[c + 1]) * sc;
+            float got = __shfl_xor_sync(0xffffffffu, odd ? a : bb, 1);
+            float gate = odd ? got : a, up = odd ? bb : got;
+            if (c < tlim && f < F) dst[(size_t)c * F] = __float2bfloat16(gelu_tanh_fast(gate) * up);
+          }
         }
-      }
       }
     }
   }

@@ -559,6 +559,7 @@ struct GemmArgs {
   const float* wscale;     // per weight row, in tile order, padded to the tile grid
   int T, N, K;             // N = logical output columns (unpadded)
   int ksplit;              // K splits; partial outputs [ksplit][T][N]
+  int chain;               // stages of a split that one accumulator takes (epilogue 0; the other one's takes all)
   float* outF;             // epilogue 0
   __nv_bfloat16* outB;     // epilogue 1 (GeGLU): [T][N/2]
   int* err;

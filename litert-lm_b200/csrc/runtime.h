@@ -56,10 +56,12 @@ struct ActMap {
 };
 CUtensorMap make_activation_map_box(const __nv_bfloat16* base, int rows, int cols, int box_rows);
 ActMap make_activation_map(const __nv_bfloat16* base, int rows, int cols);
+enum class GemmRows { kNormed, kAttention, kGeglu };
+int gemm_chain(GemmRows rows, int K);
 int pick_ksplit(int T, int N, int K, int sms, int most = 8);
 void launch_gemm(cudaStream_t st, int mode, const ActMap& a_map, const __nv_bfloat16* A, const uint4* w4t,
-                 const float* s4t, const uint8_t* w4g, const float* s4g, int T, int N, int K, int ksplit, bool geglu,
-                 float* outF, __nv_bfloat16* outB, int* err, int64_t* launches);
+                 const float* s4t, const uint8_t* w4g, const float* s4g, int T, int N, int K, int ksplit, int chain,
+                 bool geglu, float* outF, __nv_bfloat16* outB, int* err, int64_t* launches);
 
 // One session: KV cache, step counter, pending token, scratch activations.
 class Executor {

@@ -33,6 +33,35 @@ def test_tcgen05_gemm_of_several_narrow_token_tiles(pkg, orc, mio, t, n, k, kspl
     assert np.abs(got - want).max() / np.abs(want).max() < 2e-5      # exact products, fp32 sums in another order
 
 
+def unpack_int4(packed):
+    q = np.empty((packed.shape[0], packed.shape[1] * 2), np.int8)
+    q[:, 0::2], q[:, 1::2] = packed & 0xF, packed >> 4
+    return np.where(q > 7, q - 16, q)
+
+
+# 2-norm error against 64 bits of eight chains over GeGLU rows, 384 rows x 512; in one chain 2.8e-7, 1.2e-6, 2.0e-6, 5.1e-6
+EIGHT_CHAINS = {2048: 7.4e-8, 6912: 1.24e-7, 10240: 1.7e-7, 21504: 3.6e-7}
+
+
+@pytest.mark.parametrize("t,n,k,ksplit", [
+    (17, 128, 10240, 1), (30, 160, 10240, 2), (64, 640, 21504, 4), (100, 400, 2048, 1), (203, 1152, 6912, 1), (300, 5376, 21504, 1),
+    (511, 1152, 2048, 2), (600, 1152, 6912, 4),
+])
+def test_no_accumulator_takes_more_than_an_eighth_of_k(pkg, mio, t, n, k, ksplit):
+    """However K is split, the error is that of eight accumulators: they cut off what they add, so longer ones lose more.  All
+    token tiles, ragged ones too; K / ksplit of whole stages and not.  Bound: 1.5 times the measured error, which leaves
+    room for the scatter of small outputs; the next longer chains (two eighths of K) are at 1.9 times and above."""
+    packed, scale = make_matrix(mio, n, k, 7 * n + k)
+    rng = np.random.Generator(np.random.PCG64(t + 3))
+    g, u = rng.standard_normal((2, t, k), dtype=np.float32)
+    a = bf16_round(0.5 * g * (1 + np.tanh(0.7978845608028654 * (g + 0.044715 * g ** 3))) * u)
+    q = np.empty((n, k), np.int8)
+    q[:, 0::2], q[:, 1::2] = packed & 0xF, packed >> 4
+    want = a.astype(np.float64) @ (np.where(q > 7, q - 16, q) * scale.astype(np.float64)[:, None]).T
+    got, _ = pkg.ops.gemm_w4(packed, scale, a, mode=pkg.GEMM_TCGEN05, ksplit=ksplit)
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) < 1.5 * EIGHT_CHAINS[k]
+
+
 def test_tcgen05_gemm_agrees_with_check_gemm(pkg, mio):
     packed, scale = make_matrix(mio, 768, 384, 77)
     a = bf16_round(np.random.Generator(np.random.PCG64(6)).standard_normal((150, 384), dtype=np.float32))
