@@ -98,10 +98,15 @@ void launch_gemv(const Launch& l, const DecodeArgs& a, const StepPlan& pl, StepG
     *l.fits = false;
     return;
   }
-  if (nv <= 1) launch_gemv_cp<PRO, EPI, 1>(l, a, g);
-  else if (nv <= 3) launch_gemv_cp<PRO, EPI, 3>(l, a, g);
-  else if (nv <= 4) launch_gemv_cp<PRO, EPI, 4>(l, a, g);
-  else launch_gemv_cp<PRO, EPI, 12>(l, a, g);
+  // the short combine's slices are at most 256 wide, which is less than a float4 a thread in every group
+  if constexpr (PRO == kStCombineShort) {
+    launch_gemv_cp<PRO, EPI, 1>(l, a, g);
+  } else {
+    if (nv <= 1) launch_gemv_cp<PRO, EPI, 1>(l, a, g);
+    else if (nv <= 3) launch_gemv_cp<PRO, EPI, 3>(l, a, g);
+    else if (nv <= 4) launch_gemv_cp<PRO, EPI, 4>(l, a, g);
+    else launch_gemv_cp<PRO, EPI, 12>(l, a, g);
+  }
 }
 
 template <typename T, int HD, int G>
@@ -164,8 +169,8 @@ int run(Launch l, const DecodeArgs& a, const StepPlan& pl, const LayerWeights* l
     o.w = L.wo; o.wscale = L.so; o.tiles = d.d / 16; o.KT = KTo; o.slices = pl.o_slices; o.y = pl.opart;
     o.part_o = pl.part_o; o.part_ml = pl.part_ml; o.nsplit = pl.nsplit[L.is_global ? 1 : 0]; o.is_global = L.is_global;
     o.bar = 5 * i + 2;
-    // one head of 256 or two of 128 in a slice of K, and sessions that have the warps for it
-    if (d.hd >= 128 && d.nq() / pl.o_slices <= 256) launch_gemv<kStCombineShort, kStPlain>(l, a, pl, o);
+    // one head of 256, or one or two of 128 in a slice of K: a warp's 128 values belong to one head
+    if (d.hd >= 128 && d.nq() / pl.o_slices <= kStShortSlice) launch_gemv<kStCombineShort, kStPlain>(l, a, pl, o);
     else launch_gemv<kStCombine, kStPlain>(l, a, pl, o);
     if (reduce) reduce(ctx, pl.opart, (size_t)pl.o_slices * a.ncols * d.d);
     StepGemv gu{};

@@ -33,6 +33,8 @@ constexpr int kStMaxSlots = 2;            // ring slots of a warp
 constexpr int kStKeys = 32;               // keys of one attention round (one per lane of the softmax warps)
 constexpr int kStMaxSplits = 64;
 constexpr int kAtThreads = 256;
+constexpr int kStShortSlice = 256;        // widest slice of K that kStCombineShort takes
+static_assert(kStShortSlice <= kStThreads, "less than a float4 a thread with four sessions");
 
 enum StepPrologue { kStResid = 0, kStAct = 1, kStCombine = 2, kStCombineShort = 3 };
 enum StepEpilogue { kStPlain = 0, kStGeglu = 1, kStHead = 2 };
