@@ -24,7 +24,7 @@ def reference(q, k, v, table, s, window):
     (9, 257, 0), (33, 1023, 256), (64, 3000, 0),               # row tiles with a remainder; more than one tile
 ])
 @pytest.mark.parametrize("bf16", [False, True])
-def test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window, bf16):
+def test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window, bf16, nan_ahead=False):
     gen = torch.Generator(device="cuda").manual_seed(batch * 1000 + s)
     pages = -(-s // 256)
     q = torch.randn(batch, (hq + 2 * hkv) * hd, device="cuda", generator=gen)
@@ -34,6 +34,10 @@ def test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window,
     k[-1, :, s - (pages - 1) * 256:] = float("nan")            # slots past the last key are never read
     v[-1, :, s - (pages - 1) * 256:] = float("nan")
     k[-1], v[-1] = k[-1].clone(), v[-1].clone()
+    if nan_ahead:                                              # nor do those ahead of a window's first key enter
+        for p in range(pages):
+            k[p, :, :max(0, s - window - 256 * p)] = float("nan")
+            v[p, :, :max(0, s - window - 256 * p)] = float("nan")
     table = torch.randperm(pages, device="cuda", generator=gen).to(torch.int32)
     inv = torch.empty_like(table)
     inv[table.long()] = torch.arange(pages, device="cuda", dtype=torch.int32)
@@ -58,6 +62,14 @@ def test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window,
 ])
 def test_many_rows_on_tcgen05(pkg, batch, s, window, hq, hkv, hd):
     test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window, True)
+
+
+@pytest.mark.parametrize("batch,s,window,hq,hkv,hd", [
+    (33, 1023, 1001, 4, 1, 256), (64, 3000, 1500, 4, 1, 128),   # first keys 22 and 28 of a tile of 32
+    (64, 4097, 4096, 4, 1, 256), (49, 2600, 1513, 2, 2, 128),   # the second, and the last of a tile in the middle of a page
+])
+def test_nothing_ahead_of_a_window_enters_on_tcgen05(pkg, batch, s, window, hq, hkv, hd):
+    test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window, True, nan_ahead=True)
 
 
 def test_unaligned_cache_goes_through_the_plain_kernel(pkg):

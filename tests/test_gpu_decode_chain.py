@@ -60,6 +60,57 @@ def test_sessions_in_lockstep_agree_with_one_at_a_time(pkg, models, sessions):
         assert np.linalg.norm(a - b) <= 2e-3 * np.linalg.norm(b), i     # two int8 terms with three or four sessions
 
 
+@pytest.mark.parametrize("kv_dtype", [0, 1])
+@pytest.mark.parametrize("heads,kv_heads", [(1, 1), (2, 1), (2, 2), (4, 1), (4, 2)])
+@pytest.mark.parametrize("prompt", [1, 33, 1100])              # one key in one split, two splits, all 32 and a window's 20
+def test_heads_of_128_one_to_a_slice(pkg, mio, heads, kv_heads, prompt, kv_dtype):
+    """A slice of the O projection's K is one head of 128 where there are one, two or four of them: the narrowest form of the
+    short combine, alone and with two and four sessions, against the streaming kernel."""
+    cfg = dataclasses.replace(mio.config_small(), n_layers=2, n_q_heads=heads, n_kv_heads=kv_heads, head_dim=128, d_model=192, ffn=256, vocab=512,
+                              max_ctx=1280, window=600, global_period=2, kv_dtype=kv_dtype)
+    img = image(mio, cfg)
+    ids = [seeded_ids(prompt + i, cfg.vocab, max(1, prompt - 31 * i)) for i in range(4)]
+
+    def logits(sessions, mode):
+        ex = pkg.B200LlmExecutor(img, n_sessions=sessions, decode_mode=mode)
+        for i in range(sessions):
+            ex.PrefillSession(i, ids[i])
+        tokens = ex.DecodeTokensBatch(3)
+        out = []
+        for i in range(sessions):
+            ex.SelectSession(i)
+            out.append(ex.DecodeLogits().ravel().astype(np.float64))
+        return tokens, out
+
+    # fp32 sums in another order, and two int8 terms with four sessions.  Either may round a value of a bf16 cache the
+    # other way: 2^-8 of it, and at most that of a result over few rows.
+    for sessions, tol in ((1, 1e-4), (2, 1e-4), (4, 2e-3)):
+        tol += kv_dtype * 2.0 ** -8
+        (ta, la), (tb, lb) = (logits(sessions, m) for m in (pkg.DECODE_CHAINED, pkg.DECODE_PERSISTENT))
+        assert np.array_equal(ta, tb)
+        for a, b in zip(la, lb):
+            assert np.linalg.norm(a - b) <= tol * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("d_model,ffn", [(4096, 512), (4160, 512), (6144, 256), (256, 24576)])   # 4, 5 and 6 float4 a thread; down's 6
+def test_two_sessions_over_wide_vectors(pkg, mio, d_model, ffn):
+    cfg = dataclasses.replace(mio.config_small(), n_layers=2, d_model=d_model, ffn=ffn, n_q_heads=2, head_dim=128, vocab=256, max_ctx=256)
+    img = image(mio, cfg)
+    ids = [seeded_ids(80 + i, cfg.vocab, 40 - 17 * i) for i in range(2)]
+    ex = pkg.B200LlmExecutor(img, n_sessions=2, decode_mode=pkg.DECODE_CHAINED)
+    assert ex.GetDecodeMode() == pkg.DECODE_CHAINED
+    for i, p in enumerate(ids):
+        ex.PrefillSession(i, p)
+    got = ex.DecodeTokensBatch(4)
+    for i, p in enumerate(ids):
+        solo = pkg.B200LlmExecutor(img)
+        solo.Prefill(p)
+        assert list(solo.DecodeTokens(4)) == list(got[:, i])
+        ex.SelectSession(i)
+        a, b = (e.DecodeLogits().ravel().astype(np.float64) for e in (ex, solo))
+        assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(b)
+
+
 def test_timeline_covers_every_kernel_of_the_step(pkg, models):
     cfg, _, img = models("small")
     ex = pkg.B200LlmExecutor(img)
