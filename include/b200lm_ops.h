@@ -108,7 +108,8 @@ int B200LmOps_AttentionPrefillTc(int32_t device, const float* q, const float* k,
  * Otherwise the split kernel of csrc/decode_ops.cuh runs with nsplit splits.
  *
  * Limits: batch <= 16368 and batch*hq*nsplit*(hd+2)*4 bytes <= 8 MiB - 64 KiB;
- * larger requests are rejected with InvalidArgument.  The first call on a
+ * larger requests are rejected with InvalidArgument.  Pages of a bf16 cache
+ * start within 32 TB of the first.  The first call on a
  * device looks up the array's address and sets a kernel attribute; make that
  * first call before starting any stream capture.  All calls on a device share
  * the array, which keeps what the last call left in it; two calls whose kernels

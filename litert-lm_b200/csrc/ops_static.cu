@@ -15,6 +15,7 @@
 #include "attn_tc.cuh"
 #include "common.cuh"
 #include "decode_ops.cuh"
+#include "page_map.h"
 #include "prefill_ops.cuh"
 
 #include <atomic>
@@ -166,9 +167,9 @@ extern "C" int B200LmOps_AttentionDecodeStatic(int32_t device, const float* q_de
       const int cap = (int)std::min<size_t>(kTicketSplits, (kStaticScratchBytes - kStaticHeaderBytes) / per_split);
       a.part_ml = part_o + (size_t)batch * hq * cap * hd;
       if (const int ns = kv_bf16 ? atc_splits(a, hd, sc.clusters[hd == 256], cap) : 0) {
-        // the pages of a cache as [page][kv head x slot][hd]; how many there are, only the caller knows: 32 TB of them
+        // the pages of a cache as [page][kv head x slot][hd]
         const cuuint64_t strides[2] = {(cuuint64_t)hd * 2, (cuuint64_t)hkv * kPage * hd * 2};
-        const cuuint64_t dims[3] = {(cuuint64_t)hd, (cuuint64_t)hkv * kPage, std::min<cuuint64_t>(1ull << 24, (1ull << 45) / strides[1])};
+        const cuuint64_t dims[3] = {(cuuint64_t)hd, (cuuint64_t)hkv * kPage, map_pages(strides[1])};
         const cuuint32_t box[3] = {64, kAtcKeys, 1};
         const CUtensorMap tm_k = make_bf16_map(k_pages_dev, 3, dims, strides, box), tm_v = make_bf16_map(v_pages_dev, 3, dims, strides, box);
         if (hd == 256) launch_attn_tc<256>(st, tm_k, tm_v, a, ns);
