@@ -123,6 +123,14 @@ int B200LmOps_AttentionDecodeStatic(int32_t device, const float* q_dev, const vo
                                     int32_t hq, int32_t hkv, int32_t hd, int32_t window, int32_t kv_bf16,
                                     int32_t nsplit, float* out_dev, void* stream, char** err);
 
+/* Which kernel a call of this shape with aligned pointers runs on `device`: how
+ * many clusters of csrc/attn_tc.cuh share the keys of 128 query rows of a kv
+ * head, or 0 where csrc/attn_mma.cuh takes the call.  For tests and tuning; does
+ * the per-device set-up of the call above.  No counterpart in the reference. */
+int B200LmOps_AttentionDecodeStaticClusters(int32_t device, int32_t batch, int32_t s, int32_t hq, int32_t hkv,
+                                            int32_t hd, int32_t window, int32_t kv_bf16, int32_t* clusters,
+                                            char** err);
+
 /* Status of the work queued by B200LmOps_AttentionDecodeStatic on `stream`:
  * waits for the stream, then reads and clears the error word of the static
  * array (no allocation either).  Returns OK when no call since the last status

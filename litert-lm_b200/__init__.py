@@ -60,7 +60,8 @@ _EXEC_SYMBOLS = ["B200Lm_Create", "B200Lm_CreateShared", "B200Lm_Destroy", "B200
                  "B200Lm_SelectSession", "B200Lm_GetNumSessions", "B200Lm_PrefillSession", "B200Lm_DecodeTokensBatch"]
 _OPS_SYMBOLS = ["B200LmOps_RepackW4T", "B200LmOps_RepackW4G", "B200LmOps_UnpackW4", "B200LmOps_GemvW4",
                 "B200LmOps_GemmW4", "B200LmOps_GemmGegluW4", "B200LmOps_Attention", "B200LmOps_AttentionPrefillTc",
-                "B200LmOps_AttentionDecodeStatic", "B200LmOps_AttentionDecodeStaticStatus"]
+                "B200LmOps_AttentionDecodeStatic", "B200LmOps_AttentionDecodeStaticStatus",
+                "B200LmOps_AttentionDecodeStaticClusters"]
 
 
 def load_library() -> C.CDLL:
@@ -107,6 +108,7 @@ def load_library() -> C.CDLL:
         "B200LmOps_AttentionPrefillTc": [i32, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, errp],
         "B200LmOps_AttentionDecodeStatic": [i32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp, errp],
         "B200LmOps_AttentionDecodeStaticStatus": [i32, vp, vp, errp],
+        "B200LmOps_AttentionDecodeStaticClusters": [i32] * 8 + [vp, errp],
     }
     for name, args in sig.items():
         fn = getattr(lib, name)
@@ -419,6 +421,14 @@ class ops:
             stream or None, C.byref(err))
         if code != OK:
             _check(code, err)
+
+    @staticmethod
+    def attention_decode_static_clusters(batch: int, s: int, hq: int, hkv: int, hd: int, window: int = 0, kv_bf16: bool = False,
+                                         device: int = 0) -> int:
+        """Clusters per 128 query rows with which the tcgen05 kernel takes such a call, 0 where the mma.sync kernel does."""
+        n = C.c_int32(-1)
+        _call("B200LmOps_AttentionDecodeStaticClusters", device, batch, s, hq, hkv, hd, window, kv_bf16, C.byref(n))
+        return n.value
 
     @staticmethod
     def attention_decode_static_status(stream: int = 0, device: int = 0) -> int:

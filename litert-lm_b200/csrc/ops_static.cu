@@ -112,6 +112,12 @@ static void require_device(int device) {
   B2_CHECK(device >= 0 && device < ndev, kInvalidArgument, "device ordinal out of range");
 }
 
+// Splits of a batch's queries whose partials the scratch holds.
+static int scratch_splits(int batch, int hq, int hd) {
+  const size_t per_split = (size_t)batch * hq * (hd + 2) * sizeof(float);
+  return (int)std::min<size_t>(kTicketSplits, (kStaticScratchBytes - kStaticHeaderBytes) / per_split);
+}
+
 }  // namespace b200lm
 
 using namespace b200lm;
@@ -163,8 +169,7 @@ extern "C" int B200LmOps_AttentionDecodeStatic(int32_t device, const float* q_de
       a.part_o = part_o;
       a.err = hdr;
       // the caller's nsplit sized the check above; what fits the scratch is this kernel's own limit
-      const size_t per_split = (size_t)batch * hq * (hd + 2) * sizeof(float);
-      const int cap = (int)std::min<size_t>(kTicketSplits, (kStaticScratchBytes - kStaticHeaderBytes) / per_split);
+      const int cap = scratch_splits(batch, hq, hd);
       a.part_ml = part_o + (size_t)batch * hq * cap * hd;
       if (const int ns = kv_bf16 ? atc_splits(a, hd, sc.clusters[hd == 256], cap) : 0) {
         // the pages of a cache as [page][kv head x slot][hd]
@@ -210,6 +215,30 @@ extern "C" int B200LmOps_AttentionDecodeStatic(int32_t device, const float* q_de
     const int total = batch * hq * hd;
     attn_combine_kernel<<<(total + 255) / 256, 256, 0, st>>>(part_o, part_ml, batch, hq, hkv, hd, nsplit, out_dev);
     B2_CUDA(cudaGetLastError());
+  } catch (const Error& e_) {
+    return static_fail(err, e_.code, e_.msg);
+  } catch (...) {
+    return static_fail(err, kInternal, "unknown failure");
+  }
+  return kOk;
+}
+
+// What atc_splits answers for a call of this shape on this device.
+extern "C" int B200LmOps_AttentionDecodeStaticClusters(int32_t device, int32_t batch, int32_t s, int32_t hq, int32_t hkv, int32_t hd,
+                                                       int32_t window, int32_t kv_bf16, int32_t* clusters, char** err) {
+  if (err) *err = nullptr;
+  try {
+    B2_CHECK(clusters, kInvalidArgument, "null pointer");
+    B2_CHECK(batch > 0 && batch <= kStaticMaxQueries && s > 0 && hq > 0 && hkv > 0 && hq % hkv == 0 && hd > 0, kInvalidArgument, "bad shape");
+    require_device(device);
+    DeviceScope scope(device);
+    const StaticScratch sc = static_scratch_for(device);
+    AmArgs a{};
+    a.rows = batch * (hq / hkv);
+    a.hkv = hkv;
+    a.lo = window > 0 && window < s ? s - window : 0;
+    a.k1 = s;
+    *clusters = kv_bf16 ? atc_splits(a, hd, sc.clusters[hd == 256], scratch_splits(batch, hq, hd)) : 0;
   } catch (const Error& e_) {
     return static_fail(err, e_.code, e_.msg);
   } catch (...) {

@@ -61,6 +61,7 @@ def test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window,
     (64, 1100, 0, 32, 32, 128),                                 # as many units as leave one split each
 ])
 def test_many_rows_on_tcgen05(pkg, batch, s, window, hq, hkv, hd):
+    assert pkg.ops.attention_decode_static_clusters(batch, s, hq, hkv, hd, window, True) >= 1
     test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window, True)
 
 
@@ -69,7 +70,21 @@ def test_many_rows_on_tcgen05(pkg, batch, s, window, hq, hkv, hd):
     (64, 4097, 4096, 4, 1, 256), (49, 2600, 1513, 2, 2, 128),   # the second, and the last of a tile in the middle of a page
 ])
 def test_nothing_ahead_of_a_window_enters_on_tcgen05(pkg, batch, s, window, hq, hkv, hd):
+    assert pkg.ops.attention_decode_static_clusters(batch, s, hq, hkv, hd, window, True) >= 1
     test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window, True, nan_ahead=True)
+
+
+@pytest.mark.parametrize("batch,s,window,hq,hkv,hd,bf16,tcgen05", [
+    (8, 32768, 0, 4, 1, 256, True, False), (9, 32768, 0, 4, 1, 256, True, True),       # 32 and 36 rows
+    (12, 7999, 0, 4, 1, 256, True, False), (12, 8000, 0, 4, 1, 256, True, True),       # 48: keys of all kv heads
+    (20, 2499, 0, 8, 4, 128, True, False), (20, 2500, 0, 8, 4, 128, True, True),       # and of one
+    (13, 999, 0, 4, 1, 256, True, False), (13, 1000, 0, 4, 1, 256, True, True),        # 52
+    (64, 5000, 999, 4, 1, 128, True, False), (64, 5000, 1000, 4, 1, 128, True, True),  # a window's keys are what counts
+    (64, 5000, 0, 4, 1, 256, False, False), (64, 5000, 0, 2, 2, 64, True, False),      # other caches and head sizes
+])
+def test_which_calls_run_on_tcgen05(pkg, batch, s, window, hq, hkv, hd, bf16, tcgen05):
+    assert (pkg.ops.attention_decode_static_clusters(batch, s, hq, hkv, hd, window, bf16) > 0) == tcgen05
+    test_shared_cache_attention_matches_fp64(pkg, hq, hkv, hd, batch, s, window, bf16)
 
 
 def test_unaligned_cache_goes_through_the_plain_kernel(pkg):
