@@ -6,11 +6,14 @@
 //
 //   S  = Q K^T    three products a 16-wide step.  hi and mid sit in shared memory, lo is the A operand in tensor memory
 //                 (three 64 KB planes do not fit beside the ring).  The tensor core cuts its sums off rather than rounding
-//                 them, so none of its chains is long: a quarter of the head's hi products each, in two accumulators that
-//                 are read twice a tile.  Part A is two quarters; part B the third, and lo, mid and the last quarter.
+//                 them, so the leading products are spread out: a quarter of the head's hi products each, in two accumulators
+//                 that are read twice a tile.  Part A is two quarters; part B the third, and in one chain of 36 (head size 256)
+//                 lo, mid and the last quarter.
 //   P          running maximum, exp2, three terms back into tensor memory
-//   O_t = P V     V rows as they lie in the cache: the B operand with hd contiguous.  Every tile's product leaves tensor
-//                 memory and is added to fp32 registers, which is also where the running maximum rescales the sum.
+//   O_t = P V     V rows as they lie in the cache: the B operand with hd contiguous.  Every tile's product, a chain of six
+//                 over 32 keys, leaves tensor memory and is added to fp32 registers, which is also where the running
+//                 maximum rescales the sum.
+// attn_mma.cuh has shorter chains in places (P V three over 16 keys, lo and mid apart from hi); atc_splits has both errors.
 //
 // Four CTAs with neighbouring key ranges are a cluster: they exchange their sums through distributed shared memory, a
 // quarter of the head each, so that only a fourth of the splits goes through the scratch.

@@ -274,9 +274,10 @@ static CUtensorMap make_bf16_map(const void* base, int rank, const cuuint64_t* d
 // tile and K split.  The terms are what the kernel spends its time on: rounds of tiles over the CTA slots, each a row of k
 // blocks whose price depends on the tile's width (tensor-bound at 256 tokens, the expansion's chain of waits below; dearer
 // where two CTAs share an SM), then the accumulators' stores, then the partials once more out of L2.  The constants are a
-// least-squares fit to 2600 timed pairs of GEMM and residual norm (14 projections of four models, 20 - 1023 tokens): it is
-// off by 8 % on average and its choice costs 1.3 % more than the best one, where filling 90 % of the last round with the
-// widest tile cost 15 % (2560 x 2048 at 1023 tokens: 45.6 us with eight splits, 22.5 with one).
+// least-squares fit to timed pairs of GEMM and residual norm (14 projections of four models, 20 - 1023 tokens), made while
+// a split's K went into one accumulator.  With the present kernel the choice takes 1.5 % more than the best split on average and up
+// to 22 % at 36 tokens (15 projections, 2048 tokens and shards of layers among them: profiles/gemm_split_choice.md), where filling
+// 90 % of the last round with the widest tile had eight splits for 2560 x 2048 at 1023 tokens: 45.6 us with the norm, 22.5 with one.
 static double ts_cost(int T, int N, int K, bool geglu, int ntok, int ks, int sms) {
   struct Width { int ntok; double kb, kb_shared, round; };
   static const Width widths[] = {{16, 0.172, 0.325, 0.0}, {32, 0.188, 0.312, 0.0}, {64, 0.209, 0.317, 0.0}, {128, 0.281, 0.281, 0.0}, {256, 0.331, 0.331, 0.6}};

@@ -145,9 +145,9 @@ __device__ __forceinline__ void ts_load_acc(uint32_t taddr, uint32_t (&v)[EC]) {
 // EPI 0: fp32 partials outF[ks][T][N], each the sum of its chains.  EPI 1: GeGLU; tile rows alternate
 // gate (even) and up (odd) rows of one ffn feature, output bf16 outB[T][N/2].
 //
-// NTOK is the token width of a tile (the N of the MMA): 256 for prefill; 128 .. 16 when the whole GEMM has
-// no more token rows than that (the wide decode step, short prompts), which cuts the activation bytes every
-// CTA re-reads per k block and the MMA time in proportion.  tmX must have a box of min(NTOK, 128) rows.
+// NTOK is the token width of a tile (the N of the MMA): whichever of 16 .. 256 the launcher finds cheapest for the token
+// rows, several tiles with the last one ragged among them.  Narrow tiles fill more CTAs and cost less each in activation
+// bytes and MMA time; wide ones expand the weights less often.  tmX must have a box of min(NTOK, 128) rows.
 template <int EPI, int NTOK>
 __global__ void __launch_bounds__(ts_threads(NTOK), ts_ctas_per_sm(NTOK))
 gemm_w4_ts_kernel(const __grid_constant__ CUtensorMap tmX, GemmArgs g) {
