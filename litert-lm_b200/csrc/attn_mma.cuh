@@ -151,6 +151,8 @@ attn_shared_kernel(const AmArgs a) {
   // group's warps issue them, each its share of the copies, NS - 1 ahead.  Chunks start at multiples of 16, so one never
   // spans two pages and is contiguous in the cache: every copy of the loop has a constant offset.
   const int mt = warp % MT, kg = warp / MT;
+  // None of this lane's waits has given up.  A lane that gave up waits no more and asks for nothing, but goes on with what is
+  // there: the products are the whole warp's, and lanes that left would be waited for (a vote a wait cost 0.4 %).
   bool ok = true;
   int page = 0;                                // of the next chunk to issue
   auto next_page = [&](int c) {                // volatile: a load that may sink to its use is a round trip to L2 in the loop
@@ -176,7 +178,7 @@ attn_shared_kernel(const AmArgs a) {
     if (c >= c1) return;
     if (++is_slot == NS) { is_slot = 0; ++is_round; }
     uint64_t* fb = &full[kg * NS + slot];
-    if (round > 0) ok = mbar_wait(&empty[kg * NS + slot], (round - 1) & 1, a.err);
+    if (round > 0) ok = ok && mbar_wait(&empty[kg * NS + slot], (round - 1) & 1, a.err);
     if (!ok) return;
     constexpr int UPR = HD * (int)sizeof(T) / 16;               // 16-byte units per row; 32 / UPR or fewer rows per round
     const unsigned char* src = reinterpret_cast<const unsigned char*>(isv ? a.v : a.k) +
@@ -225,7 +227,6 @@ attn_shared_kernel(const AmArgs a) {
     auto advance = [&]() { if (++slot == NS) { slot = 0; phase ^= 1; } };
     for (int c = c0 + kg, n = 0; c < c1; c += KG, n += 2) {
       issue(n + NS - 1);
-      if (!ok) break;
       // ---- scores of 16 keys: two n-tiles of 8, the leading and the other terms in accumulators of their own
       float acc[2][NA][4], sum[2][4];
 #pragma unroll
@@ -234,8 +235,7 @@ attn_shared_kernel(const AmArgs a) {
 #pragma unroll
         for (int p = 0; p < NA; ++p) acc[x][p][0] = acc[x][p][1] = acc[x][p][2] = acc[x][p][3] = 0.f;
       }
-      ok = mbar_wait(&full[kg * NS + slot], phase, a.err);
-      if (!ok) break;
+      ok = ok && mbar_wait(&full[kg * NS + slot], phase, a.err);
       const unsigned char* ks = ring + (size_t)(kg * NS + slot) * S::kHalf;
       const uint32_t k_addr = smem_u32(ks) + (uint32_t)(((lane & 7) + ((lane >> 4) << 3)) * S::kKRow + ((lane >> 3) & 1) * 16);
       uint32_t af[2][QT][4], raw[2][RW];                              // fragments of this k step and the next
@@ -370,9 +370,7 @@ attn_shared_kernel(const AmArgs a) {
       }
       // ---- O += P V
       issue(n + NS);
-      if (!ok) break;
-      ok = mbar_wait(&full[kg * NS + slot], phase, a.err);
-      if (!ok) break;
+      ok = ok && mbar_wait(&full[kg * NS + slot], phase, a.err);
       const unsigned char* vs = ring + (size_t)(kg * NS + slot) * S::kHalf;
       const uint32_t v_addr = smem_u32(vs) + (uint32_t)(((lane & 7) + ((lane >> 3) & 1) * 8) * S::kVRow + (lane >> 4) * 16);
       uint32_t vraw[2][2][RW];                                        // two pairs of n-tiles at a time, fetched one step ahead

@@ -197,7 +197,7 @@ static __device__ __noinline__ void stream_producer(const DecodeArgs& a, StreamC
   StreamCursor cur{0, 0, kSA, 0};
   for (unsigned n = 0; cur.step < nsteps; ++n) {
     const unsigned h = n & 1u;
-    if (n >= 2 && !mbar_wait(&c.empty[h], ((n >> 1) - 1u) & 1u, &a.st->err)) return;
+    if (n >= 2 && !__all_sync(0xffffffffu, mbar_wait(&c.empty[h], ((n >> 1) - 1u) & 1u, &a.st->err))) return;
     unsigned char* dst = c.half[h];
     uint64_t* bar = &c.full[h];
     FillDesc d;
